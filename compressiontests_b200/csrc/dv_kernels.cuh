@@ -458,6 +458,69 @@ __global__ void __launch_bounds__(kThreads) k_csr(const int32_t *__restrict__ rp
 }
 
 // ---------------------------------------------------------------------------
+// CSR node kernel: W threads per node group of 3 consecutive rows that share one column list
+// (dv_matrix::row_group == 3, checked over the whole matrix at upload)
+//
+// HBM-bound.  Read row by row a product moves (4 + s_v) bytes an entry; here the columns and the
+// gathered x are read once for the three rows, 4/3 + s_v bytes an entry (FP64 9.33 instead of 12,
+// FP32 5.33 instead of 8), from the caller's CSR arrays as they are (the list of the group's first
+// row).  Each lane loads U columns and 3 U values, then gathers, then multiplies; the three row
+// sums are reduced over the W lanes and lanes 0 .. 2 finish one row each.  64 x 48 x 48 elements
+// (36 M entries), FP64: 84.3 -> 69.4 us (365 MB of DRAM traffic, 5.3 TB/s; the gathers and the
+// unaligned value runs make 660 MB between L2 and the SMs); 37 x 29 x 23, FP32, in cache:
+// 16.2 -> 11.2 us.  A register double buffer (the next group's loads ahead of the multiplies) left
+// both unchanged.
+// ---------------------------------------------------------------------------
+template <int W, class AT, class Gather, class Op>
+__global__ void __launch_bounds__(kThreads) k_csr_nodes(const int32_t *__restrict__ rp, const int32_t *__restrict__ ci,
+                                                        const AT *__restrict__ va, int32_t ngroups, Gather g, Op op,
+                                                        const int *__restrict__ done, double *partials,
+                                                        unsigned *ticket) {
+    if (done && *(volatile const int *)done) return;
+    constexpr int U = 3;
+    double red[Op::NRED > 0 ? Op::NRED : 1];
+#pragma unroll
+    for (int i = 0; i < (Op::NRED > 0 ? Op::NRED : 1); ++i) red[i] = 0.0;
+    const int sub = threadIdx.x % W;
+    constexpr int gpb = kThreads / W;
+    for (int32_t grp = blockIdx.x * gpb + threadIdx.x / W; grp < ngroups; grp += gridDim.x * gpb) {
+        const int32_t r0 = 3 * grp;
+        const int32_t s0 = __ldg(rp + r0), len = __ldg(rp + r0 + 1) - s0;
+        const int32_t *cp = ci + s0;
+        const AT *vp = va + s0;   // the rows' values follow each other: row d starts at d * len
+        AT s[3] = {AT(0), AT(0), AT(0)};
+        for (int32_t base = sub; base < len; base += W * U) {
+            int32_t c[U];
+            AT v[U][3], xv[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const int32_t k = base + u * W;
+                c[u] = k < len ? __ldcs(cp + k) : 0;
+#pragma unroll
+                for (int d = 0; d < 3; ++d) v[u][d] = k < len ? __ldcs(vp + (size_t)d * len + k) : AT(0);
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u) xv[u] = (base + u * W < len) ? g((uint32_t)c[u]) : AT(0);
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+                if (base + u * W < len)
+#pragma unroll
+                    for (int d = 0; d < 3; ++d) s[d] = madd<AT>(s[d], v[u][d], xv[u]);
+        }
+#pragma unroll
+        for (int d = 0; d < 3; ++d) s[d] = group_sum<W>(s[d]);
+        if (sub < 3) {
+            const AT t = sub == 0 ? s[0] : sub == 1 ? s[1] : s[2];
+            op.row(r0 + sub, op.init(r0 + sub) + t, red);
+        }
+    }
+    if constexpr (Op::NRED > 0) {
+        double tot[Op::NRED];
+        if (grid_reduce<Op::NRED, Op::MAXMASK>(red, partials, ticket, tot)) op.finish(tot);
+    }
+}
+
+// ---------------------------------------------------------------------------
 // DuVi row-bundle kernel
 //
 // One warp per bundle of <= 32 consecutive rows.  The warp copies the
@@ -1442,6 +1505,24 @@ void launch_csr_tpr(const LaunchEnv &e, const dv_matrix *m, Gather g, Op op) {
     e.ctx->count();
 }
 
+template <int W, class AT, class Gather, class Op>
+void launch_csr_nodes(const LaunchEnv &e, const dv_matrix *m, Gather g, Op op) {
+    auto kern = k_csr_nodes<W, AT, Gather, Op>;
+    const int32_t ngroups = m->n_rows / 3;
+    const int64_t need = std::max<int64_t>(1, ((int64_t)ngroups * W + kThreads - 1) / kThreads);
+    int64_t blocks = need;
+    if (Op::NRED > 0) {   // one wave of resident blocks, so that few partial sums are left to add
+        static OccupancyCache occupancy;   // per instantiation
+        const int64_t wave = (int64_t)e.ctx->num_sms * occupancy.get(kern, kThreads, 0, e.ctx->device);
+        blocks = std::min<int64_t>(need, std::min<int64_t>(wave, e.max_blocks));
+    }
+    kern<<<(unsigned)blocks, kThreads, 0, e.stream>>>(m->rowptr.as<int32_t>(), m->col.as<int32_t>(),
+                                                      static_cast<const AT *>(m->val.p), ngroups, g, op, e.done,
+                                                      e.partials, e.ticket);
+    DV_CUDA(cudaGetLastError());
+    e.ctx->count();
+}
+
 // ---------------------------------------------------------------------------
 // Matrix-free hexahedral operator (DV_FORMAT_HEX): y = K(E) x with K = sum_e f_e Ke on a
 // structured grid of unit-cube trilinear hexahedra, f_e = scale * E_e per element, the
@@ -1834,6 +1915,8 @@ void launch_rows(const LaunchEnv &e, const dv_matrix *m, Gather g, Op op) {
         case 4: launch_csr_tpr<4, AT>(e, m, g, op); break;
         case 8: launch_csr_tpr<8, AT>(e, m, g, op); break;
         case 16: launch_csr_tpr<16, AT>(e, m, g, op); break;
+        case 3 * 16: launch_csr_nodes<16, AT>(e, m, g, op); break;
+        case 3 * 32: launch_csr_nodes<32, AT>(e, m, g, op); break;
         default: launch_csr_tpr<32, AT>(e, m, g, op); break;
     }
 }

@@ -313,7 +313,9 @@ static void autotune(dv_matrix *m) {
         }
     };
     // CSR: threads per row; DuVi: 4 / 9 = staged kernel with that batch width, 100 = lane kernel
+    // (48 / 96: 16 / 32 lanes per 3-row node group, where the rows come in such groups)
     std::vector<int> cand = m->format == DV_FORMAT_CSR ? std::vector<int>{8, 16, 32} : std::vector<int>{4, 9};
+    if (m->format == DV_FORMAT_CSR && m->row_group == 3) cand = {3 * 16, 3 * 32};
     if (m->format == DV_FORMAT_DUVI && m->lanes_ok) cand.push_back(100);
     if (m->format == DV_FORMAT_DUVI && m->pat_ok) cand.push_back(200);
     if (m->format == DV_FORMAT_DUVI && m->grid_ok) cand.push_back(300);
@@ -382,8 +384,13 @@ dv_matrix *dv_matrix_build(dv_context *ctx, const dv_csr_host &a, int format, in
             upload(m->val, f.data(), 4 * (size_t)m->nnz, s);
             DV_CUDA(cudaStreamSynchronize(s));
         }
-        m->csr_tpr = pick_tpr(a.n_rows ? (double)m->nnz / a.n_rows : 1.0);
+        const double mean_nnz = a.n_rows ? (double)m->nnz / a.n_rows : 1.0;
+        m->csr_tpr = pick_tpr(mean_nnz);
         m->row_group = dv_csr_row_group(a);
+        // node groups of 3 rows: k_csr_nodes with 32 lanes a group where its 3 entries a lane fill up
+        // (81 entries: 32 lanes do them in one step), 16 below 48 entries; under 16 most lanes would
+        // idle and the row kernel stays
+        if (m->row_group == 3 && mean_nnz >= 16) m->csr_tpr = mean_nnz < 48 ? 3 * 16 : 3 * 32;
         m->device_bytes = m->nnz * (4 + (precision == DV_F64 ? 8 : 4)) + 4 * ((int64_t)a.n_rows + 1);
     } else {
         if (encoded) {

@@ -467,3 +467,35 @@ def test_matrix_free_trilinear_transfers_bit_exact(ctx, native, oracle, rng, ne)
             np.testing.assert_array_equal(Y[:, j], ref.spmv(X[:, j]))
     with pytest.raises(native.DuviError):
         native.SparseMatrix.trilinear_transfer(ctx, (8, 7, 6))
+
+
+@pytest.mark.parametrize("width", [15, 16, 47, 48, 81, 96, 97, 200])
+@pytest.mark.parametrize("prec", ["f64", "f32"])
+def test_csr_node_groups(ctx, native, rng, width, prec):
+    # Rows in groups of 3 with one column list (and a short last list): the node kernel reads the
+    # columns once a group.  Widths around its steps (3 entries a lane, 16 or 32 lanes), below
+    # which the row kernel stays.  y = A x, y += A x and r = b - A x against the 64-bit product;
+    # the bars are those of the row kernel.
+    import torch
+    ng, m = 67, 640
+    rows, cols = [], []
+    for g in range(ng):
+        c = np.sort(rng.choice(m, size=width if g < ng - 1 else 1, replace=False))
+        for d in range(3):
+            rows += [3 * g + d] * len(c)
+            cols += list(c)
+    A = sp.csr_matrix((rng.standard_normal(len(rows)), (rows, cols)), shape=(3 * ng, m))
+    A.sort_indices()
+    dt, bar = (np.float64, REL64) if prec == "f64" else (np.float32, REL32)
+    x, b = rng.standard_normal(m).astype(dt).astype(np.float64), rng.standard_normal(3 * ng).astype(dt).astype(np.float64)
+    M = native.SparseMatrix(ctx, A, "csr", prec)
+    assert M.info()["row_group"] == 3
+    scale = abs(A) @ np.abs(x) + np.abs(b)
+    assert rowwise_rel(_device_product(ctx, M, x, dt), A @ x, A, x) <= bar
+    assert np.max(np.abs(M.Multiply(x, b.copy(), clear=False) - (b + A @ x)) / scale) <= bar
+    db, dx = torch.from_numpy(b.astype(dt)).cuda(), torch.from_numpy(x.astype(dt)).cuda()
+    dr = torch.empty_like(db)
+    torch.cuda.synchronize()
+    M.residual_device(db.data_ptr(), dx.data_ptr(), dr.data_ptr(), prec)
+    ctx.synchronize()
+    assert np.max(np.abs(dr.cpu().numpy() - (b - A @ x)) / scale) <= bar

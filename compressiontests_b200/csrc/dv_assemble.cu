@@ -14,12 +14,13 @@
 // counts, so the entries before a node are sums of per-axis prefix counts.
 //
 // dv_matrix_create_hex builds the matrix-free form of the same operator (the element
-// kernel k_hex_elem): the per-element factors on the device, the value classes of Ke,
-// and the diagonal for Jacobi weights (summed on the host in the assembly's order, so it
+// kernel k_hex_elem): the per-element factors on the device, Ke's numbers in its symmetry
+// blocks, and the diagonal for Jacobi weights (summed on the host in the assembly's order, so it
 // equals the assembled matrix's diagonal bit for bit).
 #include "dv_kernels.cuh"
 
 #include <algorithm>
+#include <cmath>
 #include <vector>
 
 using namespace dvk;
@@ -136,6 +137,43 @@ extern "C" DV_API int dv_hex_assemble_device(dv_context *ctx, const int32_t *ne,
     });
 }
 
+// The numbers of Ke in its symmetry blocks (HexModes): (1/64) H Ke H with the signs (-1)^(s.b) of
+// character s and corner b.  Every entry outside the blocks is zero and every entry inside is one of
+// the eight numbers, up to rounding; another element stiffness is refused.
+static void hex_modes(const double *ke, double (&out)[8]) {
+    static const int vtk[8] = {0, 1, 3, 2, 4, 5, 7, 6};
+    auto sign = [](int s, int b) { return __builtin_popcount(s & b) & 1 ? -1.0L : 1.0L; };
+    auto mode = [&](int s, int d, int t, int c) {
+        long double m = 0.0L;
+        for (int i = 0; i < 8; ++i)
+            for (int j = 0; j < 8; ++j)
+                m += sign(s, i) * sign(t, j) * (long double)ke[24 * (3 * vtk[i] + d) + 3 * vtk[j] + c];
+        return m / 64.0L;
+    };
+    const long double normal = mode(1, 0, 2, 1), high = mode(6, 0, 5, 1);
+    const long double v[8] = {mode(1, 0, 1, 0) - normal, normal, mode(3, 1, 3, 1), mode(3, 1, 5, 2),
+                              mode(2, 0, 2, 0),          mode(7, 2, 7, 2), mode(6, 0, 6, 0) - high, high};
+    for (int i = 0; i < 8; ++i) out[i] = (double)v[i];
+    const long double tol = 1e-13L * (std::abs(v[0]) + std::abs(v[1]));
+    for (int s = 0; s < 8; ++s)
+        for (int d = 0; d < 3; ++d)
+            for (int t = 0; t < 8; ++t)
+                for (int c = 0; c < 3; ++c) {
+                    long double want = 0.0L;
+                    const int block = s ^ (1 << d), n = __builtin_popcount(block);
+                    if (block == (t ^ (1 << c))) {
+                        const bool dz = s == 0, cz = t == 0;   // a translation
+                        const bool lone_d = s == 7, lone_c = t == 7;
+                        if (n == 0) want = v[1] + (d == c ? v[0] : 0.0L);
+                        else if (n == 1) want = dz || cz ? 0.0L : d == c ? v[2] : v[3];
+                        else if (n == 2) want = lone_d != lone_c ? 0.0L : lone_d ? v[5] : v[4];
+                        else want = v[7] + (d == c ? v[6] : 0.0L);
+                    }
+                    DV_REQUIRE(std::abs(mode(s, d, t, c) - want) <= tol, DV_ERR_UNSUPPORTED,
+                               "element stiffness without the hexahedron's symmetries");
+                }
+}
+
 // Matrix-free operator of several meshes (block-diagonal, meshes in the given order); ne holds
 // 3 element counts per mesh, elem_E (or NULL) the moduli of all meshes' elements in order.
 dv_matrix *dv_hex_operator_build(dv_context *ctx, int32_t nmesh, const int32_t *ne, const double *elem_E, double scale,
@@ -146,17 +184,8 @@ dv_matrix *dv_hex_operator_build(dv_context *ctx, int32_t nmesh, const int32_t *
     std::vector<double> ke(576);
     dv_hex_ke(E, nu, ke.data());
     auto m = std::make_unique<dv_matrix>();
-    bool seen[kKeClasses] = {};
-    for (int i = 0; i < 576; ++i) {
-        const int c = ke_class(i);
-        if (!seen[c]) {
-            seen[c] = true;
-            m->hex_cls[c] = ke[i];
-        } else {
-            DV_REQUIRE(ke[i] == m->hex_cls[c], DV_ERR_UNSUPPORTED, "element stiffness without the hexahedron's symmetries");
-        }
-    }
-    // mesh table: tiles of 32 x 8 nodes over runs of z planes
+    hex_modes(ke.data(), m->hex_modes);
+    // mesh table: tiles of nodes (hex_tile) over runs of z planes
     std::vector<HexMesh> meshes(nmesh);
     int64_t rows = 0, nnz = 0, nel = 0, tiles = 0;
     int64_t plane_tiles_all = 0;
@@ -170,8 +199,9 @@ dv_matrix *dv_hex_operator_build(dv_context *ctx, int32_t nmesh, const int32_t *
         h.ne0 = n[0];
         h.ne1 = n[1];
         h.ne2 = n[2];
-        h.ntx = (n[0] + kGridTX - 1) / kGridTX;
-        h.nty = (n[1] + 1 + kGridTY - 1) / kGridTY;
+        hex_tile(n[0], n[1] + 1, h.wn, h.rn);
+        h.ntx = (n[0] + h.wn - 1) / h.wn;
+        h.nty = (n[1] + 1 + h.rn - 1) / h.rn;
         h.row0 = rows;
         h.fac0 = nel;
         h.pad = 0;
@@ -181,10 +211,13 @@ dv_matrix *dv_hex_operator_build(dv_context *ctx, int32_t nmesh, const int32_t *
         plane_tiles_all += (int64_t)h.ntx * h.nty;
     }
     DV_REQUIRE(rows < INT32_MAX, DV_ERR_ARG, "operator exceeds int32 rows");
-    // run length: one mesh from the waves x steps model; several meshes share a run of 8 planes
-    const int64_t conc = (int64_t)ctx->num_sms * (precision == DV_F64 ? 1 : 3);
+    // run length from the waves x steps model: of the mesh, or of all meshes' tiles at their mean height
+    const int64_t conc = (int64_t)ctx->num_sms * (precision == DV_F64 ? 2 : 3);
+    int64_t tall = 0;
+    for (auto &h : meshes) tall += (int64_t)h.ntx * h.nty * (h.ne2 + 1);
+    const int run = stream_run_length(plane_tiles_all, (int)std::max<int64_t>(1, tall / plane_tiles_all), conc);
     for (auto &h : meshes) {
-        h.zc = nmesh == 1 ? stream_run_length((int64_t)h.ntx * h.nty, h.ne2 + 1, conc) : 8;
+        h.zc = run;
         h.tile0 = (int32_t)tiles;
         tiles += (int64_t)h.ntx * h.nty * ((h.ne2 + 1 + h.zc - 1) / h.zc);
     }

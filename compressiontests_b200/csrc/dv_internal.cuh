@@ -235,7 +235,7 @@ struct dv_matrix {
     int32_t hex_nmesh = 0, hex_ntile = 0;
     int32_t tri_ne[3] = {0, 0, 0};       // DV_FORMAT_TRILINEAR: fine element counts (even)
     int tri_restrict = 0;                // 1: restriction P^T, 0: prolongation P
-    double hex_cls[14] = {};             // value classes of Ke (dvk::ke_class)
+    double hex_modes[8] = {};            // numbers of Ke in its symmetry blocks (dvk::HexModes)
     int lanes_ok = 0;          // lane layout built (host-encoded matrices)
     int lanes_stencil = 0;     // stencil mode: lanes_off holds the column offsets (int32)
     DevMem lanes_off;

@@ -1529,65 +1529,35 @@ void launch_csr_nodes(const LaunchEnv &e, const dv_matrix *m, Gather g, Op op) {
 // nodes of the x = 0 face clamped (FemCantileverBase.cs:87-158, FemCantilever3D.cs:27-132).
 //
 // Nothing of the matrix is stored: a product reads the element factors (one value per
-// element), x and writes y.  A block owns a tile of 32 x 8 free nodes of the xy plane and a
-// run of zc planes and streams node planes of x and layers of element factors through
-// shared memory (x planes double buffered, factor layers triple buffered because each layer
-// is read in two consecutive steps).  At plane p every thread loads its 3 x 3 x 3
-// neighbourhood of x once and forms, for the 8 elements around its node column, the
-// element rows Ke(a, b) x_b of the corners b in plane p, scaled by the element factor, into
-// the three nodes it accumulates (planes p + 1, p, p - 1).  Elements outside the mesh have
-// factor 0 and clamped or outside nodes have x = 0, so face and edge nodes need no special
-// case.  Ke enters through its 14 value classes (ke_class): equal entries share one
-// register-resident value.  The sum order differs from the assembled operator's, so FP64
-// products agree with the assembled matrix to rounding (not bit for bit).
+// element), x and writes y.  Bound by arithmetic: 24 x 24 multiply-adds an element if Ke is
+// applied as it stands (and by corner, 48 scalings of x more).  Ke commutes with the element's
+// three mirror images, so in sums and differences over opposite corners (a Walsh-Hadamard
+// transform of the 8 corner values of each component, signs (-1)^(s.b) for corner b and
+// character s) it falls apart into eight 3 x 3 blocks, one per parity t: component c of block t is
+// character s = t xor e_c.  For the isotropic cube these blocks hold 8 different numbers in all
+// (HexModes); rigid motions are exact zeros.  One element then takes 33 operations and 18
+// scalings, and the transforms 24 + 24 additions in xy (once per node plane and element
+// column) and 24 + 24 in z: about 170 operations an element instead of 670.
+//
+// A thread owns one element column of a tile of W x R columns and streams node planes: the
+// plane's four corner values (staged in shared memory, kGridStages planes in flight) are
+// transformed in xy, combined with the plane below in z, multiplied, and the two faces' parts
+// added while still transformed; the inverse in xy gives the column's share of its 4 nodes of the
+// plane.  Shares of other threads' nodes are exchanged through shared memory across the next
+// step's barrier (so a step has one), and every thread finishes the node at its column's upper
+// right corner: (W - 1) x (R - 1) nodes a tile.  W and R are chosen per mesh for the fewest tiles
+// (hex_tile).  Elements outside the mesh have factor 0 and clamped or outside nodes have x = 0,
+// so face and edge nodes need no special case.  The sum order differs from the assembled
+// operator's, so FP64 products agree with the assembled matrix to rounding (not bit for bit).
+// 128^3, log-uniform moduli, FP64 product: 212.9 -> 79.9 us (119 MB of vectors and factors: 18 us;
+// 170 FP64 operations a node: 19 us), relative error against 64 bits 4.7e-16 -> 2.1e-16.
 // ---------------------------------------------------------------------------
-
-// Value classes of the 24 x 24 unit-cube hexahedron stiffness (VTK corner order, 3 dofs per
-// corner, entry (3 a + d, 3 b + c) at 24 (3 a + d) + 3 b + c): entries of one class are equal
-// for every modulus and Poisson ratio (the element's symmetries; no entry is structurally
-// zero).  Checked against Ke when an operator is created.
-constexpr int kKeClasses = 14;
-#define DV_KE_CLASS_TABLE \
-    0,  1,  1,  2,  3,  3,  4,  5,  6,  7,  8,  9,  7,  9,  8,  4,  6,  5, 10, 11, 11, 12, 13, 13, \
-    1,  0,  1,  8,  7,  9,  5,  4,  6,  3,  2,  3,  9,  7,  8, 13, 12, 13, 11, 10, 11,  6,  4,  5, \
-    1,  1,  0,  8,  9,  7, 13, 13, 12,  9,  8,  7,  3,  3,  2,  5,  6,  4, 11, 11, 10,  6,  5,  4, \
-    2,  8,  8,  0,  5,  5,  7,  3, 11,  4,  1, 13,  4, 13,  1,  7, 11,  3, 12,  6,  6, 10,  9,  9, \
-    3,  7,  9,  5,  0,  1,  8,  2,  3,  1,  4,  6,  6, 12, 13, 11,  7,  8, 13,  4,  5,  9, 10, 11, \
-    3,  9,  7,  5,  1,  0, 11,  8,  7,  6, 13, 12,  1,  6,  4,  8,  3,  2, 13,  5,  4,  9, 11, 10, \
-    4,  5, 13,  7,  8, 11,  0,  1,  5,  2,  3,  8, 10, 11,  9, 12, 13,  6,  7,  9,  3,  4,  6,  1, \
-    5,  4, 13,  3,  2,  8,  1,  0,  5,  8,  7, 11, 11, 10,  9,  6,  4,  1,  9,  7,  3, 13, 12,  6, \
-    6,  6, 12, 11,  3,  7,  5,  5,  0,  3, 11,  7,  9,  9, 10, 13,  1,  4,  8,  8,  2,  1, 13,  4, \
-    7,  3,  9,  4,  1,  6,  2,  8,  3,  0,  5,  1, 12,  6, 13, 10,  9, 11,  4, 13,  5,  7, 11,  8, \
-    8,  2,  8,  1,  4, 13,  3,  7, 11,  5,  0,  5, 13,  4,  1,  9, 10,  9,  6, 12,  6, 11,  7,  3, \
-    9,  3,  7, 13,  6, 12,  8, 11,  7,  1,  5,  0,  6,  1,  4, 11,  9, 10,  5, 13,  4,  3,  8,  2, \
-    7,  9,  3,  4,  6,  1, 10, 11,  9, 12, 13,  6,  0,  1,  5,  2,  3,  8,  4,  5, 13,  7,  8, 11, \
-    9,  7,  3, 13, 12,  6, 11, 10,  9,  6,  4,  1,  1,  0,  5,  8,  7, 11,  5,  4, 13,  3,  2,  8, \
-    8,  8,  2,  1, 13,  4,  9,  9, 10, 13,  1,  4,  5,  5,  0,  3, 11,  7,  6,  6, 12, 11,  3,  7, \
-    4, 13,  5,  7, 11,  8, 12,  6, 13, 10,  9, 11,  2,  8,  3,  0,  5,  1,  7,  3,  9,  4,  1,  6, \
-    6, 12,  6, 11,  7,  3, 13,  4,  1,  9, 10,  9,  3,  7, 11,  5,  0,  5,  8,  2,  8,  1,  4, 13, \
-    5, 13,  4,  3,  8,  2,  6,  1,  4, 11,  9, 10,  8, 11,  7,  1,  5,  0,  9,  3,  7, 13,  6, 12, \
-    10, 11, 11, 12, 13, 13,  7,  9,  8,  4,  6,  5,  4,  5,  6,  7,  8,  9,  0,  1,  1,  2,  3,  3, \
-    11, 10, 11,  6,  4,  5,  9,  7,  8, 13, 12, 13,  5,  4,  6,  3,  2,  3,  1,  0,  1,  8,  7,  9, \
-    11, 11, 10,  6,  5,  4,  3,  3,  2,  5,  6,  4, 13, 13, 12,  9,  8,  7,  1,  1,  0,  8,  9,  7, \
-    12,  6,  6, 10,  9,  9,  4, 13,  1,  7, 11,  3,  7,  3, 11,  4,  1, 13,  2,  8,  8,  0,  5,  5, \
-    13,  4,  5,  9, 10, 11,  6, 12, 13, 11,  7,  8,  8,  2,  3,  1,  4,  6,  3,  7,  9,  5,  0,  1, \
-    13,  5,  4,  9, 11, 10,  1,  6,  4,  8,  3,  2, 11,  8,  7,  6, 13, 12,  3,  9,  7,  5,  1,  0
-// The same table in device and host memory: device code indexes the __device__ copy, which
-// the compiler folds to constants after unrolling (a table local to a constexpr function
-// would be rebuilt at every inlined call).
-__device__ constexpr signed char kKeClassDev[576] = {DV_KE_CLASS_TABLE};
-constexpr signed char kKeClassHost[576] = {DV_KE_CLASS_TABLE};
-__host__ __device__ __forceinline__ constexpr int ke_class(int i) {
-#ifdef __CUDA_ARCH__
-    return kKeClassDev[i];
-#else
-    return kKeClassHost[i];
-#endif
-}
-
 template <class AT>
-struct KeCoef {
-    AT cls[kKeClasses];
+struct HexModes {
+    AT a0, b0;   // t = 0 (the three normal strains): diagonal minus off-diagonal, off-diagonal
+    AT p, q;     // t = one axis: the two components that are not translations
+    AT r, w;     // t = two axes: shear (all four entries equal), the third component alone
+    AT g0, h0;   // t = three axes: as t = 0
 };
 
 // One mesh of a (possibly batched) matrix-free operator: its element counts, the tiles it is
@@ -1595,78 +1565,61 @@ struct KeCoef {
 struct HexMesh {
     int32_t ne0, ne1, ne2;     // elements per axis (free-node box: ne0 x (ne1 + 1) x (ne2 + 1))
     int32_t ntx, nty, zc;      // tiles per plane in x and y, planes per z run
+    int32_t wn, rn;            // nodes of a tile in x and y (one element column more in each)
     int32_t tile0, pad;        // first tile of this mesh
     int64_t row0, fac0;        // first row, first element factor
 };
 
-constexpr int kHexEX = kGridTX + 1, kHexEY = kGridTY + 1;   // element tile per layer (33 x 9)
-constexpr int kHexLayer = kHexEX * kHexEY;                  // 297 factors
-constexpr int kHexLayerLoads = (kHexLayer + 255) / 256;     // per thread (2)
+constexpr int kHexThreads = 256;
+constexpr int kHexLoads = 4;                               // staging slots per thread
+constexpr int kHexPlane = kHexLoads * kHexThreads;         // staged values of a plane, at most
 
-// Contributions of one element layer to the two accumulated nodes of the thread's column that
-// its elements contain.  L = 0: the layer above plane p (elements between p and p + 1; their
-// corners in plane p are lower corners), which holds node p + 1 as an upper corner (UP, into
-// au) and node p as a lower corner (DN, into ad).  L = 1: the layer below (p - 1 .. p; corners
-// in plane p are upper corners), holding node p as an upper corner and node p - 1 as a lower
-// one.  Each staged x value is scaled by the element factor once and applied to both nodes.
-template <class AT, bool FUSED, int L, bool UP, bool DN>
-__device__ __forceinline__ void hex_layer_terms(const AT (&xv)[27], const AT *__restrict__ el, int tx, int ty,
-                                                const KeCoef<AT> &kc, AT (&au)[3], AT (&ad)[3]) {
-    constexpr int vtk[8] = {0, 1, 3, 2, 4, 5, 7, 6};
-    constexpr int bz = L == 0 ? 0 : 1;
-#pragma unroll
-    for (int eyo = 0; eyo < 2; ++eyo)
-#pragma unroll
-        for (int exo = 0; exo < 2; ++exo) {
-            const AT f = el[(tx + exo) + kHexEX * (ty + eyo)];
-            const int a_up = vtk[(1 - exo) + 2 * (1 - eyo) + 4];   // the node as the element's upper corner
-            const int a_dn = vtk[(1 - exo) + 2 * (1 - eyo)];       // and as its lower corner
-#pragma unroll
-            for (int by = 0; by < 2; ++by)
-#pragma unroll
-                for (int bx = 0; bx < 2; ++bx) {
-                    const int b = vtk[bx + 2 * by + 4 * bz];
-                    const int dxs = exo + bx - 1, dys = eyo + by - 1;   // source node offset in the plane
-#pragma unroll
-                    for (int c = 0; c < 3; ++c) {
-                        const AT w = f * xv[9 * (dys + 1) + 3 * (dxs + 1) + c];
-#pragma unroll
-                        for (int d = 0; d < 3; ++d) {
-                            if (UP) au[d] = madd_op<AT, FUSED>(au[d], kc.cls[ke_class(24 * (3 * a_up + d) + 3 * b + c)], w);
-                            if (DN) ad[d] = madd_op<AT, FUSED>(ad[d], kc.cls[ke_class(24 * (3 * a_dn + d) + 3 * b + c)], w);
-                        }
-                    }
-                }
+// Tile of a mesh plane of lx x ly free nodes: (wn + 1) x (rn + 1) element columns, one a thread,
+// whose (wn + 2) x (rn + 2) nodes fit the staging slots; the fewest tiles, the widest at a tie.
+inline void hex_tile(int32_t lx, int32_t ly, int32_t &wn, int32_t &rn) {
+    int64_t best = INT64_MAX;
+    wn = rn = 1;
+    for (int32_t nt = 1; nt <= lx; ++nt) {
+        const int32_t w = (lx + nt - 1) / nt;
+        int32_t r = std::min<int32_t>(kHexThreads / (w + 1) - 1, ly);
+        while (r >= 1 && 3 * (w + 2) * (r + 2) > kHexPlane) --r;
+        if (r < 1) continue;
+        const int32_t my = (ly + r - 1) / r;
+        const int64_t tiles = (int64_t)((lx + w - 1) / w) * my;
+        if (tiles < best) {
+            best = tiles;
+            wn = w;
+            rn = (ly + my - 1) / my;
         }
+        if (w <= 8) break;
+    }
 }
 
-// One plane step: layer p feeds nodes p + 1 (DI) and p (DM), layer p - 1 nodes p (DM) and p - 1 (DF).
-template <class AT, bool FUSED, bool DI, bool DM, bool DF>
-__device__ __forceinline__ void hex_plane_step(const AT (&xv)[27], const AT *lay_up, const AT *lay_dn, int tx, int ty,
-                                               const KeCoef<AT> &kc, AT (&a0)[3], AT (&a1)[3], AT (&a2)[3]) {
-    if constexpr (DI || DM) hex_layer_terms<AT, FUSED, 0, DI, DM>(xv, lay_up, tx, ty, kc, a2, a1);
-    if constexpr (DM || DF) hex_layer_terms<AT, FUSED, 1, DM, DF>(xv, lay_dn, tx, ty, kc, a1, a0);
+// Corner values v[by][bx] of one component in a plane -> characters s = sx + 2 sy.
+template <class AT>
+__device__ __forceinline__ void hex_xy(AT v00, AT v10, AT v01, AT v11, AT (&s)[4]) {
+    const AT a = v00 + v10, b = v00 - v10, c = v01 + v11, d = v01 - v11;
+    s[0] = a + c;
+    s[1] = b + d;
+    s[2] = a - c;
+    s[3] = b - d;
 }
 
 template <class AT, class Gather, class Op>
-__global__ void __launch_bounds__(256, sizeof(AT) == 8 ? 1 : 3)
-    k_hex_elem(const HexMesh *__restrict__ meshes, int32_t nmesh, int32_t ntile, KeCoef<AT> kc,
+__global__ void __launch_bounds__(kHexThreads, sizeof(AT) == 8 ? 2 : 3)
+    k_hex_elem(const HexMesh *__restrict__ meshes, int32_t nmesh, int32_t ntile, HexModes<AT> kc,
                const AT *__restrict__ ef_all, Gather g, Op op, const int *__restrict__ done, double *partials,
                unsigned *ticket) {
     if (done && *(volatile const int *)done) return;
     extern __shared__ uint4 hex_smem[];
-    constexpr bool FU = op_fused<Op>::value;
     using SS = StageSrc<Gather>;
     using ST = typename SS::ST;
-    constexpr int SLOT = SS::N * kGridPlane;
-    constexpr int NL = kGridStages + 1;              // factor layers: each is read in two consecutive steps
-    ST *ring = reinterpret_cast<ST *>(hex_smem);     // kGridStages slots of node planes
-    AT *layer = reinterpret_cast<AT *>(ring + kGridStages * SLOT);   // NL slots of element factors
+    constexpr int SLOT = SS::N * kHexPlane;
+    ST *ring = reinterpret_cast<ST *>(hex_smem);                      // kGridStages slots of node planes
+    AT *share = reinterpret_cast<AT *>(ring + kGridStages * SLOT);    // 2 x 9 shares a thread
     double red[Op::NRED > 0 ? Op::NRED : 1];
 #pragma unroll
     for (int i = 0; i < (Op::NRED > 0 ? Op::NRED : 1); ++i) red[i] = 0.0;
-    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-    const StageSlots<1> slots;
     for (int t = blockIdx.x; t < ntile; t += gridDim.x) {
         int lo = 0, hi = nmesh - 1;   // the mesh of tile t: the last with tile0 <= t
         while (lo < hi) {
@@ -1676,82 +1629,144 @@ __global__ void __launch_bounds__(256, sizeof(AT) == 8 ? 1 : 3)
         }
         const HexMesh G = meshes[lo];
         const int32_t lx = G.ne0, ly = G.ne1 + 1, lz = G.ne2 + 1;
-        const int64_t lxy = (int64_t)lx * ly;
-        const int32_t plane_len = (int32_t)(3 * lxy), layer_len = G.ne0 * G.ne1;
-        const AT *ef = ef_all + G.fac0;
+        const int32_t plane_len = 3 * lx * ly, layer_len = G.ne0 * G.ne1;
+        const int W = G.wn + 1, R = G.rn + 1;   // element columns
         const int tl = t - G.tile0;
         const int txi = tl % G.ntx, tyi = (tl / G.ntx) % G.nty, tzi = tl / (G.ntx * G.nty);
-        const int x0 = txi * kGridTX, y0 = tyi * kGridTY, z0 = tzi * G.zc, z1 = min(lz, z0 + G.zc);
-        const int ix = x0 + tx, iy = y0 + ty;
-        const bool inxy = ix < lx && iy < ly;
-        const int64_t col_xy = G.row0 / 3 + ix + (int64_t)lx * iy;   // node index in the batch
-        int32_t poff[kGridLoads], loff[kHexLayerLoads];
-        slots.plane_offsets(x0, y0, lx, ly, poff);
+        const int x0 = txi * G.wn, y0 = tyi * G.rn, z0 = tzi * G.zc, z1 = min(lz, z0 + G.zc);
+        const int ty = (int)threadIdx.x / W, tx = (int)threadIdx.x - W * ty;
+        const bool column = ty < R;
+        const int ix = x0 + tx, iy = y0 + ty;   // the node this thread finishes; its element is (ix, iy - 1)
+        const bool node = column && tx < W - 1 && ty < R - 1 && ix < lx && iy < ly;
+        const bool inside = column && ix < G.ne0 && iy >= 1 && iy <= G.ne1;
+        const AT *ef = ef_all + G.fac0 + (inside ? ix + (int64_t)G.ne0 * (iy - 1) : 0);
+        auto factor = [&](int l) { return inside && l >= 0 && l < G.ne2 ? __ldg(ef + (int64_t)l * layer_len) : AT(0); };
+        const int32_t r_xy = (int32_t)G.row0 + 3 * (ix + lx * iy);
+        // staged plane: node (x0 - 1 + j, y0 - 1 + i), dof c at 3 ((W + 1) i + j) + c; offsets in the plane, -1
+        // outside the mesh, -2 past the tile
+        int32_t poff[kHexLoads];
+        const int staged = 3 * (W + 1) * (R + 1);
 #pragma unroll
-        for (int j = 0; j < kHexLayerLoads; ++j) {   // element (ex, ey) of the layer tile (x index 0 is clamped)
-            const int k = threadIdx.x + 256 * j;
-            const int ex = x0 + k % kHexEX, ey = y0 - 1 + k / kHexEX;
-            loff[j] = (k < kHexLayer && ex < G.ne0 && ey >= 0 && ey < G.ne1) ? ex + G.ne0 * ey : (k < kHexLayer ? -1 : -2);
+        for (int j = 0; j < kHexLoads; ++j) {
+            const int k = threadIdx.x + kHexThreads * j, nd = k / 3, i = nd / (W + 1);
+            const int xn = x0 - 1 + nd - (W + 1) * i, yn = y0 - 1 + i;
+            poff[j] = k >= staged ? -2 : xn >= 0 && xn < lx && yn >= 0 && yn < ly ? 3 * (xn + lx * yn) + (k - 3 * nd) : -1;
         }
-        // node plane z and element layer z (elements between planes z and z + 1), one copy group
         auto issue = [&](int z, int k) {
-            const bool lin = z >= 0 && z < G.ne2;
-            const int32_t lbase = lin ? z * layer_len : 0;
-            AT *ld = layer + (k % NL) * kHexLayer;
+            const bool zin = z >= 0 && z < lz;
+            const int64_t base = zin ? G.row0 + (int64_t)z * plane_len : 0;
+            ST *slot = ring + (k % kGridStages) * SLOT;
 #pragma unroll
-            for (int j = 0; j < kHexLayerLoads; ++j)
-                if (loff[j] > -2) {
-                    const bool v = lin && loff[j] >= 0;
-                    cp_async_zfill<sizeof(AT)>(ld + threadIdx.x + 256 * j, v ? ef + lbase + loff[j] : ef, v);
-                }
-            slots.template issue<SS>(g, ring + (k % kGridStages) * SLOT, poff, z, lz, plane_len, G.row0);   // commits
+            for (int q = 0; q < SS::N; ++q) {
+                const ST *src = SS::src(g, q);
+#pragma unroll
+                for (int j = 0; j < kHexLoads; ++j)
+                    if (poff[j] > -2) {
+                        const bool v = zin && poff[j] >= 0;
+                        cp_async_zfill<sizeof(ST)>(slot + q * kHexPlane + threadIdx.x + kHexThreads * j,
+                                                   v ? src + base + poff[j] : src, v);
+                    }
+            }
+            cp_async_commit();
         };
 #pragma unroll
         for (int q = 0; q < kGridStages - 1; ++q) {
             if (z0 - 1 + q <= z1) issue(z0 - 1 + q, q);
             else cp_async_commit();
         }
-        AT a0[3], a1[3], a2[3];
+        AT sp[3][4], up[3][4];   // the plane below, transformed; its part from the layer under it
 #pragma unroll
-        for (int d = 0; d < 3; ++d) a0[d] = a1[d] = a2[d] = AT(0);
-        for (int p = z0 - 1, k = 0; p <= z1; ++p, ++k) {
-            cp_async_wait<kGridStages - 2>();
-            __syncthreads();
+        for (int c = 0; c < 3; ++c)
+#pragma unroll
+            for (int s = 0; s < 4; ++s) sp[c][s] = up[c][s] = AT(0);
+        AT own[3] = {AT(0), AT(0), AT(0)};
+        AT fa = factor(z0 - 1), fb = factor(z0);
+        const int corner = column ? 3 * ((W + 1) * ty + tx) : 0;
+        for (int p = z0 - 1, k = 0; p <= z1 + 1; ++p, ++k) {
+            cp_async_wait<kGridStages - 2>();   // plane p has landed (this thread's copies)
+            __syncthreads();                     // ... and everyone's, and the shares of plane p - 2
+            if (p - 2 >= z0 && node) {   // finish node plane p - 2
+                const AT *sh = share + ((k + 1) & 1) * 9 * kHexThreads + threadIdx.x;
+                const int32_t r = r_xy + (p - 2) * plane_len;
+#pragma unroll
+                for (int c = 0; c < 3; ++c) {
+                    const AT s = (own[c] + sh[c * kHexThreads + 1]) +
+                                 (sh[(3 + c) * kHexThreads + W] + sh[(6 + c) * kHexThreads + W + 1]);
+                    op.row(r + c, op.init(r + c) + s, red);
+                }
+            }
+            if (p > z1) break;
             if (p + kGridStages - 1 <= z1) issue(p + kGridStages - 1, k + kGridStages - 1);
             else cp_async_commit();
-            const ST *pl = ring + (k % kGridStages) * SLOT;
-            const AT *lay_up = layer + (k % NL) * kHexLayer;             // layer p
-            const AT *lay_dn = layer + ((k + NL - 1) % NL) * kHexLayer;  // layer p - 1
-            const bool di = p + 1 >= z0 && p + 1 < z1, dm = p >= z0 && p < z1, df = p - 1 >= z0 && p - 1 < z1;
-            if (di) {
-                const int32_t r = (int32_t)(3 * (col_xy + lxy * (p + 1)));
+            const ST *pl = ring + (k % kGridStages) * SLOT + corner;
+            AT sc[3][4];
 #pragma unroll
-                for (int d = 0; d < 3; ++d) a2[d] = inxy ? op.init(r + d) : AT(0);
+            for (int c = 0; c < 3; ++c)
+                hex_xy<AT>(SS::template value<kHexPlane>(pl, c), SS::template value<kHexPlane>(pl, 3 + c),
+                           SS::template value<kHexPlane>(pl, 3 * (W + 1) + c),
+                           SS::template value<kHexPlane>(pl, 3 * (W + 1) + 3 + c), sc[c]);
+            if (p >= z0) {
+                // element layer p - 1 .. p: X+ = lower + upper (sz = 0), X- = lower - upper (sz = 1)
+                const AT f = fa;
+                fa = fb;
+                fb = factor(p + 1);
+                if (p - 1 >= z0 && node) touch_rows(op, r_xy + (p - 1) * plane_len);   // finished next step
+                AT xp[3][4], xm[3][4];
+#pragma unroll
+                for (int c = 0; c < 3; ++c)
+#pragma unroll
+                    for (int s = 0; s < 4; ++s) {
+                        xp[c][s] = sp[c][s] + sc[c][s];
+                        xm[c][s] = sp[c][s] - sc[c][s];
+                    }
+                AT yp[3][4], ym[3][4];
+                auto three = [&](AT u, AT v, AT w, AT d, AT o, AT &yu, AT &yv, AT &yw) {
+                    const AT m = o * (u + v + w);
+                    yu = f * fma(d, u, m);
+                    yv = f * fma(d, v, m);
+                    yw = f * fma(d, w, m);
+                };
+                auto two = [&](AT u, AT v, AT &yu, AT &yv) {
+                    yu = f * fma(kc.p, u, kc.q * v);
+                    yv = f * fma(kc.p, v, kc.q * u);
+                };
+                const AT fr = f * kc.r, fw = f * kc.w;
+                yp[0][0] = yp[1][0] = yp[2][0] = AT(0);                                                   // translations
+                three(xp[0][1], xp[1][2], xm[2][0], kc.a0, kc.b0, yp[0][1], yp[1][2], ym[2][0]);         // t = 000
+                two(xp[1][3], xm[2][1], yp[1][3], ym[2][1]);                                              // x
+                two(xp[0][3], xm[2][2], yp[0][3], ym[2][2]);                                              // y
+                two(xm[0][1], xm[1][2], ym[0][1], ym[1][2]);                                              // z
+                yp[0][2] = yp[1][1] = fr * (xp[0][2] + xp[1][1]);                                         // xy
+                ym[2][3] = fw * xm[2][3];
+                ym[0][0] = yp[2][1] = fr * (xm[0][0] + xp[2][1]);                                         // xz
+                ym[1][3] = fw * xm[1][3];
+                ym[1][0] = yp[2][2] = fr * (xm[1][0] + xp[2][2]);                                         // yz
+                ym[0][3] = fw * xm[0][3];
+                three(xm[0][2], xm[1][1], xp[2][3], kc.g0, kc.h0, ym[0][2], ym[1][1], yp[2][3]);         // xyz
+                // plane p - 1: the part from below and this layer's lower face, back to corners
+                if (p - 1 >= z0) {
+                    AT *sh = share + (k & 1) * 9 * kHexThreads + threadIdx.x;
+#pragma unroll
+                    for (int c = 0; c < 3; ++c) {
+                        AT n[4], T[4];
+#pragma unroll
+                        for (int s = 0; s < 4; ++s) T[s] = up[c][s] + (yp[c][s] + ym[c][s]);
+                        hex_xy<AT>(T[0], T[1], T[2], T[3], n);   // its own inverse but for the factor: n[bx + 2 by]
+                        own[c] = n[3];
+                        sh[c * kHexThreads] = n[2];         // (bx, by) = (0, 1): the node to the left
+                        sh[(3 + c) * kHexThreads] = n[1];   // (1, 0): the node below
+                        sh[(6 + c) * kHexThreads] = n[0];
+                    }
+                }
+#pragma unroll
+                for (int c = 0; c < 3; ++c)
+#pragma unroll
+                    for (int s = 0; s < 4; ++s) up[c][s] = yp[c][s] - ym[c][s];
             }
-            if (dm && inxy) touch_rows(op, (int32_t)(3 * (col_xy + lxy * p)));   // finished next step
-            AT xv[27];
 #pragma unroll
-            for (int dy = 0; dy < 3; ++dy)
+            for (int c = 0; c < 3; ++c)
 #pragma unroll
-                for (int dx = 0; dx < 3; ++dx)
-#pragma unroll
-                    for (int c = 0; c < 3; ++c) xv[9 * dy + 3 * dx + c] = SS::value(pl, ((ty + dy) * kGridPX + tx + dx) * 3 + c);
-            if (di && dm && df) hex_plane_step<AT, FU, true, true, true>(xv, lay_up, lay_dn, tx, ty, kc, a0, a1, a2);
-            else if (di && dm) hex_plane_step<AT, FU, true, true, false>(xv, lay_up, lay_dn, tx, ty, kc, a0, a1, a2);
-            else if (dm && df) hex_plane_step<AT, FU, false, true, true>(xv, lay_up, lay_dn, tx, ty, kc, a0, a1, a2);
-            else if (di) hex_plane_step<AT, FU, true, false, false>(xv, lay_up, lay_dn, tx, ty, kc, a0, a1, a2);
-            else if (dm) hex_plane_step<AT, FU, false, true, false>(xv, lay_up, lay_dn, tx, ty, kc, a0, a1, a2);
-            else if (df) hex_plane_step<AT, FU, false, false, true>(xv, lay_up, lay_dn, tx, ty, kc, a0, a1, a2);
-            if (df && inxy) {
-                const int32_t r = (int32_t)(3 * (col_xy + lxy * (p - 1)));
-#pragma unroll
-                for (int d = 0; d < 3; ++d) op.row(r + d, a0[d], red);
-            }
-#pragma unroll
-            for (int d = 0; d < 3; ++d) {
-                a0[d] = a1[d];
-                a1[d] = a2[d];
-            }
+                for (int s = 0; s < 4; ++s) sp[c][s] = sc[c][s];
         }
         cp_async_wait<0>();
         __syncthreads();   // the next tile refills the rings
@@ -1766,16 +1781,16 @@ template <class AT, class Gather, class Op>
 void launch_hex_elem(const LaunchEnv &e, const dv_matrix *m, Gather g, Op op) {
     auto kern = k_hex_elem<AT, Gather, Op>;
     using SS = StageSrc<Gather>;
-    const size_t smem = sizeof(typename SS::ST) * SS::N * kGridStages * (size_t)kGridPlane +
-                        sizeof(AT) * (kGridStages + 1) * (size_t)kHexLayer;
+    const size_t smem = sizeof(typename SS::ST) * SS::N * kGridStages * (size_t)kHexPlane +
+                        sizeof(AT) * 18 * (size_t)kHexThreads;
     static SmemLimit limit;   // per instantiation and device
     limit.raise(kern, smem, e.ctx->device);
-    KeCoef<AT> kc;
-    for (int c = 0; c < kKeClasses; ++c) kc.cls[c] = (AT)m->hex_cls[c];
+    const double *c = m->hex_modes;
+    const HexModes<AT> kc{(AT)c[0], (AT)c[1], (AT)c[2], (AT)c[3], (AT)c[4], (AT)c[5], (AT)c[6], (AT)c[7]};
     const int blocks = (int)std::min<int64_t>(m->hex_ntile, e.max_blocks);
-    kern<<<blocks, 256, smem, e.stream>>>(m->hex_meshes.as<HexMesh>(), m->hex_nmesh, m->hex_ntile, kc,
-                                          static_cast<const AT *>(m->hex_factor.p), g, op, e.done, e.partials,
-                                          e.ticket);
+    kern<<<blocks, kHexThreads, smem, e.stream>>>(m->hex_meshes.as<HexMesh>(), m->hex_nmesh, m->hex_ntile, kc,
+                                                  static_cast<const AT *>(m->hex_factor.p), g, op, e.done, e.partials,
+                                                  e.ticket);
     DV_CUDA(cudaGetLastError());
     e.ctx->count();
 }

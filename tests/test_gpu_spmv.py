@@ -499,3 +499,15 @@ def test_csr_node_groups(ctx, native, rng, width, prec):
     M.residual_device(db.data_ptr(), dx.data_ptr(), dr.data_ptr(), prec)
     ctx.synchronize()
     assert np.max(np.abs(dr.cpu().numpy() - (b - A @ x)) / scale) <= bar
+
+
+@pytest.mark.parametrize("ne", [(260, 1, 1), (2, 300, 1), (1, 2, 70), (64, 17, 5), (31, 33, 9), (23, 11, 18)])
+def test_matrix_free_hex_operator_tiles(ctx, native, rng, ne):
+    # Meshes at the edges of the element kernel's tiles (wider and higher than one tile, one node wide,
+    # several z runs): against the assembled 64-bit product, the bars of the operator's other test.
+    E = 10.0 ** rng.uniform(-2.0, 0.0, int(np.prod(ne)))
+    A = native.hex_stiffness(ne, E)
+    x = rng.standard_normal(A.shape[1])
+    for prec, bar, dt in (("f64", REL64, np.float64), ("f32", REL32, np.float32)):
+        H = native.SparseMatrix.hex_operator(ctx, ne, E, precision=prec)
+        assert rowwise_rel(_device_product(ctx, H, x, dt).astype(np.float64), A @ x, A, x) <= bar

@@ -505,7 +505,7 @@ __global__ void __launch_bounds__(kThreads) k_csr_nodes(const int32_t *__restric
             for (int u = 0; u < U; ++u)
                 if (base + u * W < len)
 #pragma unroll
-                    for (int d = 0; d < 3; ++d) s[d] = madd<AT>(s[d], v[u][d], xv[u]);
+                    for (int d = 0; d < 3; ++d) s[d] = fma(v[u][d], xv[u], s[d]);   // one rounding a term
         }
 #pragma unroll
         for (int d = 0; d < 3; ++d) s[d] = group_sum<W>(s[d]);

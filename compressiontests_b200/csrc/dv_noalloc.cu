@@ -29,6 +29,7 @@
 //    matrix format it will use before reserving it, or run with
 //    CUDA_MODULE_LOADING=EAGER, which loads everything when CUDA initialises.
 #include "dv_kernels.cuh"
+#include "dv_pcg_resident.cuh"
 
 #include <chrono>
 #include <cmath>
@@ -43,6 +44,7 @@ constexpr int kNoAllocMaxBlocks = 4096;
 constexpr size_t kHeaderBytes = 256;                                   // ticket + scalars
 constexpr size_t kPartialBytes = sizeof(double) * kMaxRed * kNoAllocMaxBlocks;
 constexpr size_t kVectorBytes = sizeof(double) * (size_t)kNoAllocMaxRows;
+static_assert(5 * (size_t)kPcgResidentRows <= 4 * (size_t)kNoAllocMaxRows, "five vectors do not fit the array");
 constexpr size_t kScratchBytes = kHeaderBytes + kPartialBytes + 4 * kVectorBytes;   // 4,325,632 bytes
 static_assert(sizeof(SolverScalars) + 16 <= kHeaderBytes, "scalars do not fit the header");
 
@@ -165,7 +167,11 @@ extern "C" DV_API int dv_pcg_solve_noalloc(dv_matrix *A, const double *d_b, doub
         SolverScalars *sc = reinterpret_cast<SolverScalars *>(base + 16);
         double *partials = reinterpret_cast<double *>(base + kHeaderBytes);
         double *r = reinterpret_cast<double *>(base + kHeaderBytes + kPartialBytes);
-        double *z = r + kNoAllocMaxRows, *p = z + kNoAllocMaxRows, *ap = p + kNoAllocMaxRows;
+        // small systems iterate in one kernel, as dv_pcg_solve's do, with a second direction vector: five
+        // vectors of n rows in the room of four of the largest system
+        const bool resident = dv_pcg_resident_ok(A);
+        const size_t len = resident ? (size_t)n : (size_t)kNoAllocMaxRows;
+        double *z = r + len, *p = z + len, *ap = p + len;
         // The ticket must start at zero; the scalars are written by k_na_init.
         DV_CUDA(cudaMemsetAsync(ticket, 0, 16, st));
         k_na_init<<<1, 1, 0, st>>>(sc, max_iterations);
@@ -194,7 +200,14 @@ extern "C" DV_API int dv_pcg_solve_noalloc(dv_matrix *A, const double *d_b, doub
         LaunchEnv ed = e;
         ed.done = &sc->done;
         SolverScalars h{};
-        for (;;) {
+        if (resident) {
+            DV_REQUIRE(dv_pcg_resident_bytes(ctx) <= kPartialBytes, DV_ERR_CUDA, "too many SMs for the fixed array");
+            dv_pcg_resident(A, A->diag.as<double>(), 1, d_x, r, z, ap + len, p, ap, partials, sc, tol, 0);
+            DV_CUDA(cudaMemcpyAsync(&h, sc, sizeof(h), cudaMemcpyDeviceToHost, st));
+            DV_CUDA(cudaStreamSynchronize(st));
+            DV_REQUIRE(h.done, DV_ERR_CUDA, "the blocks of the one-kernel PCG lost one another");
+        }
+        while (!h.done) {
             for (int k = 0; k < 8; ++k) {
                 OpPcgAp op{p, ap, sc};
                 launch_rows<double>(ed, A, GatherVec<double, double>{p}, op);
@@ -207,12 +220,15 @@ extern "C" DV_API int dv_pcg_solve_noalloc(dv_matrix *A, const double *d_b, doub
             }
             DV_CUDA(cudaMemcpyAsync(&h, sc, sizeof(h), cudaMemcpyDeviceToHost, st));
             DV_CUDA(cudaStreamSynchronize(st));
-            if (h.done) break;
         }
-        // relative residual of the returned x in FP64: z = b - A x (z is free now), ||b||, ||z||
+        // relative residual of the returned x in FP64: z = b - A x (z is free now), ||b||, ||z||.  Close to the
+        // limit of FP64 its last digits depend on the order of the row sums: a small system's CSR rows are
+        // summed one thread a row in the stored order, as DuVi rows are and as a host would.
         {
             OpResid<double> op{{}, d_b, z};
-            launch_rows<double>(e, A, GatherVec<double, double>{d_x}, op);
+            const GatherVec<double, double> x{d_x};
+            if (resident && A->format == DV_FORMAT_CSR) launch_csr_tpr<1, double>(e, A, x, op);
+            else launch_rows<double>(e, A, x, op);
             k_na_norms<<<grid, kThreads, 0, st>>>(d_b, z, n, sc, partials, ticket);
             DV_CUDA(cudaGetLastError());
             ctx->count();

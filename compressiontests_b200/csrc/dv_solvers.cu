@@ -8,6 +8,7 @@
 // iterate is frozen at the iteration that met the stop test and the host reads
 // the flag once per chunk.
 #include "dv_kernels.cuh"
+#include "dv_pcg_resident.cuh"
 #include "dv_solvers.cuh"
 #include "dv_mgpcg.cuh"
 
@@ -304,6 +305,7 @@ struct dv_pcg {
     double tol = 0;
     int32_t tol_kind = DV_TOL_ABS_MAX;
     DevMem M, b, x, r, z, p, ap;
+    DevMem p1, work;   // second direction buffer and barrier of the one-kernel iteration (small systems)
 };
 
 extern "C" DV_API int dv_pcg_set_tolerance_kind(dv_pcg *s, int32_t tol_kind) {
@@ -337,6 +339,10 @@ extern "C" DV_API int dv_pcg_create(dv_context *ctx, const dv_csr_host *A, int32
         s->M.alloc(nb);
         DV_CUDA(cudaMemcpyAsync(s->M.p, minv.data(), nb, cudaMemcpyHostToDevice, ctx->stream));
         s->b.alloc(nb); s->x.alloc(nb); s->r.alloc(nb); s->z.alloc(nb); s->p.alloc(nb); s->ap.alloc(nb);
+        if (dv_pcg_resident_ok(s->A.get())) {
+            s->p1.alloc(nb);
+            s->work.alloc(dv_pcg_resident_bytes(ctx));
+        }
         DV_CUDA(cudaStreamSynchronize(ctx->stream));
         *out = s.release();
     });
@@ -392,17 +398,27 @@ extern "C" DV_API int dv_pcg_solve(dv_pcg *s, const double *b, const double *x0,
                 ctx->count(2);
             }
         };
-        for (;;) {
+        if (s->work.p) {   // every iteration in one kernel
+            dv_pcg_resident(s->A.get(), s->M.as<double>(), 0, s->x.as<double>(), s->r.as<double>(), s->z.as<double>(),
+                            s->p1.as<double>(), s->p.as<double>(), s->ap.as<double>(), s->work.p, s->ws->sc(), s->tol,
+                            rel_l2);
+            s->ws->pull();
+            DV_REQUIRE(h.done, DV_ERR_CUDA, "the blocks of the one-kernel PCG lost one another");
+        }
+        while (!h.done) {
             s->ws->run_chunk(body, true, 3 * chunk);
             s->ws->pull();
-            if (h.done) break;
         }
         DV_CUDA(cudaEventRecord(e1, st));
         DV_CUDA(cudaMemcpyAsync(xout, s->x.p, nb, cudaMemcpyDeviceToHost, st));
-        // relative residual of the returned x, recomputed in FP64: z = b - A x, ||z||^2
+        // relative residual of the returned x, recomputed in FP64: z = b - A x, ||z||^2.  Close to the limit of
+        // FP64 its last digits depend on the order of the row sums: a small system's CSR rows are summed
+        // one thread a row in the stored order, as DuVi rows are and as a host would.
         {
             OpResid<double> op{{}, s->b.as<double>(), s->z.as<double>()};
-            launch_rows<double>(e, s->A.get(), GatherVec<double, double>{s->x.as<double>()}, op);
+            const GatherVec<double, double> x{s->x.as<double>()};
+            if (s->work.p && s->A->format == DV_FORMAT_CSR) launch_csr_tpr<1, double>(e, s->A.get(), x, op);
+            else launch_rows<double>(e, s->A.get(), x, op);
             k_norm2<<<g, kThreads, 0, st>>>(s->z.as<double>(), n, s->ws->sc(), 1, e.partials, e.ticket);
             DV_CUDA(cudaGetLastError());
             ctx->count();

@@ -349,3 +349,23 @@ def test_slab_operator_on_device_single_rank(ctx, native, oracle):
     assert conv and abs(its - it_ref) <= 1
     assert rel(xs.cpu().numpy(), x_ref) < 1e-7
     op.release()
+
+
+@pytest.mark.parametrize("fmt", ["csr", "duvi"])
+@pytest.mark.parametrize("ne", [(1, 1, 1), (5, 3, 2), (24, 24, 24), (36, 34, 34)])
+def test_pcg_sizes_match_oracle(ctx, native, oracle, fmt, ne):
+    # From fewer node groups than blocks, over several groups a warp (45,000 rows), to the first
+    # size past the one-kernel iteration (132,300 rows): iterations within 1 and the solution
+    # within 1e-7 of the oracle's, from zero and from a guess.
+    A = native.hex_stiffness(ne)
+    b = native.traction_rhs(ne)
+    K = oracle.Csr.from_scipy(A)
+    x_ref, it_ref = oracle.pcg_jacobi(K, b, 20000, 1e-9, rel_l2=True)
+    assert it_ref >= 0
+    s = native.CudaCsrPcgSolver(ctx, 20000, 1e-9, fmt=fmt, tol_kind="rel_l2").Initialize(A=A, b=b)
+    x, st = s.Solve()
+    assert st.HasConverged and abs(st.NumIterationsRequired - it_ref) <= 1
+    assert rel(x, x_ref) < 1e-7
+    x2, st2 = s.Solve(xInitialGuess=0.5 * x)
+    assert st2.HasConverged and rel(x2, x_ref) < 1e-7
+    s.ReleaseCudaResources()

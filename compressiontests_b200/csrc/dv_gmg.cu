@@ -83,7 +83,7 @@ static void smooth(dv_gmg *g, const LaunchEnv &e, GLevel &L, int sweeps) {
         }
         return;
     }
-    for (int k = 0; k < sweeps; ++k) gs_sweep<double>(e, L.A.get(), L.gs, L.b.as<double>(), L.x.as<double>());
+    gs_sweeps<double>(e, L.A.get(), L.gs, L.b.as<double>(), L.x.as<double>(), sweeps);
 }
 
 // One V-cycle pass over the path (the step loop of Solve).
@@ -203,7 +203,10 @@ extern "C" DV_API int dv_gmg_create(dv_context *ctx, int32_t n_levels, const dv_
             }
             const size_t nb = 8 * (size_t)L.n;
             L.b.alloc(nb); L.x.alloc(nb); L.t.alloc(nb); L.r.alloc(nb); L.D.alloc(nb);
-            if (cfg->smoother != DV_SMOOTHER_JACOBI) gs_build_order(A[l], cfg->smoother == DV_SMOOTHER_GS_LEX, s, L.gs);
+            if (cfg->smoother != DV_SMOOTHER_JACOBI) {
+                gs_build_order(A[l], cfg->smoother == DV_SMOOTHER_GS_LEX, s, L.gs);
+                gs_prepare_block<double>(L.A.get(), L.gs);
+            }
         }
         // relaxation (GeometricMultigridSolver.cs:209-214 / :109-121 / OpenCLCsrGeometricMultigridSolver.cs:164-171)
         if (cfg->coarse_relaxation) {

@@ -123,6 +123,130 @@ __global__ void __launch_bounds__(256) k_gs_pattern(const uint16_t *__restrict__
     }
 }
 
+// ---------------------------------------------------------------------------
+// Forward sweeps in the reference's row order by one block, for systems whose x fits its shared
+// memory
+//
+// A dependency level of a small system holds a few dozen rows, and a launch per level waits for the
+// launch before and then walks each row's entries one after another in one thread.  Here one block
+// runs all levels of all sweeps with x in shared memory and a barrier between levels.  A warp takes
+// a row: the lanes load its entries (those of the warp's next row are in flight across the
+// barrier), form the products a_ij x_j side by side and leave them in shared memory, from where
+// they are subtracted one after another in column order: products and differences are rounded
+// one by one as in gs_row_csr, so the result is the same bit for bit (the diagonal and the padding
+// subtract +0, which changes nothing).  Bound by that chain of dependent subtractions.
+// 12 x 4 x 4 elements, two levels, to 1e-3: 1,040 -> 109 ms (13.8 -> about 1.2 us a dependency level).
+// ---------------------------------------------------------------------------
+constexpr int kGsWarps = 32;
+constexpr int kGsLane = 3;   // entries of a row a lane holds at a time (96 a warp)
+
+template <class T>
+__global__ void __launch_bounds__(kGsWarps * 32) k_gs_block(const int32_t *__restrict__ rp, const int32_t *__restrict__ ci,
+                                                            const T *__restrict__ va, const T *__restrict__ b, T *x,
+                                                            const int32_t *__restrict__ rows,
+                                                            const int32_t *__restrict__ off, int32_t nlevels, int32_t n,
+                                                            int sweeps, const int *__restrict__ done) {
+    if (done && *(volatile const int *)done) return;
+    extern __shared__ uint4 gsb_smem[];
+    constexpr int W = 32 * kGsLane;
+    T *prod = reinterpret_cast<T *>(gsb_smem) + (threadIdx.x >> 5) * W;   // this warp's products
+    T *xs = reinterpret_cast<T *>(gsb_smem) + kGsWarps * W;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int32_t i = threadIdx.x; i < n; i += kGsWarps * 32) xs[i] = x[i];
+    // a row and the first W of its entries, held by the warp
+    struct Row {
+        int32_t i, s, len, c[kGsLane];
+        T v[kGsLane], b;
+    } q;
+    auto load = [&](int32_t t) {
+        q.i = __ldg(rows + t);
+        q.s = __ldg(rp + q.i);
+        q.len = __ldg(rp + q.i + 1) - q.s;
+        q.b = b[q.i];
+#pragma unroll
+        for (int u = 0; u < kGsLane; ++u) {
+            const int32_t k = lane + 32 * u;
+            q.c[u] = k < q.len ? __ldg(ci + q.s + k) : q.i;   // padding: as the diagonal, but without a value
+            q.v[u] = k < q.len ? __ldg(va + q.s + k) : T(0);
+        }
+    };
+    const int32_t last = sweeps * nlevels;
+    int32_t t0 = __ldg(off), t1 = __ldg(off + 1);
+    if (t0 + warp < t1) load(t0 + warp);
+    for (int32_t l = 0; l < last; ++l) {
+        __syncthreads();   // the rows of the level before are in xs
+        int32_t n0 = 0, n1 = 0;   // the next level's rows
+        if (l + 1 < last) {
+            const int32_t m = (l + 1) % nlevels;
+            n0 = __ldg(off + m);
+            n1 = __ldg(off + m + 1);
+        }
+        for (int32_t t = t0 + warp; t < t1; t += kGsWarps) {
+            T s = q.b, d = T(0);
+            const int32_t i = q.i;
+            for (int32_t k0 = 0;; k0 += W) {
+                const int32_t cnt = min(W, q.len - k0);
+#pragma unroll
+                for (int u = 0; u < kGsLane; ++u) {
+                    const bool diag = q.c[u] == i;
+                    if (diag && k0 + lane + 32 * u < q.len) d = q.v[u];
+                    prod[lane + 32 * u] = diag ? T(0) : rn_mul<T>(q.v[u], xs[q.c[u]]);
+                }
+                __syncwarp();
+#pragma unroll 4
+                for (int32_t k = 0; k < cnt; k += 4) {   // W is a multiple of 4: the padding subtracts +0
+                    T p[4];
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) p[u] = prod[k + u];
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) s = rn_sub<T>(s, p[u]);
+                }
+                __syncwarp();
+                if (k0 + W >= q.len) break;
+#pragma unroll
+                for (int u = 0; u < kGsLane; ++u) {   // the next W entries of a longer row
+                    const int32_t k = k0 + W + lane + 32 * u;
+                    q.c[u] = k < q.len ? __ldg(ci + q.s + k) : i;
+                    q.v[u] = k < q.len ? __ldg(va + q.s + k) : T(0);
+                }
+            }
+            // the next row of this warp, in this level or the next one
+            const bool more = t + kGsWarps < t1;
+            const unsigned has = __ballot_sync(0xffffffffu, d != T(0));
+            d = __shfl_sync(0xffffffffu, d, has ? __ffs(has) - 1 : 0);
+            if (more) load(t + kGsWarps);
+            else if (n0 + warp < n1) load(n0 + warp);
+            if (lane == 0) xs[i] = rn_div<T>(s, d);
+        }
+        if (t0 + warp >= t1 && n0 + warp < n1) load(n0 + warp);   // no row in this level
+        t0 = n0;
+        t1 = n1;
+    }
+    __syncthreads();
+    for (int32_t i = threadIdx.x; i < n; i += kGsWarps * 32) x[i] = xs[i];
+}
+
+// Columns and values of a DuVi matrix, entry by entry (the one-block sweep walks them side by side).
+template <class VI, class T>
+__global__ void k_gs_decode(DuviArgs A, int32_t n, int32_t *__restrict__ col, T *__restrict__ val) {
+    const T *tab = static_cast<const T *>(A.values);
+    const VI *vi = static_cast<const VI *>(A.vidx);
+    for (int32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        uint32_t di = A.row_to_dist[i];
+        for (uint32_t bl = A.row_to_col[i]; bl < A.row_to_col[i + 1]; ++bl) {
+            uint32_t c = A.col_idx[bl];
+            const int cnt = A.dist[di];
+            for (int k = 0;; ++k) {
+                col[di] = (int32_t)c;
+                val[di] = tab[vi[di]];
+                ++di;
+                if (k == cnt) break;
+                c += A.dist[di] + 1u;
+            }
+        }
+    }
+}
+
 inline DuviArgs gs_duvi_args(const dv_matrix *m) {
     DuviArgs a;
     a.row_to_col = m->row_to_col.as<uint32_t>();
@@ -142,12 +266,16 @@ struct GsOrder {
     DevMem rows;
     std::vector<int32_t> off;
     int bs = 1;
+    bool lex = false;
+    bool block = false;          // swept by one block (k_gs_block): level offsets and, for DuVi, the entries
+    DevMem d_off, col, val;
 };
 
 // Builds the ordering: lex = dependency levels of the forward sweep (rows);
 // otherwise a greedy coloring of node blocks (3 or 2 consecutive rows when the size allows).
 inline void gs_build_order(const dv_csr_host &a, bool lex, cudaStream_t s, GsOrder &o) {
     std::vector<int32_t> rows;
+    o.lex = lex;
     if (lex) {
         dv_gs_level_sets(a, rows, o.off);
         o.bs = 1;
@@ -165,6 +293,35 @@ inline void gs_build_order(const dv_csr_host &a, bool lex, cudaStream_t s, GsOrd
     o.rows.alloc(4 * rows.size());
     DV_CUDA(cudaMemcpyAsync(o.rows.p, rows.data(), 4 * rows.size(), cudaMemcpyHostToDevice, s));
     DV_CUDA(cudaStreamSynchronize(s));
+}
+
+template <class T>
+constexpr size_t gs_block_smem(int32_t n) {
+    return sizeof(T) * ((size_t)n + kGsWarps * 32 * kGsLane);
+}
+
+// Prepares the one-block sweep of A's row-order levels where x fits a block's shared memory (FP64 up
+// to 25,984 rows).  There a level has a few dozen rows and one block is enough for it; a level of a
+// larger system has hundreds to thousands, and every level stays a launch over all SMs.
+template <class T>
+void gs_prepare_block(const dv_matrix *A, GsOrder &o) {
+    dv_context *ctx = A->ctx;
+    if (!o.lex || A->n_rows == 0 || gs_block_smem<T>(A->n_rows) > (size_t)ctx->max_smem_optin - 1024) return;
+    cudaStream_t s = ctx->stream;
+    o.d_off.alloc(4 * o.off.size());
+    DV_CUDA(cudaMemcpyAsync(o.d_off.p, o.off.data(), 4 * o.off.size(), cudaMemcpyHostToDevice, s));
+    if (A->format == DV_FORMAT_DUVI) {
+        o.col.alloc(4 * (size_t)A->nnz);
+        o.val.alloc(sizeof(T) * (size_t)A->nnz);
+        const int grid = (A->n_rows + 255) / 256;
+        if (A->vi_bits == 8) k_gs_decode<uint8_t, T><<<grid, 256, 0, s>>>(gs_duvi_args(A), A->n_rows, o.col.as<int32_t>(), o.val.as<T>());
+        else if (A->vi_bits == 16) k_gs_decode<uint16_t, T><<<grid, 256, 0, s>>>(gs_duvi_args(A), A->n_rows, o.col.as<int32_t>(), o.val.as<T>());
+        else k_gs_decode<uint32_t, T><<<grid, 256, 0, s>>>(gs_duvi_args(A), A->n_rows, o.col.as<int32_t>(), o.val.as<T>());
+        DV_CUDA(cudaGetLastError());
+        ctx->count();
+    }
+    DV_CUDA(cudaStreamSynchronize(s));
+    o.block = true;
 }
 
 // One forward sweep over all groups of the ordering (x updated in place).
@@ -198,6 +355,26 @@ void gs_sweep(const LaunchEnv &e, const dv_matrix *A, const GsOrder &o, const T 
         DV_CUDA(cudaGetLastError());
         ctx->count();
     }
+}
+
+// `sweeps` forward sweeps.
+template <class T>
+void gs_sweeps(const LaunchEnv &e, const dv_matrix *A, const GsOrder &o, const T *b, T *x, int sweeps) {
+    if (!o.block) {
+        for (int k = 0; k < sweeps; ++k) gs_sweep<T>(e, A, o, b, x);
+        return;
+    }
+    if (sweeps < 1) return;
+    const bool csr = A->format == DV_FORMAT_CSR;
+    const size_t smem = gs_block_smem<T>(A->n_rows);
+    static SmemLimit limit;   // per instantiation and device
+    limit.raise(k_gs_block<T>, smem, e.ctx->device);
+    k_gs_block<T><<<1, kGsWarps * 32, smem, e.stream>>>(
+        csr ? A->rowptr.as<int32_t>() : A->row_to_dist.as<int32_t>(), csr ? A->col.as<int32_t>() : o.col.as<int32_t>(),
+        csr ? static_cast<const T *>(A->val.p) : o.val.as<T>(), b, x, o.rows.as<int32_t>(), o.d_off.as<int32_t>(),
+        (int32_t)o.off.size() - 1, A->n_rows, sweeps, e.done);
+    DV_CUDA(cudaGetLastError());
+    e.ctx->count();
 }
 
 }  // namespace dvk

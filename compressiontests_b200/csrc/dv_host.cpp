@@ -838,13 +838,19 @@ int dv_gs_level_sets(const dv_csr_host &a, std::vector<int32_t> &perm, std::vect
     int32_t n = a.n_rows;
     std::vector<int32_t> lev(n, 0);
     int32_t maxl = 0;
+    // row i comes after the rows j < i it reads, and before the rows j > i whose old value it reads (the
+    // same rows where the structure is symmetric); lev[j] of a later row holds its bound so far
     for (int32_t i = 0; i < n; ++i) {
-        int32_t l = 0;
+        int32_t l = lev[i];
         for (int32_t k = a.rowptr[i]; k < a.rowptr[i + 1]; ++k) {
             int32_t j = a.col[k];
             if (j < i) l = std::max(l, lev[j] + 1);
         }
         lev[i] = l;
+        for (int32_t k = a.rowptr[i]; k < a.rowptr[i + 1]; ++k) {
+            int32_t j = a.col[k];
+            if (j > i && j < n) lev[j] = std::max(lev[j], l + 1);
+        }
         maxl = std::max(maxl, l);
     }
     offsets.assign(maxl + 2, 0);

@@ -118,7 +118,7 @@ struct VCycle {
         k_fill<T><<<grid_for(ctx, L.n), kThreads, 0, s>>>(x, T(0), L.n, e.done);
         DV_CUDA(cudaGetLastError());
         ctx->count();
-        for (int k = 0; k < nu; ++k) gs_sweep<T>(e, L.A.get(), L.gs, b, x);
+        gs_sweeps<T>(e, L.A.get(), L.gs, b, x, nu);
         OpResid<T> orr{{}, b, L.r.template as<T>()};
         launch_rows<T>(e, L.A.get(), GatherVec<T, T>{x}, orr);
         T *bn = l + 1 < lv.size() ? lv[l + 1].b.template as<T>() : bc.template as<T>();
@@ -131,7 +131,7 @@ struct VCycle {
         opro.y = x;
         opro.clear = 0;
         launch_rows<T>(e, L.P.get(), GatherVec<T, T>{xn}, opro);
-        for (int k = 0; k < nu; ++k) gs_sweep<T>(e, L.A.get(), L.gs, b, x);
+        gs_sweeps<T>(e, L.A.get(), L.gs, b, x, nu);
         return x;
     }
 };

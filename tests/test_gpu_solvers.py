@@ -369,3 +369,40 @@ def test_pcg_sizes_match_oracle(ctx, native, oracle, fmt, ne):
     x2, st2 = s.Solve(xInitialGuess=0.5 * x)
     assert st2.HasConverged and rel(x2, x_ref) < 1e-7
     s.ReleaseCudaResources()
+
+
+@pytest.mark.parametrize("fmt", ["csr", "duvi"])
+@pytest.mark.parametrize("n,width", [(1, 1), (40, 3), (300, 95), (300, 96), (300, 97), (500, 250), (3000, 4)])
+def test_gauss_seidel_row_order_sweeps(ctx, native, fmt, n, width):
+    # Forward sweeps in row order by one block (x in shared memory, a warp a row, 96 entries at a
+    # time): rows around that width and levels from one row to hundreds, against the sequential sweep
+    # in numpy.  Two cycles of one sweep with a coarse level that corrects nothing (R = 0), so the
+    # result is two sweeps from zero; values from a small pool (DuVi merges values within 1e-10).
+    import scipy.sparse as sp
+    rng = np.random.default_rng(7)
+    rows = []
+    for i in range(n):
+        c = np.union1d(rng.choice(n, size=min(n, width), replace=False), [i])
+        v = rng.integers(-8, 9, len(c)) / 16.0
+        v[c == i] = 2.0 * len(c)
+        rows.append((c, v))
+    A = sp.csr_matrix((np.concatenate([v for _, v in rows]), np.concatenate([c for c, _ in rows]),
+                       np.concatenate([[0], np.cumsum([len(c) for c, _ in rows])])), shape=(n, n))
+    R = sp.csr_matrix((np.zeros(1), [0], [0, 1]), shape=(1, n))
+    P = sp.csr_matrix((np.zeros(n), np.zeros(n, int), np.arange(n + 1)), shape=(n, 1))
+    b = rng.standard_normal(n)
+    x = np.zeros(n)
+    for _ in range(2):
+        for i, (c, v) in enumerate(rows):
+            s = b[i]
+            for k in range(len(c)):
+                if c[k] != i:
+                    s -= v[k] * x[c[k]]
+            x[i] = s / v[c == i][0]
+    cls = native.CudaDuViGeometricMultigridSolver if fmt == "duvi" else native.CudaCsrGeometricMultigridSolver
+    s = cls(ctx, 0, 0.0, [True, False], [1], GaussSeidel=True)
+    s.b = b
+    s.initialize_from_levels([A, sp.identity(1, format="csr")], [R], [P], False)
+    got, st, _ = s.Solve()
+    np.testing.assert_array_equal(got, x)
+    s.ReleaseCudaResources()

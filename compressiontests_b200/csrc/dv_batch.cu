@@ -61,14 +61,19 @@ __device__ __forceinline__ void seg_reduce(double (&v)[NQ], const SegPlan &sp, d
     __syncthreads();
     if (!is_last) return;
     __threadfence();
-    for (int s = threadIdx.x; s < sp.nseg; s += blockDim.x) {
+    // a warp per mesh: the lanes stride over its chunks, then a fixed butterfly (one thread per mesh took
+    // 10 us of the kernel for 60 chunks, one load after another)
+    const int lane = threadIdx.x & 31;
+    for (int s = threadIdx.x >> 5; s < sp.nseg; s += blockDim.x >> 5) {
         double t[NQ];
 #pragma unroll
         for (int q = 0; q < NQ; ++q) t[q] = 0.0;
-        for (int32_t c = sp.seg_chunk[s]; c < sp.seg_chunk[s + 1]; ++c)
+        for (int32_t c = sp.seg_chunk[s] + lane; c < sp.seg_chunk[s + 1]; c += 32)
 #pragma unroll
             for (int q = 0; q < NQ; ++q) t[q] += __ldcg(partials + (size_t)c * NQ + q);
-        fin(s, t);
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) t[q] = dvk::warp_sum(t[q]);
+        if (lane == 0) fin(s, t);
     }
     __syncthreads();
     if (threadIdx.x == 0) *ticket = 0;
@@ -164,13 +169,17 @@ __global__ void __launch_bounds__(256) k_seg_update(double *__restrict__ x, doub
     seg_reduce<1>(v, sp, partials, ticket, FinUpdate{ms, tol2, sc});
 }
 
-__global__ void k_seg_stop(const MeshScalars *ms, int nseg, dvk::SolverScalars *sc) {
+// stop decision after an update, one warp over the meshes
+__global__ void __launch_bounds__(32) k_seg_stop(const MeshScalars *ms, int nseg, dvk::SolverScalars *sc) {
     if (sc->done) return;
-    int all = 1, bad = 0;
-    for (int s = 0; s < nseg; ++s) {
-        all &= ms[s].converged;
+    int open = 0, bad = 0;
+    for (int s = threadIdx.x; s < nseg; s += 32) {
+        open |= !ms[s].converged;
         bad |= isnan(ms[s].rr) ? 1 : 0;
     }
+    const int all = !__any_sync(0xffffffffu, open);
+    bad = __any_sync(0xffffffffu, bad);
+    if (threadIdx.x != 0) return;
     sc->it += 1;
     if (all || bad || sc->it >= sc->max_it) {
         sc->done = 1;
@@ -504,7 +513,7 @@ void batch_solve_impl(dv_batch *B, BCycle<T> &vc, int32_t *conv_per_mesh, int32_
             k_seg_update<T><<<B->nchunks, 256, 0, st>>>(Xd, Rd, rl, Pd, Qd, sp, ms, tol2, ws.sc(), ed.done,
                                                         ed.partials, ed.ticket);
             DV_CUDA(cudaGetLastError());
-            k_seg_stop<<<1, 1, 0, st>>>(ms, B->nmesh, ws.sc());
+            k_seg_stop<<<1, 32, 0, st>>>(ms, B->nmesh, ws.sc());
             DV_CUDA(cudaGetLastError());
             ctx->count(3);
             zz = vc.level(ed, 0, rin);
@@ -589,14 +598,18 @@ void run(dv_batch *B, int32_t *conv, int32_t *its, dv_stats *stats) {
     if (stats) stats->solve_ms = ms;
 }
 
-// user-order <-> internal-order copies of the fine-level vectors
+// user-order <-> internal-order copies of the fine-level vectors, one copy for every run of meshes that
+// follow each other in both orders (meshes of one depth do)
 void permute(dv_batch *B, const double *src, double *dst, bool to_internal, cudaMemcpyKind kind) {
-    for (int32_t pos = 0; pos < B->nmesh; ++pos) {
+    for (int32_t pos = 0; pos < B->nmesh;) {
         const int32_t m = B->order[pos];
-        const size_t bytes = 8 * (size_t)B->nfine[m];
+        int32_t run = 1;
+        size_t rows = B->nfine[m];
+        while (pos + run < B->nmesh && B->order[pos + run] == m + run) rows += B->nfine[m + run++];
         const double *s = src + (to_internal ? B->user_off[m] : B->int_off[pos]);
         double *d = dst + (to_internal ? B->int_off[pos] : B->user_off[m]);
-        DV_CUDA(cudaMemcpyAsync(d, s, bytes, kind, B->ctx->stream));
+        DV_CUDA(cudaMemcpyAsync(d, s, 8 * rows, kind, B->ctx->stream));
+        pos += run;
     }
 }
 

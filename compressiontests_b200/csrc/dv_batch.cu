@@ -393,6 +393,7 @@ std::unique_ptr<BCycle<T>> build_bcycle(dv_batch *B, const int32_t *nlev, const 
             hr.nc = pv.n_rows;
             dv_csr_host rv = hr.view();
             L.R.reset(dv_matrix_build(ctx, rv, B->cfg.format, prec, 0, 1e-10));
+            for (dv_matrix *m : {L.A.get(), L.P.get(), L.R.get()}) dv_use_entries(m);
             for (double d : L.A->host_diag) DV_REQUIRE(d != 0.0, DV_ERR_SINGULAR, "zero diagonal entry");
             double om = B->cfg.omega;
             if (B->cfg.omega_mode == DV_OMEGA_SPECTRAL) {
@@ -657,6 +658,7 @@ extern "C" DV_API int dv_batch_create(dv_context *ctx, int32_t n_meshes, const i
             HostCsr h = blockdiag(a0);
             dv_csr_host v = h.view();
             B->Aout.reset(dv_matrix_build(ctx, v, cfg->outer_format, DV_F64, 0, 1e-10));
+            dv_use_entries(B->Aout.get());
         }
         if (cfg->precision == DV_MIXED) B->c32 = build_bcycle<float>(B.get(), n_levels, A, P);
         else B->c64 = build_bcycle<double>(B.get(), n_levels, A, P);

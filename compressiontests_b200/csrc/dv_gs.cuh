@@ -226,41 +226,6 @@ __global__ void __launch_bounds__(kGsWarps * 32) k_gs_block(const int32_t *__res
     for (int32_t i = threadIdx.x; i < n; i += kGsWarps * 32) x[i] = xs[i];
 }
 
-// Columns and values of a DuVi matrix, entry by entry (the one-block sweep walks them side by side).
-template <class VI, class T>
-__global__ void k_gs_decode(DuviArgs A, int32_t n, int32_t *__restrict__ col, T *__restrict__ val) {
-    const T *tab = static_cast<const T *>(A.values);
-    const VI *vi = static_cast<const VI *>(A.vidx);
-    for (int32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        uint32_t di = A.row_to_dist[i];
-        for (uint32_t bl = A.row_to_col[i]; bl < A.row_to_col[i + 1]; ++bl) {
-            uint32_t c = A.col_idx[bl];
-            const int cnt = A.dist[di];
-            for (int k = 0;; ++k) {
-                col[di] = (int32_t)c;
-                val[di] = tab[vi[di]];
-                ++di;
-                if (k == cnt) break;
-                c += A.dist[di] + 1u;
-            }
-        }
-    }
-}
-
-inline DuviArgs gs_duvi_args(const dv_matrix *m) {
-    DuviArgs a;
-    a.row_to_col = m->row_to_col.as<uint32_t>();
-    a.row_to_dist = m->row_to_dist.as<uint32_t>();
-    a.col_idx = m->col_idx.as<uint32_t>();
-    a.dist = m->dist.as<uint8_t>();
-    a.vidx = m->vidx.p;
-    a.values = m->values.p;
-    a.bundles = m->bundles.as<int32_t>();
-    a.nbundles = m->nbundles;
-    a.nuniq = (int32_t)m->nuniq;
-    return a;
-}
-
 // Row groups of one Gauss-Seidel ordering (device rows + host group offsets).
 struct GsOrder {
     DevMem rows;
@@ -313,12 +278,7 @@ void gs_prepare_block(const dv_matrix *A, GsOrder &o) {
     if (A->format == DV_FORMAT_DUVI) {
         o.col.alloc(4 * (size_t)A->nnz);
         o.val.alloc(sizeof(T) * (size_t)A->nnz);
-        const int grid = (A->n_rows + 255) / 256;
-        if (A->vi_bits == 8) k_gs_decode<uint8_t, T><<<grid, 256, 0, s>>>(gs_duvi_args(A), A->n_rows, o.col.as<int32_t>(), o.val.as<T>());
-        else if (A->vi_bits == 16) k_gs_decode<uint16_t, T><<<grid, 256, 0, s>>>(gs_duvi_args(A), A->n_rows, o.col.as<int32_t>(), o.val.as<T>());
-        else k_gs_decode<uint32_t, T><<<grid, 256, 0, s>>>(gs_duvi_args(A), A->n_rows, o.col.as<int32_t>(), o.val.as<T>());
-        DV_CUDA(cudaGetLastError());
-        ctx->count();
+        duvi_decode<T>(A, o.col.as<int32_t>(), o.val.as<T>());
     }
     DV_CUDA(cudaStreamSynchronize(s));
     o.block = true;
@@ -346,11 +306,11 @@ void gs_sweep(const LaunchEnv &e, const dv_matrix *A, const GsOrder &o, const T 
             k_gs_csr<T><<<grid, kThreads, 0, e.stream>>>(A->rowptr.as<int32_t>(), A->col.as<int32_t>(),
                                                          static_cast<const T *>(A->val.p), b, x, rows, cnt, o.bs, e.done);
         } else if (A->vi_bits == 8) {
-            k_gs_duvi<uint8_t, T><<<grid, kThreads, 0, e.stream>>>(gs_duvi_args(A), b, x, rows, cnt, o.bs, e.done);
+            k_gs_duvi<uint8_t, T><<<grid, kThreads, 0, e.stream>>>(duvi_args(A), b, x, rows, cnt, o.bs, e.done);
         } else if (A->vi_bits == 16) {
-            k_gs_duvi<uint16_t, T><<<grid, kThreads, 0, e.stream>>>(gs_duvi_args(A), b, x, rows, cnt, o.bs, e.done);
+            k_gs_duvi<uint16_t, T><<<grid, kThreads, 0, e.stream>>>(duvi_args(A), b, x, rows, cnt, o.bs, e.done);
         } else {
-            k_gs_duvi<uint32_t, T><<<grid, kThreads, 0, e.stream>>>(gs_duvi_args(A), b, x, rows, cnt, o.bs, e.done);
+            k_gs_duvi<uint32_t, T><<<grid, kThreads, 0, e.stream>>>(duvi_args(A), b, x, rows, cnt, o.bs, e.done);
         }
         DV_CUDA(cudaGetLastError());
         ctx->count();

@@ -201,6 +201,7 @@ struct dv_matrix {
     // CSR
     DevMem rowptr, col, val;
     int csr_tpr = 16;          // threads per row (autotuned)
+    int entries_ok = 0;        // DuVi: columns and values also decoded into col / val (dv_use_entries)
     // DuVi SoA
     int vi_bits = 8;
     int64_t nblocks = 0, nuniq = 0;
@@ -349,6 +350,9 @@ dv_matrix *dv_trilinear_build(dv_context *ctx, const int32_t *ne_fine, int restr
 // Matrix-free hexahedral operator of nmesh meshes placed block-diagonally (dv_assemble.cu).
 dv_matrix *dv_hex_operator_build(dv_context *ctx, int32_t nmesh, const int32_t *ne, const double *elem_E, double scale,
                                  double E, double nu, int32_t precision);
+// Decodes a solver's own small DuVi operator into columns and values and lets its products run on
+// them (dv_matrix.cu).
+void dv_use_entries(dv_matrix *m);
 // Times the launch shapes of m's product and keeps the fastest (matrices of >= 100k rows).
 void dv_autotune(dv_matrix *m);
 

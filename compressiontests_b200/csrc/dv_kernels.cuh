@@ -423,7 +423,9 @@ __global__ void __launch_bounds__(kThreads) k_csr(const int32_t *__restrict__ rp
                                                   const MT *__restrict__ va, int32_t n, Gather g, Op op,
                                                   const int *__restrict__ done, double *partials, unsigned *ticket) {
     if (done && *(volatile const int *)done) return;
-    constexpr int U = 4;   // entries per lane per step: all index/value loads, then all gathers, then the FMAs
+    // entries per lane per step: all index/value loads, then all gathers, then the FMAs (one lane a row: the
+    // 27 entries of a restriction row in three steps, summed in order)
+    constexpr int U = TPR == 1 ? 9 : 4;
     double red[Op::NRED > 0 ? Op::NRED : 1];
 #pragma unroll
     for (int i = 0; i < (Op::NRED > 0 ? Op::NRED : 1); ++i) red[i] = 0.0;
@@ -1492,6 +1494,58 @@ void launch_duvi_vi(const LaunchEnv &e, const dv_matrix *m, Gather g, Op op) {
     e.ctx->count();
 }
 
+// Columns and values of a DuVi matrix, entry by entry, for kernels that walk a row's entries side by
+// side (row offsets: row_to_dist).
+template <class VI, class T>
+__global__ void k_duvi_decode(DuviArgs A, int32_t n, int32_t *__restrict__ col, T *__restrict__ val) {
+    const T *tab = static_cast<const T *>(A.values);
+    const VI *vi = static_cast<const VI *>(A.vidx);
+    for (int32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        uint32_t di = A.row_to_dist[i];
+        for (uint32_t bl = A.row_to_col[i]; bl < A.row_to_col[i + 1]; ++bl) {
+            uint32_t c = A.col_idx[bl];
+            const int cnt = A.dist[di];
+            for (int k = 0;; ++k) {
+                col[di] = (int32_t)c;
+                val[di] = tab[vi[di]];
+                ++di;
+                if (k == cnt) break;
+                c += A.dist[di] + 1u;
+            }
+        }
+    }
+}
+
+inline DuviArgs duvi_args(const dv_matrix *m) {
+    DuviArgs a;
+    a.row_to_col = m->row_to_col.as<uint32_t>();
+    a.row_to_dist = m->row_to_dist.as<uint32_t>();
+    a.col_idx = m->col_idx.as<uint32_t>();
+    a.dist = m->dist.as<uint8_t>();
+    a.vidx = m->vidx.p;
+    a.values = m->values.p;
+    a.bundles = m->bundles.as<int32_t>();
+    a.nbundles = m->nbundles;
+    a.nuniq = (int32_t)m->nuniq;
+    return a;
+}
+
+template <class T>
+void duvi_decode(const dv_matrix *m, int32_t *col, T *val) {
+    const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(((int64_t)m->n_rows + 255) / 256, m->ctx->num_sms * 16));
+    cudaStream_t s = m->ctx->stream;
+    if (m->vi_bits == 8) k_duvi_decode<uint8_t, T><<<grid, 256, 0, s>>>(duvi_args(m), m->n_rows, col, val);
+    else if (m->vi_bits == 16) k_duvi_decode<uint16_t, T><<<grid, 256, 0, s>>>(duvi_args(m), m->n_rows, col, val);
+    else k_duvi_decode<uint32_t, T><<<grid, 256, 0, s>>>(duvi_args(m), m->n_rows, col, val);
+    DV_CUDA(cudaGetLastError());
+    m->ctx->count();
+}
+
+// Row offsets of a CSR matrix, or of a DuVi matrix's decoded entries.
+inline const int32_t *row_offsets(const dv_matrix *m) {
+    return (m->format == DV_FORMAT_CSR ? m->rowptr : m->row_to_dist).as<int32_t>();
+}
+
 template <int TPR, class AT, class Gather, class Op>
 void launch_csr_tpr(const LaunchEnv &e, const dv_matrix *m, Gather g, Op op) {
     const int gpb = kThreads / TPR;
@@ -1499,7 +1553,7 @@ void launch_csr_tpr(const LaunchEnv &e, const dv_matrix *m, Gather g, Op op) {
     if (blocks > e.max_blocks) blocks = e.max_blocks;
     if (blocks < 1) blocks = 1;
     k_csr<TPR, AT, AT, Gather, Op><<<blocks, kThreads, 0, e.stream>>>(
-        m->rowptr.as<int32_t>(), m->col.as<int32_t>(), static_cast<const AT *>(m->val.p), m->n_rows, g, op, e.done,
+        row_offsets(m), m->col.as<int32_t>(), static_cast<const AT *>(m->val.p), m->n_rows, g, op, e.done,
         e.partials, e.ticket);
     DV_CUDA(cudaGetLastError());
     e.ctx->count();
@@ -1516,7 +1570,7 @@ void launch_csr_nodes(const LaunchEnv &e, const dv_matrix *m, Gather g, Op op) {
         const int64_t wave = (int64_t)e.ctx->num_sms * occupancy.get(kern, kThreads, 0, e.ctx->device);
         blocks = std::min<int64_t>(need, std::min<int64_t>(wave, e.max_blocks));
     }
-    kern<<<(unsigned)blocks, kThreads, 0, e.stream>>>(m->rowptr.as<int32_t>(), m->col.as<int32_t>(),
+    kern<<<(unsigned)blocks, kThreads, 0, e.stream>>>(row_offsets(m), m->col.as<int32_t>(),
                                                       static_cast<const AT *>(m->val.p), ngroups, g, op, e.done,
                                                       e.partials, e.ticket);
     DV_CUDA(cudaGetLastError());
@@ -1887,6 +1941,20 @@ void launch_trilinear(const LaunchEnv &e, const dv_matrix *m, Gather g, Op op) {
     e.ctx->count();
 }
 
+// CSR rows, or the decoded entries of a DuVi matrix.
+template <class AT, class Gather, class Op>
+void launch_csr(const LaunchEnv &e, const dv_matrix *m, Gather g, Op op) {
+    switch (m->csr_tpr) {
+        case 1: launch_csr_tpr<1, AT>(e, m, g, op); break;
+        case 4: launch_csr_tpr<4, AT>(e, m, g, op); break;
+        case 8: launch_csr_tpr<8, AT>(e, m, g, op); break;
+        case 16: launch_csr_tpr<16, AT>(e, m, g, op); break;
+        case 3 * 16: launch_csr_nodes<16, AT>(e, m, g, op); break;
+        case 3 * 32: launch_csr_nodes<32, AT>(e, m, g, op); break;
+        default: launch_csr_tpr<32, AT>(e, m, g, op); break;
+    }
+}
+
 // Runs op over every row of m with the accumulator type AT (= value precision).
 template <class AT, class Gather, class Op>
 void launch_rows(const LaunchEnv &e, const dv_matrix *m, Gather g, Op op) {
@@ -1896,6 +1964,10 @@ void launch_rows(const LaunchEnv &e, const dv_matrix *m, Gather g, Op op) {
     }
     if (m->format == DV_FORMAT_TRILINEAR) {
         launch_trilinear<AT>(e, m, g, op);
+        return;
+    }
+    if (m->entries_ok) {
+        launch_csr<AT>(e, m, g, op);
         return;
     }
     if (m->format == DV_FORMAT_DUVI && m->duvi_variant == 3) {
@@ -1925,15 +1997,7 @@ void launch_rows(const LaunchEnv &e, const dv_matrix *m, Gather g, Op op) {
         }
         return;
     }
-    switch (m->csr_tpr) {
-        case 1: launch_csr_tpr<1, AT>(e, m, g, op); break;
-        case 4: launch_csr_tpr<4, AT>(e, m, g, op); break;
-        case 8: launch_csr_tpr<8, AT>(e, m, g, op); break;
-        case 16: launch_csr_tpr<16, AT>(e, m, g, op); break;
-        case 3 * 16: launch_csr_nodes<16, AT>(e, m, g, op); break;
-        case 3 * 32: launch_csr_nodes<32, AT>(e, m, g, op); break;
-        default: launch_csr_tpr<32, AT>(e, m, g, op); break;
-    }
+    launch_csr<AT>(e, m, g, op);
 }
 
 // ---------------------------------------------------------------------------

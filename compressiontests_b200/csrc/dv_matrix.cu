@@ -89,6 +89,14 @@ static int pick_tpr(double mean_nnz) {
     return 32;
 }
 
+// csr_tpr of a matrix: threads per row, or 3 x the lanes per node group of 3 rows.  k_csr_nodes takes 32
+// lanes a group where its 3 entries a lane fill up (81 entries: 32 lanes do them in one step), 16
+// below 48 entries; under 16 most lanes would idle and the row kernel stays.
+static int row_lanes(int row_group, double mean_nnz) {
+    if (row_group == 3 && mean_nnz >= 16) return mean_nnz < 48 ? 3 * 16 : 3 * 32;
+    return pick_tpr(mean_nnz);
+}
+
 // Uploads the SoA arrays of encoding h and derives the device layouts; h is only read
 // here (export reads the device arrays back), so callers keep it only while building.
 void dv_upload_patterns(dv_matrix *m, const DuviPatternHost &P, const std::vector<double> &values, cudaStream_t s) {
@@ -358,6 +366,32 @@ static void autotune(dv_matrix *m) {
 
 void dv_autotune(dv_matrix *m) { autotune(m); }
 
+// The derived DuVi layouts give a node (81 entries) to one thread: right where the operator is too
+// large for the caches, but a small level has too few nodes to hide 81 dependent steps.  Its products
+// run on the decoded entries instead, as long as those stay in the 126 MB L2 cache beside the vectors:
+// node groups a warp each (k_csr_nodes), the short rows of the transfers a thread each, in the stored
+// order (so that they equal the matrix-free transfers).  Only operators that a solver built for itself:
+// the order of a node group's sums is not the stored one.  Measured with against without: solve of 12
+// uneven meshes 3.43 -> 2.53 ms, adjoint pair 48x24x24 10.4 -> 6.6 ms, mixed solve 16^3 1.31 -> 0.99 ms
+// (a 12,168-row level's sweep 25.7 us on the lane layout, 16 blocks).
+// DV_ENTRIES=<MB> moves the line (0: never; A/B comparisons).
+void dv_use_entries(dv_matrix *m) {
+    int64_t limit = 32ll << 20;
+    if (const char *v = getenv("DV_ENTRIES")) limit = atoll(v) << 20;
+    if (m->format != DV_FORMAT_DUVI || m->entries_ok || m->n_rows == 0) return;
+    const int64_t vs = m->precision == DV_F64 ? 8 : 4;
+    const bool nodes = m->row_group == 3 && !m->lanes_shift && !m->pat_shift && m->n_rows % 3 == 0;
+    const double mean_nnz = (double)m->nnz / m->n_rows;
+    if (m->nnz * vs + m->nnz * 4 / (nodes ? 3 : 1) > limit || (!nodes && mean_nnz > 32)) return;
+    m->col.alloc(4 * (size_t)m->nnz);
+    m->val.alloc(vs * (size_t)m->nnz);
+    if (m->precision == DV_F64) dvk::duvi_decode<double>(m, m->col.as<int32_t>(), m->val.as<double>());
+    else dvk::duvi_decode<float>(m, m->col.as<int32_t>(), m->val.as<float>());
+    m->csr_tpr = nodes ? row_lanes(3, mean_nnz) : 1;
+    DV_CUDA(cudaStreamSynchronize(m->ctx->stream));
+    m->entries_ok = 1;
+}
+
 dv_matrix *dv_matrix_build(dv_context *ctx, const dv_csr_host &a, int format, int precision, int vi_bits, double tol,
                            const DuviHost *encoded) {
     dv_ctx_check(ctx);
@@ -384,13 +418,8 @@ dv_matrix *dv_matrix_build(dv_context *ctx, const dv_csr_host &a, int format, in
             upload(m->val, f.data(), 4 * (size_t)m->nnz, s);
             DV_CUDA(cudaStreamSynchronize(s));
         }
-        const double mean_nnz = a.n_rows ? (double)m->nnz / a.n_rows : 1.0;
-        m->csr_tpr = pick_tpr(mean_nnz);
         m->row_group = dv_csr_row_group(a);
-        // node groups of 3 rows: k_csr_nodes with 32 lanes a group where its 3 entries a lane fill up
-        // (81 entries: 32 lanes do them in one step), 16 below 48 entries; under 16 most lanes would
-        // idle and the row kernel stays
-        if (m->row_group == 3 && mean_nnz >= 16) m->csr_tpr = mean_nnz < 48 ? 3 * 16 : 3 * 32;
+        m->csr_tpr = row_lanes(m->row_group, a.n_rows ? (double)m->nnz / a.n_rows : 1.0);
         m->device_bytes = m->nnz * (4 + (precision == DV_F64 ? 8 : 4)) + 4 * ((int64_t)a.n_rows + 1);
     } else {
         if (encoded) {

@@ -490,6 +490,7 @@ static std::unique_ptr<VCycle<T>> build_vcycle(dv_context *ctx, SolverWs &ws, in
             dv_csr_host rt{P[l].n_cols, P[l].n_rows, rp.data(), ci.data(), va.data()};
             lv.R.reset(dv_matrix_build(ctx, rt, cfg.format, prec, 0, 1e-10));
         }
+        for (dv_matrix *m : {lv.A.get(), lv.P.get(), lv.R.get()}) dv_use_entries(m);
         for (double d : lv.A->host_diag) DV_REQUIRE(d != 0.0, DV_ERR_SINGULAR, "zero diagonal entry");
         double om = cfg.omega;
         if (cfg.omega_mode == DV_OMEGA_SPECTRAL) {
@@ -598,7 +599,10 @@ extern "C" DV_API int dv_mgpcg_create_hex(dv_context *ctx, const int32_t *ne, do
                 dv_autotune(m.get());
                 return m;
             };
-            if (l == 0) s->Aout = build(DV_F64);
+            if (l == 0) {
+                s->Aout = build(DV_F64);
+                dv_use_entries(s->Aout.get());
+            }
             prebuilt.push_back(build(prec));
             Ash[l] = dv_csr_host{nr, nr, nullptr, nullptr, nullptr};
             // trilinear prolongation to this level from the next: matrix-free, or host CSR when
@@ -657,6 +661,7 @@ extern "C" DV_API int dv_mgpcg_create(dv_context *ctx, int32_t L, const dv_csr_h
         }
         const DuviHost *shared = outer_duvi && inner_duvi ? &h0 : nullptr;
         s->Aout.reset(dv_matrix_build(ctx, A[0], cfg->outer_format, DV_F64, 0, 1e-10, shared));
+        dv_use_entries(s->Aout.get());
         if (cfg->precision == DV_MIXED) s->v32 = build_vcycle<float>(ctx, *s->ws, L, A, P, *cfg, s->omega_eff, shared);
         else s->v64 = build_vcycle<double>(ctx, *s->ws, L, A, P, *cfg, s->omega_eff, shared);
         const size_t nb = 8 * (size_t)s->n;

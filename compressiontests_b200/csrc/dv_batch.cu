@@ -93,7 +93,7 @@ template <class ZT>
 __global__ void __launch_bounds__(256) k_seg_fcg_red(const ZT *__restrict__ z, const double *__restrict__ q,
                                                      const double *__restrict__ r, SegPlan sp, MeshScalars *ms,
                                                      const int *__restrict__ done, double *partials, unsigned *ticket) {
-    if (*(volatile const int *)done) return;
+    if (dvk::chain_done(done)) return;
     const int32_t rb = sp.chunk_begin[blockIdx.x], re = sp.chunk_end[blockIdx.x];
     double v[2] = {0.0, 0.0};
     for (int32_t i = rb + threadIdx.x; i < re; i += blockDim.x) {
@@ -130,7 +130,7 @@ struct FinPq {
 __global__ void __launch_bounds__(256) k_seg_pq(const double *__restrict__ p, const double *__restrict__ q, SegPlan sp,
                                                 MeshScalars *ms, const int *__restrict__ done, double *partials,
                                                 unsigned *ticket) {
-    if (*(volatile const int *)done) return;
+    if (dvk::chain_done(done)) return;
     const int32_t rb = sp.chunk_begin[blockIdx.x], re = sp.chunk_end[blockIdx.x];
     double v[1] = {0.0};
     for (int32_t i = rb + threadIdx.x; i < re; i += blockDim.x) v[0] += p[i] * q[i];
@@ -155,7 +155,7 @@ __global__ void __launch_bounds__(256) k_seg_update(double *__restrict__ x, doub
                                                     const double *__restrict__ p, const double *__restrict__ q,
                                                     SegPlan sp, MeshScalars *ms, double tol2, const dvk::SolverScalars *sc,
                                                     const int *__restrict__ done, double *partials, unsigned *ticket) {
-    if (*(volatile const int *)done) return;
+    if (dvk::chain_done(done)) return;
     const int32_t rb = sp.chunk_begin[blockIdx.x], re = sp.chunk_end[blockIdx.x];
     const double a = ms[sp.chunk_seg[blockIdx.x]].alpha;
     double v[1] = {0.0};
@@ -171,7 +171,7 @@ __global__ void __launch_bounds__(256) k_seg_update(double *__restrict__ x, doub
 
 // stop decision after an update, one warp over the meshes
 __global__ void __launch_bounds__(32) k_seg_stop(const MeshScalars *ms, int nseg, dvk::SolverScalars *sc) {
-    if (sc->done) return;
+    if (dvk::chain_done(&sc->done)) return;
     int open = 0, bad = 0;
     for (int s = threadIdx.x; s < nseg; s += 32) {
         open |= !ms[s].converged;
@@ -218,7 +218,7 @@ __global__ void __launch_bounds__(256) k_block_coarse(const T *__restrict__ ainv
                                                       const int32_t *__restrict__ bstart,
                                                       const int32_t *__restrict__ bsize, const T *__restrict__ b,
                                                       T *__restrict__ y, int32_t nrows, const int *__restrict__ done) {
-    if (done && *(volatile const int *)done) return;
+    if (dvk::chain_done(done)) return;
     const int lane = threadIdx.x & 31;
     const int32_t nw = (gridDim.x * blockDim.x) >> 5;
     for (int32_t row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; row < nrows; row += nw) {
@@ -257,7 +257,7 @@ struct BCycle {
         if (L.s > 0) {
             const T *w = L.w.template as<T>();
             if (nu == 1) {
-                k_scale<T><<<grid_for(ctx, L.s), kThreads, 0, st>>>(w, b, x, L.s, e.done);
+                dvk::launch_chain(k_scale<T>, grid_for(ctx, L.s), kThreads, 0, st, w, b, x, L.s, e.done);
                 DV_CUDA(cudaGetLastError());
                 ctx->count();
             } else {
@@ -290,7 +290,7 @@ struct BCycle {
         if (L.t > L.s) {
             const int32_t nr = L.t - L.s;
             const int grid = std::max(1, std::min((nr * 32 + 255) / 256, ctx->num_sms * 16));
-            k_block_coarse<T><<<grid, 256, 0, st>>>(L.ainv.template as<T>(), L.aoff.template as<int64_t>(),
+            dvk::launch_chain(k_block_coarse<T>, grid, 256, 0, st, L.ainv.template as<T>(), L.aoff.template as<int64_t>(),
                                                     L.bstart.template as<int32_t>(), L.bsize.template as<int32_t>(),
                                                     b + L.s, x + L.s, nr, e.done);
             DV_CUDA(cudaGetLastError());
@@ -489,7 +489,7 @@ void batch_solve_impl(dv_batch *B, BCycle<T> &vc, int32_t *conv_per_mesh, int32_
     T *rin = kMixed ? reinterpret_cast<T *>(B->r32.p) : reinterpret_cast<T *>(B->r.p);
     auto to_low = [&] {
         if (kMixed) {
-            dvk::k_convert<double, float><<<grid_for(ctx, n), kThreads, 0, st>>>(B->r.as<double>(), B->r32.as<float>(), n);
+            dvk::launch_chain(dvk::k_convert<double, float>, grid_for(ctx, n), kThreads, 0, st, B->r.as<double>(), B->r32.as<float>(), n);
             DV_CUDA(cudaGetLastError());
             ctx->count();
         }
@@ -503,18 +503,18 @@ void batch_solve_impl(dv_batch *B, BCycle<T> &vc, int32_t *conv_per_mesh, int32_
     auto body = [&] {
         const T *zz = z;
         for (int it = 0; it < per; ++it) {
-            k_seg_fcg_red<T><<<B->nchunks, 256, 0, st>>>(zz, Qd, Rd, sp, ms, ed.done, ed.partials, ed.ticket);
+            dvk::launch_chain(k_seg_fcg_red<T>, B->nchunks, 256, 0, st, zz, Qd, Rd, sp, ms, ed.done, ed.partials, ed.ticket);
             DV_CUDA(cudaGetLastError());
             ctx->count();
             OpFcgSeg<T> op{{}, zz, Pd, Qd, B->seg_of.as<int32_t>(), ms};
             launch_rows<double>(ed, B->Aout.get(), GatherVec<T, double>{zz}, op);
-            k_seg_pq<<<B->nchunks, 256, 0, st>>>(Pd, Qd, sp, ms, ed.done, ed.partials, ed.ticket);
+            dvk::launch_chain(k_seg_pq, B->nchunks, 256, 0, st, Pd, Qd, sp, ms, ed.done, ed.partials, ed.ticket);
             DV_CUDA(cudaGetLastError());
             T *rl = kMixed ? reinterpret_cast<T *>(B->r32.p) : nullptr;
-            k_seg_update<T><<<B->nchunks, 256, 0, st>>>(Xd, Rd, rl, Pd, Qd, sp, ms, tol2, ws.sc(), ed.done,
+            dvk::launch_chain(k_seg_update<T>, B->nchunks, 256, 0, st, Xd, Rd, rl, Pd, Qd, sp, ms, tol2, ws.sc(), ed.done,
                                                         ed.partials, ed.ticket);
             DV_CUDA(cudaGetLastError());
-            k_seg_stop<<<1, 32, 0, st>>>(ms, B->nmesh, ws.sc());
+            dvk::launch_chain(k_seg_stop, 1, 32, 0, st, ms, B->nmesh, ws.sc());
             DV_CUDA(cudaGetLastError());
             ctx->count(3);
             zz = vc.level(ed, 0, rin);

@@ -196,7 +196,7 @@ __global__ void __launch_bounds__(kThreads) k_bprod_csr(const int32_t *__restric
                                                         const AT *__restrict__ va, int32_t ngroups, int kc, Gather g,
                                                         Epi ep, const int *__restrict__ done, double *partials,
                                                         unsigned *ticket) {
-    if (done && *(volatile const int *)done) return;
+    if (dvk::chain_done(done)) return;
     __shared__ Rec<AT, G> srec[kWarps][32];
     constexpr int NC = Epi::NC > 0 ? Epi::NC : 1;
     double red[U][NC];
@@ -264,7 +264,7 @@ template <class AT, int G, int U, bool EXACT, class Gather, class Epi>
 __global__ void __launch_bounds__(kThreads) k_bprod_duvi(BDuviArgs A, int32_t ngroups, int kc, Gather g, Epi ep,
                                                          const int *__restrict__ done, double *partials,
                                                          unsigned *ticket) {
-    if (done && *(volatile const int *)done) return;
+    if (dvk::chain_done(done)) return;
     __shared__ Rec<AT, G> srec[kWarps][32];
     __shared__ AT stab[256];
     constexpr int NC = Epi::NC > 0 ? Epi::NC : 1;
@@ -364,13 +364,13 @@ void launch_bprod_gu(const LaunchEnv &e, const dv_matrix *m, int kc, Gather g, E
     const int32_t ngroups = m->n_rows / G;
     const int blocks = bprod_blocks(e, ngroups, Epi::NC > 0);
     if (m->format == DV_FORMAT_CSR) {
-        k_bprod_csr<AT, G, U, EXACT, Gather, Epi><<<blocks, kThreads, 0, e.stream>>>(
+        dvk::launch_chain(k_bprod_csr<AT, G, U, EXACT, Gather, Epi>, blocks, kThreads, 0, e.stream, 
             m->rowptr.as<int32_t>(), m->col.as<int32_t>(), static_cast<const AT *>(m->val.p), ngroups, kc, g, ep,
             e.done, e.partials, e.ticket);
     } else {
         BDuviArgs a{m->row_to_col.as<uint32_t>(), m->row_to_dist.as<uint32_t>(), m->col_idx.as<uint32_t>(),
                     m->dist.as<uint8_t>(), m->vidx.p, m->values.p, m->vi_bits, (int)m->nuniq};
-        k_bprod_duvi<AT, G, U, EXACT, Gather, Epi><<<blocks, kThreads, 0, e.stream>>>(a, ngroups, kc, g, ep, e.done,
+        dvk::launch_chain(k_bprod_duvi<AT, G, U, EXACT, Gather, Epi>, blocks, kThreads, 0, e.stream, a, ngroups, kc, g, ep, e.done,
                                                                                       e.partials, e.ticket);
     }
     DV_CUDA(cudaGetLastError());
@@ -390,7 +390,7 @@ __global__ void __launch_bounds__(kThreads) k_bprod_pattern(const uint16_t *__re
                                                             int32_t nrec, int32_t ngroups, int kc, Gather g, Epi ep,
                                                             const int *__restrict__ done, double *partials,
                                                             unsigned *ticket, const uint32_t *__restrict__ list) {
-    if (done && *(volatile const int *)done) return;
+    if (dvk::chain_done(done)) return;
     extern __shared__ uint4 bpat_smem[];
     dvk::PatRec<AT> *rec = reinterpret_cast<dvk::PatRec<AT> *>(bpat_smem);
     uint32_t *st = reinterpret_cast<uint32_t *>(rec + nrec);
@@ -458,7 +458,7 @@ void launch_bprod_pattern_u(const LaunchEnv &e, const dv_matrix *m, int kc, Gath
     limit.raise(kern, smem, e.ctx->device);
     const int32_t ngroups = list ? (int32_t)nlist : m->n_rows / G;
     const int blocks = bprod_blocks(e, ngroups, Epi::NC > 0);
-    kern<<<blocks, kThreads, smem, e.stream>>>(m->pat_id.as<uint16_t>(), m->pat_start.as<uint32_t>(),
+    dvk::launch_chain(kern, blocks, kThreads, smem, e.stream, m->pat_id.as<uint16_t>(), m->pat_start.as<uint32_t>(),
                                                static_cast<const dvk::PatRec<AT> *>(m->pat_rec.p),
                                                m->pat_base.as<uint32_t>(), m->pat_count, m->pat_entries, ngroups, kc,
                                                g, ep, e.done, e.partials, e.ticket, list);
@@ -550,7 +550,7 @@ __global__ void __launch_bounds__(kThreads, 3) k_bprod_grid(BGridGeom G, dvk::Gr
                                                              int ld, int kc, Gather g, Epi ep,
                                                              const int *__restrict__ done) {
     static_assert(Epi::NC == 0, "column reductions run on the pattern kernel");
-    if (done && *(volatile const int *)done) return;
+    if (dvk::chain_done(done)) return;
     extern __shared__ uint4 bgrid_smem[];
     float *ring = reinterpret_cast<float *>(bgrid_smem);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -674,7 +674,7 @@ void launch_bprod_grid(const LaunchEnv &e, const dv_matrix *m, int kc, Gather g,
         static dvk::SmemLimit limit;   // per instantiation and device
         limit.raise(kern, smem, e.ctx->device);
         const dim3 grid((unsigned)G.ntile, (unsigned)((kc + 31) / 32));
-        kern<<<grid, kThreads, smem, e.stream>>>(G, cf, m->pat_id.as<uint16_t>(), BGridSrc<Gather>::block(g), g.ld, kc,
+        dvk::launch_chain(kern, grid, kThreads, smem, e.stream, G, cf, m->pat_id.as<uint16_t>(), BGridSrc<Gather>::block(g), g.ld, kc,
                                                  g, ep, e.done);
         DV_CUDA(cudaGetLastError());
         e.ctx->count();
@@ -692,7 +692,7 @@ template <bool RESTRICT, class AT, class Gather, class Epi>
 __global__ void __launch_bounds__(kThreads) k_bprod_tri(dvk::TriGeom G, int kc, Gather g, Epi ep,
                                                          const int *__restrict__ done) {
     static_assert(Epi::NC == 0, "transfers carry no reductions");
-    if (done && *(volatile const int *)done) return;
+    if (dvk::chain_done(done)) return;
     const int64_t work = G.nodes(RESTRICT) * kc;
     for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < work; t += (int64_t)gridDim.x * blockDim.x) {
         const uint32_t q = (uint32_t)(t / kc);
@@ -716,8 +716,8 @@ void launch_bprod(const LaunchEnv &e, const dv_matrix *m, int kc, Gather g, Epi 
             const dvk::TriGeom G{m->tri_ne[0], m->tri_ne[1], m->tri_ne[2]};
             const int64_t work = G.nodes(m->tri_restrict) * kc;
             const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>((work + kThreads - 1) / kThreads, e.max_blocks));
-            if (m->tri_restrict) k_bprod_tri<true, AT><<<blocks, kThreads, 0, e.stream>>>(G, kc, g, ep, e.done);
-            else k_bprod_tri<false, AT><<<blocks, kThreads, 0, e.stream>>>(G, kc, g, ep, e.done);
+            if (m->tri_restrict) dvk::launch_chain(k_bprod_tri<true, AT, Gather, Epi>, blocks, kThreads, 0, e.stream, G, kc, g, ep, e.done);
+            else dvk::launch_chain(k_bprod_tri<false, AT, Gather, Epi>, blocks, kThreads, 0, e.stream, G, kc, g, ep, e.done);
             DV_CUDA(cudaGetLastError());
             e.ctx->count();
             return;

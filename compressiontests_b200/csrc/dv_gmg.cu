@@ -77,7 +77,7 @@ static void smooth(dv_gmg *g, const LaunchEnv &e, GLevel &L, int sweeps) {
             std::swap(x, t);
         }
         if (x != L.x.as<double>()) {
-            k_copy<double><<<grid_n(ctx, L.n), kThreads, 0, s>>>(x, L.x.as<double>(), L.n, e.done);
+            dvk::launch_chain(k_copy<double>, grid_n(ctx, L.n), kThreads, 0, s, x, L.x.as<double>(), L.n, e.done);
             DV_CUDA(cudaGetLastError());
             ctx->count();
         }
@@ -95,7 +95,7 @@ static void cycle(dv_gmg *g, const LaunchEnv &e) {
     for (size_t step = 0; step < g->path.size(); ++step) {
         if (cur == TL - 1) {
             GLevel &Lp = g->lv[cur - 1];
-            k_dense_gemv<double><<<std::max(1, std::min(g->nc / 8 + 1, ctx->num_sms * 8)), kThreads, 0, s>>>(
+            dvk::launch_chain(k_dense_gemv<double>, std::max(1, std::min(g->nc / 8 + 1, ctx->num_sms * 8)), kThreads, 0, s, 
                 g->ainv.as<double>(), g->bc.as<double>(), g->xc.as<double>(), g->nc, e.done);
             DV_CUDA(cudaGetLastError());
             ctx->count();
@@ -122,7 +122,7 @@ static void cycle(dv_gmg *g, const LaunchEnv &e) {
                 launch_rows<double>(e, L.R.get(), GatherVec<double, double>{L.r.as<double>()}, op);
                 if (cur < TL - 2) {
                     GLevel &N = g->lv[cur + 1];
-                    k_fill<double><<<grid_n(ctx, N.n), kThreads, 0, s>>>(N.x.as<double>(), 0.0, N.n, e.done);
+                    dvk::launch_chain(k_fill<double>, grid_n(ctx, N.n), kThreads, 0, s, N.x.as<double>(), 0.0, N.n, e.done);
                     DV_CUDA(cudaGetLastError());
                     ctx->count();
                 }

@@ -60,7 +60,7 @@ template <class T>
 __global__ void k_gs_csr(const int32_t *__restrict__ rp, const int32_t *__restrict__ ci, const T *__restrict__ va,
                          const T *__restrict__ b, T *x, const int32_t *__restrict__ rows, int32_t count, int bs,
                          const int *__restrict__ done) {
-    if (done && *(volatile const int *)done) return;
+    if (chain_done(done)) return;
     for (int32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < count; t += gridDim.x * blockDim.x) {
         const int32_t r0 = rows[t];
         for (int q = 0; q < bs; ++q) gs_row_csr<T>(rp, ci, va, b, x, r0 + q);
@@ -69,7 +69,7 @@ __global__ void k_gs_csr(const int32_t *__restrict__ rp, const int32_t *__restri
 template <class VI, class T>
 __global__ void k_gs_duvi(DuviArgs A, const T *__restrict__ b, T *x, const int32_t *__restrict__ rows, int32_t count,
                           int bs, const int *__restrict__ done) {
-    if (done && *(volatile const int *)done) return;
+    if (chain_done(done)) return;
     for (int32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < count; t += gridDim.x * blockDim.x) {
         const int32_t r0 = rows[t];
         for (int q = 0; q < bs; ++q) gs_row_duvi<VI, T>(A, b, x, r0 + q);
@@ -87,7 +87,7 @@ __global__ void __launch_bounds__(256) k_gs_pattern(const uint16_t *__restrict__
                                                     const PatRec<T> *__restrict__ grec, int32_t npat, int32_t nrec,
                                                     const T *__restrict__ b, T *x, const int32_t *__restrict__ rows,
                                                     int32_t count, const int *__restrict__ done) {
-    if (done && *(volatile const int *)done) return;
+    if (chain_done(done)) return;
     extern __shared__ uint4 gs_smem[];
     const PatRec<T> *rec = reinterpret_cast<const PatRec<T> *>(gs_smem);
     const uint32_t *st = reinterpret_cast<const uint32_t *>(rec + nrec);
@@ -146,7 +146,7 @@ __global__ void __launch_bounds__(kGsWarps * 32) k_gs_block(const int32_t *__res
                                                             const int32_t *__restrict__ rows,
                                                             const int32_t *__restrict__ off, int32_t nlevels, int32_t n,
                                                             int sweeps, const int *__restrict__ done) {
-    if (done && *(volatile const int *)done) return;
+    if (chain_done(done)) return;
     extern __shared__ uint4 gsb_smem[];
     constexpr int W = 32 * kGsLane;
     T *prod = reinterpret_cast<T *>(gsb_smem) + (threadIdx.x >> 5) * W;   // this warp's products
@@ -299,18 +299,18 @@ void gs_sweep(const LaunchEnv &e, const dv_matrix *A, const GsOrder &o, const T 
             const size_t smem = sizeof(PatRec<T>) * (size_t)A->pat_entries + 4 * ((size_t)A->pat_count + 1);
             static SmemLimit limit;   // per instantiation and device
             limit.raise(k_gs_pattern<T>, smem, ctx->device);
-            k_gs_pattern<T><<<grid, kThreads, smem, e.stream>>>(A->pat_id.as<uint16_t>(), A->pat_start.as<uint32_t>(),
+            launch_chain(k_gs_pattern<T>, grid, kThreads, smem, e.stream, A->pat_id.as<uint16_t>(), A->pat_start.as<uint32_t>(),
                                                                static_cast<const PatRec<T> *>(A->pat_rec.p),
                                                                A->pat_count, A->pat_entries, b, x, rows, cnt, e.done);
         } else if (A->format == DV_FORMAT_CSR) {
-            k_gs_csr<T><<<grid, kThreads, 0, e.stream>>>(A->rowptr.as<int32_t>(), A->col.as<int32_t>(),
+            launch_chain(k_gs_csr<T>, grid, kThreads, 0, e.stream, A->rowptr.as<int32_t>(), A->col.as<int32_t>(),
                                                          static_cast<const T *>(A->val.p), b, x, rows, cnt, o.bs, e.done);
         } else if (A->vi_bits == 8) {
-            k_gs_duvi<uint8_t, T><<<grid, kThreads, 0, e.stream>>>(duvi_args(A), b, x, rows, cnt, o.bs, e.done);
+            launch_chain(k_gs_duvi<uint8_t, T>, grid, kThreads, 0, e.stream, duvi_args(A), b, x, rows, cnt, o.bs, e.done);
         } else if (A->vi_bits == 16) {
-            k_gs_duvi<uint16_t, T><<<grid, kThreads, 0, e.stream>>>(duvi_args(A), b, x, rows, cnt, o.bs, e.done);
+            launch_chain(k_gs_duvi<uint16_t, T>, grid, kThreads, 0, e.stream, duvi_args(A), b, x, rows, cnt, o.bs, e.done);
         } else {
-            k_gs_duvi<uint32_t, T><<<grid, kThreads, 0, e.stream>>>(duvi_args(A), b, x, rows, cnt, o.bs, e.done);
+            launch_chain(k_gs_duvi<uint32_t, T>, grid, kThreads, 0, e.stream, duvi_args(A), b, x, rows, cnt, o.bs, e.done);
         }
         DV_CUDA(cudaGetLastError());
         ctx->count();
@@ -329,7 +329,7 @@ void gs_sweeps(const LaunchEnv &e, const dv_matrix *A, const GsOrder &o, const T
     const size_t smem = gs_block_smem<T>(A->n_rows);
     static SmemLimit limit;   // per instantiation and device
     limit.raise(k_gs_block<T>, smem, e.ctx->device);
-    k_gs_block<T><<<1, kGsWarps * 32, smem, e.stream>>>(
+    launch_chain(k_gs_block<T>, 1, kGsWarps * 32, smem, e.stream, 
         csr ? A->rowptr.as<int32_t>() : A->row_to_dist.as<int32_t>(), csr ? A->col.as<int32_t>() : o.col.as<int32_t>(),
         csr ? static_cast<const T *>(A->val.p) : o.val.as<T>(), b, x, o.rows.as<int32_t>(), o.d_off.as<int32_t>(),
         (int32_t)o.off.size() - 1, A->n_rows, sweeps, e.done);

@@ -9,6 +9,7 @@
 #pragma once
 
 #include <cstddef>
+#include <cstdlib>
 #include <mutex>
 #include <type_traits>
 #include <utility>
@@ -74,6 +75,46 @@ struct OccupancyCache {
         return occ;
     }
 };
+
+// ---------------------------------------------------------------------------
+// chains of dependent kernels
+//
+// The kernels of an iteration depend on one another and are short on all but the finest levels, so the
+// time from the last block of one to the first of the next counts.  They are launched with
+// programmatic stream serialisation: a kernel's blocks may be set up when the blocks of the one before
+// have left, and wait (griddepcontrol.wait) for that kernel's writes to be visible before they touch
+// anything but constant tables.  Every kernel launched by launch_chain calls chain_done first (a kernel
+// that did not wait could complete before the one it depends on, and release the next), and what it
+// reads comes after the branch on its result.  With against without: mixed solve 16^3 963 -> 845 us,
+// 12 uneven meshes 2.34 -> 2.13 ms, adjoint pair 48x24x24 8.10 -> 7.50 ms, mixed solve 128^3 7.49 -> 7.27
+// ms, a product of 1,200 rows called over and over 4.0 -> 3.5 us.  Letting the next kernel's blocks in
+// as soon as all of this one's have started (griddepcontrol.launch_dependents) was slower for all but
+// the smallest: they settle on the SMs that happen to have room and stay there (adjoint pair 9.3 ms).
+// DV_CHAIN=0 launches plainly (A/B comparisons).
+// ---------------------------------------------------------------------------
+// waits for the kernel before; then whether the solve has stopped
+__device__ __forceinline__ bool chain_done(const int *done) {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    return done && *(volatile const int *)done;
+}
+template <class... P, class... A>
+void launch_chain(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A &&...args) {
+    static const bool on = [] {
+        const char *v = getenv("DV_CHAIN");
+        return !(v && v[0] == '0');
+    }();
+    cudaLaunchConfig_t c = {};
+    c.gridDim = grid;
+    c.blockDim = block;
+    c.dynamicSmemBytes = smem;
+    c.stream = stream;
+    cudaLaunchAttribute serial = {};
+    serial.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    serial.val.programmaticStreamSerializationAllowed = 1;
+    c.attrs = &serial;
+    c.numAttrs = on ? 1 : 0;
+    DV_CUDA(cudaLaunchKernelEx(&c, kern, static_cast<P>(args)...));
+}
 
 // ---------------------------------------------------------------------------
 // reductions
@@ -422,7 +463,7 @@ template <int TPR, class MT, class AT, class Gather, class Op>
 __global__ void __launch_bounds__(kThreads) k_csr(const int32_t *__restrict__ rp, const int32_t *__restrict__ ci,
                                                   const MT *__restrict__ va, int32_t n, Gather g, Op op,
                                                   const int *__restrict__ done, double *partials, unsigned *ticket) {
-    if (done && *(volatile const int *)done) return;
+    if (chain_done(done)) return;
     // entries per lane per step: all index/value loads, then all gathers, then the FMAs (one lane a row: the
     // 27 entries of a restriction row in three steps, summed in order)
     constexpr int U = TPR == 1 ? 9 : 4;
@@ -478,7 +519,7 @@ __global__ void __launch_bounds__(kThreads) k_csr_nodes(const int32_t *__restric
                                                         const AT *__restrict__ va, int32_t ngroups, Gather g, Op op,
                                                         const int *__restrict__ done, double *partials,
                                                         unsigned *ticket) {
-    if (done && *(volatile const int *)done) return;
+    if (chain_done(done)) return;
     constexpr int U = 3;
     double red[Op::NRED > 0 ? Op::NRED : 1];
 #pragma unroll
@@ -554,7 +595,7 @@ __device__ __forceinline__ void copy16(void *dst, const void *src, int nbytes16,
 template <class VI, class AT, class Gather, class Op, int WARPS, int BATCH>
 __global__ void __launch_bounds__(WARPS * 32, 2) k_duvi(DuviArgs A, Gather g, Op op, const int *__restrict__ done,
                                                      double *partials, unsigned *ticket) {
-    if (done && *(volatile const int *)done) return;
+    if (chain_done(done)) return;
     extern __shared__ __align__(16) unsigned char smem[];
     constexpr bool kSmemTable = sizeof(VI) == 1;
     AT *tab = reinterpret_cast<AT *>(smem);
@@ -735,7 +776,7 @@ __device__ __forceinline__ AT lane_value(const AT *tab, const AT *gtab, const Ch
 template <class VI, class AT, class Gather, class Op, int G, bool SCALED, bool SHIFT, bool TUP, bool STEN>
 __global__ void __launch_bounds__(256) k_duvi_lanes(DuviLanesArgs A, Gather g, Op op, const int *__restrict__ done,
                                                     double *partials, unsigned *ticket) {
-    if (done && *(volatile const int *)done) return;
+    if (chain_done(done)) return;
     using Chunk = typename ViChunk<VI>::T;
     constexpr bool kSmemTable = sizeof(VI) == 1;
     constexpr int NV = TUP ? 1 : G;   // index chunks per word
@@ -901,23 +942,23 @@ void launch_duvi_lanes_g(const LaunchEnv &e, const dv_matrix *m, Gather g, Op op
     if constexpr (sizeof(VI) == 1) {
         if constexpr (G > 1) {
             if (m->lanes_stencil) {
-                k_duvi_lanes<VI, AT, Gather, Op, G, false, false, true, true><<<blocks, 256, 0, e.stream>>>(a, g, op, e.done, e.partials, e.ticket);
+                launch_chain(k_duvi_lanes<VI, AT, Gather, Op, G, false, false, true, true>, blocks, 256, 0, e.stream, a, g, op, e.done, e.partials, e.ticket);
                 done_launch = true;
             } else if (m->lanes_tuples) {
-                if (sh) k_duvi_lanes<VI, AT, Gather, Op, G, false, true, true, false><<<blocks, 256, 0, e.stream>>>(a, g, op, e.done, e.partials, e.ticket);
-                else k_duvi_lanes<VI, AT, Gather, Op, G, false, false, true, false><<<blocks, 256, 0, e.stream>>>(a, g, op, e.done, e.partials, e.ticket);
+                if (sh) launch_chain(k_duvi_lanes<VI, AT, Gather, Op, G, false, true, true, false>, blocks, 256, 0, e.stream, a, g, op, e.done, e.partials, e.ticket);
+                else launch_chain(k_duvi_lanes<VI, AT, Gather, Op, G, false, false, true, false>, blocks, 256, 0, e.stream, a, g, op, e.done, e.partials, e.ticket);
                 done_launch = true;
             }
         }
         if (!done_launch && m->lanes_scaled) {
-            if (sh) k_duvi_lanes<VI, AT, Gather, Op, G, true, G != 1, false, false><<<blocks, 256, 0, e.stream>>>(a, g, op, e.done, e.partials, e.ticket);
-            else k_duvi_lanes<VI, AT, Gather, Op, G, true, false, false, false><<<blocks, 256, 0, e.stream>>>(a, g, op, e.done, e.partials, e.ticket);
+            if (sh) launch_chain(k_duvi_lanes<VI, AT, Gather, Op, G, true, G != 1, false, false>, blocks, 256, 0, e.stream, a, g, op, e.done, e.partials, e.ticket);
+            else launch_chain(k_duvi_lanes<VI, AT, Gather, Op, G, true, false, false, false>, blocks, 256, 0, e.stream, a, g, op, e.done, e.partials, e.ticket);
             done_launch = true;
         }
     }
     if (!done_launch) {
-        if (sh) k_duvi_lanes<VI, AT, Gather, Op, G, false, G != 1, false, false><<<blocks, 256, 0, e.stream>>>(a, g, op, e.done, e.partials, e.ticket);
-        else k_duvi_lanes<VI, AT, Gather, Op, G, false, false, false, false><<<blocks, 256, 0, e.stream>>>(a, g, op, e.done, e.partials, e.ticket);
+        if (sh) launch_chain(k_duvi_lanes<VI, AT, Gather, Op, G, false, G != 1, false, false>, blocks, 256, 0, e.stream, a, g, op, e.done, e.partials, e.ticket);
+        else launch_chain(k_duvi_lanes<VI, AT, Gather, Op, G, false, false, false, false>, blocks, 256, 0, e.stream, a, g, op, e.done, e.partials, e.ticket);
     }
     DV_CUDA(cudaGetLastError());
     e.ctx->count();
@@ -1013,11 +1054,11 @@ __global__ void __launch_bounds__(256) k_duvi_pattern(const uint16_t *__restrict
                                                       const PatRec<AT> *__restrict__ grec, const uint32_t *__restrict__ base,
                                                       int32_t npat, int32_t nrec, int64_t ngroups, Gather g, Op op,
                                                       const int *__restrict__ done, double *partials, unsigned *ticket) {
-    if (done && *(volatile const int *)done) return;
     extern __shared__ uint4 pat_smem[];
     const PatRec<AT> *rec = reinterpret_cast<const PatRec<AT> *>(pat_smem);
     const uint32_t *st = reinterpret_cast<const uint32_t *>(rec + nrec);
     stage_patterns<AT>(pat_smem, grec, pstart, npat, nrec);
+    if (chain_done(done)) return;
     __syncthreads();
     double red[Op::NRED > 0 ? Op::NRED : 1];
 #pragma unroll
@@ -1239,7 +1280,6 @@ __global__ void __launch_bounds__(256, 3)   // 3 blocks an SM: FP64 fits 80 regi
     k_duvi_grid(GridGeom G, GridCoef<AT> cf, const uint16_t *__restrict__ pid, const uint32_t *__restrict__ pstart,
                 const PatRec<AT> *__restrict__ grec, const uint32_t *__restrict__ bnode, int32_t npat, int32_t nrec,
                 Gather g, Op op, const int *__restrict__ done, double *partials, unsigned *ticket) {
-    if (done && *(volatile const int *)done) return;
     extern __shared__ uint4 grid_smem[];
     constexpr bool FU = op_fused<Op>::value;
     constexpr bool S0 = FU || sizeof(AT) == 4;   // FP64 parity epilogues multiply the zeros too
@@ -1251,11 +1291,13 @@ __global__ void __launch_bounds__(256, 3)   // 3 blocks an SM: FP64 fits 80 regi
         const PatRec<AT> *rec = reinterpret_cast<const PatRec<AT> *>(grid_smem);
         const uint32_t *st = reinterpret_cast<const uint32_t *>(rec + nrec);
         stage_patterns<AT>(grid_smem, grec, pstart, npat, nrec);
+        if (chain_done(done)) return;
         __syncthreads();
         for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < G.nbound;
              i += (int64_t)G.bound_blocks * blockDim.x)
             pattern_group<AT, Gather, Op, 3, false, false>((int64_t)__ldg(bnode + i), rec, st, pid, nullptr, g, op, red);
     } else {
+        if (chain_done(done)) return;
         using SS = StageSrc<Gather>;
         using ST = typename SS::ST;
         using SL = StageSlots<NY>;
@@ -1411,7 +1453,7 @@ void launch_duvi_grid_h(const LaunchEnv &e, const dv_matrix *m, Gather g, Op op)
     G.ntile = G.lz > 2 ? (int32_t)(plane_tiles * ((lzi + G.zc - 1) / G.zc)) : 0;
     const int64_t tile_blocks = std::min<int64_t>(G.ntile, std::max<int64_t>(1, e.max_blocks - G.bound_blocks));
     const int blocks = (int)std::max<int64_t>(1, G.bound_blocks + tile_blocks);
-    kern<<<blocks, 256, smem, e.stream>>>(G, cf, m->pat_id.as<uint16_t>(), m->pat_start.as<uint32_t>(),
+    launch_chain(kern, blocks, 256, smem, e.stream, G, cf, m->pat_id.as<uint16_t>(), m->pat_start.as<uint32_t>(),
                                           static_cast<const PatRec<AT> *>(m->pat_rec.p), m->grid_bnode.as<uint32_t>(),
                                           m->pat_count, m->pat_entries, g, op, e.done, e.partials, e.ticket);
     DV_CUDA(cudaGetLastError());
@@ -1434,7 +1476,7 @@ void launch_duvi_pattern_gbs(const LaunchEnv &e, const dv_matrix *m, Gather g, O
     const int64_t need = std::max<int64_t>(1, (ng + 255) / 256), wave = (int64_t)e.ctx->num_sms * occ;
     const int64_t cap = std::min<int64_t>(need, e.max_blocks);
     const int blocks = (int)(cap <= wave ? cap : cap / wave * wave);
-    kern<<<blocks, 256, smem, e.stream>>>(m->pat_id.as<uint16_t>(), m->pat_start.as<uint32_t>(),
+    launch_chain(kern, blocks, 256, smem, e.stream, m->pat_id.as<uint16_t>(), m->pat_start.as<uint32_t>(),
                                           static_cast<const PatRec<AT> *>(m->pat_rec.p), m->pat_base.as<uint32_t>(),
                                           m->pat_count, m->pat_entries, ng, g, op, e.done, e.partials, e.ticket);
     DV_CUDA(cudaGetLastError());
@@ -1489,7 +1531,7 @@ void launch_duvi_vi(const LaunchEnv &e, const dv_matrix *m, Gather g, Op op) {
     int blocks = (m->nbundles + W - 1) / W;
     if (blocks > e.max_blocks) blocks = e.max_blocks;
     if (blocks < 1) blocks = 1;
-    kern<<<blocks, W * 32, smem, e.stream>>>(a, g, op, e.done, e.partials, e.ticket);
+    launch_chain(kern, blocks, W * 32, smem, e.stream, a, g, op, e.done, e.partials, e.ticket);
     DV_CUDA(cudaGetLastError());
     e.ctx->count();
 }
@@ -1552,7 +1594,7 @@ void launch_csr_tpr(const LaunchEnv &e, const dv_matrix *m, Gather g, Op op) {
     int blocks = (m->n_rows + gpb - 1) / gpb;
     if (blocks > e.max_blocks) blocks = e.max_blocks;
     if (blocks < 1) blocks = 1;
-    k_csr<TPR, AT, AT, Gather, Op><<<blocks, kThreads, 0, e.stream>>>(
+    launch_chain(k_csr<TPR, AT, AT, Gather, Op>, blocks, kThreads, 0, e.stream, 
         row_offsets(m), m->col.as<int32_t>(), static_cast<const AT *>(m->val.p), m->n_rows, g, op, e.done,
         e.partials, e.ticket);
     DV_CUDA(cudaGetLastError());
@@ -1570,7 +1612,7 @@ void launch_csr_nodes(const LaunchEnv &e, const dv_matrix *m, Gather g, Op op) {
         const int64_t wave = (int64_t)e.ctx->num_sms * occupancy.get(kern, kThreads, 0, e.ctx->device);
         blocks = std::min<int64_t>(need, std::min<int64_t>(wave, e.max_blocks));
     }
-    kern<<<(unsigned)blocks, kThreads, 0, e.stream>>>(row_offsets(m), m->col.as<int32_t>(),
+    launch_chain(kern, (unsigned)blocks, kThreads, 0, e.stream, row_offsets(m), m->col.as<int32_t>(),
                                                       static_cast<const AT *>(m->val.p), ngroups, g, op, e.done,
                                                       e.partials, e.ticket);
     DV_CUDA(cudaGetLastError());
@@ -1664,7 +1706,7 @@ __global__ void __launch_bounds__(kHexThreads, sizeof(AT) == 8 ? 2 : 3)
     k_hex_elem(const HexMesh *__restrict__ meshes, int32_t nmesh, int32_t ntile, HexModes<AT> kc,
                const AT *__restrict__ ef_all, Gather g, Op op, const int *__restrict__ done, double *partials,
                unsigned *ticket) {
-    if (done && *(volatile const int *)done) return;
+    if (chain_done(done)) return;
     extern __shared__ uint4 hex_smem[];
     using SS = StageSrc<Gather>;
     using ST = typename SS::ST;
@@ -1842,7 +1884,7 @@ void launch_hex_elem(const LaunchEnv &e, const dv_matrix *m, Gather g, Op op) {
     const double *c = m->hex_modes;
     const HexModes<AT> kc{(AT)c[0], (AT)c[1], (AT)c[2], (AT)c[3], (AT)c[4], (AT)c[5], (AT)c[6], (AT)c[7]};
     const int blocks = (int)std::min<int64_t>(m->hex_ntile, e.max_blocks);
-    kern<<<blocks, kHexThreads, smem, e.stream>>>(m->hex_meshes.as<HexMesh>(), m->hex_nmesh, m->hex_ntile, kc,
+    launch_chain(kern, blocks, kHexThreads, smem, e.stream, m->hex_meshes.as<HexMesh>(), m->hex_nmesh, m->hex_ntile, kc,
                                                   static_cast<const AT *>(m->hex_factor.p), g, op, e.done, e.partials,
                                                   e.ticket);
     DV_CUDA(cudaGetLastError());
@@ -1906,7 +1948,7 @@ __device__ __forceinline__ void tri_walk(const TriGeom &G, uint32_t q, F &&f) {
 template <bool RESTRICT, class AT, class Gather, class Op>
 __global__ void __launch_bounds__(256) k_tri(TriGeom G, Gather g, Op op, const int *__restrict__ done,
                                              double *partials, unsigned *ticket) {
-    if (done && *(volatile const int *)done) return;
+    if (chain_done(done)) return;
     constexpr bool FU = op_fused<Op>::value;
     double red[Op::NRED > 0 ? Op::NRED : 1];
 #pragma unroll
@@ -1935,8 +1977,8 @@ void launch_trilinear(const LaunchEnv &e, const dv_matrix *m, Gather g, Op op) {
     const TriGeom G{m->tri_ne[0], m->tri_ne[1], m->tri_ne[2]};
     const int64_t nodes = m->n_rows / 3;
     const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>((nodes + 255) / 256, e.max_blocks));
-    if (m->tri_restrict) k_tri<true, AT, Gather, Op><<<blocks, 256, 0, e.stream>>>(G, g, op, e.done, e.partials, e.ticket);
-    else k_tri<false, AT, Gather, Op><<<blocks, 256, 0, e.stream>>>(G, g, op, e.done, e.partials, e.ticket);
+    if (m->tri_restrict) launch_chain(k_tri<true, AT, Gather, Op>, blocks, 256, 0, e.stream, G, g, op, e.done, e.partials, e.ticket);
+    else launch_chain(k_tri<false, AT, Gather, Op>, blocks, 256, 0, e.stream, G, g, op, e.done, e.partials, e.ticket);
     DV_CUDA(cudaGetLastError());
     e.ctx->count();
 }
@@ -2006,17 +2048,17 @@ void launch_rows(const LaunchEnv &e, const dv_matrix *m, Gather g, Op op) {
 template <class T>
 __global__ void k_scale(const T *__restrict__ w, const T *__restrict__ b, T *__restrict__ x, int32_t n,
                         const int *__restrict__ done) {
-    if (done && *(volatile const int *)done) return;
+    if (chain_done(done)) return;
     for (int32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) x[i] = w[i] * b[i];
 }
 template <class T>
 __global__ void k_copy(const T *__restrict__ a, T *__restrict__ b, int32_t n, const int *__restrict__ done) {
-    if (done && *(volatile const int *)done) return;
+    if (chain_done(done)) return;
     for (int32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) b[i] = a[i];
 }
 template <class T>
 __global__ void k_fill(T *__restrict__ a, T v, int32_t n, const int *__restrict__ done) {
-    if (done && *(volatile const int *)done) return;
+    if (chain_done(done)) return;
     for (int32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) a[i] = v;
 }
 template <class A, class B>
@@ -2026,7 +2068,7 @@ __global__ void k_convert(const A *__restrict__ a, B *__restrict__ b, int32_t n)
 // x += y
 template <class T>
 __global__ void k_axpy1(const T *__restrict__ y, T *__restrict__ x, int32_t n, const int *__restrict__ done) {
-    if (done && *(volatile const int *)done) return;
+    if (chain_done(done)) return;
     for (int32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) x[i] = x[i] + y[i];
 }
 
@@ -2034,7 +2076,7 @@ __global__ void k_axpy1(const T *__restrict__ y, T *__restrict__ x, int32_t n, c
 template <class T>
 __global__ void k_dense_gemv(const T *__restrict__ a, const T *__restrict__ b, T *__restrict__ y, int32_t n,
                              const int *__restrict__ done) {
-    if (done && *(volatile const int *)done) return;
+    if (chain_done(done)) return;
     const int lane = threadIdx.x & 31;
     const int32_t nw = (gridDim.x * blockDim.x) >> 5;
     for (int32_t r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < n; r += nw) {
@@ -2051,7 +2093,7 @@ __global__ void k_dense_gemv(const T *__restrict__ a, const T *__restrict__ b, T
 template <class T>
 __global__ void __launch_bounds__(128) k_dense_gemv_rows(const T *__restrict__ a, const T *__restrict__ b,
                                                          T *__restrict__ y, int32_t n, const int *__restrict__ done) {
-    if (done && *(volatile const int *)done) return;
+    if (chain_done(done)) return;
     __shared__ T part[4];
     for (int32_t r = blockIdx.x; r < n; r += gridDim.x) {
         const T *ar = a + (size_t)r * n;

@@ -54,7 +54,7 @@ struct VCycle {
     T *level(const LaunchEnv &e, size_t l, const T *b, const T *wb = nullptr) {
         cudaStream_t s = e.stream;
         if (l == lv.size()) {
-            k_dense_gemv_rows<T><<<std::max(1, std::min(nc, ctx->num_sms * 16)), 128, 0, s>>>(
+            dvk::launch_chain(k_dense_gemv_rows<T>, std::max(1, std::min(nc, ctx->num_sms * 16)), 128, 0, s, 
                 ainv.template as<T>(), b, xc.template as<T>(), nc, e.done);
             DV_CUDA(cudaGetLastError());
             ctx->count();
@@ -65,7 +65,7 @@ struct VCycle {
         T *x = L.x.template as<T>(), *t = L.t.template as<T>();
         const T *w = L.w.template as<T>();
         if (nu == 1) {
-            k_scale<T><<<grid_for(ctx, L.n), kThreads, 0, s>>>(w, b, x, L.n, e.done);
+            dvk::launch_chain(k_scale<T>, grid_for(ctx, L.n), kThreads, 0, s, w, b, x, L.n, e.done);
             DV_CUDA(cudaGetLastError());
             ctx->count();
         } else {
@@ -115,7 +115,7 @@ struct VCycle {
         cudaStream_t s = e.stream;
         VLevel<T> &L = lv[l];
         T *x = L.x.template as<T>();
-        k_fill<T><<<grid_for(ctx, L.n), kThreads, 0, s>>>(x, T(0), L.n, e.done);
+        dvk::launch_chain(k_fill<T>, grid_for(ctx, L.n), kThreads, 0, s, x, T(0), L.n, e.done);
         DV_CUDA(cudaGetLastError());
         ctx->count();
         gs_sweeps<T>(e, L.A.get(), L.gs, b, x, nu);

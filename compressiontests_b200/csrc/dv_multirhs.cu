@@ -75,7 +75,7 @@ __global__ void __launch_bounds__(dvb::kThreads) k_bfcg_red(const ZT *__restrict
                                                             const double *__restrict__ r, int32_t n, int k,
                                                             ColScalars *cs, const int *__restrict__ done,
                                                             double *partials, unsigned *ticket) {
-    if (*(volatile const int *)done) return;
+    if (dvk::chain_done(done)) return;
     double red[U][2];
 #pragma unroll
     for (int u = 0; u < U; ++u) red[u][0] = red[u][1] = 0.0;
@@ -110,7 +110,7 @@ __global__ void __launch_bounds__(dvb::kThreads) k_bfcg_update(double *__restric
                                                                const double *__restrict__ q, int32_t n, int k,
                                                                ColScalars *cs, double tol2, const int *__restrict__ done,
                                                                double *partials, unsigned *ticket) {
-    if (*(volatile const int *)done) return;
+    if (dvk::chain_done(done)) return;
     double red[U][1];
 #pragma unroll
     for (int u = 0; u < U; ++u) red[u][0] = 0.0;
@@ -137,7 +137,7 @@ __global__ void __launch_bounds__(dvb::kThreads) k_bfcg_update(double *__restric
 
 // stop decision after an update: every column converged, a NaN, or the iteration limit
 __global__ void k_bfcg_stop(const ColScalars *cs, int k, dvk::SolverScalars *sc) {
-    if (sc->done) return;
+    if (dvk::chain_done(&sc->done)) return;
     int all = 1, bad = 0;
     for (int j = 0; j < k; ++j) {
         all &= cs[j].converged;
@@ -187,7 +187,7 @@ __global__ void __launch_bounds__(dvb::kThreads) k_bnorm(const double *__restric
 template <class T>
 __global__ void k_bscale(const T *__restrict__ w, const T *__restrict__ b, T *__restrict__ x, int32_t n, int k,
                          const int *__restrict__ done) {
-    if (done && *(volatile const int *)done) return;
+    if (dvk::chain_done(done)) return;
     const size_t tot = (size_t)n * k;
     for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < tot; q += (size_t)gridDim.x * blockDim.x)
         x[q] = w[q / k] * b[q];
@@ -199,7 +199,7 @@ __global__ void k_bscale(const T *__restrict__ w, const T *__restrict__ b, T *__
 template <class T>
 __global__ void __launch_bounds__(256) k_bcoarse(const T *__restrict__ a, const T *__restrict__ b, T *__restrict__ y,
                                                  int32_t nc, int k, const int *__restrict__ done) {
-    if (done && *(volatile const int *)done) return;
+    if (dvk::chain_done(done)) return;
     __shared__ T As[8][33];
     __shared__ T Bs[32][33];
     const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
@@ -236,7 +236,7 @@ T *block_vcycle(const LaunchEnv &e, VCycle<T> &vc, BlockLevels<T> &W, size_t l, 
     cudaStream_t s = e.stream;
     dv_context *ctx = vc.ctx;
     if (l == vc.lv.size()) {
-        k_bcoarse<T><<<dim3((vc.nc + 7) / 8, (k + 31) / 32), 256, 0, s>>>(vc.ainv.template as<T>(), b,
+        dvk::launch_chain(k_bcoarse<T>, dim3((vc.nc + 7) / 8, (k + 31) / 32), 256, 0, s, vc.ainv.template as<T>(), b,
                                                                           W.xc.template as<T>(), vc.nc, k, e.done);
         DV_CUDA(cudaGetLastError());
         ctx->count();
@@ -246,7 +246,7 @@ T *block_vcycle(const LaunchEnv &e, VCycle<T> &vc, BlockLevels<T> &W, size_t l, 
     T *x = W.x[l].template as<T>(), *t = W.t[l].template as<T>();
     const T *w = L.w.template as<T>();
     if (vc.nu == 1) {
-        k_bscale<T><<<vec_grid(ctx, (size_t)L.n * k), 256, 0, s>>>(w, b, x, L.n, k, e.done);
+        dvk::launch_chain(k_bscale<T>, vec_grid(ctx, (size_t)L.n * k), 256, 0, s, w, b, x, L.n, k, e.done);
         DV_CUDA(cudaGetLastError());
         ctx->count();
     } else {
@@ -351,7 +351,7 @@ void multi_solve(dv_mgpcg *s, VCycle<T> &vc, MultiState<T> &M, int k, const doub
     T *rin = kMixed ? reinterpret_cast<T *>(M.Rlow.p) : reinterpret_cast<T *>(M.R.p);
     auto to_low = [&] {
         if (kMixed) {
-            dvk::k_convert<double, float><<<vec_grid(ctx, nk), 256, 0, st>>>(M.R.template as<double>(),
+            dvk::launch_chain(dvk::k_convert<double, float>, vec_grid(ctx, nk), 256, 0, st, M.R.template as<double>(),
                                                                              M.Rlow.template as<float>(), (int32_t)nk);
             DV_CUDA(cudaGetLastError());
             ctx->count();
@@ -365,19 +365,19 @@ void multi_solve(dv_mgpcg *s, VCycle<T> &vc, MultiState<T> &M, int k, const doub
     double *Xd = M.X.template as<double>(), *Rd = M.R.template as<double>();
     double *Pd = M.Pv.template as<double>(), *Qd = M.Q.template as<double>();
     auto launch_red = [&](const T *zz) {
-        if (k <= 32) k_bfcg_red<T, 1><<<gw, dvb::kThreads, 0, st>>>(zz, Qd, Rd, n, k, cs, ed.done, ed.partials, ed.ticket);
-        else if (k <= 64) k_bfcg_red<T, 2><<<gw, dvb::kThreads, 0, st>>>(zz, Qd, Rd, n, k, cs, ed.done, ed.partials, ed.ticket);
-        else k_bfcg_red<T, 4><<<gw, dvb::kThreads, 0, st>>>(zz, Qd, Rd, n, k, cs, ed.done, ed.partials, ed.ticket);
+        if (k <= 32) dvk::launch_chain(k_bfcg_red<T, 1>, gw, dvb::kThreads, 0, st, zz, Qd, Rd, n, k, cs, ed.done, ed.partials, ed.ticket);
+        else if (k <= 64) dvk::launch_chain(k_bfcg_red<T, 2>, gw, dvb::kThreads, 0, st, zz, Qd, Rd, n, k, cs, ed.done, ed.partials, ed.ticket);
+        else dvk::launch_chain(k_bfcg_red<T, 4>, gw, dvb::kThreads, 0, st, zz, Qd, Rd, n, k, cs, ed.done, ed.partials, ed.ticket);
         DV_CUDA(cudaGetLastError());
         ctx->count();
     };
     auto launch_update = [&] {
         T *rl = kMixed ? reinterpret_cast<T *>(M.Rlow.p) : nullptr;
-        if (k <= 32) k_bfcg_update<T, 1><<<gw, dvb::kThreads, 0, st>>>(Xd, Rd, rl, Pd, Qd, n, k, cs, tol2, ed.done, ed.partials, ed.ticket);
-        else if (k <= 64) k_bfcg_update<T, 2><<<gw, dvb::kThreads, 0, st>>>(Xd, Rd, rl, Pd, Qd, n, k, cs, tol2, ed.done, ed.partials, ed.ticket);
-        else k_bfcg_update<T, 4><<<gw, dvb::kThreads, 0, st>>>(Xd, Rd, rl, Pd, Qd, n, k, cs, tol2, ed.done, ed.partials, ed.ticket);
+        if (k <= 32) dvk::launch_chain(k_bfcg_update<T, 1>, gw, dvb::kThreads, 0, st, Xd, Rd, rl, Pd, Qd, n, k, cs, tol2, ed.done, ed.partials, ed.ticket);
+        else if (k <= 64) dvk::launch_chain(k_bfcg_update<T, 2>, gw, dvb::kThreads, 0, st, Xd, Rd, rl, Pd, Qd, n, k, cs, tol2, ed.done, ed.partials, ed.ticket);
+        else dvk::launch_chain(k_bfcg_update<T, 4>, gw, dvb::kThreads, 0, st, Xd, Rd, rl, Pd, Qd, n, k, cs, tol2, ed.done, ed.partials, ed.ticket);
         DV_CUDA(cudaGetLastError());
-        k_bfcg_stop<<<1, 1, 0, st>>>(cs, k, ws.sc());
+        dvk::launch_chain(k_bfcg_stop, 1, 1, 0, st, cs, k, ws.sc());
         DV_CUDA(cudaGetLastError());
         ctx->count(2);
     };

@@ -91,7 +91,7 @@ __global__ void k_na_pcg_init(const double *__restrict__ diag, const double *__r
 __global__ void k_na_update(const double *__restrict__ diag, const double *__restrict__ ap, const double *__restrict__ p,
                             double *__restrict__ x, double *__restrict__ r, double *__restrict__ z, int32_t n,
                             double tol, SolverScalars *sc, double *partials, unsigned *ticket) {
-    if (*(volatile const int *)&sc->done) return;
+    if (dvk::chain_done(&sc->done)) return;
     const double a = sc->alpha;
     double red[4] = {0.0, 0.0, 0.0, 0.0};
     for (int32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
@@ -125,7 +125,7 @@ __global__ void k_na_update(const double *__restrict__ diag, const double *__res
 }
 
 __global__ void k_na_p(const double *__restrict__ z, double *__restrict__ p, int32_t n, const SolverScalars *sc) {
-    if (*(volatile const int *)&sc->done) return;
+    if (dvk::chain_done(&sc->done)) return;
     const double b = sc->beta;
     for (int32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) p[i] = z[i] + b * p[i];
 }
@@ -211,10 +211,10 @@ extern "C" DV_API int dv_pcg_solve_noalloc(dv_matrix *A, const double *d_b, doub
             for (int k = 0; k < 8; ++k) {
                 OpPcgAp op{p, ap, sc};
                 launch_rows<double>(ed, A, GatherVec<double, double>{p}, op);
-                k_na_update<<<grid, kThreads, 0, st>>>(A->diag.as<double>(), ap, p, d_x, r, z, n, tol, sc, partials,
+                dvk::launch_chain(k_na_update, grid, kThreads, 0, st, A->diag.as<double>(), ap, p, d_x, r, z, n, tol, sc, partials,
                                                        ticket);
                 DV_CUDA(cudaGetLastError());
-                k_na_p<<<grid, kThreads, 0, st>>>(z, p, n, sc);
+                dvk::launch_chain(k_na_p, grid, kThreads, 0, st, z, p, n, sc);
                 DV_CUDA(cudaGetLastError());
                 ctx->count(2);
             }

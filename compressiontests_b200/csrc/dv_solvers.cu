@@ -116,7 +116,7 @@ __global__ void k_pcg_update(const double *__restrict__ M, const double *__restr
                              double *__restrict__ x, double *__restrict__ r, double *__restrict__ z, int32_t n,
                              double tol, int rel_l2, SolverScalars *sc, const int *__restrict__ done,
                              double *partials, unsigned *ticket) {
-    if (*(volatile const int *)done) return;
+    if (dvk::chain_done(done)) return;
     const double a = sc->alpha;
     double red[4] = {0.0, 0.0, 0.0, 0.0};   // max|r|, failed flag, r.z, r.r
     for (int32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
@@ -152,7 +152,7 @@ __global__ void k_pcg_update(const double *__restrict__ M, const double *__restr
 // p = z + beta p (update_p, CsrCG.cl:311-320)
 __global__ void k_pcg_p(const double *__restrict__ z, double *__restrict__ p, int32_t n, const SolverScalars *sc,
                         const int *__restrict__ done) {
-    if (*(volatile const int *)done) return;
+    if (dvk::chain_done(done)) return;
     const double b = sc->beta;
     for (int32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) p[i] = z[i] + b * p[i];
 }
@@ -162,7 +162,7 @@ template <class ZT>
 __global__ void k_fcg_red(const ZT *__restrict__ z, const double *__restrict__ q, const double *__restrict__ r,
                           int32_t n, SolverScalars *sc, const int *__restrict__ done, double *partials,
                           unsigned *ticket) {
-    if (*(volatile const int *)done) return;
+    if (dvk::chain_done(done)) return;
     double red[2] = {0.0, 0.0};
     for (int32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         double zi = (double)z[i];
@@ -185,7 +185,7 @@ __global__ void k_fcg_update(double *__restrict__ x, double *__restrict__ r, RT 
                              const RT *__restrict__ w0, RT *__restrict__ wb, const double *__restrict__ p,
                              const double *__restrict__ q, int32_t n, SolverScalars *sc, const int *__restrict__ done,
                              double *partials, unsigned *ticket) {
-    if (*(volatile const int *)done) return;
+    if (dvk::chain_done(done)) return;
     const double a = sc->alpha;
     double red[1] = {0.0};
     for (int32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
@@ -389,11 +389,11 @@ extern "C" DV_API int dv_pcg_solve(dv_pcg *s, const double *b, const double *x0,
             for (int k = 0; k < chunk; ++k) {
                 OpPcgAp op{s->p.as<double>(), s->ap.as<double>(), s->ws->sc()};
                 launch_rows<double>(ed, s->A.get(), GatherVec<double, double>{s->p.as<double>()}, op);
-                k_pcg_update<<<g, kThreads, 0, st>>>(s->M.as<double>(), s->ap.as<double>(), s->p.as<double>(),
+                dvk::launch_chain(k_pcg_update, g, kThreads, 0, st, s->M.as<double>(), s->ap.as<double>(), s->p.as<double>(),
                                                      s->x.as<double>(), s->r.as<double>(), s->z.as<double>(), n, s->tol,
                                                      rel_l2, s->ws->sc(), ed.done, ed.partials, ed.ticket);
                 DV_CUDA(cudaGetLastError());
-                k_pcg_p<<<g, kThreads, 0, st>>>(s->z.as<double>(), s->p.as<double>(), n, s->ws->sc(), ed.done);
+                dvk::launch_chain(k_pcg_p, g, kThreads, 0, st, s->z.as<double>(), s->p.as<double>(), n, s->ws->sc(), ed.done);
                 DV_CUDA(cudaGetLastError());
                 ctx->count(2);
             }
@@ -682,7 +682,7 @@ static const T *fcg_step(dv_mgpcg *s, const LaunchEnv &e, VCycle<T> &vc, const T
     cudaStream_t st = e.stream;
     const int g = grid_for(s->ctx, s->n);
     if (!vc.fused_red()) {   // otherwise z.q, z.r and beta came with the V-cycle's last sweep
-        k_fcg_red<T><<<g, kThreads, 0, st>>>(z, s->q.as<double>(), s->r.as<double>(), s->n, s->ws->sc(), e.done,
+        dvk::launch_chain(k_fcg_red<T>, g, kThreads, 0, st, z, s->q.as<double>(), s->r.as<double>(), s->n, s->ws->sc(), e.done,
                                              e.partials, e.ticket);
         DV_CUDA(cudaGetLastError());
         s->ctx->count();
@@ -694,7 +694,7 @@ static const T *fcg_step(dv_mgpcg *s, const LaunchEnv &e, VCycle<T> &vc, const T
     const bool form_wb = mixed && vc.nu > 1 && vc.smoother == DV_SMOOTHER_JACOBI && !vc.lv.empty();
     T *wb = form_wb ? reinterpret_cast<T *>(s->wb32.p) : nullptr;
     const T *w0 = wb ? vc.lv[0].w.template as<T>() : nullptr;
-    k_fcg_update<T><<<g, kThreads, 0, st>>>(s->x.as<double>(), s->r.as<double>(), rl, w0, wb, s->p.as<double>(),
+    dvk::launch_chain(k_fcg_update<T>, g, kThreads, 0, st, s->x.as<double>(), s->r.as<double>(), rl, w0, wb, s->p.as<double>(),
                                             s->q.as<double>(), s->n, s->ws->sc(), e.done, e.partials, e.ticket);
     DV_CUDA(cudaGetLastError());
     s->ctx->count();
@@ -747,7 +747,7 @@ static void mgpcg_solve_impl(dv_mgpcg *s, VCycle<T> &vc, dv_stats *stats) {
     DV_CUDA(cudaMemcpyAsync(s->r.p, s->b.p, nb, cudaMemcpyDeviceToDevice, st));
     T *rin;
     if (std::is_same<T, float>::value) {
-        k_convert<double, float><<<g, kThreads, 0, st>>>(s->b.as<double>(), s->r32.as<float>(), n);
+        dvk::launch_chain(k_convert<double, float>, g, kThreads, 0, st, s->b.as<double>(), s->r32.as<float>(), n);
         DV_CUDA(cudaGetLastError());
         ctx->count();
         rin = reinterpret_cast<T *>(s->r32.p);
@@ -793,7 +793,7 @@ static void mgpcg_solve_impl(dv_mgpcg *s, VCycle<T> &vc, dv_stats *stats) {
         ++refinements;
         DV_CUDA(cudaMemcpyAsync(s->r.p, s->p.p, nb, cudaMemcpyDeviceToDevice, st));
         if (std::is_same<T, float>::value) {
-            k_convert<double, float><<<g, kThreads, 0, st>>>(s->r.as<double>(), s->r32.as<float>(), n);
+            dvk::launch_chain(k_convert<double, float>, g, kThreads, 0, st, s->r.as<double>(), s->r32.as<float>(), n);
             DV_CUDA(cudaGetLastError());
             ctx->count();
         }

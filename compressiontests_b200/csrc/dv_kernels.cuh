@@ -1016,28 +1016,33 @@ __device__ __forceinline__ void pattern_group(int64_t gi, const PatRec<AT> *rec,
 #pragma unroll
     for (int d = 0; d < G; ++d) s[d] = op.init(r0 + d);
     uint32_t k = b;
-    for (; k + 4 <= e; k += 4) {
-        PatRec<AT> q[4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) q[u] = rec[k + u];
+    // B records at a time: their columns, then all gathers, then the multiply-adds.  A group's walk is a chain of
+    // B-wide steps, each as long as a gather from L2; hex patterns have 81, 54, 36 or 24 records.
+    constexpr int B = SHIFT ? 4 : 9;
+    for (; k + B <= e; k += B) {
         if constexpr (SHIFT) {
-            AT x[4][G];
+            PatRec<AT> q[B];
 #pragma unroll
-            for (int u = 0; u < 4; ++u)
+            for (int u = 0; u < B; ++u) q[u] = rec[k + u];
+            AT x[B][G];
+#pragma unroll
+            for (int u = 0; u < B; ++u)
 #pragma unroll
                 for (int d = 0; d < G; ++d) x[u][d] = g((uint32_t)(c0 + q[u].off + d));
 #pragma unroll
-            for (int u = 0; u < 4; ++u)
+            for (int u = 0; u < B; ++u)
 #pragma unroll
                 for (int d = 0; d < G; ++d) s[d] = madd_op<AT, op_fused<Op>::value>(s[d], q[u].v[d], x[u][d]);
         } else {
-            AT x[4];
+            AT x[B];
 #pragma unroll
-            for (int u = 0; u < 4; ++u) x[u] = g((uint32_t)(c0 + q[u].off));
+            for (int u = 0; u < B; ++u) x[u] = g((uint32_t)(c0 + rec[k + u].off));
 #pragma unroll
-            for (int u = 0; u < 4; ++u)
+            for (int u = 0; u < B; ++u) {
+                const PatRec<AT> q = rec[k + u];
 #pragma unroll
-                for (int d = 0; d < G; ++d) s[d] = madd_op<AT, op_fused<Op>::value>(s[d], q[u].v[d], x[u]);
+                for (int d = 0; d < G; ++d) s[d] = madd_op<AT, op_fused<Op>::value>(s[d], q.v[d], x[u]);
+            }
         }
     }
     for (; k < e; ++k) {
@@ -1142,7 +1147,7 @@ struct GridGeom {
     int32_t lx, ly, lz;        // group box
     int32_t ntx, nty, zc;      // tiles per plane in x and y, planes per z run
     int32_t ntile;             // ntx * nty * ceil((lz - 2) / zc): tiles over the interior nodes
-    int32_t bound_blocks;      // blocks [0, bound_blocks) run the boundary list, the rest the tiles
+    int32_t tile_blocks;       // blocks [0, tile_blocks) run the tiles, the rest the boundary list
     int32_t hot, all_hot;      // interior pattern id; 1 when no interior group has another pattern
     int64_t nbound;
 };
@@ -1286,15 +1291,16 @@ __global__ void __launch_bounds__(256, 3)   // 3 blocks an SM: FP64 fits 80 regi
     double red[Op::NRED > 0 ? Op::NRED : 1];
 #pragma unroll
     for (int i = 0; i < (Op::NRED > 0 ? Op::NRED : 1); ++i) red[i] = 0.0;
-    if ((int32_t)blockIdx.x < G.bound_blocks) {
-        // boundary groups from their pattern records
+    if ((int32_t)blockIdx.x >= G.tile_blocks) {
+        // boundary groups from their pattern records: short blocks, last, so that they fill the SMs that
+        // finish their tiles first
         const PatRec<AT> *rec = reinterpret_cast<const PatRec<AT> *>(grid_smem);
         const uint32_t *st = reinterpret_cast<const uint32_t *>(rec + nrec);
         stage_patterns<AT>(grid_smem, grec, pstart, npat, nrec);
         if (chain_done(done)) return;
         __syncthreads();
-        for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < G.nbound;
-             i += (int64_t)G.bound_blocks * blockDim.x)
+        const int64_t bblk = (int64_t)blockIdx.x - G.tile_blocks, nbblk = (int64_t)gridDim.x - G.tile_blocks;
+        for (int64_t i = bblk * blockDim.x + threadIdx.x; i < G.nbound; i += nbblk * blockDim.x)
             pattern_group<AT, Gather, Op, 3, false, false>((int64_t)__ldg(bnode + i), rec, st, pid, nullptr, g, op, red);
     } else {
         if (chain_done(done)) return;
@@ -1307,8 +1313,7 @@ __global__ void __launch_bounds__(256, 3)   // 3 blocks an SM: FP64 fits 80 regi
         const SL slots;
         const int64_t lxy = (int64_t)G.lx * G.ly;
         const int32_t plane_len = (int32_t)(3 * lxy);
-        const int nblk = (int)gridDim.x - G.bound_blocks;
-        for (int t = (int)blockIdx.x - G.bound_blocks; t < G.ntile; t += nblk) {
+        for (int t = (int)blockIdx.x; t < G.ntile; t += G.tile_blocks) {
             const int txi = t % G.ntx, tyi = (t / G.ntx) % G.nty, tzi = t / (G.ntx * G.nty);
             // tiles cover the interior nodes 1 .. l-2 of each axis (the faces are boundary groups)
             const int x0 = 1 + txi * kGridTX, y0 = 1 + tyi * PlaneDims<NY>::TY, z0 = 1 + tzi * G.zc,
@@ -1414,8 +1419,29 @@ inline int stream_run_length(int64_t plane_tiles, int lz, int64_t conc) {
     return best;
 }
 
-// Grid-stencil launch: boundary blocks first (they run alongside the tiles), then tile blocks over
-// runs of zc planes.
+// Planes per z run of the grid stencil's tiles.  A tile of zc planes takes zc + 2 steps, a boundary block
+// about kBoundSteps; tiles start first, boundary blocks fill in.  The time is at least the tiles' waves and at
+// least all work spread over the wave; the run with the smallest bound, the longer one at a tie (fewer
+// planes staged twice).  128^3 FP32 residual 45.1 -> 38.7 us, mixed solve 8.09 -> 7.55 ms: with the boundary
+// blocks first and runs of a power of two, 68 of 512 tiles were left to a second wave.
+constexpr int kBoundSteps = 3;
+inline int grid_run_length(int64_t plane_tiles, int lz, int64_t wave, int64_t bound_blocks) {
+    int best = 1;
+    double best_cost = 1e300;
+    for (int zc = 1; zc <= std::min(lz, 64); ++zc) {
+        const int64_t tiles = plane_tiles * ((lz + zc - 1) / zc);
+        const double waves = (double)((tiles + wave - 1) / wave) * (zc + 2);
+        const double spread = ((double)tiles * (zc + 2) + (double)bound_blocks * kBoundSteps) / (double)wave;
+        const double cost = std::max(waves, spread);
+        if (cost <= best_cost) {
+            best_cost = cost;
+            best = zc;
+        }
+    }
+    return best;
+}
+
+// Grid-stencil launch: tile blocks over runs of zc planes, then the boundary blocks.
 template <class AT, class Gather, class Op, bool HEX>
 void launch_duvi_grid_h(const LaunchEnv &e, const dv_matrix *m, Gather g, Op op) {
     // FP32: two nodes per thread in y (staged rows shared, per-step work amortised); FP64: one
@@ -1443,16 +1469,15 @@ void launch_duvi_grid_h(const LaunchEnv &e, const dv_matrix *m, Gather g, Op op)
     G.all_hot = m->grid_all_hot;
     G.nbound = m->grid_nb;
     const int64_t wave = (int64_t)e.ctx->num_sms * occ;
-    // one boundary group a thread: more per thread puts the boundary blocks on the critical path
-    // (measured: two or four a thread slowed the solve by 6 and 14 %)
-    G.bound_blocks = G.nbound == 0 ? 0
-                     : (int32_t)std::min<int64_t>((G.nbound + 255) / 256, std::max<int64_t>(1, e.max_blocks / 4));
+    // one boundary group a thread (measured: two or four a thread slowed the solve by 6 and 14 %)
+    const int64_t bound_blocks = G.nbound == 0 ? 0
+                                 : std::min<int64_t>((G.nbound + 255) / 256, std::max<int64_t>(1, e.max_blocks / 4));
     const int64_t plane_tiles = (int64_t)G.ntx * G.nty;
     const int lzi = std::max(1, G.lz - 2);
-    G.zc = stream_run_length(plane_tiles, lzi, std::max<int64_t>(1, wave - G.bound_blocks / 2));
+    G.zc = grid_run_length(plane_tiles, lzi, wave, bound_blocks);
     G.ntile = G.lz > 2 ? (int32_t)(plane_tiles * ((lzi + G.zc - 1) / G.zc)) : 0;
-    const int64_t tile_blocks = std::min<int64_t>(G.ntile, std::max<int64_t>(1, e.max_blocks - G.bound_blocks));
-    const int blocks = (int)std::max<int64_t>(1, G.bound_blocks + tile_blocks);
+    G.tile_blocks = (int32_t)std::min<int64_t>(G.ntile, std::max<int64_t>(1, e.max_blocks - bound_blocks));
+    const int blocks = (int)std::max<int64_t>(1, G.tile_blocks + bound_blocks);
     launch_chain(kern, blocks, 256, smem, e.stream, G, cf, m->pat_id.as<uint16_t>(), m->pat_start.as<uint32_t>(),
                                           static_cast<const PatRec<AT> *>(m->pat_rec.p), m->grid_bnode.as<uint32_t>(),
                                           m->pat_count, m->pat_entries, g, op, e.done, e.partials, e.ticket);

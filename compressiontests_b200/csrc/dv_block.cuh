@@ -89,7 +89,8 @@ struct BGatherWB {
 };
 
 // ---------------------------------------------------------------------------
-// epilogues: apply(row, column, row sum, this lane's reduction slots)
+// epilogues: apply(row, column, row sum, this lane's reduction slots); touch(row, column) prefetches what
+// apply will read, issued by the streaming kernel one plane ahead
 // ---------------------------------------------------------------------------
 struct NoFin {
     __device__ void operator()(int, const double *) const {}
@@ -104,6 +105,9 @@ struct BEpiSpmm {   // Y = A X, or Y += A X
         T *p = y + (size_t)i * ld + j;
         *p = clear ? s : *p + s;
     }
+    __device__ __forceinline__ void touch(int32_t i, int j) const {
+        if (!clear) dvk::prefetch_l1(y + (size_t)i * ld + j);
+    }
 };
 template <class T>
 struct BEpiResid {   // R = B - A X
@@ -116,6 +120,7 @@ struct BEpiResid {   // R = B - A X
         const size_t q = (size_t)i * ld + j;
         r[q] = b[q] - s;
     }
+    __device__ __forceinline__ void touch(int32_t i, int j) const { dvk::prefetch_l1(b + (size_t)i * ld + j); }
 };
 template <class T>
 struct BEpiJacobi {   // Y = X + w (B - A X)
@@ -127,6 +132,10 @@ struct BEpiJacobi {   // Y = X + w (B - A X)
     __device__ __forceinline__ void apply(int32_t i, int j, T s, double *) const {
         const size_t q = (size_t)i * ld + j;
         y[q] = x[q] + w[i] * (b[q] - s);
+    }
+    __device__ __forceinline__ void touch(int32_t i, int j) const {
+        dvk::prefetch_l1(x + (size_t)i * ld + j);
+        dvk::prefetch_l1(b + (size_t)i * ld + j);
     }
 };
 template <class T>
@@ -141,6 +150,7 @@ struct BEpiJacobiFromZero {   // two sweeps from zero: Y = wB + w (B - A (wB))
         const T wi = w[i], bi = b[q];
         y[q] = wi * bi + wi * (bi - s);
     }
+    __device__ __forceinline__ void touch(int32_t i, int j) const { dvk::prefetch_l1(b + (size_t)i * ld + j); }
 };
 
 // ---------------------------------------------------------------------------
@@ -389,7 +399,7 @@ __global__ void __launch_bounds__(kThreads) k_bprod_pattern(const uint16_t *__re
                                                             const uint32_t *__restrict__ base, int32_t npat,
                                                             int32_t nrec, int32_t ngroups, int kc, Gather g, Epi ep,
                                                             const int *__restrict__ done, double *partials,
-                                                            unsigned *ticket, const uint32_t *__restrict__ list) {
+                                                            unsigned *ticket) {
     if (dvk::chain_done(done)) return;
     extern __shared__ uint4 bpat_smem[];
     dvk::PatRec<AT> *rec = reinterpret_cast<dvk::PatRec<AT> *>(bpat_smem);
@@ -409,8 +419,7 @@ __global__ void __launch_bounds__(kThreads) k_bprod_pattern(const uint16_t *__re
         for (int c = 0; c < NC; ++c) red[u][c] = 0.0;
     const int lane = threadIdx.x & 31;
     const int32_t nw = (gridDim.x * blockDim.x) >> 5;
-    for (int32_t gi = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; gi < ngroups; gi += nw) {
-        const int32_t grp = list ? (int32_t)__ldg(list + gi) : gi;   // list: the groups to run (ngroups of them)
+    for (int32_t grp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; grp < ngroups; grp += nw) {
         const uint32_t p = __ldg(pid + grp);
         const uint32_t b = st[p], e = st[p + 1];
         const int32_t r0 = grp * G;
@@ -449,26 +458,20 @@ __global__ void __launch_bounds__(kThreads) k_bprod_pattern(const uint16_t *__re
 }
 
 template <class AT, int U, bool EXACT, bool BASED, bool SHIFT, class Gather, class Epi>
-void launch_bprod_pattern_u(const LaunchEnv &e, const dv_matrix *m, int kc, Gather g, Epi ep,
-                            const uint32_t *list = nullptr, int64_t nlist = 0) {
+void launch_bprod_pattern_u(const LaunchEnv &e, const dv_matrix *m, int kc, Gather g, Epi ep) {
     constexpr int G = 3;
     auto kern = k_bprod_pattern<AT, G, U, EXACT, BASED, SHIFT, Gather, Epi>;
     const size_t smem = sizeof(dvk::PatRec<AT>) * (size_t)m->pat_entries + 4 * ((size_t)m->pat_count + 1);
     static dvk::SmemLimit limit;   // per instantiation and device
     limit.raise(kern, smem, e.ctx->device);
-    const int32_t ngroups = list ? (int32_t)nlist : m->n_rows / G;
+    const int32_t ngroups = m->n_rows / G;
     const int blocks = bprod_blocks(e, ngroups, Epi::NC > 0);
     dvk::launch_chain(kern, blocks, kThreads, smem, e.stream, m->pat_id.as<uint16_t>(), m->pat_start.as<uint32_t>(),
                                                static_cast<const dvk::PatRec<AT> *>(m->pat_rec.p),
                                                m->pat_base.as<uint32_t>(), m->pat_count, m->pat_entries, ngroups, kc,
-                                               g, ep, e.done, e.partials, e.ticket, list);
+                                               g, ep, e.done, e.partials, e.ticket);
     DV_CUDA(cudaGetLastError());
     e.ctx->count();
-}
-
-template <int U, class Gather, class Epi>
-void launch_bprod_boundary(const LaunchEnv &e, const dv_matrix *m, int kc, Gather g, Epi ep) {
-    launch_bprod_pattern_u<float, U, true, false, false>(e, m, kc, g, ep, m->grid_bnode.as<uint32_t>(), m->grid_nb);
 }
 
 template <class AT, bool EXACT, bool BASED, bool SHIFT, class Gather, class Epi>
@@ -479,16 +482,19 @@ void launch_bprod_pattern(const LaunchEnv &e, const dv_matrix *m, int kc, Gather
 }
 
 // ---------------------------------------------------------------------------
-// Block products on the grid-stencil layout (FP32 hex operators, epilogues without column
-// reductions).  A block owns a tile of 8 x 4 interior nodes of a plane, streams a run of z planes
-// and covers 32 right-hand sides (lane = column).  Each plane of the tile with its one-node halo
-// (10 x 6 nodes, 3 dofs, 32 columns: 180 rows of 128 bytes) is copied into a ring of shared-memory
-// slots with 16-byte cp.async copies, two planes ahead; warp w takes the 4 nodes x = 4 (w % 2) .. +3
-// of tile row w / 2 and applies every staged value of the plane to the nodes it couples in z - 1,
-// z and z + 1 (the streaming accumulators of k_duvi_grid) with the hex stencil's class values.
-// Each row sums its terms in column order with one FMA each, as the pattern kernel does (the
-// stencil's structural zeros skipped: they add exact zeros).  Face groups and interior groups of
-// other patterns run on the pattern kernel over the boundary list.
+// Block products on the grid-stencil layout (hex operators, a staged FP32 block, FP32 or FP64 sums).  A
+// block owns a tile of 8 x 4 interior nodes of a plane, streams a run of z planes and covers 32
+// right-hand sides (lane = column).  Each plane of the tile with its one-node halo (10 x 6 nodes, 3
+// dofs, 32 columns: 180 rows of 128 bytes) is copied into a ring of shared-memory slots with 16-byte
+// cp.async copies, two planes ahead; warp w takes the 4 nodes x = 4 (w % 2) .. +3 of tile row w / 2
+// and applies every staged value of the plane to the nodes it couples in z - 1, z and z + 1 (the
+// streaming accumulators of k_duvi_grid) with the hex stencil's class values.  Each row sums its
+// terms in column order with one multiply-add each, as the pattern kernel does (the stencil's
+// structural zeros skipped: they add exact zeros).  Face groups and interior groups of other patterns
+// are walked from their pattern records by the launch's last blocks, a warp a group, which fill in
+// beside the tiles (as a second launch they cost 19 to 34 us a product, whatever the level's size).
+// 64 load cases on 48^3, whole solve: 39.1 -> 34.9 ms (the FP64 outer product alone, in place of the
+// patterns with the column sums fused in: 31.2 -> 28.6 ms).
 // ---------------------------------------------------------------------------
 // DV_BGRID=0 keeps the pattern kernel for block products on grid layouts (A/B comparisons).
 inline bool bgrid_enabled() {
@@ -500,146 +506,207 @@ constexpr int kBgHX = kBgTX + 2, kBgHY = kBgTY + 2;      // with the halo
 constexpr int kBgRows = kBgHX * kBgHY * 3;               // staged rows of a plane (node dofs)
 constexpr int kBgStages = 3;
 constexpr int kBgSlot = kBgRows * 32 + kBgRows;          // floats of a slot: the rows, then w (Jacobi from zero)
+constexpr int kBgCopies = (kBgRows * 8 + kThreads - 1) / kThreads;   // 16-byte copies per thread and plane
 
 struct BGridGeom {
     int32_t lx, ly, lz, ntx, nty, zc, ntile, hot, all_hot;
+    int32_t tile_blocks;   // blocks [0, tile_blocks) run the tiles, the rest the boundary list
+    int32_t nbound;
+};
+template <class AT>
+struct BGridCoef {
+    AT cls[dvk::kHexClasses];
 };
 
 template <class Gather>
 struct BGridSrc;   // the block array a gather stages, and its per-row weight (w .* B)
-template <class T>
-struct BGridSrc<BGatherVec<T, T>> {
+template <class AT>
+struct BGridSrc<BGatherVec<float, AT>> {
     static constexpr bool WB = false;
-    static const T *block(const BGatherVec<T, T> &g) { return g.x; }
-    __device__ static const T *weights(const BGatherVec<T, T> &) { return nullptr; }
+    static const float *block(const BGatherVec<float, AT> &g) { return g.x; }
+    __device__ static const float *weights(const BGatherVec<float, AT> &) { return nullptr; }
 };
-template <class T>
-struct BGridSrc<BGatherWB<T>> {
+template <>
+struct BGridSrc<BGatherWB<float>> {
     static constexpr bool WB = true;
-    static const T *block(const BGatherWB<T> &g) { return g.b; }
-    __device__ static const T *weights(const BGatherWB<T> &g) { return g.w; }
+    static const float *block(const BGatherWB<float> &g) { return g.b; }
+    __device__ static const float *weights(const BGatherWB<float> &g) { return g.w; }
 };
 
-template <class Gather>
-__device__ __forceinline__ void bgrid_issue(const Gather &g, const float *__restrict__ X, int ld, float *slot, int x0,
-                                            int y0, int z, const BGridGeom &G, int j0, int kc) {
-    const bool zin = z >= 0 && z < G.lz;
-    for (int c = threadIdx.x; c < kBgRows * 8; c += kThreads) {
-        const int row = c >> 3, sub = c & 7, hn = row / 3, comp = row - 3 * hn;
-        const int gx = x0 - 1 + hn % kBgHX, gy = y0 - 1 + hn / kBgHX;
-        const bool v = zin && gx >= 0 && gx < G.lx && gy >= 0 && gy < G.ly && j0 + 4 * sub < kc;
-        const int64_t grow = 3 * ((int64_t)gx + (int64_t)G.lx * (gy + (int64_t)G.ly * z)) + comp;
-        dvk::cp_async_zfill<16>(slot + row * 32 + 4 * sub, v ? X + grow * ld + j0 + 4 * sub : X, v);
-    }
-    if constexpr (BGridSrc<Gather>::WB) {
-        const float *w = BGridSrc<Gather>::weights(g);
-        for (int row = threadIdx.x; row < kBgRows; row += kThreads) {
-            const int hn = row / 3, comp = row - 3 * hn;
-            const int gx = x0 - 1 + hn % kBgHX, gy = y0 - 1 + hn / kBgHX;
-            const bool v = zin && gx >= 0 && gx < G.lx && gy >= 0 && gy < G.ly;
-            const int64_t grow = 3 * ((int64_t)gx + (int64_t)G.lx * (gy + (int64_t)G.ly * z)) + comp;
-            dvk::cp_async_zfill<4>(slot + kBgRows * 32 + row, v ? w + grow : w, v);
-        }
-    }
-    dvk::cp_async_commit();
-}
-
-template <class Gather, class Epi>
-__global__ void __launch_bounds__(kThreads, 3) k_bprod_grid(BGridGeom G, dvk::GridCoef<float> cf,
-                                                             const uint16_t *__restrict__ pid, const float *__restrict__ X,
-                                                             int ld, int kc, Gather g, Epi ep,
-                                                             const int *__restrict__ done) {
-    static_assert(Epi::NC == 0, "column reductions run on the pattern kernel");
-    if (dvk::chain_done(done)) return;
+template <class AT, class Gather, class Epi>
+__global__ void __launch_bounds__(kThreads, sizeof(AT) == 8 ? 2 : 3)
+    k_bprod_grid(BGridGeom G, BGridCoef<AT> cf, const uint16_t *__restrict__ pid, const uint32_t *__restrict__ pstart,
+                 const dvk::PatRec<AT> *__restrict__ grec, const uint32_t *__restrict__ bnode, int32_t npat, int32_t nrec,
+                 const float *__restrict__ X, int ld, int kc, Gather g, Epi ep, const int *__restrict__ done) {
+    static_assert(Epi::NC == 0, "column reductions run on the other kernels");
     extern __shared__ uint4 bgrid_smem[];
-    float *ring = reinterpret_cast<float *>(bgrid_smem);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int yw = warp >> 1, xs = (warp & 1) * 4;   // the warp's 4 nodes: tile x xs .. xs+3, tile row yw
-    const int j0 = blockIdx.y * 32;
-    const int64_t lxy = (int64_t)G.lx * G.ly;
+    const int j0 = blockIdx.y * 32, j = j0 + lane;
     double nored[1];
-    for (int t = blockIdx.x; t < G.ntile; t += gridDim.x) {
-        const int txi = t % G.ntx, tyi = (t / G.ntx) % G.nty, tzi = t / (G.ntx * G.nty);
-        const int x0 = 1 + txi * kBgTX, y0 = 1 + tyi * kBgTY, z0 = 1 + tzi * G.zc, z1 = min(G.lz - 1, z0 + G.zc);
-        const int gy = y0 + yw;
-        bool inxy[4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) inxy[i] = x0 + xs + i <= G.lx - 2 && gy <= G.ly - 2;
-        auto active = [&](int i, int z) {
-            if (!inxy[i] || z < 1 || z > G.lz - 2) return false;
-            return G.all_hot || (int)__ldg(pid + (x0 + xs + i) + (int64_t)G.lx * gy + lxy * z) == G.hot;
-        };
-        bgrid_issue(g, X, ld, ring, x0, y0, z0 - 1, G, j0, kc);
-        if (z0 <= z1) bgrid_issue(g, X, ld, ring + kBgSlot, x0, y0, z0, G, j0, kc);
-        else dvk::cp_async_commit();
-        float a0[4][3], a1[4][3], a2[4][3];
-        bool act0[4], act1[4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            act0[i] = act1[i] = false;
-#pragma unroll
-            for (int d = 0; d < 3; ++d) a0[i][d] = a1[i][d] = a2[i][d] = 0.f;
-        }
-        for (int p = z0 - 1, k = 0; p <= z1; ++p, ++k) {
-            dvk::cp_async_wait<kBgStages - 2>();
-            __syncthreads();
-            if (p + 2 <= z1) bgrid_issue(g, X, ld, ring + ((k + 2) % kBgStages) * kBgSlot, x0, y0, p + 2, G, j0, kc);
-            else dvk::cp_async_commit();
-            const float *pl = ring + (k % kBgStages) * kBgSlot;
-            const bool di = p + 1 >= z0 && p + 1 < z1, dm = p >= z0 && p < z1, df = p - 1 >= z0 && p - 1 < z1;
-            bool act2[4];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                act2[i] = di && active(i, p + 1);
-#pragma unroll
-                for (int d = 0; d < 3; ++d) a2[i][d] = 0.f;
-            }
-#pragma unroll
-            for (int dy = 0; dy < 3; ++dy)
-#pragma unroll
-                for (int hx = 0; hx < 6; ++hx)
-#pragma unroll
-                    for (int c = 0; c < 3; ++c) {
-                        const int row = ((yw + dy) * kBgHX + xs + hx) * 3 + c;
-                        float v = pl[row * 32 + lane];
-                        if constexpr (BGridSrc<Gather>::WB) v = pl[kBgRows * 32 + row] * v;
-#pragma unroll
-                        for (int i = 0; i < 4; ++i) {
-                            const int dx = hx - i;   // neighbour offset + 1
-                            if (dx < 0 || dx > 2) continue;
-                            const int e = 9 * dy + 3 * dx + c;
-#pragma unroll
-                            for (int d = 0; d < 3; ++d) {
-                                const int ci = dvk::hex_class(3 * e + d), cm = dvk::hex_class(3 * (27 + e) + d),
-                                          cz = dvk::hex_class(3 * (54 + e) + d);
-                                if (ci >= 0 && di) a2[i][d] = fmaf(cf.cls[ci], v, a2[i][d]);
-                                if (cm >= 0 && dm) a1[i][d] = fmaf(cf.cls[cm], v, a1[i][d]);
-                                if (cz >= 0 && df) a0[i][d] = fmaf(cf.cls[cz], v, a0[i][d]);
-                            }
-                        }
-                    }
-            if (df && lane < kc - j0) {
-#pragma unroll
-                for (int i = 0; i < 4; ++i)
-                    if (act0[i]) {
-                        const int32_t r = (int32_t)(3 * ((x0 + xs + i) + G.lx * (int64_t)gy + lxy * (p - 1)));
-#pragma unroll
-                        for (int d = 0; d < 3; ++d) ep.apply(r + d, j0 + lane, a0[i][d], nored);
-                    }
-            }
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-#pragma unroll
-                for (int d = 0; d < 3; ++d) {
-                    a0[i][d] = a1[i][d];
-                    a1[i][d] = a2[i][d];
-                }
-                act0[i] = act1[i];
-                act1[i] = act2[i];
-            }
-        }
-        dvk::cp_async_wait<0>();
+    if ((int)blockIdx.x >= G.tile_blocks) {
+        // boundary groups from their pattern records, a warp a group
+        dvk::PatRec<AT> *rec = reinterpret_cast<dvk::PatRec<AT> *>(bgrid_smem);
+        const uint32_t *st = reinterpret_cast<const uint32_t *>(rec + nrec);
+        dvk::stage_patterns<AT>(bgrid_smem, grec, pstart, npat, nrec);
+        if (dvk::chain_done(done)) return;
         __syncthreads();
+        const int32_t nw = ((int32_t)gridDim.x - G.tile_blocks) * kWarps;
+        for (int32_t i = ((int32_t)blockIdx.x - G.tile_blocks) * kWarps + warp; i < G.nbound; i += nw) {
+            const int32_t r0 = 3 * (int32_t)__ldg(bnode + i);
+            const uint32_t p = __ldg(pid + r0 / 3);
+            AT acc[3] = {AT(0), AT(0), AT(0)};
+            const uint32_t end = st[p + 1];
+            uint32_t k = st[p];
+            if (j < kc) {
+                for (; k + 9 <= end; k += 9) {   // hex patterns have 81, 54, 36 or 24 records
+                    AT x[9];
+#pragma unroll
+                    for (int u = 0; u < 9; ++u) x[u] = g((uint32_t)(r0 + rec[k + u].off), j);
+#pragma unroll
+                    for (int u = 0; u < 9; ++u)
+#pragma unroll
+                        for (int d = 0; d < 3; ++d) acc[d] = fma(rec[k + u].v[d], x[u], acc[d]);
+                }
+                for (; k < end; ++k) {
+                    const AT x = g((uint32_t)(r0 + rec[k].off), j);
+#pragma unroll
+                    for (int d = 0; d < 3; ++d) acc[d] = fma(rec[k].v[d], x, acc[d]);
+                }
+#pragma unroll
+                for (int d = 0; d < 3; ++d) ep.apply(r0 + d, j, acc[d], nored);
+            }
+        }
+    } else {
+        if (dvk::chain_done(done)) return;
+        float *ring = reinterpret_cast<float *>(bgrid_smem);
+        const int yw = warp >> 1, xs = (warp & 1) * 4;   // the warp's 4 nodes: tile x xs .. xs+3, tile row yw
+        const int32_t lxy = G.lx * G.ly;
+        constexpr bool WB = BGridSrc<Gather>::WB;
+        for (int t = blockIdx.x; t < G.ntile; t += G.tile_blocks) {
+            const int txi = t % G.ntx, tyi = (t / G.ntx) % G.nty, tzi = t / (G.ntx * G.nty);
+            const int x0 = 1 + txi * kBgTX, y0 = 1 + tyi * kBgTY, z0 = 1 + tzi * G.zc, z1 = min(G.lz - 1, z0 + G.zc);
+            const int gy = y0 + yw;
+            bool inxy[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) inxy[i] = x0 + xs + i <= G.lx - 2 && gy <= G.ly - 2;
+            auto active = [&](int i, int z) {
+                if (!inxy[i] || z < 1 || z > G.lz - 2) return false;
+                return G.all_hot || (int)__ldg(pid + (x0 + xs + i) + G.lx * gy + (int64_t)lxy * z) == G.hot;
+            };
+            // this thread's copies of a plane: row of the plane (-1: zero, -2: none); columns 4 (c % 8) .. +3
+            int32_t prow[kBgCopies], wrow = -2;
+            const int sub = threadIdx.x & 7;
+#pragma unroll
+            for (int q = 0; q < kBgCopies; ++q) {
+                const int row = (threadIdx.x + kThreads * q) >> 3, hn = row / 3;
+                const int gx = x0 - 1 + hn % kBgHX, hy = y0 - 1 + hn / kBgHX;
+                prow[q] = row >= kBgRows ? -2
+                          : gx >= 0 && gx < G.lx && hy >= 0 && hy < G.ly && j0 + 4 * sub < kc ? 3 * (gx + G.lx * hy) + row - 3 * hn
+                                                                                            : -1;
+            }
+            if constexpr (WB)
+                if (threadIdx.x < kBgRows) {
+                    const int hn = threadIdx.x / 3, gx = x0 - 1 + hn % kBgHX, hy = y0 - 1 + hn / kBgHX;
+                    wrow = gx >= 0 && gx < G.lx && hy >= 0 && hy < G.ly ? 3 * (gx + G.lx * hy) + (int)threadIdx.x - 3 * hn : -1;
+                }
+            auto issue = [&](int z, int k) {
+                const bool zin = z >= 0 && z < G.lz;
+                const int64_t base = zin ? 3 * (int64_t)lxy * z : 0;
+                float *slot = ring + (k % kBgStages) * kBgSlot;
+                const float *src = X + base * ld + j0 + 4 * sub;
+#pragma unroll
+                for (int q = 0; q < kBgCopies; ++q)
+                    if (prow[q] > -2) {
+                        const bool v = zin && prow[q] >= 0;
+                        dvk::cp_async_zfill<16>(slot + (threadIdx.x + kThreads * q) * 4, v ? src + (int64_t)prow[q] * ld : X, v);
+                    }
+                if constexpr (WB)
+                    if (wrow > -2) {
+                        const bool v = zin && wrow >= 0;
+                        const float *w = BGridSrc<Gather>::weights(g);
+                        dvk::cp_async_zfill<4>(slot + kBgRows * 32 + threadIdx.x, v ? w + base + wrow : w, v);
+                    }
+                dvk::cp_async_commit();
+            };
+            issue(z0 - 1, 0);
+            if (z0 <= z1) issue(z0, 1);
+            else dvk::cp_async_commit();
+            AT a0[4][3], a1[4][3], a2[4][3];
+            bool act0[4], act1[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                act0[i] = act1[i] = false;
+#pragma unroll
+                for (int d = 0; d < 3; ++d) a0[i][d] = a1[i][d] = a2[i][d] = AT(0);
+            }
+            const int32_t r_xy = 3 * (x0 + xs + G.lx * gy);
+            for (int p = z0 - 1, k = 0; p <= z1; ++p, ++k) {
+                dvk::cp_async_wait<kBgStages - 2>();
+                __syncthreads();
+                if (p + 2 <= z1) issue(p + 2, k + 2);
+                else dvk::cp_async_commit();
+                const float *pl = ring + (k % kBgStages) * kBgSlot;
+                const bool di = p + 1 >= z0 && p + 1 < z1, dm = p >= z0 && p < z1, df = p - 1 >= z0 && p - 1 < z1;
+                bool act2[4];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    act2[i] = di && active(i, p + 1);
+#pragma unroll
+                    for (int d = 0; d < 3; ++d) a2[i][d] = AT(0);
+                    if (dm && act1[i] && j < kc)   // finished next step
+#pragma unroll
+                        for (int d = 0; d < 3; ++d) ep.touch(r_xy + 3 * i + d + 3 * lxy * p, j);
+                }
+                auto step = [&](auto DI, auto DM, auto DF) {
+#pragma unroll
+                    for (int dy = 0; dy < 3; ++dy)
+#pragma unroll
+                        for (int hx = 0; hx < 6; ++hx)
+#pragma unroll
+                            for (int c = 0; c < 3; ++c) {
+                                const int row = ((yw + dy) * kBgHX + xs + hx) * 3 + c;
+                                float f = pl[row * 32 + lane];
+                                if constexpr (WB) f = pl[kBgRows * 32 + row] * f;
+                                const AT v = (AT)f;
+#pragma unroll
+                                for (int i = 0; i < 4; ++i) {
+                                    const int dx = hx - i;   // neighbour offset + 1
+                                    if (dx < 0 || dx > 2) continue;
+                                    const int e = 9 * dy + 3 * dx + c;
+#pragma unroll
+                                    for (int d = 0; d < 3; ++d) {
+                                        const int ci = dvk::hex_class(3 * e + d), cm = dvk::hex_class(3 * (27 + e) + d),
+                                                  cz = dvk::hex_class(3 * (54 + e) + d);
+                                        if (ci >= 0 && DI) a2[i][d] = fma(cf.cls[ci], v, a2[i][d]);
+                                        if (cm >= 0 && DM) a1[i][d] = fma(cf.cls[cm], v, a1[i][d]);
+                                        if (cz >= 0 && DF) a0[i][d] = fma(cf.cls[cz], v, a0[i][d]);
+                                    }
+                                }
+                            }
+                };
+                if (di && dm && df) step(std::true_type{}, std::true_type{}, std::true_type{});
+                else step(di, dm, df);
+                if (df && j < kc) {
+#pragma unroll
+                    for (int i = 0; i < 4; ++i)
+                        if (act0[i])
+#pragma unroll
+                            for (int d = 0; d < 3; ++d) ep.apply(r_xy + 3 * i + d + 3 * lxy * (p - 1), j, a0[i][d], nored);
+                }
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+#pragma unroll
+                    for (int d = 0; d < 3; ++d) {
+                        a0[i][d] = a1[i][d];
+                        a1[i][d] = a2[i][d];
+                    }
+                    act0[i] = act1[i];
+                    act1[i] = act2[i];
+                }
+            }
+            dvk::cp_async_wait<0>();
+            __syncthreads();
+        }
     }
 }
 
@@ -648,42 +715,48 @@ struct bgrid_gather : std::false_type {};
 template <>
 struct bgrid_gather<BGatherVec<float, float>> : std::true_type {};
 template <>
+struct bgrid_gather<BGatherVec<float, double>> : std::true_type {};
+template <>
 struct bgrid_gather<BGatherWB<float>> : std::true_type {};
 
-// The grid-stencil block product and the boundary groups' pattern walk (two launches, disjoint rows).
-template <class Gather, class Epi>
+// Whether m's block products run on the grid-stencil layout, given an aligned block of rows of ld columns.
+inline bool bgrid_layout(const dv_matrix *m, int precision, int ld) {
+    return m->format == DV_FORMAT_DUVI && m->duvi_variant == 3 && m->grid_hex && m->precision == precision && ld % 4 == 0;
+}
+
+template <class AT, class Gather, class Epi>
 void launch_bprod_grid(const LaunchEnv &e, const dv_matrix *m, int kc, Gather g, Epi ep) {
+    auto kern = k_bprod_grid<AT, Gather, Epi>;
+    const size_t smem = std::max(sizeof(float) * (size_t)kBgStages * kBgSlot,
+                                 sizeof(dvk::PatRec<AT>) * (size_t)m->pat_entries + 4 * ((size_t)m->pat_count + 1));
+    static dvk::SmemLimit limit;   // per instantiation and device
+    limit.raise(kern, smem, e.ctx->device);
+    static dvk::OccupancyCache occupancy;   // per instantiation
+    const int64_t wave = (int64_t)e.ctx->num_sms * occupancy.get(kern, kThreads, smem, e.ctx->device);
     BGridGeom G;
     G.lx = m->grid_lx;
     G.ly = m->grid_ly;
     G.lz = m->grid_lz;
     G.ntx = std::max(0, (G.lx - 2 + kBgTX - 1) / kBgTX);   // tiles over the interior nodes 1 .. l-2
     G.nty = std::max(0, (G.ly - 2 + kBgTY - 1) / kBgTY);
-    G.zc = 8;
-    const int lzi = std::max(1, G.lz - 2);
-    G.ntile = G.lz > 2 ? G.ntx * G.nty * ((lzi + G.zc - 1) / G.zc) : 0;
     G.hot = m->grid_hot;
     G.all_hot = m->grid_all_hot;
-    dvk::GridCoef<float> cf;
-    for (int k = 0; k < 81; ++k)
-        for (int d = 0; d < 3; ++d) cf.v[k][d] = (float)m->grid_coef[3 * k + d];
-    for (int c = 0; c < dvk::kHexClasses; ++c) cf.cls[c] = (float)m->grid_cls[c];
-    if (G.ntile > 0) {
-        auto kern = k_bprod_grid<Gather, Epi>;
-        const size_t smem = sizeof(float) * (size_t)kBgStages * kBgSlot;
-        static dvk::SmemLimit limit;   // per instantiation and device
-        limit.raise(kern, smem, e.ctx->device);
-        const dim3 grid((unsigned)G.ntile, (unsigned)((kc + 31) / 32));
-        dvk::launch_chain(kern, grid, kThreads, smem, e.stream, G, cf, m->pat_id.as<uint16_t>(), BGridSrc<Gather>::block(g), g.ld, kc,
-                                                 g, ep, e.done);
-        DV_CUDA(cudaGetLastError());
-        e.ctx->count();
-    }
-    if (m->grid_nb > 0) {
-        if (kc <= 32) launch_bprod_boundary<1>(e, m, kc, g, ep);
-        else if (kc <= 64) launch_bprod_boundary<2>(e, m, kc, g, ep);
-        else launch_bprod_boundary<4>(e, m, kc, g, ep);
-    }
+    G.nbound = (int32_t)m->grid_nb;
+    const int64_t slabs = (kc + 31) / 32, plane_tiles = (int64_t)G.ntx * G.nty;
+    const int lzi = std::max(1, G.lz - 2);
+    // two boundary groups a warp; a block of them takes about as long as three plane steps of a tile
+    const int64_t bound_blocks = std::min<int64_t>((G.nbound + 2 * kWarps - 1) / (2 * kWarps), wave);
+    G.zc = dvk::grid_run_length(plane_tiles * slabs, lzi, wave, bound_blocks * slabs);
+    G.ntile = G.lz > 2 ? (int32_t)(plane_tiles * ((lzi + G.zc - 1) / G.zc)) : 0;
+    G.tile_blocks = G.ntile;
+    BGridCoef<AT> cf;
+    for (int c = 0; c < dvk::kHexClasses; ++c) cf.cls[c] = (AT)m->grid_cls[c];
+    const dim3 grid((unsigned)std::max<int64_t>(1, G.tile_blocks + bound_blocks), (unsigned)slabs);
+    dvk::launch_chain(kern, grid, kThreads, smem, e.stream, G, cf, m->pat_id.as<uint16_t>(), m->pat_start.as<uint32_t>(),
+                      static_cast<const dvk::PatRec<AT> *>(m->pat_rec.p), m->grid_bnode.as<uint32_t>(), m->pat_count,
+                      m->pat_entries, BGridSrc<Gather>::block(g), g.ld, kc, g, ep, e.done);
+    DV_CUDA(cudaGetLastError());
+    e.ctx->count();
 }
 
 // Matrix-free trilinear transfer (DV_FORMAT_TRILINEAR): one thread per (node, column j), the
@@ -725,12 +798,12 @@ void launch_bprod(const LaunchEnv &e, const dv_matrix *m, int kc, Gather g, Epi 
     }
     DV_REQUIRE(m->format == DV_FORMAT_CSR || m->format == DV_FORMAT_DUVI, DV_ERR_UNSUPPORTED,
                "block products need an assembled matrix");
-    if constexpr (Epi::NC == 0 && std::is_same<AT, float>::value && bgrid_gather<Gather>::value) {
-        // FP32 hex operators on the grid-stencil layout; 16-byte copies need an aligned block and ld
-        const void *xb = BGridSrc<Gather>::block(g);
-        if (m->format == DV_FORMAT_DUVI && m->duvi_variant == 3 && m->grid_hex && m->precision == DV_F32 &&
-            (reinterpret_cast<uintptr_t>(xb) & 15) == 0 && g.ld % 4 == 0 && bgrid_enabled()) {
-            launch_bprod_grid(e, m, kc, g, ep);
+    if constexpr (Epi::NC == 0 && bgrid_gather<Gather>::value && !(EXACT && sizeof(AT) == 8)) {
+        // hex operators on the grid-stencil layout, FP32 block staged; 16-byte copies need an aligned block and
+        // ld.  FP64 products that have to round as the oracle does stay on the patterns.
+        if (bgrid_layout(m, sizeof(AT) == 4 ? DV_F32 : DV_F64, g.ld) &&
+            (reinterpret_cast<uintptr_t>(BGridSrc<Gather>::block(g)) & 15) == 0 && bgrid_enabled()) {
+            launch_bprod_grid<AT>(e, m, kc, g, ep);
             return;
         }
     }

@@ -39,9 +39,10 @@ struct FinFcg {
         cs[j].alpha = cs[j].converged ? 0.0 : cs[j].zr / t[0];
     }
 };
-template <class ZT>
+// RED: with p.q; without, k_bfcg_pq sums it afterwards (the grid-stencil products carry no column sums).
+template <class ZT, bool RED>
 struct BEpiFcg {
-    static constexpr int NC = 1;
+    static constexpr int NC = RED ? 1 : 0;
     const ZT *z;
     double *p, *q;
     const ColScalars *cs;
@@ -54,7 +55,13 @@ struct BEpiFcg {
         const double pi = (double)z[o] + bt * p[o];
         q[o] = qi;
         p[o] = pi;
-        red[0] += pi * qi;
+        if constexpr (RED) red[0] += pi * qi;
+    }
+    __device__ __forceinline__ void touch(int32_t i, int j) const {
+        const size_t o = (size_t)i * ld + j;
+        dvk::prefetch_l1(z + o);
+        dvk::prefetch_l1(p + o);
+        dvk::prefetch_l1(q + o);
     }
 };
 
@@ -72,7 +79,7 @@ struct FinRed {   // beta_j = -(z.q)/(p.q) (FCG(1)), 0 on a restart or a frozen 
 };
 template <class ZT, int U>
 __global__ void __launch_bounds__(dvb::kThreads) k_bfcg_red(const ZT *__restrict__ z, const double *__restrict__ q,
-                                                            const double *__restrict__ r, int32_t n, int k,
+                                                            const double *__restrict__ r, int32_t n, int k, int ld,
                                                             ColScalars *cs, const int *__restrict__ done,
                                                             double *partials, unsigned *ticket) {
     if (dvk::chain_done(done)) return;
@@ -86,13 +93,36 @@ __global__ void __launch_bounds__(dvb::kThreads) k_bfcg_red(const ZT *__restrict
         for (int u = 0; u < U; ++u) {
             const int j = lane + 32 * u;
             if (j < k) {
-                const size_t o = (size_t)i * k + j;
+                const size_t o = (size_t)i * ld + j;
                 const double zi = (double)z[o];
                 red[u][0] += zi * q[o];
                 red[u][1] += zi * r[o];
             }
         }
     dvb::col_reduce<2, U>(red, k, partials, ticket, FinRed{cs});
+}
+// p.q and alpha of every column
+template <int U>
+__global__ void __launch_bounds__(dvb::kThreads) k_bfcg_pq(const double *__restrict__ p, const double *__restrict__ q,
+                                                           int32_t n, int k, int ld, ColScalars *cs,
+                                                           const int *__restrict__ done, double *partials,
+                                                           unsigned *ticket) {
+    if (dvk::chain_done(done)) return;
+    double red[U][1];
+#pragma unroll
+    for (int u = 0; u < U; ++u) red[u][0] = 0.0;
+    const int lane = threadIdx.x & 31;
+    const int32_t nw = (gridDim.x * blockDim.x) >> 5;
+    for (int32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < n; i += nw)
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int j = lane + 32 * u;
+            if (j < k) {
+                const size_t o = (size_t)i * ld + j;
+                red[u][0] += p[o] * q[o];
+            }
+        }
+    dvb::col_reduce<1, U>(red, k, partials, ticket, FinFcg{cs});
 }
 
 struct FinUpdate {   // ||r_j||^2 and the per-column stop test
@@ -107,7 +137,7 @@ struct FinUpdate {   // ||r_j||^2 and the per-column stop test
 template <class RT, int U>
 __global__ void __launch_bounds__(dvb::kThreads) k_bfcg_update(double *__restrict__ x, double *__restrict__ r,
                                                                RT *__restrict__ rlow, const double *__restrict__ p,
-                                                               const double *__restrict__ q, int32_t n, int k,
+                                                               const double *__restrict__ q, int32_t n, int k, int ld,
                                                                ColScalars *cs, double tol2, const int *__restrict__ done,
                                                                double *partials, unsigned *ticket) {
     if (dvk::chain_done(done)) return;
@@ -124,7 +154,7 @@ __global__ void __launch_bounds__(dvb::kThreads) k_bfcg_update(double *__restric
         for (int u = 0; u < U; ++u) {
             const int j = lane + 32 * u;
             if (j < k) {
-                const size_t o = (size_t)i * k + j;
+                const size_t o = (size_t)i * ld + j;
                 x[o] = x[o] + al[u] * p[o];
                 const double ri = r[o] - al[u] * q[o];
                 r[o] = ri;
@@ -165,7 +195,7 @@ struct FinNorm {
     }
 };
 template <int U>
-__global__ void __launch_bounds__(dvb::kThreads) k_bnorm(const double *__restrict__ v, int32_t n, int k, ColScalars *cs,
+__global__ void __launch_bounds__(dvb::kThreads) k_bnorm(const double *__restrict__ v, int32_t n, int k, int ld, ColScalars *cs,
                                                          int slot, double *partials, unsigned *ticket) {
     double red[U][1];
 #pragma unroll
@@ -177,7 +207,7 @@ __global__ void __launch_bounds__(dvb::kThreads) k_bnorm(const double *__restric
         for (int u = 0; u < U; ++u) {
             const int j = lane + 32 * u;
             if (j < k) {
-                const double a = v[(size_t)i * k + j];
+                const double a = v[(size_t)i * ld + j];
                 red[u][0] += a * a;
             }
         }
@@ -198,7 +228,7 @@ __global__ void k_bscale(const T *__restrict__ w, const T *__restrict__ b, T *__
 // 32-wide tiles of Ainv and B staged in shared memory.
 template <class T>
 __global__ void __launch_bounds__(256) k_bcoarse(const T *__restrict__ a, const T *__restrict__ b, T *__restrict__ y,
-                                                 int32_t nc, int k, const int *__restrict__ done) {
+                                                 int32_t nc, int k, int ld, const int *__restrict__ done) {
     if (dvk::chain_done(done)) return;
     __shared__ T As[8][33];
     __shared__ T Bs[32][33];
@@ -208,13 +238,13 @@ __global__ void __launch_bounds__(256) k_bcoarse(const T *__restrict__ a, const 
     T s = 0;
     for (int32_t c0 = 0; c0 < nc; c0 += 32) {
         As[ty][tx] = (row < nc && c0 + tx < nc) ? a[(size_t)row * nc + c0 + tx] : T(0);
-        for (int q = ty; q < 32; q += 8) Bs[q][tx] = (c0 + q < nc && col < k) ? b[(size_t)(c0 + q) * k + col] : T(0);
+        for (int q = ty; q < 32; q += 8) Bs[q][tx] = (c0 + q < nc && col < k) ? b[(size_t)(c0 + q) * ld + col] : T(0);
         __syncthreads();
 #pragma unroll
         for (int q = 0; q < 32; ++q) s += As[ty][q] * Bs[q][tx];
         __syncthreads();
     }
-    if (row < nc && col < k) y[(size_t)row * k + col] = s;
+    if (row < nc && col < k) y[(size_t)row * ld + col] = s;
 }
 
 // ---------------------------------------------------------------------------
@@ -231,13 +261,13 @@ inline int vec_grid(dv_context *ctx, size_t tot) {
 }
 
 template <class T>
-T *block_vcycle(const LaunchEnv &e, VCycle<T> &vc, BlockLevels<T> &W, size_t l, const T *b, int k) {
+T *block_vcycle(const LaunchEnv &e, VCycle<T> &vc, BlockLevels<T> &W, size_t l, const T *b, int k, int ld) {
     using namespace dvb;
     cudaStream_t s = e.stream;
     dv_context *ctx = vc.ctx;
     if (l == vc.lv.size()) {
         dvk::launch_chain(k_bcoarse<T>, dim3((vc.nc + 7) / 8, (k + 31) / 32), 256, 0, s, vc.ainv.template as<T>(), b,
-                                                                          W.xc.template as<T>(), vc.nc, k, e.done);
+                                                                          W.xc.template as<T>(), vc.nc, k, ld, e.done);
         DV_CUDA(cudaGetLastError());
         ctx->count();
         return W.xc.template as<T>();
@@ -246,24 +276,24 @@ T *block_vcycle(const LaunchEnv &e, VCycle<T> &vc, BlockLevels<T> &W, size_t l, 
     T *x = W.x[l].template as<T>(), *t = W.t[l].template as<T>();
     const T *w = L.w.template as<T>();
     if (vc.nu == 1) {
-        dvk::launch_chain(k_bscale<T>, vec_grid(ctx, (size_t)L.n * k), 256, 0, s, w, b, x, L.n, k, e.done);
+        dvk::launch_chain(k_bscale<T>, vec_grid(ctx, (size_t)L.n * ld), 256, 0, s, w, b, x, L.n, ld, e.done);
         DV_CUDA(cudaGetLastError());
         ctx->count();
     } else {
-        launch_bprod<T>(e, L.A.get(), k, BGatherWB<T>{w, b, k}, BEpiJacobiFromZero<T>{w, b, x, k, {}});
+        launch_bprod<T>(e, L.A.get(), k, BGatherWB<T>{w, b, ld}, BEpiJacobiFromZero<T>{w, b, x, ld, {}});
         for (int q = 2; q < vc.nu; ++q) {
-            launch_bprod<T>(e, L.A.get(), k, BGatherVec<T, T>{x, k}, BEpiJacobi<T>{x, w, b, t, k, {}});
+            launch_bprod<T>(e, L.A.get(), k, BGatherVec<T, T>{x, ld}, BEpiJacobi<T>{x, w, b, t, ld, {}});
             std::swap(x, t);
         }
     }
     T *r = W.r[l].template as<T>();
-    launch_bprod<T>(e, L.A.get(), k, BGatherVec<T, T>{x, k}, BEpiResid<T>{b, r, k, {}});
+    launch_bprod<T>(e, L.A.get(), k, BGatherVec<T, T>{x, ld}, BEpiResid<T>{b, r, ld, {}});
     T *bn = l + 1 < vc.lv.size() ? W.b[l + 1].template as<T>() : W.bc.template as<T>();
-    launch_bprod<T>(e, L.R.get(), k, BGatherVec<T, T>{r, k}, BEpiSpmm<T>{bn, k, 1, {}});
-    T *xn = block_vcycle<T>(e, vc, W, l + 1, bn, k);
-    launch_bprod<T>(e, L.P.get(), k, BGatherVec<T, T>{xn, k}, BEpiSpmm<T>{x, k, 0, {}});
+    launch_bprod<T>(e, L.R.get(), k, BGatherVec<T, T>{r, ld}, BEpiSpmm<T>{bn, ld, 1, {}});
+    T *xn = block_vcycle<T>(e, vc, W, l + 1, bn, k, ld);
+    launch_bprod<T>(e, L.P.get(), k, BGatherVec<T, T>{xn, ld}, BEpiSpmm<T>{x, ld, 0, {}});
     for (int q = 0; q < vc.nu; ++q) {
-        launch_bprod<T>(e, L.A.get(), k, BGatherVec<T, T>{x, k}, BEpiJacobi<T>{x, w, b, t, k, {}});
+        launch_bprod<T>(e, L.A.get(), k, BGatherVec<T, T>{x, ld}, BEpiJacobi<T>{x, w, b, t, ld, {}});
         std::swap(x, t);
     }
     return x;
@@ -288,20 +318,23 @@ void multi_solve(dv_mgpcg *s, VCycle<T> &vc, MultiState<T> &M, int k, const doub
     dv_context *ctx = s->ctx;
     cudaStream_t st = ctx->stream;
     const int32_t n = s->n;
-    const size_t nk = (size_t)n * k;
     constexpr bool kMixed = std::is_same<T, float>::value;
+    // rows of the mixed solver's blocks are padded to 16 bytes, which the grid-stencil products copy by; the
+    // padding columns stay zero
+    const int ld = kMixed ? (k + 3) & ~3 : k;
+    const size_t nk = (size_t)n * ld;
     if (M.k != k) {   // (re)size the block buffers
         M = MultiState<T>();
         M.k = k;
         for (auto &L : vc.lv) {
-            const size_t b = sizeof(T) * (size_t)L.n * k;
+            const size_t b = sizeof(T) * (size_t)L.n * ld;
             M.W.x.emplace_back(b);
             M.W.t.emplace_back(b);
             M.W.r.emplace_back(b);
             M.W.b.emplace_back(b);
         }
-        M.W.bc.alloc(sizeof(T) * (size_t)vc.nc * k);
-        M.W.xc.alloc(sizeof(T) * (size_t)vc.nc * k);
+        M.W.bc.alloc(sizeof(T) * (size_t)vc.nc * ld);
+        M.W.xc.alloc(sizeof(T) * (size_t)vc.nc * ld);
         M.B.alloc(8 * nk);
         M.X.alloc(8 * nk);
         M.R.alloc(8 * nk);
@@ -313,8 +346,6 @@ void multi_solve(dv_mgpcg *s, VCycle<T> &vc, MultiState<T> &M, int k, const doub
         M.ws = std::make_unique<SolverWs>(ctx);
     }
     SolverWs &ws = *M.ws;
-    ws.reset_graph();
-    ws.warmed = false;
     dvk::SolverScalars &h = *ws.host_scal;
     std::memset(&h, 0, sizeof(h));
     h.max_it = s->cfg.max_iterations;
@@ -329,9 +360,9 @@ void multi_solve(dv_mgpcg *s, VCycle<T> &vc, MultiState<T> &M, int k, const doub
     const int gw = (int)std::max<int64_t>(1, std::min<int64_t>(((int64_t)n * 32 + 255) / 256,
                                                                 (int64_t)ctx->num_sms * dvb::kReduceBlocksPerSm));
     auto norms = [&](const double *v, int slot) {
-        if (k <= 32) k_bnorm<1><<<gw, dvb::kThreads, 0, st>>>(v, n, k, cs, slot, e0.partials, e0.ticket);
-        else if (k <= 64) k_bnorm<2><<<gw, dvb::kThreads, 0, st>>>(v, n, k, cs, slot, e0.partials, e0.ticket);
-        else k_bnorm<4><<<gw, dvb::kThreads, 0, st>>>(v, n, k, cs, slot, e0.partials, e0.ticket);
+        if (k <= 32) k_bnorm<1><<<gw, dvb::kThreads, 0, st>>>(v, n, k, ld, cs, slot, e0.partials, e0.ticket);
+        else if (k <= 64) k_bnorm<2><<<gw, dvb::kThreads, 0, st>>>(v, n, k, ld, cs, slot, e0.partials, e0.ticket);
+        else k_bnorm<4><<<gw, dvb::kThreads, 0, st>>>(v, n, k, ld, cs, slot, e0.partials, e0.ticket);
         DV_CUDA(cudaGetLastError());
         ctx->count();
     };
@@ -342,7 +373,8 @@ void multi_solve(dv_mgpcg *s, VCycle<T> &vc, MultiState<T> &M, int k, const doub
         c.pq = 1.0;
     }
     DV_CUDA(cudaMemcpyAsync(cs, hc.data(), sizeof(ColScalars) * k, cudaMemcpyHostToDevice, st));
-    DV_CUDA(cudaMemcpyAsync(M.B.p, dB, 8 * nk, cudaMemcpyDeviceToDevice, st));
+    if (ld == k) DV_CUDA(cudaMemcpyAsync(M.B.p, dB, 8 * nk, cudaMemcpyDeviceToDevice, st));
+    else DV_CUDA(cudaMemcpy2DAsync(M.B.p, 8 * (size_t)ld, dB, 8 * (size_t)k, 8 * (size_t)k, n, cudaMemcpyDeviceToDevice, st));
     norms(M.B.template as<double>(), 0);
     DV_CUDA(cudaMemsetAsync(M.X.p, 0, 8 * nk, st));
     DV_CUDA(cudaMemcpyAsync(M.R.p, M.B.p, 8 * nk, cudaMemcpyDeviceToDevice, st));
@@ -358,24 +390,40 @@ void multi_solve(dv_mgpcg *s, VCycle<T> &vc, MultiState<T> &M, int k, const doub
         }
     };
     to_low();
-    const T *z = block_vcycle<T>(ed, vc, M.W, 0, rin, k);
+    const T *z = block_vcycle<T>(ed, vc, M.W, 0, rin, k, ld);
     const int per = s->cfg.iterations_per_sync > 0 ? s->cfg.iterations_per_sync : 4;
     const double tol2 = h.tol2;
     const T *zfinal = z;
     double *Xd = M.X.template as<double>(), *Rd = M.R.template as<double>();
     double *Pd = M.Pv.template as<double>(), *Qd = M.Q.template as<double>();
     auto launch_red = [&](const T *zz) {
-        if (k <= 32) dvk::launch_chain(k_bfcg_red<T, 1>, gw, dvb::kThreads, 0, st, zz, Qd, Rd, n, k, cs, ed.done, ed.partials, ed.ticket);
-        else if (k <= 64) dvk::launch_chain(k_bfcg_red<T, 2>, gw, dvb::kThreads, 0, st, zz, Qd, Rd, n, k, cs, ed.done, ed.partials, ed.ticket);
-        else dvk::launch_chain(k_bfcg_red<T, 4>, gw, dvb::kThreads, 0, st, zz, Qd, Rd, n, k, cs, ed.done, ed.partials, ed.ticket);
+        if (k <= 32) dvk::launch_chain(k_bfcg_red<T, 1>, gw, dvb::kThreads, 0, st, zz, Qd, Rd, n, k, ld, cs, ed.done, ed.partials, ed.ticket);
+        else if (k <= 64) dvk::launch_chain(k_bfcg_red<T, 2>, gw, dvb::kThreads, 0, st, zz, Qd, Rd, n, k, ld, cs, ed.done, ed.partials, ed.ticket);
+        else dvk::launch_chain(k_bfcg_red<T, 4>, gw, dvb::kThreads, 0, st, zz, Qd, Rd, n, k, ld, cs, ed.done, ed.partials, ed.ticket);
+        DV_CUDA(cudaGetLastError());
+        ctx->count();
+    };
+    // q = A z + beta q, p = z + beta p and p.q: on the grid-stencil layout a product without column sums and a
+    // pass over p and q, elsewhere in one
+    const bool grid_outer = kMixed && bgrid_layout(s->Aout.get(), DV_F64, ld);
+    auto launch_outer = [&](const T *zz) {
+        const BGatherVec<T, double> g{zz, ld};
+        if (!grid_outer) {
+            launch_bprod<double, false>(ed, s->Aout.get(), k, g, BEpiFcg<T, true>{zz, Pd, Qd, cs, ld, FinFcg{cs}});
+            return;
+        }
+        launch_bprod<double, false>(ed, s->Aout.get(), k, g, BEpiFcg<T, false>{zz, Pd, Qd, cs, ld, FinFcg{cs}});
+        if (k <= 32) dvk::launch_chain(k_bfcg_pq<1>, gw, dvb::kThreads, 0, st, Pd, Qd, n, k, ld, cs, ed.done, ed.partials, ed.ticket);
+        else if (k <= 64) dvk::launch_chain(k_bfcg_pq<2>, gw, dvb::kThreads, 0, st, Pd, Qd, n, k, ld, cs, ed.done, ed.partials, ed.ticket);
+        else dvk::launch_chain(k_bfcg_pq<4>, gw, dvb::kThreads, 0, st, Pd, Qd, n, k, ld, cs, ed.done, ed.partials, ed.ticket);
         DV_CUDA(cudaGetLastError());
         ctx->count();
     };
     auto launch_update = [&] {
         T *rl = kMixed ? reinterpret_cast<T *>(M.Rlow.p) : nullptr;
-        if (k <= 32) dvk::launch_chain(k_bfcg_update<T, 1>, gw, dvb::kThreads, 0, st, Xd, Rd, rl, Pd, Qd, n, k, cs, tol2, ed.done, ed.partials, ed.ticket);
-        else if (k <= 64) dvk::launch_chain(k_bfcg_update<T, 2>, gw, dvb::kThreads, 0, st, Xd, Rd, rl, Pd, Qd, n, k, cs, tol2, ed.done, ed.partials, ed.ticket);
-        else dvk::launch_chain(k_bfcg_update<T, 4>, gw, dvb::kThreads, 0, st, Xd, Rd, rl, Pd, Qd, n, k, cs, tol2, ed.done, ed.partials, ed.ticket);
+        if (k <= 32) dvk::launch_chain(k_bfcg_update<T, 1>, gw, dvb::kThreads, 0, st, Xd, Rd, rl, Pd, Qd, n, k, ld, cs, tol2, ed.done, ed.partials, ed.ticket);
+        else if (k <= 64) dvk::launch_chain(k_bfcg_update<T, 2>, gw, dvb::kThreads, 0, st, Xd, Rd, rl, Pd, Qd, n, k, ld, cs, tol2, ed.done, ed.partials, ed.ticket);
+        else dvk::launch_chain(k_bfcg_update<T, 4>, gw, dvb::kThreads, 0, st, Xd, Rd, rl, Pd, Qd, n, k, ld, cs, tol2, ed.done, ed.partials, ed.ticket);
         DV_CUDA(cudaGetLastError());
         dvk::launch_chain(k_bfcg_stop, 1, 1, 0, st, cs, k, ws.sc());
         DV_CUDA(cudaGetLastError());
@@ -385,16 +433,15 @@ void multi_solve(dv_mgpcg *s, VCycle<T> &vc, MultiState<T> &M, int k, const doub
         const T *zz = z;
         for (int it = 0; it < per; ++it) {
             launch_red(zz);
-            launch_bprod<double, false>(ed, s->Aout.get(), k, BGatherVec<T, double>{zz, k},
-                                 BEpiFcg<T>{zz, Pd, Qd, cs, k, FinFcg{cs}});
+            launch_outer(zz);
             launch_update();
-            zz = block_vcycle<T>(ed, vc, M.W, 0, rin, k);
+            zz = block_vcycle<T>(ed, vc, M.W, 0, rin, k, ld);
         }
         zfinal = zz;
     };
     auto true_residual = [&] {   // into Pd (free once the recurrence stopped)
-        launch_bprod<double>(e0, s->Aout.get(), k, BGatherVec<double, double>{Xd, k},
-                             BEpiResid<double>{M.B.template as<double>(), Pd, k, {}});
+        launch_bprod<double>(e0, s->Aout.get(), k, BGatherVec<double, double>{Xd, ld},
+                             BEpiResid<double>{M.B.template as<double>(), Pd, ld, {}});
         norms(Pd, 1);
         DV_CUDA(cudaMemcpyAsync(hc.data(), cs, sizeof(ColScalars) * k, cudaMemcpyDeviceToHost, st));
         DV_CUDA(cudaStreamSynchronize(st));
@@ -427,11 +474,12 @@ void multi_solve(dv_mgpcg *s, VCycle<T> &vc, MultiState<T> &M, int k, const doub
         h.done = 0;
         h.converged = 0;
         ws.push();
-        z = block_vcycle<T>(ed, vc, M.W, 0, rin, k);
+        z = block_vcycle<T>(ed, vc, M.W, 0, rin, k, ld);
     }
     // final FP64 true residual of every column (already taken when the loop ended on a verification)
     if (!verified) true_residual();
-    DV_CUDA(cudaMemcpyAsync(dX, Xd, 8 * nk, cudaMemcpyDeviceToDevice, st));
+    if (ld == k) DV_CUDA(cudaMemcpyAsync(dX, Xd, 8 * nk, cudaMemcpyDeviceToDevice, st));
+    else DV_CUDA(cudaMemcpy2DAsync(dX, 8 * (size_t)k, Xd, 8 * (size_t)ld, 8 * (size_t)k, n, cudaMemcpyDeviceToDevice, st));
     DV_CUDA(cudaStreamSynchronize(st));
     double worst = 0.0, worst_abs = 0.0;
     int all = 1;

@@ -113,10 +113,14 @@ struct OpFcgSeg : dvk::NoRed {
     const int32_t *__restrict__ seg_of;
     const MeshScalars *ms;
     __device__ __forceinline__ double init(int32_t) const { return 0.0; }
-    __device__ __forceinline__ void row(int32_t i, double s, double *) const {
-        const double bt = ms[seg_of[i]].beta;
-        q[i] = s + bt * q[i];
-        p[i] = (double)z[i] + bt * p[i];
+    struct In {
+        double bt, q, p;
+        ZT z;
+    };
+    __device__ __forceinline__ In load(int32_t i) const { return {ms[seg_of[i]].beta, q[i], p[i], z[i]}; }
+    __device__ __forceinline__ void store(int32_t i, double s, const In &a, double *) const {
+        q[i] = s + a.bt * a.q;
+        p[i] = (double)a.z + a.bt * a.p;
     }
 };
 

@@ -89,8 +89,10 @@ struct BGatherWB {
 };
 
 // ---------------------------------------------------------------------------
-// epilogues: apply(row, column, row sum, this lane's reduction slots); touch(row, column) prefetches what
-// apply will read, issued by the streaming kernel one plane ahead
+// epilogues: load(row, column) reads what an element needs and store(row, column, row sum, loaded, this
+// lane's reduction slots) finishes it; all rows' loads come before the first store (see the row
+// operators of dv_kernels.cuh).  touch(row, column) prefetches what load will read, issued by the
+// streaming kernel one plane ahead
 // ---------------------------------------------------------------------------
 struct NoFin {
     __device__ void operator()(int, const double *) const {}
@@ -101,9 +103,9 @@ struct BEpiSpmm {   // Y = A X, or Y += A X
     T *y;
     int ld, clear;
     NoFin fin;
-    __device__ __forceinline__ void apply(int32_t i, int j, T s, double *) const {
-        T *p = y + (size_t)i * ld + j;
-        *p = clear ? s : *p + s;
+    __device__ __forceinline__ T load(int32_t i, int j) const { return clear ? T(0) : y[(size_t)i * ld + j]; }
+    __device__ __forceinline__ void store(int32_t i, int j, T s, T y0, double *) const {
+        y[(size_t)i * ld + j] = clear ? s : y0 + s;
     }
     __device__ __forceinline__ void touch(int32_t i, int j) const {
         if (!clear) dvk::prefetch_l1(y + (size_t)i * ld + j);
@@ -116,10 +118,8 @@ struct BEpiResid {   // R = B - A X
     T *r;
     int ld;
     NoFin fin;
-    __device__ __forceinline__ void apply(int32_t i, int j, T s, double *) const {
-        const size_t q = (size_t)i * ld + j;
-        r[q] = b[q] - s;
-    }
+    __device__ __forceinline__ T load(int32_t i, int j) const { return b[(size_t)i * ld + j]; }
+    __device__ __forceinline__ void store(int32_t i, int j, T s, T bi, double *) const { r[(size_t)i * ld + j] = bi - s; }
     __device__ __forceinline__ void touch(int32_t i, int j) const { dvk::prefetch_l1(b + (size_t)i * ld + j); }
 };
 template <class T>
@@ -129,9 +129,15 @@ struct BEpiJacobi {   // Y = X + w (B - A X)
     T *y;
     int ld;
     NoFin fin;
-    __device__ __forceinline__ void apply(int32_t i, int j, T s, double *) const {
+    struct In {
+        T x, w, b;
+    };
+    __device__ __forceinline__ In load(int32_t i, int j) const {
         const size_t q = (size_t)i * ld + j;
-        y[q] = x[q] + w[i] * (b[q] - s);
+        return {x[q], w[i], b[q]};
+    }
+    __device__ __forceinline__ void store(int32_t i, int j, T s, const In &a, double *) const {
+        y[(size_t)i * ld + j] = a.x + a.w * (a.b - s);
     }
     __device__ __forceinline__ void touch(int32_t i, int j) const {
         dvk::prefetch_l1(x + (size_t)i * ld + j);
@@ -145,10 +151,12 @@ struct BEpiJacobiFromZero {   // two sweeps from zero: Y = wB + w (B - A (wB))
     T *y;
     int ld;
     NoFin fin;
-    __device__ __forceinline__ void apply(int32_t i, int j, T s, double *) const {
-        const size_t q = (size_t)i * ld + j;
-        const T wi = w[i], bi = b[q];
-        y[q] = wi * bi + wi * (bi - s);
+    struct In {
+        T w, b;
+    };
+    __device__ __forceinline__ In load(int32_t i, int j) const { return {w[i], b[(size_t)i * ld + j]}; }
+    __device__ __forceinline__ void store(int32_t i, int j, T s, const In &a, double *) const {
+        y[(size_t)i * ld + j] = a.w * a.b + a.w * (a.b - s);
     }
     __device__ __forceinline__ void touch(int32_t i, int j) const { dvk::prefetch_l1(b + (size_t)i * ld + j); }
 };
@@ -195,9 +203,13 @@ __device__ __forceinline__ void group_epilogue(int32_t r0, int kc, int lane, con
 #pragma unroll
     for (int u = 0; u < U; ++u) {
         const int j = lane + 32 * u;
-        if (j < kc)
+        if (j < kc) {
+            decltype(ep.load(0, 0)) in[G];
 #pragma unroll
-            for (int t = 0; t < G; ++t) ep.apply(r0 + t, j, acc[t][u], red[u]);
+            for (int t = 0; t < G; ++t) in[t] = ep.load(r0 + t, j);
+#pragma unroll
+            for (int t = 0; t < G; ++t) ep.store(r0 + t, j, acc[t][u], in[t], red[u]);
+        }
     }
 }
 
@@ -572,8 +584,11 @@ __global__ void __launch_bounds__(kThreads, sizeof(AT) == 8 ? 2 : 3)
 #pragma unroll
                     for (int d = 0; d < 3; ++d) acc[d] = fma(rec[k].v[d], x, acc[d]);
                 }
+                decltype(ep.load(0, 0)) in[3];
 #pragma unroll
-                for (int d = 0; d < 3; ++d) ep.apply(r0 + d, j, acc[d], nored);
+                for (int d = 0; d < 3; ++d) in[d] = ep.load(r0 + d, j);
+#pragma unroll
+                for (int d = 0; d < 3; ++d) ep.store(r0 + d, j, acc[d], in[d], nored);
             }
         }
     } else {
@@ -687,11 +702,21 @@ __global__ void __launch_bounds__(kThreads, sizeof(AT) == 8 ? 2 : 3)
                 if (di && dm && df) step(std::true_type{}, std::true_type{}, std::true_type{});
                 else step(di, dm, df);
                 if (df && j < kc) {
+                    const int32_t r = r_xy + 3 * lxy * (p - 1);
 #pragma unroll
-                    for (int i = 0; i < 4; ++i)
-                        if (act0[i])
+                    for (int h = 0; h < 4; h += 2) {   // two nodes' loads, then their stores
+                        decltype(ep.load(0, 0)) in[2][3];
 #pragma unroll
-                            for (int d = 0; d < 3; ++d) ep.apply(r_xy + 3 * i + d + 3 * lxy * (p - 1), j, a0[i][d], nored);
+                        for (int i = 0; i < 2; ++i)
+                            if (act0[h + i])
+#pragma unroll
+                                for (int d = 0; d < 3; ++d) in[i][d] = ep.load(r + 3 * (h + i) + d, j);
+#pragma unroll
+                        for (int i = 0; i < 2; ++i)
+                            if (act0[h + i])
+#pragma unroll
+                                for (int d = 0; d < 3; ++d) ep.store(r + 3 * (h + i) + d, j, a0[h + i][d], in[i][d], nored);
+                    }
                 }
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
@@ -775,8 +800,11 @@ __global__ void __launch_bounds__(kThreads) k_bprod_tri(dvk::TriGeom G, int kc, 
 #pragma unroll
             for (int d = 0; d < 3; ++d) s[d] = madd<AT>(s[d], w, g(col + d, j));
         });
+        decltype(ep.load(0, 0)) in[3];
 #pragma unroll
-        for (int d = 0; d < 3; ++d) ep.apply((int32_t)(3 * q + d), j, s[d], nullptr);
+        for (int d = 0; d < 3; ++d) in[d] = ep.load((int32_t)(3 * q + d), j);
+#pragma unroll
+        for (int d = 0; d < 3; ++d) ep.store((int32_t)(3 * q + d), j, s[d], in[d], nullptr);
     }
 }
 

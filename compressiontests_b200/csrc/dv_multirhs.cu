@@ -48,11 +48,18 @@ struct BEpiFcg {
     const ColScalars *cs;
     int ld;
     FinFcg fin;
-    __device__ __forceinline__ void apply(int32_t i, int j, double s, double *red) const {
+    struct In {
+        double bt, q, p;
+        ZT z;
+    };
+    __device__ __forceinline__ In load(int32_t i, int j) const {
         const size_t o = (size_t)i * ld + j;
-        const double bt = cs[j].beta;
-        const double qi = s + bt * q[o];
-        const double pi = (double)z[o] + bt * p[o];
+        return {cs[j].beta, q[o], p[o], z[o]};
+    }
+    __device__ __forceinline__ void store(int32_t i, int j, double s, const In &a, double *red) const {
+        const size_t o = (size_t)i * ld + j;
+        const double qi = s + a.bt * a.q;
+        const double pi = (double)a.z + a.bt * a.p;
         q[o] = qi;
         p[o] = pi;
         if constexpr (RED) red[0] += pi * qi;

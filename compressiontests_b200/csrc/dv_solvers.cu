@@ -234,8 +234,9 @@ struct OpPower {
     T *__restrict__ y;
     SolverScalars *sc;
     __device__ __forceinline__ T init(int32_t) const { return T(0); }
-    __device__ __forceinline__ void row(int32_t i, T s, double *red) const {
-        T v = (T)((double)s / diag[i]);
+    __device__ __forceinline__ double load(int32_t i) const { return diag[i]; }
+    __device__ __forceinline__ void store(int32_t i, T s, double d, double *red) const {
+        T v = (T)((double)s / d);
         y[i] = v;
         red[0] += (double)v * (double)v;
     }

@@ -91,8 +91,7 @@ struct BGatherWB {
 // ---------------------------------------------------------------------------
 // epilogues: load(row, column) reads what an element needs and store(row, column, row sum, loaded, this
 // lane's reduction slots) finishes it; all rows' loads come before the first store (see the row
-// operators of dv_kernels.cuh).  touch(row, column) prefetches what load will read, issued by the
-// streaming kernel one plane ahead
+// operators of dv_kernels.cuh).
 // ---------------------------------------------------------------------------
 struct NoFin {
     __device__ void operator()(int, const double *) const {}
@@ -107,9 +106,6 @@ struct BEpiSpmm {   // Y = A X, or Y += A X
     __device__ __forceinline__ void store(int32_t i, int j, T s, T y0, double *) const {
         y[(size_t)i * ld + j] = clear ? s : y0 + s;
     }
-    __device__ __forceinline__ void touch(int32_t i, int j) const {
-        if (!clear) dvk::prefetch_l1(y + (size_t)i * ld + j);
-    }
 };
 template <class T>
 struct BEpiResid {   // R = B - A X
@@ -120,7 +116,6 @@ struct BEpiResid {   // R = B - A X
     NoFin fin;
     __device__ __forceinline__ T load(int32_t i, int j) const { return b[(size_t)i * ld + j]; }
     __device__ __forceinline__ void store(int32_t i, int j, T s, T bi, double *) const { r[(size_t)i * ld + j] = bi - s; }
-    __device__ __forceinline__ void touch(int32_t i, int j) const { dvk::prefetch_l1(b + (size_t)i * ld + j); }
 };
 template <class T>
 struct BEpiJacobi {   // Y = X + w (B - A X)
@@ -139,10 +134,6 @@ struct BEpiJacobi {   // Y = X + w (B - A X)
     __device__ __forceinline__ void store(int32_t i, int j, T s, const In &a, double *) const {
         y[(size_t)i * ld + j] = a.x + a.w * (a.b - s);
     }
-    __device__ __forceinline__ void touch(int32_t i, int j) const {
-        dvk::prefetch_l1(x + (size_t)i * ld + j);
-        dvk::prefetch_l1(b + (size_t)i * ld + j);
-    }
 };
 template <class T>
 struct BEpiJacobiFromZero {   // two sweeps from zero: Y = wB + w (B - A (wB))
@@ -158,7 +149,6 @@ struct BEpiJacobiFromZero {   // two sweeps from zero: Y = wB + w (B - A (wB))
     __device__ __forceinline__ void store(int32_t i, int j, T s, const In &a, double *) const {
         y[(size_t)i * ld + j] = a.w * a.b + a.w * (a.b - s);
     }
-    __device__ __forceinline__ void touch(int32_t i, int j) const { dvk::prefetch_l1(b + (size_t)i * ld + j); }
 };
 
 // ---------------------------------------------------------------------------
@@ -668,9 +658,6 @@ __global__ void __launch_bounds__(kThreads, sizeof(AT) == 8 ? 2 : 3)
                     act2[i] = di && active(i, p + 1);
 #pragma unroll
                     for (int d = 0; d < 3; ++d) a2[i][d] = AT(0);
-                    if (dm && act1[i] && j < kc)   // finished next step
-#pragma unroll
-                        for (int d = 0; d < 3; ++d) ep.touch(r_xy + 3 * i + d + 3 * lxy * p, j);
                 }
                 auto step = [&](auto DI, auto DM, auto DF) {
 #pragma unroll

@@ -64,12 +64,6 @@ struct BEpiFcg {
         p[o] = pi;
         if constexpr (RED) red[0] += pi * qi;
     }
-    __device__ __forceinline__ void touch(int32_t i, int j) const {
-        const size_t o = (size_t)i * ld + j;
-        dvk::prefetch_l1(z + o);
-        dvk::prefetch_l1(p + o);
-        dvk::prefetch_l1(q + o);
-    }
 };
 
 // ---------------------------------------------------------------------------

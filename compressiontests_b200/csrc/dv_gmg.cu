@@ -205,7 +205,7 @@ extern "C" DV_API int dv_gmg_create(dv_context *ctx, int32_t n_levels, const dv_
             L.b.alloc(nb); L.x.alloc(nb); L.t.alloc(nb); L.r.alloc(nb); L.D.alloc(nb);
             if (cfg->smoother != DV_SMOOTHER_JACOBI) {
                 gs_build_order(A[l], cfg->smoother == DV_SMOOTHER_GS_LEX, s, L.gs);
-                gs_prepare_block<double>(L.A.get(), L.gs);
+                gs_prepare_block<double>(L.A.get(), A[l], L.gs);
             }
         }
         // relaxation (GeometricMultigridSolver.cs:209-214 / :109-121 / OpenCLCsrGeometricMultigridSolver.cs:164-171)

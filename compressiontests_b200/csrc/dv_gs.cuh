@@ -226,6 +226,112 @@ __global__ void __launch_bounds__(kGsWarps * 32) k_gs_block(const int32_t *__res
     for (int32_t i = threadIdx.x; i < n; i += kGsWarps * 32) x[i] = xs[i];
 }
 
+// ---------------------------------------------------------------------------
+// The same by node groups: 3 consecutive rows with one column list of at most 96 columns.  A warp takes
+// a node, with a barrier per level of nodes (a third of the rows' levels).  Every product with another
+// node's value is formed at once; lanes 0 .. 2 subtract the three rows' products up to the node's own
+// columns side by side, then row by row the node's own terms (new values of the rows before, old ones
+// of the rows after), the rest of the row and the division: 39 + 3 x 41 subtractions after one
+// another for a hex node instead of 3 x 81, in each row's own order.  The next node's entries are
+// loaded while they run.  12 x 4 x 4 elements, two levels, to 1e-3: 91.9 -> 82.0 ms (3.1 us a level of nodes).
+// ---------------------------------------------------------------------------
+constexpr int kGsCols = 96;          // columns of a node, 3 a lane
+constexpr int kGsStride = kGsCols + 2;   // a row's products in shared memory: the three lanes' loads in different banks
+
+template <class T>
+__global__ void __launch_bounds__(kGsWarps * 32) k_gs_block_nodes(const int32_t *__restrict__ rp, const int32_t *__restrict__ ci,
+                                                                  const T *__restrict__ va, const T *__restrict__ b, T *x,
+                                                                  const int32_t *__restrict__ nodes,
+                                                                  const int32_t *__restrict__ off, int32_t nlevels,
+                                                                  int32_t n, int sweeps, const int *__restrict__ done) {
+    if (chain_done(done)) return;
+    extern __shared__ uint4 gsb_smem[];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    T *prod = reinterpret_cast<T *>(gsb_smem) + warp * (3 * kGsStride + 9);   // this warp's products, own 3 x 3 block
+    T *block = prod + 3 * kGsStride;
+    T *xs = reinterpret_cast<T *>(gsb_smem) + kGsWarps * (3 * kGsStride + 9);
+    for (int32_t i = threadIdx.x; i < n; i += kGsWarps * 32) xs[i] = x[i];
+    const int row = min(lane, 2);
+    struct Node {
+        int32_t node, len, c[3];
+        T v[3][3], b;
+    } q;
+    auto load = [&](int32_t t) {
+        q.node = __ldg(nodes + t);
+        const int32_t s = __ldg(rp + 3 * q.node);
+        q.len = __ldg(rp + 3 * q.node + 1) - s;
+        q.b = b[3 * q.node + row];
+#pragma unroll
+        for (int u = 0; u < 3; ++u) {
+            const int32_t k = lane + 32 * u;
+            q.c[u] = k < q.len ? __ldg(ci + s + k) : 0;
+#pragma unroll
+            for (int d = 0; d < 3; ++d) q.v[u][d] = k < q.len ? __ldg(va + s + d * q.len + k) : T(0);
+        }
+    };
+    const int32_t last = sweeps * nlevels;
+    int32_t t0 = __ldg(off), t1 = __ldg(off + 1);
+    if (t0 + warp < t1) load(t0 + warp);
+    for (int32_t l = 0; l < last; ++l) {
+        __syncthreads();   // the nodes of the level before are in xs
+        int32_t n0 = 0, n1 = 0;   // the next level's nodes
+        if (l + 1 < last) {
+            const int32_t m = (l + 1) % nlevels;
+            n0 = __ldg(off + m);
+            n1 = __ldg(off + m + 1);
+        }
+        for (int32_t t = t0 + warp; t < t1; t += kGsWarps) {
+            const int32_t r0 = 3 * q.node, len = q.len;
+            int first = len, own = 0;   // the node's own columns: position of the first, and which of the three are there
+#pragma unroll
+            for (int u = 0; u < 3; ++u) {
+                const int32_t k = lane + 32 * u, o = q.c[u] - r0;
+                const bool mine = k < len && o >= 0 && o < 3;
+                const unsigned m = __ballot_sync(0xffffffffu, mine);
+                if (m && first == len) first = 32 * u + __ffs(m) - 1;
+#pragma unroll
+                for (int e = 0; e < 3; ++e)
+                    if (__ballot_sync(0xffffffffu, mine && o == e)) own |= 1 << e;
+                const T xv = xs[q.c[u]];
+#pragma unroll
+                for (int d = 0; d < 3; ++d) {
+                    if (mine) block[3 * d + o] = q.v[u][d];
+                    prod[d * kGsStride + k] = mine || k >= len ? T(0) : rn_mul<T>(q.v[u][d], xv);
+                }
+            }
+            T s = q.b;
+            __syncwarp();
+            const bool more = t + kGsWarps < t1;
+            if (more) load(t + kGsWarps);
+            else if (n0 + warp < n1) load(n0 + warp);
+            const T *pr = prod + row * kGsStride;
+            const T *ar = block + 3 * row;
+#pragma unroll 8
+            for (int k = 0; k < first; ++k) s = rn_sub<T>(s, pr[k]);
+            T xn[3] = {xs[r0], xs[r0 + 1], xs[r0 + 2]};   // old values, replaced row by row
+            const int rest = first + __popc(own);
+#pragma unroll
+            for (int d = 0; d < 3; ++d) {   // row d: lane d's result counts
+                T w = s;
+#pragma unroll
+                for (int o = 0; o < 3; ++o)
+                    if (o != d && ((own >> o) & 1)) w = rn_sub<T>(w, rn_mul<T>(ar[o], xn[o]));
+#pragma unroll 8
+                for (int k = rest; k < len; ++k) w = rn_sub<T>(w, pr[k]);
+                w = rn_div<T>(w, (own >> d) & 1 ? block[4 * d] : T(0));
+                xn[d] = __shfl_sync(0xffffffffu, w, d);
+            }
+            if (lane < 3) xs[r0 + lane] = lane == 0 ? xn[0] : lane == 1 ? xn[1] : xn[2];
+            __syncwarp();
+        }
+        if (t0 + warp >= t1 && n0 + warp < n1) load(n0 + warp);   // no node in this level
+        t0 = n0;
+        t1 = n1;
+    }
+    __syncthreads();
+    for (int32_t i = threadIdx.x; i < n; i += kGsWarps * 32) x[i] = xs[i];
+}
+
 // Row groups of one Gauss-Seidel ordering (device rows + host group offsets).
 struct GsOrder {
     DevMem rows;
@@ -233,7 +339,9 @@ struct GsOrder {
     int bs = 1;
     bool lex = false;
     bool block = false;          // swept by one block (k_gs_block): level offsets and, for DuVi, the entries
-    DevMem d_off, col, val;
+    bool nodes = false;          // ... by node groups (k_gs_block_nodes): d_nodes in levels d_off
+    int32_t nlevels = 0;
+    DevMem d_off, d_nodes, col, val;
 };
 
 // Builds the ordering: lex = dependency levels of the forward sweep (rows);
@@ -261,20 +369,33 @@ inline void gs_build_order(const dv_csr_host &a, bool lex, cudaStream_t s, GsOrd
 }
 
 template <class T>
-constexpr size_t gs_block_smem(int32_t n) {
-    return sizeof(T) * ((size_t)n + kGsWarps * 32 * kGsLane);
+constexpr size_t gs_block_smem(int32_t n, bool nodes) {
+    return sizeof(T) * ((size_t)n + kGsWarps * (nodes ? 3 * kGsStride + 9 : 32 * kGsLane));
 }
 
-// Prepares the one-block sweep of A's row-order levels where x fits a block's shared memory (FP64 up
-// to 25,984 rows).  There a level has a few dozen rows and one block is enough for it; a level of a
-// larger system has hundreds to thousands, and every level stays a launch over all SMs.
+// Prepares the one-block sweep of A's row-order levels (a: its host copy) where x fits a block's shared
+// memory (FP64 up to 25,856 rows, by node groups up to 19,352).  There a level has a few dozen rows and
+// one block is enough for it; a level of a larger system has hundreds to thousands, and every level
+// stays a launch over all SMs.
 template <class T>
-void gs_prepare_block(const dv_matrix *A, GsOrder &o) {
+void gs_prepare_block(const dv_matrix *A, const dv_csr_host &a, GsOrder &o) {
     dv_context *ctx = A->ctx;
-    if (!o.lex || A->n_rows == 0 || gs_block_smem<T>(A->n_rows) > (size_t)ctx->max_smem_optin - 1024) return;
+    const size_t room = (size_t)ctx->max_smem_optin - 1024;
+    if (!o.lex || A->n_rows == 0 || gs_block_smem<T>(A->n_rows, false) > room) return;
     cudaStream_t s = ctx->stream;
-    o.d_off.alloc(4 * o.off.size());
-    DV_CUDA(cudaMemcpyAsync(o.d_off.p, o.off.data(), 4 * o.off.size(), cudaMemcpyHostToDevice, s));
+    std::vector<int32_t> perm, off;
+    o.nodes = gs_block_smem<T>(A->n_rows, true) <= room && dv_csr_row_group(a) == 3;
+    for (int32_t i = 0; i < a.n_rows && o.nodes; i += 3) o.nodes = a.rowptr[i + 1] - a.rowptr[i] <= kGsCols;
+    if (o.nodes) {
+        dv_gs_node_level_sets(a, perm, off);
+        o.d_nodes.alloc(4 * perm.size());
+        DV_CUDA(cudaMemcpyAsync(o.d_nodes.p, perm.data(), 4 * perm.size(), cudaMemcpyHostToDevice, s));
+    } else {
+        off = o.off;
+    }
+    o.nlevels = (int32_t)off.size() - 1;
+    o.d_off.alloc(4 * off.size());
+    DV_CUDA(cudaMemcpyAsync(o.d_off.p, off.data(), 4 * off.size(), cudaMemcpyHostToDevice, s));
     if (A->format == DV_FORMAT_DUVI) {
         o.col.alloc(4 * (size_t)A->nnz);
         o.val.alloc(sizeof(T) * (size_t)A->nnz);
@@ -326,13 +447,15 @@ void gs_sweeps(const LaunchEnv &e, const dv_matrix *A, const GsOrder &o, const T
     }
     if (sweeps < 1) return;
     const bool csr = A->format == DV_FORMAT_CSR;
-    const size_t smem = gs_block_smem<T>(A->n_rows);
-    static SmemLimit limit;   // per instantiation and device
-    limit.raise(k_gs_block<T>, smem, e.ctx->device);
-    launch_chain(k_gs_block<T>, 1, kGsWarps * 32, smem, e.stream, 
-        csr ? A->rowptr.as<int32_t>() : A->row_to_dist.as<int32_t>(), csr ? A->col.as<int32_t>() : o.col.as<int32_t>(),
-        csr ? static_cast<const T *>(A->val.p) : o.val.as<T>(), b, x, o.rows.as<int32_t>(), o.d_off.as<int32_t>(),
-        (int32_t)o.off.size() - 1, A->n_rows, sweeps, e.done);
+    const int32_t *rp = csr ? A->rowptr.as<int32_t>() : A->row_to_dist.as<int32_t>();
+    const int32_t *col = csr ? A->col.as<int32_t>() : o.col.as<int32_t>();
+    const T *val = csr ? static_cast<const T *>(A->val.p) : o.val.as<T>();
+    const size_t smem = gs_block_smem<T>(A->n_rows, o.nodes);
+    auto kern = o.nodes ? k_gs_block_nodes<T> : k_gs_block<T>;
+    static SmemLimit limit[2];   // per kernel, instantiation and device
+    limit[o.nodes].raise(kern, smem, e.ctx->device);
+    launch_chain(kern, 1, kGsWarps * 32, smem, e.stream, rp, col, val, b, x, (o.nodes ? o.d_nodes : o.rows).template as<int32_t>(),
+                 o.d_off.as<int32_t>(), o.nlevels, A->n_rows, sweeps, e.done);
     DV_CUDA(cudaGetLastError());
     e.ctx->count();
 }

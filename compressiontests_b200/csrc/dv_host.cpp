@@ -834,21 +834,22 @@ int dv_block_coloring(const dv_csr_host &a, int bs, std::vector<int32_t> &color)
     return ncolors;
 }
 
-int dv_gs_level_sets(const dv_csr_host &a, std::vector<int32_t> &perm, std::vector<int32_t> &offsets) {
-    int32_t n = a.n_rows;
+// Level sets of the forward sweep over n units (rows, or nodes of g rows with one column list): unit i
+// comes after the units j < i it reads, and before the units j > i whose old value it reads (the same
+// units where the structure is symmetric); lev[j] of a later unit holds its bound so far.
+static int level_sets(const dv_csr_host &a, int g, std::vector<int32_t> &perm, std::vector<int32_t> &offsets) {
+    const int32_t n = a.n_rows / g;
     std::vector<int32_t> lev(n, 0);
     int32_t maxl = 0;
-    // row i comes after the rows j < i it reads, and before the rows j > i whose old value it reads (the
-    // same rows where the structure is symmetric); lev[j] of a later row holds its bound so far
     for (int32_t i = 0; i < n; ++i) {
         int32_t l = lev[i];
-        for (int32_t k = a.rowptr[i]; k < a.rowptr[i + 1]; ++k) {
-            int32_t j = a.col[k];
+        for (int32_t k = a.rowptr[g * i]; k < a.rowptr[g * i + 1]; ++k) {
+            int32_t j = a.col[k] / g;
             if (j < i) l = std::max(l, lev[j] + 1);
         }
         lev[i] = l;
-        for (int32_t k = a.rowptr[i]; k < a.rowptr[i + 1]; ++k) {
-            int32_t j = a.col[k];
+        for (int32_t k = a.rowptr[g * i]; k < a.rowptr[g * i + 1]; ++k) {
+            int32_t j = a.col[k] / g;
             if (j > i && j < n) lev[j] = std::max(lev[j], l + 1);
         }
         maxl = std::max(maxl, l);
@@ -860,6 +861,14 @@ int dv_gs_level_sets(const dv_csr_host &a, std::vector<int32_t> &perm, std::vect
     std::vector<int32_t> fill(offsets.begin(), offsets.end() - 1);
     for (int32_t i = 0; i < n; ++i) perm[fill[lev[i]]++] = i;
     return maxl + 1;
+}
+
+int dv_gs_level_sets(const dv_csr_host &a, std::vector<int32_t> &perm, std::vector<int32_t> &offsets) {
+    return level_sets(a, 1, perm, offsets);
+}
+
+int dv_gs_node_level_sets(const dv_csr_host &a, std::vector<int32_t> &perm, std::vector<int32_t> &offsets) {
+    return level_sets(a, 3, perm, offsets);
 }
 
 // ---------------------------------------------------------------------------

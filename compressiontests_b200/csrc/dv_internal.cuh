@@ -333,6 +333,8 @@ void dv_hex_ke(double E, double nu, double *ke);
 int dv_block_coloring(const dv_csr_host &a, int bs, std::vector<int32_t> &color_of_block);
 // Level sets of the forward Gauss-Seidel dependency graph (row i depends on j < i).
 int dv_gs_level_sets(const dv_csr_host &a, std::vector<int32_t> &perm, std::vector<int32_t> &offsets);
+// The same for nodes of 3 rows that share one column list.
+int dv_gs_node_level_sets(const dv_csr_host &a, std::vector<int32_t> &perm, std::vector<int32_t> &offsets);
 
 // Pattern tables (records, starts, bases) of P with the given value table, and the grid-stencil
 // fields of Gd (false when the stencil does not apply to this matrix); pattern ids and the

@@ -504,7 +504,7 @@ static std::unique_ptr<VCycle<T>> build_vcycle(dv_context *ctx, SolverWs &ws, in
         if (l > 0 && cfg.smoother == DV_SMOOTHER_JACOBI && cfg.nu > 1) lv.wb.alloc(vs);
         if (cfg.smoother != DV_SMOOTHER_JACOBI) {
             gs_build_order(A[l], cfg.smoother == DV_SMOOTHER_GS_LEX, s, lv.gs);
-            gs_prepare_block<T>(lv.A.get(), lv.gs);
+            gs_prepare_block<T>(lv.A.get(), A[l], lv.gs);
         }
         k_make_weights<T><<<grid_for(ctx, lv.n), kThreads, 0, s>>>(lv.A->diag.template as<double>(), lv.w.template as<T>(), om, lv.n);
         DV_CUDA(cudaGetLastError());

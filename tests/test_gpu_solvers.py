@@ -406,3 +406,46 @@ def test_gauss_seidel_row_order_sweeps(ctx, native, fmt, n, width):
     got, st, _ = s.Solve()
     np.testing.assert_array_equal(got, x)
     s.ReleaseCudaResources()
+
+
+@pytest.mark.parametrize("fmt", ["csr", "duvi"])
+@pytest.mark.parametrize("nodes,width", [(1, 1), (9, 2), (120, 31), (120, 32), (120, 33), (900, 5), (6600, 3)])
+def test_gauss_seidel_row_order_node_groups(ctx, native, fmt, nodes, width):
+    # The same for node groups of 3 rows with one column list (whole or partial own blocks): lists up to
+    # 96 columns run on the node kernel, longer ones and systems past its shared memory (19,800 rows)
+    # on the row kernel.
+    import scipy.sparse as sp
+    rng = np.random.default_rng(11)
+    n = 3 * nodes
+    indptr, cols, vals = [0], [], []
+    for g in range(nodes):
+        other = rng.choice(nodes, size=min(nodes, width), replace=False)
+        c = np.sort(np.concatenate([np.arange(3 * h, 3 * h + 3) for h in np.union1d(other, [g])]))
+        if width % 2 == 0:
+            c = c[(c // 3 == g) | (c % 3 != 1)]   # other nodes' middle columns missing
+        for d in range(3):
+            v = rng.integers(-8, 9, len(c)) / 16.0
+            v[c == 3 * g + d] = 2.0 * len(c)
+            cols.append(c)
+            vals.append(v)
+            indptr.append(indptr[-1] + len(c))
+    A = sp.csr_matrix((np.concatenate(vals), np.concatenate(cols), indptr), shape=(n, n))
+    R = sp.csr_matrix((np.zeros(1), [0], [0, 1]), shape=(1, n))
+    P = sp.csr_matrix((np.zeros(n), np.zeros(n, int), np.arange(n + 1)), shape=(n, 1))
+    b = rng.standard_normal(n)
+    x = np.zeros(n)
+    for _ in range(2):
+        for i in range(n):
+            c, v = cols[i], vals[i]
+            s = b[i]
+            for k in range(len(c)):
+                if c[k] != i:
+                    s -= v[k] * x[c[k]]
+            x[i] = s / v[c == i][0]
+    cls = native.CudaDuViGeometricMultigridSolver if fmt == "duvi" else native.CudaCsrGeometricMultigridSolver
+    s = cls(ctx, 0, 0.0, [True, False], [1], GaussSeidel=True)
+    s.b = b
+    s.initialize_from_levels([A, sp.identity(1, format="csr")], [R], [P], False)
+    got, st, _ = s.Solve()
+    np.testing.assert_array_equal(got, x)
+    s.ReleaseCudaResources()

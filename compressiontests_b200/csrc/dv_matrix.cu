@@ -368,15 +368,17 @@ void dv_autotune(dv_matrix *m) { autotune(m); }
 
 // The derived DuVi layouts give a node (81 entries) to one thread: right where the operator is too
 // large for the caches, but a small level has too few nodes to hide 81 dependent steps.  Its products
-// run on the decoded entries instead, as long as those stay in the 126 MB L2 cache beside the vectors:
-// node groups a warp each (k_csr_nodes), the short rows of the transfers a thread each, in the stored
-// order (so that they equal the matrix-free transfers).  Only operators that a solver built for itself:
-// the order of a node group's sums is not the stored one.  Measured with against without: solve of 12
-// uneven meshes 3.43 -> 2.53 ms, adjoint pair 48x24x24 10.4 -> 6.6 ms, mixed solve 16^3 1.31 -> 0.99 ms
-// (a 12,168-row level's sweep 25.7 us on the lane layout, 16 blocks).
+// run on the decoded entries instead: node groups a warp each (k_csr_nodes), the short rows of the
+// transfers a thread each, in the stored order (so that they equal the matrix-free transfers).  Only
+// operators that a solver built for itself: the order of a node group's sums is not the stored one.
+// Measured with against without: solve of 12 uneven meshes 3.43 -> 2.53 ms, adjoint pair 48x24x24 10.4
+// -> 6.6 ms, mixed solve 16^3 1.31 -> 0.99 ms (a 12,168-row level's sweep 25.7 us on the lane layout, 16
+// blocks).  The line against the grid stencil, by mixed and FP64 solves: 6.0 and 9.4 MB of entries (16^3
+// in FP32 and FP64) gain 12 and 16 %, 20 MB (24^3 in FP32) lose 14 %; the other layouts are further behind
+// and give way as long as the entries stay in the 126 MB L2 cache beside the vectors.
 // DV_ENTRIES=<MB> moves the line (0: never; A/B comparisons).
 void dv_use_entries(dv_matrix *m) {
-    int64_t limit = 32ll << 20;
+    int64_t limit = (m->duvi_variant == 3 ? 12ll : 48ll) << 20;
     if (const char *v = getenv("DV_ENTRIES")) limit = atoll(v) << 20;
     if (m->format != DV_FORMAT_DUVI || m->entries_ok || m->n_rows == 0) return;
     const int64_t vs = m->precision == DV_F64 ? 8 : 4;

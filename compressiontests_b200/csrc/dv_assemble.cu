@@ -211,11 +211,13 @@ dv_matrix *dv_hex_operator_build(dv_context *ctx, int32_t nmesh, const int32_t *
         plane_tiles_all += (int64_t)h.ntx * h.nty;
     }
     DV_REQUIRE(rows < INT32_MAX, DV_ERR_ARG, "operator exceeds int32 rows");
-    // run length from the waves x steps model: of the mesh, or of all meshes' tiles at their mean height
+    // run length by the waves it leaves: of the mesh, or of all meshes' tiles at their mean height (128^3 FP64
+    // product 76.4 -> 70.4 us, adjoint pair 48 x 24 x 24 7.30 -> 7.04 ms: runs of a power of two left the last wave
+    // nearly empty)
     const int64_t conc = (int64_t)ctx->num_sms * (precision == DV_F64 ? 2 : 3);
     int64_t tall = 0;
     for (auto &h : meshes) tall += (int64_t)h.ntx * h.nty * (h.ne2 + 1);
-    const int run = stream_run_length(plane_tiles_all, (int)std::max<int64_t>(1, tall / plane_tiles_all), conc);
+    const int run = grid_run_length(plane_tiles_all, (int)std::max<int64_t>(1, tall / plane_tiles_all), conc, 0);
     for (auto &h : meshes) {
         h.zc = run;
         h.tile0 = (int32_t)tiles;

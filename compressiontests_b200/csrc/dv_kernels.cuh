@@ -1161,15 +1161,15 @@ __host__ __device__ __forceinline__ constexpr int hex_class(int i) {
 
 constexpr int kGridTX = 32, kGridTY = 8;   // tile of groups per block: one warp per row (of NY rows each)
 constexpr int kGridPX = kGridTX + 2;       // with halo
+constexpr int kGridPitch = 104;            // staged values of a tile row: 3 x 34, padded to whole 16-byte copies
 template <int NY>
 struct PlaneDims {
     static constexpr int TY = kGridTY * NY;             // tile rows
     static constexpr int PY = TY + 2;                   // with halo
-    static constexpr int PLANE = kGridPX * PY * 3;      // staged values per plane
+    static constexpr int PLANE = kGridPitch * PY;       // staged values per plane
     static constexpr int LOADS = (PLANE + 255) / 256;   // staging slots per thread
 };
-constexpr int kGridPlane = PlaneDims<1>::PLANE;   // 1020
-constexpr int kGridLoads = PlaneDims<1>::LOADS;   // 4
+constexpr int kGridPlane = PlaneDims<1>::PLANE;   // 1040
 
 template <class AT>
 struct GridCoef {
@@ -1209,6 +1209,12 @@ __device__ __forceinline__ void cp_async_zfill(void *dst, const void *src, bool 
     asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;\n" ::"r"(d), "l"(src), "n"(BYTES), "r"(valid ? BYTES : 0)
                  : "memory");
 }
+// 16 bytes, of which the first `bytes` are read and the rest zero; through the L1 cache (.ca), where an epilogue
+// that reads x at its own rows finds it again
+__device__ __forceinline__ void cp_async_part16(void *dst, const void *src, int bytes) {
+    const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 16, %2;\n" ::"r"(d), "l"(src), "r"(bytes) : "memory");
+}
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 template <int N>
 __device__ __forceinline__ void cp_async_wait() {
@@ -1238,50 +1244,83 @@ struct StageSrc<GatherWB<T>> {
 };
 constexpr int kGridStages = 4;   // staged planes in flight per block (a plane is consumed 3 steps after its copy)
 
-// Staging slots of a thread: plane value k = threadIdx.x + 256 j is node (sx, sy) of the halo tile
-// (offsets from the tile's first node), dof sc; sy = -1000000 past the plane.
-template <int NY = 1>
+// Staging of a thread: values k = threadIdx.x + 256 j of the plane (row k / kGridPitch, x-dof k % kGridPitch) ...
+template <int NY, class ST, bool VEC>
 struct StageSlots {
-    static constexpr int LOADS = PlaneDims<NY>::LOADS, PLANE = PlaneDims<NY>::PLANE;
-    int sx[LOADS], sy[LOADS], sc[LOADS];
-    __device__ StageSlots() {
+    static constexpr int PLANE = PlaneDims<NY>::PLANE;
+    static constexpr int LOADS = PlaneDims<NY>::LOADS;
+    int32_t poff[LOADS];   // offset in a plane of the lx x ly node box (-1: outside the box, -2: past the plane)
+    __device__ void plane_offsets(int x0, int y0, int lx, int ly) {
 #pragma unroll
         for (int j = 0; j < LOADS; ++j) {
-            const int k = threadIdx.x + 256 * j;
-            const int row = k / (kGridPX * 3), col = k - row * (kGridPX * 3);
-            sx[j] = col / 3 - 1;
-            sc[j] = col - 3 * (col / 3);
-            sy[j] = k < PLANE ? row - 1 : -1000000;
-        }
-    }
-    // per tile: offset of each slot inside a plane of the lx x ly node box (-1: outside the box)
-    __device__ void plane_offsets(int x0, int y0, int lx, int ly, int32_t (&poff)[LOADS]) const {
-#pragma unroll
-        for (int j = 0; j < LOADS; ++j) {
-            const int xn = x0 + sx[j], yn = y0 + sy[j];
-            poff[j] = (xn >= 0 && xn < lx && yn >= 0 && yn < ly) ? 3 * (xn + lx * yn) + sc[j] : -1;
+            const int k = threadIdx.x + 256 * j, row = k / kGridPitch, col = 3 * (x0 - 1) + k - kGridPitch * row;
+            const int yn = y0 - 1 + row;
+            poff[j] = k >= PLANE ? -2 : yn >= 0 && yn < ly && col >= 0 && col < 3 * lx ? 3 * lx * yn + col : -1;
         }
     }
     // copies plane z (zero outside 0 <= z < lz) of every source of the gather into one ring slot
     template <class SS, class Gather>
-    __device__ void issue(const Gather &g, typename SS::ST *slot, const int32_t (&poff)[LOADS], int z, int lz,
-                          int32_t plane_len, int64_t origin = 0) const {
+    __device__ void issue(const Gather &g, ST *slot, int z, int lz, int32_t plane_len) const {
         const bool zin = z >= 0 && z < lz;
-        const int64_t base = zin ? origin + (int64_t)z * plane_len : 0;
+        const int64_t base = zin ? (int64_t)z * plane_len : 0;
 #pragma unroll
         for (int k = 0; k < SS::N; ++k) {
-            const typename SS::ST *src = SS::src(g, k);
+            const ST *src = SS::src(g, k);
 #pragma unroll
             for (int j = 0; j < LOADS; ++j)
-                if (sy[j] > -2) {
+                if (poff[j] > -2) {
                     const bool v = zin && poff[j] >= 0;
-                    cp_async_zfill<sizeof(typename SS::ST)>(slot + k * PLANE + threadIdx.x + 256 * j,
-                                                            v ? src + base + poff[j] : src, v);
+                    cp_async_zfill<sizeof(ST)>(slot + k * PLANE + threadIdx.x + 256 * j, v ? src + base + poff[j] : src, v);
                 }
         }
         cp_async_commit();
     }
 };
+// ... or, where every row of an FP32 vector starts on a 16-byte boundary (an lx that is a multiple of 4), the
+// 16-byte pieces k = threadIdx.x + 256 j: two copies a thread and plane instead of eight
+// (FP32 residual 128^3 36.2 -> 33.6 us, mixed solve 6.78 -> 6.58 ms).
+template <int NY, class ST>
+struct StageSlots<NY, ST, true> {
+    static constexpr int PLANE = PlaneDims<NY>::PLANE;
+    static constexpr int E = 16 / (int)sizeof(ST);
+    static constexpr int LOADS = (PLANE / E + 255) / 256;
+    int32_t poff[LOADS], bytes[LOADS];   // bytes: of the piece, inside the box's row
+    __device__ void plane_offsets(int x0, int y0, int lx, int ly) {
+#pragma unroll
+        for (int j = 0; j < LOADS; ++j) {
+            const int k = E * (threadIdx.x + 256 * j), row = k / kGridPitch, col = 3 * (x0 - 1) + k - kGridPitch * row;
+            const int yn = y0 - 1 + row, have = max(0, min(E, 3 * lx - col));
+            poff[j] = k >= PLANE ? -2 : yn >= 0 && yn < ly && have > 0 ? 3 * lx * yn + col : -1;
+            bytes[j] = have * (int)sizeof(ST);
+        }
+    }
+    template <class SS, class Gather>
+    __device__ void issue(const Gather &g, ST *slot, int z, int lz, int32_t plane_len) const {
+        const bool zin = z >= 0 && z < lz;
+        const int64_t base = zin ? (int64_t)z * plane_len : 0;
+#pragma unroll
+        for (int k = 0; k < SS::N; ++k) {
+            const ST *src = SS::src(g, k);
+#pragma unroll
+            for (int j = 0; j < LOADS; ++j)
+                if (poff[j] > -2) {
+                    const bool v = zin && poff[j] >= 0;
+                    cp_async_part16(slot + k * PLANE + E * (threadIdx.x + 256 * j), v ? src + base + poff[j] : src,
+                                    v ? bytes[j] : 0);
+                }
+        }
+        cp_async_commit();
+    }
+};
+// Whether every row of a gather's sources starts on a 16-byte boundary (host).
+template <class ST>
+inline bool rows_aligned16(const ST *p, int32_t lx) {
+    return (reinterpret_cast<uintptr_t>(p) & 15) == 0 && (3 * (int64_t)lx * (int64_t)sizeof(ST)) % 16 == 0;
+}
+template <class XT, class AT>
+inline bool stage_aligned16(const GatherVec<XT, AT> &g, int32_t lx) { return rows_aligned16(g.x, lx); }
+template <class T>
+inline bool stage_aligned16(const GatherWB<T> &g, int32_t lx) { return rows_aligned16(g.w, lx) && rows_aligned16(g.b, lx); }
 
 // One staged plane applied to the three accumulated groups of each of the thread's NY nodes
 // (rows q = 0 .. NY-1 of its column of the tile): below (DI: group p+1 takes the plane as its
@@ -1298,7 +1337,7 @@ __device__ __forceinline__ void grid_plane_step(const typename SS::ST *__restric
         for (int dx = 0; dx < 3; ++dx)
 #pragma unroll
             for (int c = 0; c < 3; ++c) {
-                const AT v = SS::template value<PLANE>(pl, ((NY * ty + r) * kGridPX + tx + dx) * 3 + c);
+                const AT v = SS::template value<PLANE>(pl, (NY * ty + r) * kGridPitch + (tx + dx) * 3 + c);
 #pragma unroll
                 for (int q = 0; q < NY; ++q) {
                     const int dy = r - q;
@@ -1314,7 +1353,7 @@ __device__ __forceinline__ void grid_plane_step(const typename SS::ST *__restric
             }
 }
 
-template <class AT, class Gather, class Op, bool HEX, int NY>
+template <class AT, class Gather, class Op, bool HEX, int NY, bool VEC>
 __global__ void __launch_bounds__(256, 3)   // 3 blocks an SM: FP64 fits 80 registers without spills
     k_duvi_grid(GridGeom G, GridCoef<AT> cf, const uint16_t *__restrict__ pid, const uint32_t *__restrict__ pstart,
                 const PatRec<AT> *__restrict__ grec, const uint32_t *__restrict__ bnode, int32_t npat, int32_t nrec,
@@ -1340,11 +1379,11 @@ __global__ void __launch_bounds__(256, 3)   // 3 blocks an SM: FP64 fits 80 regi
         if (chain_done(done)) return;
         using SS = StageSrc<Gather>;
         using ST = typename SS::ST;
-        using SL = StageSlots<NY>;
+        using SL = StageSlots<NY, ST, VEC>;
         constexpr int SLOT = SS::N * SL::PLANE;
         ST *ring = reinterpret_cast<ST *>(grid_smem);   // kGridStages slots of SS::N staged planes
         const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-        const SL slots;
+        SL slots;
         const int64_t lxy = (int64_t)G.lx * G.ly;
         const int32_t plane_len = (int32_t)(3 * lxy);
         for (int t = (int)blockIdx.x; t < G.ntile; t += G.tile_blocks) {
@@ -1361,8 +1400,7 @@ __global__ void __launch_bounds__(256, 3)   // 3 blocks an SM: FP64 fits 80 regi
                 col_xy[q] = ix + G.lx * iy;
                 inxy[q] = ix >= 1 && ix <= G.lx - 2 && iy >= 1 && iy <= G.ly - 2;
             }
-            int32_t poff[SL::LOADS];
-            slots.plane_offsets(x0, y0, G.lx, G.ly, poff);
+            slots.plane_offsets(x0, y0, G.lx, G.ly);
             // a stencil group (off the faces, interior pattern) that this thread finishes
             auto active = [&](int q, int z) {
                 if (!inxy[q] || z < 1 || z > G.lz - 2) return false;
@@ -1370,7 +1408,7 @@ __global__ void __launch_bounds__(256, 3)   // 3 blocks an SM: FP64 fits 80 regi
             };
 #pragma unroll
             for (int s2 = 0; s2 < kGridStages - 1; ++s2) {
-                if (z0 - 1 + s2 <= z1) slots.template issue<SS>(g, ring + s2 * SLOT, poff, z0 - 1 + s2, G.lz, plane_len);
+                if (z0 - 1 + s2 <= z1) slots.template issue<SS>(g, ring + s2 * SLOT, z0 - 1 + s2, G.lz, plane_len);
                 else cp_async_commit();
             }
             AT a0[NY][3], a1[NY][3], a2[NY][3];
@@ -1385,8 +1423,8 @@ __global__ void __launch_bounds__(256, 3)   // 3 blocks an SM: FP64 fits 80 regi
                 cp_async_wait<kGridStages - 2>();   // plane p has landed (this thread's copies)
                 __syncthreads();                     // ... and everyone's; the slot of plane p-1 is free
                 if (p + kGridStages - 1 <= z1)
-                    slots.template issue<SS>(g, ring + ((k + kGridStages - 1) % kGridStages) * SLOT, poff,
-                                             p + kGridStages - 1, G.lz, plane_len);
+                    slots.template issue<SS>(g, ring + ((k + kGridStages - 1) % kGridStages) * SLOT, p + kGridStages - 1,
+                                             G.lz, plane_len);
                 else
                     cp_async_commit();
                 const ST *pl = ring + (k % kGridStages) * SLOT;
@@ -1466,12 +1504,12 @@ inline int grid_run_length(int64_t plane_tiles, int lz, int64_t wave, int64_t bo
 }
 
 // Grid-stencil launch: tile blocks over runs of zc planes, then the boundary blocks.
-template <class AT, class Gather, class Op, bool HEX>
+template <class AT, class Gather, class Op, bool HEX, bool VEC>
 void launch_duvi_grid_h(const LaunchEnv &e, const dv_matrix *m, Gather g, Op op) {
     // FP32: two nodes per thread in y (staged rows shared, per-step work amortised); FP64: one
     // (registers)
     constexpr int NY = sizeof(AT) == 4 ? 2 : 1;
-    auto kern = k_duvi_grid<AT, Gather, Op, HEX, NY>;
+    auto kern = k_duvi_grid<AT, Gather, Op, HEX, NY, VEC>;
     using SS = StageSrc<Gather>;
     const size_t smem = std::max(sizeof(typename SS::ST) * SS::N * kGridStages * (size_t)PlaneDims<NY>::PLANE,
                                  sizeof(PatRec<AT>) * (size_t)m->pat_entries + 4 * ((size_t)m->pat_count + 1));
@@ -1541,8 +1579,15 @@ void launch_duvi_pattern_g(const LaunchEnv &e, const dv_matrix *m, Gather g, Op 
 // not set for them); the fallback below only guards against a stale variant.
 template <class AT, class Gather, class Op>
 void launch_duvi_grid(const LaunchEnv &e, const dv_matrix *m, Gather g, Op op) {
-    if (m->grid_hex) launch_duvi_grid_h<AT, Gather, Op, true>(e, m, g, op);
-    else if constexpr (sizeof(AT) == 4) launch_duvi_grid_h<AT, Gather, Op, false>(e, m, g, op);
+    if (m->grid_hex) {
+        if constexpr (sizeof(typename StageSrc<Gather>::ST) == 4) {
+            if (stage_aligned16(g, m->grid_lx)) {
+                launch_duvi_grid_h<AT, Gather, Op, true, true>(e, m, g, op);
+                return;
+            }
+        }
+        launch_duvi_grid_h<AT, Gather, Op, true, false>(e, m, g, op);
+    } else if constexpr (sizeof(AT) == 4) launch_duvi_grid_h<AT, Gather, Op, false, false>(e, m, g, op);
     else launch_duvi_pattern_g<AT, Gather, Op, 3>(e, m, g, op);
 }
 

@@ -511,3 +511,34 @@ def test_matrix_free_hex_operator_tiles(ctx, native, rng, ne):
     for prec, bar, dt in (("f64", REL64, np.float64), ("f32", REL32, np.float32)):
         H = native.SparseMatrix.hex_operator(ctx, ne, E, precision=prec)
         assert rowwise_rel(_device_product(ctx, H, x, dt).astype(np.float64), A @ x, A, x) <= bar
+
+
+@pytest.mark.parametrize("ne", [(32, 9, 7), (36, 20, 6), (35, 9, 7), (64, 18, 9), (100, 5, 5)])
+def test_grid_stencil_f32_row_alignment(ctx, native, rng, ne, monkeypatch):
+    # FP32 planes are staged in 16-byte copies where every row of the node box starts on a 16-byte boundary
+    # (node counts in x that are multiples of 4, an aligned vector) and value by value elsewhere: both give
+    # the node-pattern kernel's floats, also for r = b - A x, at tiles cut off in x and y.
+    import torch
+    monkeypatch.setenv("DV_AUTOTUNE", "0")
+    A = native.hex_stiffness(ne, scale=2.0)
+    n = A.shape[0]
+    monkeypatch.setenv("DV_GRID", "0")
+    P = native.SparseMatrix(ctx, A, "duvi", "f32")
+    monkeypatch.setenv("DV_GRID", "1")
+    G = native.SparseMatrix(ctx, A, "duvi", "f32")
+    assert (P.info()["kernel_variant"], G.info()["kernel_variant"]) == (203, 303)
+    x, b = (torch.from_numpy(rng.standard_normal(n).astype(np.float32)).cuda() for _ in range(2))
+    out = []
+    for M in (P, G):
+        for shift in (0, 1, 4):   # elements past a 256-byte boundary
+            bx = torch.full((n + 8,), float("nan"), dtype=torch.float32, device="cuda")
+            bx[shift:shift + n] = x
+            y, r = torch.empty_like(x), torch.empty_like(x)
+            torch.cuda.synchronize()
+            M.multiply_device(bx.data_ptr() + 4 * shift, y.data_ptr(), "f32")
+            M.residual_device(b.data_ptr(), bx.data_ptr() + 4 * shift, r.data_ptr(), "f32")
+            ctx.synchronize()
+            out.append((y.cpu().numpy(), r.cpu().numpy()))
+    for y, r in out[1:]:
+        np.testing.assert_array_equal(y, out[0][0])
+        np.testing.assert_array_equal(r, out[0][1])

@@ -488,8 +488,8 @@ void launch_bprod_pattern(const LaunchEnv &e, const dv_matrix *m, int kc, Gather
 // block owns a tile of 8 x 4 interior nodes of a plane, streams a run of z planes and covers 32
 // right-hand sides (lane = column).  Each plane of the tile with its one-node halo (10 x 6 nodes, 3
 // dofs, 32 columns: 180 rows of 128 bytes) is copied into a ring of shared-memory slots with 16-byte
-// cp.async copies, two planes ahead; warp w takes the 4 nodes x = 4 (w % 2) .. +3 of tile row w / 2
-// and applies every staged value of the plane to the nodes it couples in z - 1, z and z + 1 (the
+// cp.async copies, two planes ahead; a warp takes two neighbouring nodes of a tile row and applies
+// every staged value of the plane to the nodes it couples in z - 1, z and z + 1 (the
 // streaming accumulators of k_duvi_grid) with the hex stencil's class values.  Each row sums its
 // terms in column order with one multiply-add each, as the pattern kernel does (the stencil's
 // structural zeros skipped: they add exact zeros).  Face groups and interior groups of other patterns
@@ -508,7 +508,12 @@ constexpr int kBgHX = kBgTX + 2, kBgHY = kBgTY + 2;      // with the halo
 constexpr int kBgRows = kBgHX * kBgHY * 3;               // staged rows of a plane (node dofs)
 constexpr int kBgStages = 3;
 constexpr int kBgSlot = kBgRows * 32 + kBgRows;          // floats of a slot: the rows, then w (Jacobi from zero)
-constexpr int kBgCopies = (kBgRows * 8 + kThreads - 1) / kThreads;   // 16-byte copies per thread and plane
+// Nodes in x a warp takes, in blocks of 16 warps (FP32: two an SM at 64 registers, FP64: one at 128).  With 4 a warp
+// reads the staged rows of 4.5 neighbours a node instead of 6, but in FP32 24 warps an SM hide less of the
+// epilogues' loads than 32 do, and in FP64 the sums of 4 nodes spill (424 bytes a thread): 64 load cases on
+// 48^3 29.0 ms with 4, 27.4 with 2 in FP32 alone, 26.1 with 2 in both.
+constexpr int kBgNX = 2;
+constexpr int kBgThreads = 32 * kBgTX * kBgTY / kBgNX;
 
 struct BGridGeom {
     int32_t lx, ly, lz, ntx, nty, zc, ntile, hot, all_hot;
@@ -536,12 +541,14 @@ struct BGridSrc<BGatherWB<float>> {
 };
 
 template <class AT, class Gather, class Epi>
-__global__ void __launch_bounds__(kThreads, sizeof(AT) == 8 ? 2 : 3)
+__global__ void __launch_bounds__(kBgThreads, sizeof(AT) == 8 ? 1 : 2)
     k_bprod_grid(BGridGeom G, BGridCoef<AT> cf, const uint16_t *__restrict__ pid, const uint32_t *__restrict__ pstart,
                  const dvk::PatRec<AT> *__restrict__ grec, const uint32_t *__restrict__ bnode, int32_t npat, int32_t nrec,
                  const float *__restrict__ X, int ld, int kc, Gather g, Epi ep, const int *__restrict__ done) {
     static_assert(Epi::NC == 0, "column reductions run on the other kernels");
     extern __shared__ uint4 bgrid_smem[];
+    constexpr int NX = kBgNX, THREADS = kBgThreads, WARPS = THREADS / 32;
+    constexpr int COPIES = (kBgRows * 8 + THREADS - 1) / THREADS;   // 16-byte copies per thread and plane
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int j0 = blockIdx.y * 32, j = j0 + lane;
     double nored[1];
@@ -552,8 +559,8 @@ __global__ void __launch_bounds__(kThreads, sizeof(AT) == 8 ? 2 : 3)
         dvk::stage_patterns<AT>(bgrid_smem, grec, pstart, npat, nrec);
         if (dvk::chain_done(done)) return;
         __syncthreads();
-        const int32_t nw = ((int32_t)gridDim.x - G.tile_blocks) * kWarps;
-        for (int32_t i = ((int32_t)blockIdx.x - G.tile_blocks) * kWarps + warp; i < G.nbound; i += nw) {
+        const int32_t nw = ((int32_t)gridDim.x - G.tile_blocks) * WARPS;
+        for (int32_t i = ((int32_t)blockIdx.x - G.tile_blocks) * WARPS + warp; i < G.nbound; i += nw) {
             const int32_t r0 = 3 * (int32_t)__ldg(bnode + i);
             const uint32_t p = __ldg(pid + r0 / 3);
             AT acc[3] = {AT(0), AT(0), AT(0)};
@@ -584,26 +591,26 @@ __global__ void __launch_bounds__(kThreads, sizeof(AT) == 8 ? 2 : 3)
     } else {
         if (dvk::chain_done(done)) return;
         float *ring = reinterpret_cast<float *>(bgrid_smem);
-        const int yw = warp >> 1, xs = (warp & 1) * 4;   // the warp's 4 nodes: tile x xs .. xs+3, tile row yw
+        const int yw = warp / (kBgTX / NX), xs = (warp % (kBgTX / NX)) * NX;   // the warp's nodes: tile x xs .., tile row yw
         const int32_t lxy = G.lx * G.ly;
         constexpr bool WB = BGridSrc<Gather>::WB;
         for (int t = blockIdx.x; t < G.ntile; t += G.tile_blocks) {
             const int txi = t % G.ntx, tyi = (t / G.ntx) % G.nty, tzi = t / (G.ntx * G.nty);
             const int x0 = 1 + txi * kBgTX, y0 = 1 + tyi * kBgTY, z0 = 1 + tzi * G.zc, z1 = min(G.lz - 1, z0 + G.zc);
             const int gy = y0 + yw;
-            bool inxy[4];
+            bool inxy[NX];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) inxy[i] = x0 + xs + i <= G.lx - 2 && gy <= G.ly - 2;
+            for (int i = 0; i < NX; ++i) inxy[i] = x0 + xs + i <= G.lx - 2 && gy <= G.ly - 2;
             auto active = [&](int i, int z) {
                 if (!inxy[i] || z < 1 || z > G.lz - 2) return false;
                 return G.all_hot || (int)__ldg(pid + (x0 + xs + i) + G.lx * gy + (int64_t)lxy * z) == G.hot;
             };
             // this thread's copies of a plane: row of the plane (-1: zero, -2: none); columns 4 (c % 8) .. +3
-            int32_t prow[kBgCopies], wrow = -2;
+            int32_t prow[COPIES], wrow = -2;
             const int sub = threadIdx.x & 7;
 #pragma unroll
-            for (int q = 0; q < kBgCopies; ++q) {
-                const int row = (threadIdx.x + kThreads * q) >> 3, hn = row / 3;
+            for (int q = 0; q < COPIES; ++q) {
+                const int row = (threadIdx.x + THREADS * q) >> 3, hn = row / 3;
                 const int gx = x0 - 1 + hn % kBgHX, hy = y0 - 1 + hn / kBgHX;
                 prow[q] = row >= kBgRows ? -2
                           : gx >= 0 && gx < G.lx && hy >= 0 && hy < G.ly && j0 + 4 * sub < kc ? 3 * (gx + G.lx * hy) + row - 3 * hn
@@ -620,10 +627,10 @@ __global__ void __launch_bounds__(kThreads, sizeof(AT) == 8 ? 2 : 3)
                 float *slot = ring + (k % kBgStages) * kBgSlot;
                 const float *src = X + base * ld + j0 + 4 * sub;
 #pragma unroll
-                for (int q = 0; q < kBgCopies; ++q)
+                for (int q = 0; q < COPIES; ++q)
                     if (prow[q] > -2) {
                         const bool v = zin && prow[q] >= 0;
-                        dvk::cp_async_zfill<16>(slot + (threadIdx.x + kThreads * q) * 4, v ? src + (int64_t)prow[q] * ld : X, v);
+                        dvk::cp_async_zfill<16>(slot + (threadIdx.x + THREADS * q) * 4, v ? src + (int64_t)prow[q] * ld : X, v);
                     }
                 if constexpr (WB)
                     if (wrow > -2) {
@@ -636,10 +643,10 @@ __global__ void __launch_bounds__(kThreads, sizeof(AT) == 8 ? 2 : 3)
             issue(z0 - 1, 0);
             if (z0 <= z1) issue(z0, 1);
             else dvk::cp_async_commit();
-            AT a0[4][3], a1[4][3], a2[4][3];
-            bool act0[4], act1[4];
+            AT a0[NX][3], a1[NX][3], a2[NX][3];
+            bool act0[NX], act1[NX];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
+            for (int i = 0; i < NX; ++i) {
                 act0[i] = act1[i] = false;
 #pragma unroll
                 for (int d = 0; d < 3; ++d) a0[i][d] = a1[i][d] = a2[i][d] = AT(0);
@@ -652,9 +659,9 @@ __global__ void __launch_bounds__(kThreads, sizeof(AT) == 8 ? 2 : 3)
                 else dvk::cp_async_commit();
                 const float *pl = ring + (k % kBgStages) * kBgSlot;
                 const bool di = p + 1 >= z0 && p + 1 < z1, dm = p >= z0 && p < z1, df = p - 1 >= z0 && p - 1 < z1;
-                bool act2[4];
+                bool act2[NX];
 #pragma unroll
-                for (int i = 0; i < 4; ++i) {
+                for (int i = 0; i < NX; ++i) {
                     act2[i] = di && active(i, p + 1);
 #pragma unroll
                     for (int d = 0; d < 3; ++d) a2[i][d] = AT(0);
@@ -663,7 +670,7 @@ __global__ void __launch_bounds__(kThreads, sizeof(AT) == 8 ? 2 : 3)
 #pragma unroll
                     for (int dy = 0; dy < 3; ++dy)
 #pragma unroll
-                        for (int hx = 0; hx < 6; ++hx)
+                        for (int hx = 0; hx < NX + 2; ++hx)
 #pragma unroll
                             for (int c = 0; c < 3; ++c) {
                                 const int row = ((yw + dy) * kBgHX + xs + hx) * 3 + c;
@@ -671,7 +678,7 @@ __global__ void __launch_bounds__(kThreads, sizeof(AT) == 8 ? 2 : 3)
                                 if constexpr (WB) f = pl[kBgRows * 32 + row] * f;
                                 const AT v = (AT)f;
 #pragma unroll
-                                for (int i = 0; i < 4; ++i) {
+                                for (int i = 0; i < NX; ++i) {
                                     const int dx = hx - i;   // neighbour offset + 1
                                     if (dx < 0 || dx > 2) continue;
                                     const int e = 9 * dy + 3 * dx + c;
@@ -690,23 +697,20 @@ __global__ void __launch_bounds__(kThreads, sizeof(AT) == 8 ? 2 : 3)
                 else step(di, dm, df);
                 if (df && j < kc) {
                     const int32_t r = r_xy + 3 * lxy * (p - 1);
+                    decltype(ep.load(0, 0)) in[NX][3];   // all loads before the first store
 #pragma unroll
-                    for (int h = 0; h < 4; h += 2) {   // two nodes' loads, then their stores
-                        decltype(ep.load(0, 0)) in[2][3];
+                    for (int i = 0; i < NX; ++i)
+                        if (act0[i])
 #pragma unroll
-                        for (int i = 0; i < 2; ++i)
-                            if (act0[h + i])
+                            for (int d = 0; d < 3; ++d) in[i][d] = ep.load(r + 3 * i + d, j);
 #pragma unroll
-                                for (int d = 0; d < 3; ++d) in[i][d] = ep.load(r + 3 * (h + i) + d, j);
+                    for (int i = 0; i < NX; ++i)
+                        if (act0[i])
 #pragma unroll
-                        for (int i = 0; i < 2; ++i)
-                            if (act0[h + i])
-#pragma unroll
-                                for (int d = 0; d < 3; ++d) ep.store(r + 3 * (h + i) + d, j, a0[h + i][d], in[i][d], nored);
-                    }
+                            for (int d = 0; d < 3; ++d) ep.store(r + 3 * i + d, j, a0[i][d], in[i][d], nored);
                 }
 #pragma unroll
-                for (int i = 0; i < 4; ++i) {
+                for (int i = 0; i < NX; ++i) {
 #pragma unroll
                     for (int d = 0; d < 3; ++d) {
                         a0[i][d] = a1[i][d];
@@ -739,12 +743,13 @@ inline bool bgrid_layout(const dv_matrix *m, int precision, int ld) {
 template <class AT, class Gather, class Epi>
 void launch_bprod_grid(const LaunchEnv &e, const dv_matrix *m, int kc, Gather g, Epi ep) {
     auto kern = k_bprod_grid<AT, Gather, Epi>;
+    constexpr int THREADS = kBgThreads, WARPS = THREADS / 32;
     const size_t smem = std::max(sizeof(float) * (size_t)kBgStages * kBgSlot,
                                  sizeof(dvk::PatRec<AT>) * (size_t)m->pat_entries + 4 * ((size_t)m->pat_count + 1));
     static dvk::SmemLimit limit;   // per instantiation and device
     limit.raise(kern, smem, e.ctx->device);
     static dvk::OccupancyCache occupancy;   // per instantiation
-    const int64_t wave = (int64_t)e.ctx->num_sms * occupancy.get(kern, kThreads, smem, e.ctx->device);
+    const int64_t wave = (int64_t)e.ctx->num_sms * occupancy.get(kern, THREADS, smem, e.ctx->device);
     BGridGeom G;
     G.lx = m->grid_lx;
     G.ly = m->grid_ly;
@@ -757,14 +762,14 @@ void launch_bprod_grid(const LaunchEnv &e, const dv_matrix *m, int kc, Gather g,
     const int64_t slabs = (kc + 31) / 32, plane_tiles = (int64_t)G.ntx * G.nty;
     const int lzi = std::max(1, G.lz - 2);
     // two boundary groups a warp; a block of them takes about as long as three plane steps of a tile
-    const int64_t bound_blocks = std::min<int64_t>((G.nbound + 2 * kWarps - 1) / (2 * kWarps), wave);
+    const int64_t bound_blocks = std::min<int64_t>((G.nbound + 2 * WARPS - 1) / (2 * WARPS), wave);
     G.zc = dvk::grid_run_length(plane_tiles * slabs, lzi, wave, bound_blocks * slabs);
     G.ntile = G.lz > 2 ? (int32_t)(plane_tiles * ((lzi + G.zc - 1) / G.zc)) : 0;
     G.tile_blocks = G.ntile;
     BGridCoef<AT> cf;
     for (int c = 0; c < dvk::kHexClasses; ++c) cf.cls[c] = (AT)m->grid_cls[c];
     const dim3 grid((unsigned)std::max<int64_t>(1, G.tile_blocks + bound_blocks), (unsigned)slabs);
-    dvk::launch_chain(kern, grid, kThreads, smem, e.stream, G, cf, m->pat_id.as<uint16_t>(), m->pat_start.as<uint32_t>(),
+    dvk::launch_chain(kern, grid, THREADS, smem, e.stream, G, cf, m->pat_id.as<uint16_t>(), m->pat_start.as<uint32_t>(),
                       static_cast<const dvk::PatRec<AT> *>(m->pat_rec.p), m->grid_bnode.as<uint32_t>(), m->pat_count,
                       m->pat_entries, BGridSrc<Gather>::block(g), g.ld, kc, g, ep, e.done);
     DV_CUDA(cudaGetLastError());

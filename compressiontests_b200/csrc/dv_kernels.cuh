@@ -1361,6 +1361,11 @@ __global__ void __launch_bounds__(256, 3)   // 3 blocks an SM: FP64 fits 80 regi
     extern __shared__ uint4 grid_smem[];
     constexpr bool FU = op_fused<Op>::value;
     constexpr bool S0 = FU || sizeof(AT) == 4;   // FP64 parity epilogues multiply the zeros too
+    // What the epilogue reads is loaded before the step's multiplies where the staged vector is FP32 (mixed solve
+    // 128^3 6.58 -> 6.49 ms); elsewhere it is prefetched a step ahead and loaded after them: with FP64 staging the
+    // early loads' registers cost more than they hide (FP64 solve 96 x 48 x 48 2.73 -> 2.79 ms), and the full
+    // coefficient table leaves none.
+    constexpr bool EARLY = HEX && sizeof(typename StageSrc<Gather>::ST) == 4;
     double red[Op::NRED > 0 ? Op::NRED : 1];
 #pragma unroll
     for (int i = 0; i < (Op::NRED > 0 ? Op::NRED : 1); ++i) red[i] = 0.0;
@@ -1438,8 +1443,19 @@ __global__ void __launch_bounds__(256, 3)   // 3 blocks an SM: FP64 fits 80 regi
 #pragma unroll
                         for (int d = 0; d < 3; ++d) a2[q][d] = act2[q] ? op.init(r + d) : AT(0);
                     }
-                    if (dm && act1[q]) touch_rows(op, (int32_t)(3 * (col_xy[q] + lxy * p)));   // finished next step
+                    if (!EARLY && dm && act1[q])
+                        touch_rows(op, (int32_t)(3 * (col_xy[q] + lxy * p)));   // finished next step
                 }
+                const int64_t below = lxy * (p - 1);
+                decltype(op.load(0)) in[NY][3];
+                auto load_below = [&] {
+#pragma unroll
+                    for (int q = 0; q < NY; ++q)
+                        if (act0[q])
+#pragma unroll
+                            for (int d = 0; d < 3; ++d) in[q][d] = op.load((int32_t)(3 * (col_xy[q] + below)) + d);
+                };
+                if (EARLY && df) load_below();
                 if (di && dm && df) grid_plane_step<AT, SS, NY, FU, HEX, S0, true, true, true>(pl, tx, ty, cf, a0, a1, a2);
                 else if (di && dm) grid_plane_step<AT, SS, NY, FU, HEX, S0, true, true, false>(pl, tx, ty, cf, a0, a1, a2);
                 else if (dm && df) grid_plane_step<AT, SS, NY, FU, HEX, S0, false, true, true>(pl, tx, ty, cf, a0, a1, a2);
@@ -1447,13 +1463,7 @@ __global__ void __launch_bounds__(256, 3)   // 3 blocks an SM: FP64 fits 80 regi
                 else if (dm) grid_plane_step<AT, SS, NY, FU, HEX, S0, false, true, false>(pl, tx, ty, cf, a0, a1, a2);
                 else if (df) grid_plane_step<AT, SS, NY, FU, HEX, S0, false, false, true>(pl, tx, ty, cf, a0, a1, a2);
                 if (df) {
-                    const int64_t below = lxy * (p - 1);
-                    decltype(op.load(0)) in[NY][3];
-#pragma unroll
-                    for (int q = 0; q < NY; ++q)
-                        if (act0[q])
-#pragma unroll
-                            for (int d = 0; d < 3; ++d) in[q][d] = op.load((int32_t)(3 * (col_xy[q] + below)) + d);
+                    if (!EARLY) load_below();
 #pragma unroll
                     for (int q = 0; q < NY; ++q)
                         if (act0[q])

@@ -52,10 +52,11 @@ sys.path.insert(0, ROOT)
 METRIC = "MG-PCG time to 1e-8 rel. residual (mixed FP32/FP64, 128^3 hex elasticity)"
 
 # dv_matrix_info.kernel_variant -> kernel (DuVi: 100 + g lane layout, 200 + g node patterns,
-# 300 + g grid stencil; CSR: threads per row; DuVi 4 / 9: staged row bundles)
+# 300 + g grid stencil; CSR: threads per row, 48 / 96: 16 / 32 lanes per 3-row node group; DuVi 4 / 9: staged
+# row bundles)
 KERNEL_NAMES = {101: "k_duvi_lanes", 102: "k_duvi_lanes", 103: "k_duvi_lanes", 201: "k_duvi_pattern",
                 202: "k_duvi_pattern", 203: "k_duvi_pattern", 303: "k_duvi_grid", 400: "k_hex_elem", 4: "k_duvi",
-                9: "k_duvi"}
+                9: "k_duvi", 48: "k_csr_nodes", 96: "k_csr_nodes"}
 # derived layouts whose matrix costs ~2 bytes per node group: their algorithmic bytes are the vectors
 DERIVED_SHAPES = {201, 202, 203, 303}
 OMEGA_EFF = (2.0 / 3.0) * 2.0 / (1.1 * 3.09)   # 2/3 of the spectrally normalised Jacobi weight (lambda ~ 3.09)
@@ -286,6 +287,8 @@ def spmv_table(cb, ctx, A0, reps, peak, cases=(("duvi", "f32"), ("duvi", "f64"),
         fmt_bytes = info["device_bytes"] + 2 * vs * n      # the caller's format: matrix arrays + x + y
         derived = info["kernel_variant"] in DERIVED_SHAPES  # node patterns / grid stencil: x + y + 2 B per node
         alg = (2 * vs * n + 2 * (n // 3)) if derived else fmt_bytes
+        if info["kernel_variant"] in (48, 96):   # one column list per node group is read, not three
+            alg -= 8 * info["nnz"] // 3
         gbs = alg / ms / 1e6
         out[f"{fmt}_{prec}"] = {"ms": round(ms, 4), "algorithmic_bytes": int(alg), "GBps": round(gbs, 1),
                                 "frac_of_peak": round(gbs / peak, 3), "value_index_bits": info["value_index_bits"],

@@ -4,15 +4,17 @@
 // solve: host applications that reserve all their device memory once at
 // start-up (a pool owned by another allocator) and forbid allocations
 // afterwards, and time-critical loops that cannot afford cudaFree, which
-// synchronises the whole device.  dv_pcg_solve_noalloc serves them: it runs the same kernels as dv_pcg_solve,
-// but its work vectors (r, z, p, Ap), reduction partials and scalars live in
-// one file-scope device array of fixed size, so the call itself allocates
+// synchronises the whole device.  dv_pcg_solve_noalloc serves them: it runs the
+// same kernels as dv_pcg_solve, but its work vectors (r, z, p, Ap; a second p where
+// one launch runs the whole solve), reduction partials and scalars live in one
+// file-scope device array of fixed size, so the call itself allocates
 // nothing.  The caller passes the matrix (already uploaded) and device
 // pointers for b and x.
 //
 // Limits and sharing:
 //  - at most kNoAllocMaxRows rows (the array holds four FP64 work vectors of
-//    that length); larger systems are rejected with DV_ERR_ARG;
+//    that length, or five of the shorter systems' solved in one launch); larger
+//    systems are rejected with DV_ERR_ARG;
 //  - the array exists once per device in every process that loads the library
 //    and lives until exit; every call on that device uses the same array, so
 //    calls whose work overlaps on the GPU (other threads, other streams)

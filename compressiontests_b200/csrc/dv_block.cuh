@@ -776,27 +776,27 @@ void launch_bprod_grid(const LaunchEnv &e, const dv_matrix *m, int kc, Gather g,
     e.ctx->count();
 }
 
-// Matrix-free trilinear transfer (DV_FORMAT_TRILINEAR): one thread per (node, column j), the
-// node's three rows summed from zero in column order like the stored kernels.
+// Matrix-free trilinear transfer (DV_FORMAT_TRILINEAR): one thread per (pair of fine nodes or coarse node, column
+// j), its rows summed from zero in column order like the stored kernels (tri_rows).
 template <bool RESTRICT, class AT, class Gather, class Epi>
 __global__ void __launch_bounds__(kThreads) k_bprod_tri(dvk::TriGeom G, int kc, Gather g, Epi ep,
                                                          const int *__restrict__ done) {
     static_assert(Epi::NC == 0, "transfers carry no reductions");
     if (dvk::chain_done(done)) return;
-    const int64_t work = G.nodes(RESTRICT) * kc;
+    constexpr int R = RESTRICT ? 3 : 6;
+    const int64_t work = G.items(RESTRICT) * kc;
     for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < work; t += (int64_t)gridDim.x * blockDim.x) {
         const uint32_t q = (uint32_t)(t / kc);
         const int j = (int)(t - (int64_t)q * kc);
-        AT s[3] = {AT(0), AT(0), AT(0)};
-        dvk::tri_walk<RESTRICT, AT>(G, q, [&](uint32_t col, AT w) {
+        AT s[R];
 #pragma unroll
-            for (int d = 0; d < 3; ++d) s[d] = madd<AT>(s[d], w, g(col + d, j));
-        });
-        decltype(ep.load(0, 0)) in[3];
+        for (int d = 0; d < R; ++d) s[d] = AT(0);
+        dvk::tri_rows<RESTRICT, AT, false>(G, q, [&](uint32_t col) { return g(col, j); }, s);
+        decltype(ep.load(0, 0)) in[R];
 #pragma unroll
-        for (int d = 0; d < 3; ++d) in[d] = ep.load((int32_t)(3 * q + d), j);
+        for (int d = 0; d < R; ++d) in[d] = ep.load((int32_t)(R * q) + d, j);
 #pragma unroll
-        for (int d = 0; d < 3; ++d) ep.store((int32_t)(3 * q + d), j, s[d], in[d], nullptr);
+        for (int d = 0; d < R; ++d) ep.store((int32_t)(R * q) + d, j, s[d], in[d], nullptr);
     }
 }
 
@@ -807,7 +807,7 @@ void launch_bprod(const LaunchEnv &e, const dv_matrix *m, int kc, Gather g, Epi 
     if constexpr (Epi::NC == 0) {
         if (m->format == DV_FORMAT_TRILINEAR) {
             const dvk::TriGeom G{m->tri_ne[0], m->tri_ne[1], m->tri_ne[2]};
-            const int64_t work = G.nodes(m->tri_restrict) * kc;
+            const int64_t work = G.items(m->tri_restrict) * kc;
             const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>((work + kThreads - 1) / kThreads, e.max_blocks));
             if (m->tri_restrict) dvk::launch_chain(k_bprod_tri<true, AT, Gather, Epi>, blocks, kThreads, 0, e.stream, G, kc, g, ep, e.done);
             else dvk::launch_chain(k_bprod_tri<false, AT, Gather, Epi>, blocks, kThreads, 0, e.stream, G, kc, g, ep, e.done);

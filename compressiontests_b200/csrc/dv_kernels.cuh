@@ -2008,126 +2008,99 @@ struct TriGeom {
     __host__ __device__ int64_t nodes(bool restrict_) const {   // rows / 3
         return restrict_ ? (int64_t)(f0 / 2) * (f1 / 2 + 1) * (f2 / 2 + 1) : (int64_t)f0 * (f1 + 1) * (f2 + 1);
     }
+    __host__ __device__ int64_t items(bool restrict_) const { return restrict_ ? nodes(true) : nodes(false) / 2; }
 };
 
-// Calls f(first column, weight) for the coarse nodes of fine free node q (prolongation, a row of P)
-// or the fine nodes of coarse free node q (restriction, a row of P^T), in increasing column order.
-template <bool RESTRICT, class AT, class F>
-__device__ __forceinline__ void tri_walk(const TriGeom &G, uint32_t q, F &&f) {
+// Adds to s the rows of the fine nodes 2 q and 2 q + 1 (prolongation; fine element counts are even, so X = 2 m + 1
+// and 2 m + 2 lie in one row and share the coarse nodes m and m + 1 of up to four coarse rows), or of coarse
+// node q (restriction), in increasing column order.  g(column) gathers; dof d takes column d of each node.  All of a
+// pair's values (restriction: a fine plane's) are loaded before the first is added: added one after another
+// as they come, a row waits for up to 8 (27) loads in turn.  Mixed solve 128^3 6.50 -> 6.27 ms, 16^3 0.86 -> 0.82 ms,
+// FP64 solve 96 x 48 x 48 2.80 -> 2.67 ms; 64 load cases on 48^3
+// (k_bprod_tri) 26.3 -> 25.2 ms.
+template <class AT, bool FU, class F>
+__device__ __forceinline__ void tri_prolong(const TriGeom &G, uint32_t q, F &&g, AT (&s)[6]) {
     // 32-bit index arithmetic throughout: rows and columns are below 2^31
     const uint32_t ny = G.f1 + 1, cx = G.f0 / 2, cy = G.f1 / 2 + 1;
-    if constexpr (!RESTRICT) {
-        const uint32_t t = q / (uint32_t)G.f0, Zy = t / ny;
-        const int32_t X = (int32_t)(q - t * (uint32_t)G.f0) + 1, Y = (int32_t)(t - Zy * ny), Z = (int32_t)Zy;
-        const int nx_ = (X & 1) ? 2 : 1, ny_ = (Y & 1) ? 2 : 1, nz_ = (Z & 1) ? 2 : 1;
-        const AT w = (nx_ == 2 ? AT(0.5) : AT(1)) * (ny_ == 2 ? AT(0.5) : AT(1)) * (nz_ == 2 ? AT(0.5) : AT(1));
-        for (int c = 0; c < nz_; ++c)
-            for (int b = 0; b < ny_; ++b)
-                for (int a = 0; a < nx_; ++a) {
-                    const int32_t xc = X / 2 + a;
-                    if (xc == 0) continue;   // clamped coarse node
-                    f(3u * ((uint32_t)(xc - 1) + cx * ((uint32_t)(Y / 2 + b) + cy * (uint32_t)(Z / 2 + c))), w);
-                }
-    } else {
-        const uint32_t t = q / cx, Zc_ = t / cy;
-        const int32_t Xc = (int32_t)(q - t * cx) + 1, Yc = (int32_t)(t - Zc_ * cy), Zc = (int32_t)Zc_;
-        for (int c = -1; c <= 1; ++c) {
-            const int32_t Z = 2 * Zc + c;
-            if (Z < 0 || Z > G.f2) continue;
-            for (int b = -1; b <= 1; ++b) {
-                const int32_t Y = 2 * Yc + b;
-                if (Y < 0 || Y > G.f1) continue;
-                for (int a = -1; a <= 1; ++a) {
-                    const int32_t X = 2 * Xc + a;
-                    if (X > G.f0) continue;   // X >= 1 always (Xc >= 1)
-                    const AT w = (a ? AT(0.5) : AT(1)) * (b ? AT(0.5) : AT(1)) * (c ? AT(0.5) : AT(1));
-                    f(3u * ((uint32_t)(X - 1) + (uint32_t)G.f0 * ((uint32_t)Y + ny * (uint32_t)Z)), w);
-                }
+    const uint32_t t = q / cx, m = q - t * cx, Z = t / ny, Y = t - Z * ny;
+    const bool oy = Y & 1, oz = Z & 1;   // between two coarse nodes: weights 1/2
+    AT v[4][2][3];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)   // coarse rows, y fastest
+        if ((!(i & 1) || oy) && (!(i & 2) || oz)) {
+            const uint32_t col = 3u * (m + cx * (Y / 2 + (i & 1) + cy * (Z / 2 + (i >> 1))));
+#pragma unroll
+            for (int d = 0; d < 3; ++d) {
+                v[i][0][d] = m > 0 ? g(col - 3 + d) : AT(0);   // coarse node 0 is clamped
+                v[i][1][d] = g(col + d);
             }
+        }
+    const AT w = (oy ? AT(0.5) : AT(1)) * (oz ? AT(0.5) : AT(1)), wh = AT(0.5) * w;
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+        if ((!(i & 1) || oy) && (!(i & 2) || oz))
+#pragma unroll
+            for (int d = 0; d < 3; ++d) {
+                if (m > 0) s[d] = madd_op<AT, FU>(s[d], wh, v[i][0][d]);
+                s[d] = madd_op<AT, FU>(s[d], wh, v[i][1][d]);
+                s[3 + d] = madd_op<AT, FU>(s[3 + d], w, v[i][1][d]);
+            }
+}
+template <class AT, bool FU, class F>
+__device__ __forceinline__ void tri_restrict(const TriGeom &G, uint32_t q, F &&g, AT (&s)[3]) {
+    const uint32_t ny = G.f1 + 1, cx = G.f0 / 2, cy = G.f1 / 2 + 1;
+    const uint32_t t = q / cx, m = q - t * cx;
+    const int32_t Zc = (int32_t)(t / cy), Yc = (int32_t)(t - (uint32_t)Zc * cy), X0 = 2 * (int32_t)m + 1;
+#pragma unroll
+    for (int c = -1; c <= 1; ++c) {
+        const int32_t Z = 2 * Zc + c;
+        if (Z < 0 || Z > G.f2) continue;
+        AT v[3][9];   // the fine nodes X0 .. X0 + 2 of three rows
+#pragma unroll
+        for (int b = -1; b <= 1; ++b) {
+            const int32_t Y = 2 * Yc + b;
+            if (Y < 0 || Y > G.f1) continue;
+            const uint32_t col = 3u * ((uint32_t)(X0 - 1) + (uint32_t)G.f0 * ((uint32_t)Y + ny * (uint32_t)Z));
+#pragma unroll
+            for (int k = 0; k < 9; ++k) v[b + 1][k] = X0 + k / 3 <= G.f0 ? g(col + k) : AT(0);
+        }
+#pragma unroll
+        for (int b = -1; b <= 1; ++b) {
+            const int32_t Y = 2 * Yc + b;
+            if (Y < 0 || Y > G.f1) continue;
+#pragma unroll
+            for (int k = 0; k < 9; ++k)
+                if (X0 + k / 3 <= G.f0) {
+                    const AT w = (k / 3 != 1 ? AT(0.5) : AT(1)) * (b ? AT(0.5) : AT(1)) * (c ? AT(0.5) : AT(1));
+                    s[k % 3] = madd_op<AT, FU>(s[k % 3], w, v[b + 1][k]);
+                }
         }
     }
 }
+template <bool RESTRICT, class AT, bool FU, class F, int R>
+__device__ __forceinline__ void tri_rows(const TriGeom &G, uint32_t q, F &&g, AT (&s)[R]) {
+    static_assert(R == (RESTRICT ? 3 : 6), "rows of an item");
+    if constexpr (RESTRICT) tri_restrict<AT, FU>(G, q, g, s);
+    else tri_prolong<AT, FU>(G, q, g, s);
+}
 
-// Prolongation: one thread per pair of fine nodes in x (fine element counts are even, so X = 2 m + 1 and 2 m + 2
-// lie in one row), which share the coarse nodes m and m + 1 of up to four coarse rows.  Restriction: one thread
-// per coarse node.  Dof d takes column d of each node.  All of a pair's values (restriction: a fine
-// plane's) are loaded before the first is added: added one after another as they come, a row waits for
-// up to 8 (27) loads in turn.  Mixed solve 128^3 6.50 -> 6.27 ms, 16^3 0.86 -> 0.82 ms, FP64 solve 96 x 48 x 48
-// 2.80 -> 2.67 ms.
+// One thread per pair of fine nodes (prolongation) or coarse node (restriction).
 template <bool RESTRICT, class AT, class Gather, class Op>
 __global__ void __launch_bounds__(256) k_tri(TriGeom G, Gather g, Op op, const int *__restrict__ done,
                                              double *partials, unsigned *ticket) {
     if (chain_done(done)) return;
     constexpr bool FU = op_fused<Op>::value;
+    constexpr int R = RESTRICT ? 3 : 6;
     double red[Op::NRED > 0 ? Op::NRED : 1];
 #pragma unroll
     for (int i = 0; i < (Op::NRED > 0 ? Op::NRED : 1); ++i) red[i] = 0.0;
-    const uint32_t ny = G.f1 + 1, cx = G.f0 / 2, cy = G.f1 / 2 + 1;
-    const uint32_t items = (uint32_t)(RESTRICT ? G.nodes(true) : G.nodes(false) / 2);
+    const uint32_t items = (uint32_t)G.items(RESTRICT);
     for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < items; q += gridDim.x * blockDim.x) {
-        const uint32_t t = q / cx, m = q - t * cx;
-        if constexpr (!RESTRICT) {
-            const uint32_t Z = t / ny, Y = t - Z * ny;
-            const bool oy = Y & 1, oz = Z & 1;   // between two coarse nodes: weights 1/2
-            AT v[4][2][3];
+        AT s[R];
 #pragma unroll
-            for (int i = 0; i < 4; ++i)   // coarse rows, y fastest
-                if ((!(i & 1) || oy) && (!(i & 2) || oz)) {
-                    const uint32_t col = 3u * (m + cx * (Y / 2 + (i & 1) + cy * (Z / 2 + (i >> 1))));
-#pragma unroll
-                    for (int d = 0; d < 3; ++d) {
-                        v[i][0][d] = m > 0 ? g(col - 3 + d) : AT(0);   // coarse node 0 is clamped
-                        v[i][1][d] = g(col + d);
-                    }
-                }
-            const AT w = (oy ? AT(0.5) : AT(1)) * (oz ? AT(0.5) : AT(1)), wh = AT(0.5) * w;
-            const int32_t r0 = (int32_t)(6 * q);
-            AT s[6];
-#pragma unroll
-            for (int d = 0; d < 6; ++d) s[d] = op.init(r0 + d);
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-                if ((!(i & 1) || oy) && (!(i & 2) || oz))
-#pragma unroll
-                    for (int d = 0; d < 3; ++d) {
-                        if (m > 0) s[d] = madd_op<AT, FU>(s[d], wh, v[i][0][d]);
-                        s[d] = madd_op<AT, FU>(s[d], wh, v[i][1][d]);
-                        s[3 + d] = madd_op<AT, FU>(s[3 + d], w, v[i][1][d]);
-                    }
-            finish_rows(op, r0, s, red);
-        } else {
-            const int32_t Zc = (int32_t)(t / cy), Yc = (int32_t)(t - (uint32_t)Zc * cy), X0 = 2 * (int32_t)m + 1;
-            const int32_t r0 = (int32_t)(3 * q);
-            AT s[3];
-#pragma unroll
-            for (int d = 0; d < 3; ++d) s[d] = op.init(r0 + d);
-#pragma unroll
-            for (int c = -1; c <= 1; ++c) {
-                const int32_t Z = 2 * Zc + c;
-                if (Z < 0 || Z > G.f2) continue;
-                AT v[3][9];   // the fine nodes X0 .. X0 + 2 of three rows
-#pragma unroll
-                for (int b = -1; b <= 1; ++b) {
-                    const int32_t Y = 2 * Yc + b;
-                    if (Y < 0 || Y > G.f1) continue;
-                    const uint32_t col = 3u * ((uint32_t)(X0 - 1) + (uint32_t)G.f0 * ((uint32_t)Y + ny * (uint32_t)Z));
-#pragma unroll
-                    for (int k = 0; k < 9; ++k) v[b + 1][k] = X0 + k / 3 <= G.f0 ? g(col + k) : AT(0);
-                }
-#pragma unroll
-                for (int b = -1; b <= 1; ++b) {
-                    const int32_t Y = 2 * Yc + b;
-                    if (Y < 0 || Y > G.f1) continue;
-#pragma unroll
-                    for (int k = 0; k < 9; ++k)
-                        if (X0 + k / 3 <= G.f0) {
-                            const AT w = (k / 3 != 1 ? AT(0.5) : AT(1)) * (b ? AT(0.5) : AT(1)) * (c ? AT(0.5) : AT(1));
-                            s[k % 3] = madd_op<AT, FU>(s[k % 3], w, v[b + 1][k]);
-                        }
-                }
-            }
-            finish_rows(op, r0, s, red);
-        }
+        for (int d = 0; d < R; ++d) s[d] = op.init((int32_t)(R * q) + d);
+        tri_rows<RESTRICT, AT, FU>(G, q, g, s);
+        finish_rows(op, (int32_t)(R * q), s, red);
     }
     if constexpr (Op::NRED > 0) {
         double tot[Op::NRED];
@@ -2138,7 +2111,7 @@ __global__ void __launch_bounds__(256) k_tri(TriGeom G, Gather g, Op op, const i
 template <class AT, class Gather, class Op>
 void launch_trilinear(const LaunchEnv &e, const dv_matrix *m, Gather g, Op op) {
     const TriGeom G{m->tri_ne[0], m->tri_ne[1], m->tri_ne[2]};
-    const int64_t items = m->tri_restrict ? m->n_rows / 3 : m->n_rows / 6;
+    const int64_t items = G.items(m->tri_restrict);
     const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>((items + 255) / 256, e.max_blocks));
     if (m->tri_restrict) launch_chain(k_tri<true, AT, Gather, Op>, blocks, 256, 0, e.stream, G, g, op, e.done, e.partials, e.ticket);
     else launch_chain(k_tri<false, AT, Gather, Op>, blocks, 256, 0, e.stream, G, g, op, e.done, e.partials, e.ticket);

@@ -2199,6 +2199,7 @@ __global__ void k_fill(T *__restrict__ a, T v, int32_t n, const int *__restrict_
 }
 template <class A, class B>
 __global__ void k_convert(const A *__restrict__ a, B *__restrict__ b, int32_t n) {
+    chain_done(nullptr);   // launched in a chain, whatever comes before it
     for (int32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) b[i] = (B)a[i];
 }
 // x += y

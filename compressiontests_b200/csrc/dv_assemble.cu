@@ -237,16 +237,16 @@ dv_matrix *dv_hex_operator_build(dv_context *ctx, int32_t nmesh, const int32_t *
     cudaStream_t s = ctx->stream;
     m->hex_meshes.alloc(sizeof(HexMesh) * meshes.size());
     DV_CUDA(cudaMemcpyAsync(m->hex_meshes.p, meshes.data(), sizeof(HexMesh) * meshes.size(), cudaMemcpyHostToDevice, s));
-    if (precision == DV_F64) {
-        m->hex_factor.alloc(8 * (size_t)nel);
-        DV_CUDA(cudaMemcpyAsync(m->hex_factor.p, f.data(), 8 * (size_t)nel, cudaMemcpyHostToDevice, s));
+    auto upload = [&](const auto &k, const auto &factors) {   // Ke, then the factors
+        const size_t vs = sizeof(k[0]);
+        m->hex_factor.alloc(vs * (576 + (size_t)nel));
+        DV_CUDA(cudaMemcpyAsync(m->hex_factor.p, k.data(), vs * 576, cudaMemcpyHostToDevice, s));
+        DV_CUDA(cudaMemcpyAsync(m->hex_factor.template as<char>() + vs * 576, factors.data(), vs * (size_t)nel,
+                                cudaMemcpyHostToDevice, s));
         DV_CUDA(cudaStreamSynchronize(s));
-    } else {
-        std::vector<float> f32(f.begin(), f.end());
-        m->hex_factor.alloc(4 * (size_t)nel);
-        DV_CUDA(cudaMemcpyAsync(m->hex_factor.p, f32.data(), 4 * (size_t)nel, cudaMemcpyHostToDevice, s));
-        DV_CUDA(cudaStreamSynchronize(s));
-    }
+    };
+    if (precision == DV_F64) upload(ke, f);
+    else upload(std::vector<float>(ke.begin(), ke.end()), std::vector<float>(f.begin(), f.end()));
     // diagonal: sum over the node's elements in increasing id of (scale E_e) Ke(a, a), as assembled
     static const int vtk[8] = {0, 1, 3, 2, 4, 5, 7, 6};
     m->host_diag.assign(rows, 0.0);

@@ -231,7 +231,8 @@ struct dv_matrix {
     DevMem grid_bnode;                   // u32 boundary groups
     int64_t grid_nb = 0;
     int32_t hex_ne[3] = {0, 0, 0};       // DV_FORMAT_HEX: elements per axis (of the first mesh)
-    DevMem hex_factor;                   // per-element factor scale * E_e, matrix precision, meshes in order
+    DevMem hex_factor;                   // the 576 entries of Ke, then the factor scale * E_e of every element (meshes
+                                         // in order), matrix precision
     DevMem hex_meshes;                   // dvk::HexMesh per mesh (tiles, first row, first factor)
     int32_t hex_nmesh = 0, hex_ntile = 0;
     int32_t tri_ne[3] = {0, 0, 0};       // DV_FORMAT_TRILINEAR: fine element counts (even)

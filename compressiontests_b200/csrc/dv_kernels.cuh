@@ -1751,6 +1751,9 @@ void launch_csr_nodes(const LaunchEnv &e, const dv_matrix *m, Gather g, Op op) {
 // operator's, so FP64 products agree with the assembled matrix to rounding (not bit for bit).
 // 128^3, log-uniform moduli, FP64 product: 212.9 -> 79.9 us (119 MB of vectors and factors: 18 us;
 // 170 FP64 operations a node: 19 us), relative error against 64 bits 4.7e-16 -> 2.1e-16.
+// Sums and differences over corners turn an infinite x into Inf - Inf, and overflow for a finite x near
+// the type's limit: a node whose sums are not finite is formed again from the entries of Ke
+// (hex_node_direct), so it has the signed infinity, the NaN or the finite value of Ke times x.
 // ---------------------------------------------------------------------------
 template <class AT>
 struct HexModes {
@@ -1805,11 +1808,71 @@ __device__ __forceinline__ void hex_xy(AT v00, AT v10, AT v01, AT v11, AT (&s)[4
     s[3] = b - d;
 }
 
+// The mesh of tile t: the last with tile0 <= t.
+__device__ __forceinline__ int hex_mesh_of(const HexMesh *__restrict__ meshes, int32_t nmesh, int t) {
+    int lo = 0, hi = nmesh - 1;
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (meshes[mid].tile0 <= t) lo = mid;
+        else hi = mid - 1;
+    }
+    return lo;
+}
+
+// The three rows from r of tile t's mesh, added to s entry by entry: the element layer below the node
+// and the one above, each by its lower and its upper corners (plane z - 1; z, above and below; z + 1).  As
+// everywhere, an element outside the mesh has factor 0 and a node outside it x = 0.  Out of line: it
+// takes no registers from the kernel's step.
+template <class AT>
+struct HexRows {
+    AT v[3];
+};
+template <class AT, bool FUSED, class Gather>
+__device__ __noinline__ HexRows<AT> hex_node_direct(const HexMesh *__restrict__ meshes, int32_t nmesh, int t,
+                                                    const AT *__restrict__ ef_all, const AT *__restrict__ ke, Gather g,
+                                                    int32_t r, HexRows<AT> s) {
+    constexpr int vtk[8] = {0, 1, 3, 2, 4, 5, 7, 6};
+    const HexMesh G = meshes[hex_mesh_of(meshes, nmesh, t)];
+    const int32_t lx = G.ne0, ly = G.ne1 + 1, q = (int32_t)(r - G.row0) / 3;
+    const int iz = q / (lx * ly), iy = q / lx - ly * iz, ix = q % lx;
+#pragma unroll 1
+    for (int part = 0; part < 4; ++part) {
+        const int above = part & 1, bz = part >> 1, layer = iz - 1 + above, z = layer + bz;
+#pragma unroll 1
+        for (int el = 0; el < 4; ++el) {
+            const int ex = ix + (el & 1), ey = iy - 1 + (el >> 1);
+            const bool inside = ex < G.ne0 && ey >= 0 && ey < G.ne1 && layer >= 0 && layer < G.ne2;
+            const AT f = inside ? ef_all[G.fac0 + ex + (int64_t)G.ne0 * (ey + (int64_t)G.ne1 * layer)] : AT(0);
+            const int a = vtk[3 - el + (above ? 0 : 4)];   // the node among the element's corners
+#pragma unroll 1
+            for (int c = 0; c < 12; ++c) {   // corner c / 3 of the plane, dof c % 3
+                const int corner = c / 3, d = c - 3 * corner;
+                const int x = ex - 1 + (corner & 1), y = ey + (corner >> 1);
+                const bool node = x >= 0 && x < lx && y >= 0 && y < ly && z >= 0 && z <= G.ne2;
+                const AT w = f * (node ? g((uint32_t)(G.row0 + 3 * (x + (int64_t)lx * (y + (int64_t)ly * z)) + d)) : AT(0));
+                const AT *col = ke + 72 * a + 3 * vtk[corner + 4 * bz] + d;
+#pragma unroll
+                for (int i = 0; i < 3; ++i) s.v[i] = madd_op<AT, FUSED>(s.v[i], col[24 * i], w);
+            }
+        }
+    }
+    return s;
+}
+// Whether any of the sums is an infinity or a NaN.
+__device__ __forceinline__ bool any_nonfinite(const double (&s)[3]) {
+    const int a = __double2hiint(s[0]) & 0x7fffffff, b = __double2hiint(s[1]) & 0x7fffffff, c = __double2hiint(s[2]) & 0x7fffffff;
+    return max(a, max(b, c)) >= 0x7ff00000;
+}
+__device__ __forceinline__ bool any_nonfinite(const float (&s)[3]) {
+    const int a = __float_as_int(s[0]) & 0x7fffffff, b = __float_as_int(s[1]) & 0x7fffffff, c = __float_as_int(s[2]) & 0x7fffffff;
+    return max(a, max(b, c)) >= 0x7f800000;
+}
+
 template <class AT, class Gather, class Op>
 __global__ void __launch_bounds__(kHexThreads, sizeof(AT) == 8 ? 2 : 3)
     k_hex_elem(const HexMesh *__restrict__ meshes, int32_t nmesh, int32_t ntile, HexModes<AT> kc,
-               const AT *__restrict__ ef_all, Gather g, Op op, const int *__restrict__ done, double *partials,
-               unsigned *ticket) {
+               const AT *__restrict__ ke, const AT *__restrict__ ef_all, Gather g, Op op, const int *__restrict__ done,
+               double *partials, unsigned *ticket) {
     if (chain_done(done)) return;
     extern __shared__ uint4 hex_smem[];
     using SS = StageSrc<Gather>;
@@ -1821,13 +1884,7 @@ __global__ void __launch_bounds__(kHexThreads, sizeof(AT) == 8 ? 2 : 3)
 #pragma unroll
     for (int i = 0; i < (Op::NRED > 0 ? Op::NRED : 1); ++i) red[i] = 0.0;
     for (int t = blockIdx.x; t < ntile; t += gridDim.x) {
-        int lo = 0, hi = nmesh - 1;   // the mesh of tile t: the last with tile0 <= t
-        while (lo < hi) {
-            const int mid = (lo + hi + 1) >> 1;
-            if (meshes[mid].tile0 <= t) lo = mid;
-            else hi = mid - 1;
-        }
-        const HexMesh G = meshes[lo];
+        const HexMesh G = meshes[hex_mesh_of(meshes, nmesh, t)];
         const int32_t lx = G.ne0, ly = G.ne1 + 1, lz = G.ne2 + 1;
         const int32_t plane_len = 3 * lx * ly, layer_len = G.ne0 * G.ne1;
         const int W = G.wn + 1, R = G.rn + 1;   // element columns
@@ -1893,6 +1950,12 @@ __global__ void __launch_bounds__(kHexThreads, sizeof(AT) == 8 ? 2 : 3)
                 for (int c = 0; c < 3; ++c)
                     s[c] = op.init(r + c) + ((own[c] + sh[c * kHexThreads + 1]) +
                                              (sh[(3 + c) * kHexThreads + W] + sh[(6 + c) * kHexThreads + W + 1]));
+                if (any_nonfinite(s)) {
+                    const HexRows<AT> v = hex_node_direct<AT, op_fused<Op>::value>(
+                        meshes, nmesh, t, ef_all, ke, g, r, HexRows<AT>{{op.init(r), op.init(r + 1), op.init(r + 2)}});
+#pragma unroll
+                    for (int c = 0; c < 3; ++c) s[c] = v.v[c];
+                }
                 finish_rows(op, r, s, red);
             }
             if (p > z1) break;
@@ -1989,8 +2052,8 @@ void launch_hex_elem(const LaunchEnv &e, const dv_matrix *m, Gather g, Op op) {
     const HexModes<AT> kc{(AT)c[0], (AT)c[1], (AT)c[2], (AT)c[3], (AT)c[4], (AT)c[5], (AT)c[6], (AT)c[7]};
     const int blocks = (int)std::min<int64_t>(m->hex_ntile, e.max_blocks);
     launch_chain(kern, blocks, kHexThreads, smem, e.stream, m->hex_meshes.as<HexMesh>(), m->hex_nmesh, m->hex_ntile, kc,
-                                                  static_cast<const AT *>(m->hex_factor.p), g, op, e.done, e.partials,
-                                                  e.ticket);
+                                                  m->hex_factor.as<AT>(), m->hex_factor.as<AT>() + 576, g, op, e.done,
+                                                  e.partials, e.ticket);
     DV_CUDA(cudaGetLastError());
     e.ctx->count();
 }

@@ -542,3 +542,71 @@ def test_grid_stencil_f32_row_alignment(ctx, native, rng, ne, monkeypatch):
     for y, r in out[1:]:
         np.testing.assert_array_equal(y, out[0][0])
         np.testing.assert_array_equal(r, out[0][1])
+
+
+def _element_sums(native, ne, E, x):
+    """K(E) x entry by entry over the elements in IEEE arithmetic: what an infinity or a NaN in x makes of each row."""
+    Ke = native.hex_stiffness((2, 1, 1), np.array([0.0, 1.0])).toarray()   # nodes x-fastest, all free
+    x0 = np.zeros((ne[2] + 1, ne[1] + 1, ne[0] + 1, 3))
+    x0[:, :, 1:] = x.reshape(ne[2] + 1, ne[1] + 1, ne[0], 3)
+    y = np.zeros_like(x0)
+    f = E.reshape(ne[2], ne[1], ne[0])
+
+    def corner(t, a):
+        i, j, k = a & 1, (a >> 1) & 1, a >> 2
+        return t[k:ne[2] + k, j:ne[1] + j, i:ne[0] + i]
+
+    for a in range(8):
+        for b in range(8):
+            for d in range(3):
+                for c in range(3):
+                    corner(y, a)[..., d] += Ke[3 * a + d, 3 * b + c] * (f * corner(x0, b)[..., c])
+    return y[:, :, 1:].ravel()
+
+
+@pytest.mark.parametrize("prec", ["f64", "f32"])
+def test_matrix_free_hex_operator_nonfinite(ctx, native, rng, prec):
+    # Infinities and a NaN in x, off the faces: every row has the signed infinity or the NaN that Ke times x has, the
+    # rows of other elements are untouched; y = A x, y += A x and r = b - A x.
+    import torch
+    ne = (40, 9, 8)
+    dt, bar = (np.float64, REL64) if prec == "f64" else (np.float32, REL32)
+    E = 10.0 ** rng.uniform(-2.0, 0.0, int(np.prod(ne)))
+    x = rng.standard_normal((ne[2] + 1, ne[1] + 1, ne[0], 3)).astype(dt).astype(np.float64)
+    x[3, 4, 7, 0], x[4, 4, 20, 1], x[5, 5, 30, 2], x[5, 5, 32, 0], x[3, 6, 14, 1] = np.inf, -np.inf, np.inf, np.inf, np.nan
+    x = x.ravel()
+    b = rng.standard_normal(x.size).astype(dt).astype(np.float64)
+    A = native.hex_stiffness(ne, E)
+    H = native.SparseMatrix.hex_operator(ctx, ne, E, precision=prec)
+    with np.errstate(invalid="ignore"):
+        ref = _element_sums(native, ne, E, x)
+    assert np.isposinf(ref).sum() > 50 and np.isneginf(ref).sum() > 50 and np.isnan(ref).sum() > 80
+    scale = abs(A) @ np.abs(np.where(np.isfinite(x), x, 0.0)) + np.abs(b)
+    db, dx = torch.from_numpy(b.astype(dt)).cuda(), torch.from_numpy(x.astype(dt)).cuda()
+    dr = torch.empty_like(db)
+    torch.cuda.synchronize()
+    H.residual_device(db.data_ptr(), dx.data_ptr(), dr.data_ptr(), prec)
+    ctx.synchronize()
+    for got, want in ((_device_product(ctx, H, x, dt), ref), (H.Multiply(x, b.copy(), clear=False), b + ref),
+                      (dr.cpu().numpy(), b - ref)):
+        got = got.astype(np.float64)
+        fin = np.isfinite(want)
+        np.testing.assert_array_equal(got[~fin], want[~fin])
+        assert np.max(np.abs(got[fin] - want[fin]) / scale[fin]) <= bar
+
+
+@pytest.mark.parametrize("prec", ["f64", "f32"])
+def test_matrix_free_hex_operator_near_overflow(ctx, native, prec):
+    # x near the type's limit, alternating in x: sums over an element's corners overflow, the rows of a soft material
+    # do not.
+    ne = (33, 6, 5)
+    dt, bar = (np.float64, REL64) if prec == "f64" else (np.float32, REL32)
+    E = np.full(int(np.prod(ne)), 1e-3)
+    x = np.zeros((ne[2] + 1, ne[1] + 1, ne[0], 3))
+    x[:] = (0.2 * float(np.finfo(dt).max) * (-1.0) ** np.arange(ne[0]))[:, None]
+    x = x.ravel().astype(dt).astype(np.float64)
+    A = native.hex_stiffness(ne, E)
+    H = native.SparseMatrix.hex_operator(ctx, ne, E, precision=prec)
+    got = _device_product(ctx, H, x, dt).astype(np.float64)
+    assert np.all(np.isfinite(got))
+    assert rowwise_rel(got * 2.0 ** -12, A @ (x * 2.0 ** -12), A, x * 2.0 ** -12) <= bar

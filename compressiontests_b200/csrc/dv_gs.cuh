@@ -373,10 +373,21 @@ constexpr size_t gs_block_smem(int32_t n, bool nodes) {
     return sizeof(T) * ((size_t)n + kGsWarps * (nodes ? 3 * kGsStride + 9 : 32 * kGsLane));
 }
 
+// Whether one block sweeps these levels faster than a launch a level does: its warps take 32 rows or nodes at a
+// time, at most `passes` times a level on average.  Measured at 19,200 rows, a level by the block against a launch
+// (FP64, 5 / 27 / 81 entries a row): 96 rows 3.4 / 4.2 / 5.7 against 8.4 / 12 / 18 us, 192 rows 6.4 / 7.8 / 12
+// against 7.0 / 11 / 19, 384 rows 12 / 15 / 25 against 7.1 / 11 / 20: six passes of rows.  By node groups (9 / 81
+// entries a row, a level of nodes against three of rows): 256 nodes 20 / 36 against 26 / 68 us, 512 nodes
+// 36 / 68 against 27 / 67: ten passes of nodes.
+inline bool gs_levels_narrow(const std::vector<int32_t> &off, int passes) {
+    int64_t need = 0;
+    for (size_t l = 0; l + 1 < off.size(); ++l) need += (off[l + 1] - off[l] + kGsWarps - 1) / kGsWarps;
+    return need <= passes * (int64_t)(off.size() - 1);
+}
+
 // Prepares the one-block sweep of A's row-order levels (a: its host copy) where x fits a block's shared
-// memory (FP64 up to 25,856 rows, by node groups up to 19,352).  There a level has a few dozen rows and
-// one block is enough for it; a level of a larger system has hundreds to thousands, and every level
-// stays a launch over all SMs.
+// memory (FP64 up to 25,856 rows, by node groups up to 19,232) and the levels are narrow; wide levels (a
+// red-black or a nearly diagonal matrix, as against a hex grid's few dozen rows) stay a launch each over all SMs.
 template <class T>
 void gs_prepare_block(const dv_matrix *A, const dv_csr_host &a, GsOrder &o) {
     dv_context *ctx = A->ctx;
@@ -384,10 +395,12 @@ void gs_prepare_block(const dv_matrix *A, const dv_csr_host &a, GsOrder &o) {
     if (!o.lex || A->n_rows == 0 || gs_block_smem<T>(A->n_rows, false) > room) return;
     cudaStream_t s = ctx->stream;
     std::vector<int32_t> perm, off;
-    o.nodes = gs_block_smem<T>(A->n_rows, true) <= room && dv_csr_row_group(a) == 3;
-    for (int32_t i = 0; i < a.n_rows && o.nodes; i += 3) o.nodes = a.rowptr[i + 1] - a.rowptr[i] <= kGsCols;
+    bool nodes = gs_block_smem<T>(A->n_rows, true) <= room && dv_csr_row_group(a) == 3;
+    for (int32_t i = 0; i < a.n_rows && nodes; i += 3) nodes = a.rowptr[i + 1] - a.rowptr[i] <= kGsCols;
+    if (nodes) dv_gs_node_level_sets(a, perm, off);
+    if (nodes ? !gs_levels_narrow(off, 10) : !gs_levels_narrow(o.off, 6)) return;
+    o.nodes = nodes;
     if (o.nodes) {
-        dv_gs_node_level_sets(a, perm, off);
         o.d_nodes.alloc(4 * perm.size());
         DV_CUDA(cudaMemcpyAsync(o.d_nodes.p, perm.data(), 4 * perm.size(), cudaMemcpyHostToDevice, s));
     } else {

@@ -449,3 +449,61 @@ def test_gauss_seidel_row_order_node_groups(ctx, native, fmt, nodes, width):
     got, st, _ = s.Solve()
     np.testing.assert_array_equal(got, x)
     s.ReleaseCudaResources()
+
+
+def _layered(rng, levels, width, group, entries):
+    """A matrix whose forward-sweep levels have `width` units each (rows, or nodes of 3 rows with one column list): a
+    unit reads units of the level before it."""
+    import scipy.sparse as sp
+    n = levels * width
+    indptr, cols, vals = [0], [], []
+    for i in range(n):
+        l = i // width
+        prev = rng.integers((l - 1) * width, l * width, entries) if l else np.zeros(0, int)
+        units = np.union1d(np.union1d(prev, [i]), [i - width] if l else [])
+        c = (units[:, None] * group + np.arange(group)).ravel()
+        for d in range(group):
+            v = rng.integers(-8, 9, len(c)) / 16.0
+            v[c == group * i + d] = 2.0 * len(c)
+            cols.append(c)
+            vals.append(v)
+            indptr.append(indptr[-1] + len(c))
+    return sp.csr_matrix((np.concatenate(vals), np.concatenate(cols), indptr), shape=(n * group, n * group))
+
+
+@pytest.mark.parametrize("fmt", ["csr", "duvi"])
+@pytest.mark.parametrize("levels,width,group,block", [(12, 33, 1, True), (6, 192, 1, True), (6, 193, 1, False), (2, 3000, 1, False),
+                                                      (5, 64, 3, True), (4, 320, 3, True), (4, 321, 3, False), (1, 2000, 3, False)])
+def test_gauss_seidel_row_order_wide_levels(ctx, native, fmt, levels, width, group, block):
+    # Levels of more units than the block has warps: swept by one block up to six passes of rows (ten of nodes) a level, one
+    # launch a level beyond, where one block would be several to fifty times slower; the sequential sweep's bits either way.
+    import scipy.sparse as sp
+    A = _layered(np.random.default_rng(5), levels, width, group, 2)
+    n = A.shape[0]
+    R = sp.csr_matrix((np.zeros(1), [0], [0, 1]), shape=(1, n))
+    P = sp.csr_matrix((np.zeros(n), np.zeros(n, int), np.arange(n + 1)), shape=(n, 1))
+    b = np.random.default_rng(6).standard_normal(n)
+    x = np.zeros(n)
+    for _ in range(2):
+        for i in range(n):
+            s, d = b[i], 0.0
+            for k in range(A.indptr[i], A.indptr[i + 1]):
+                if A.indices[k] != i:
+                    s -= A.data[k] * x[A.indices[k]]
+                else:
+                    d = A.data[k]
+            x[i] = s / d
+    cls = native.CudaDuViGeometricMultigridSolver if fmt == "duvi" else native.CudaCsrGeometricMultigridSolver
+    launches = []
+    for sweeps in (1, 3):
+        s = cls(ctx, 0, 0.0, [True, False], [sweeps], GaussSeidel=True)
+        s.b = b
+        s.initialize_from_levels([A, sp.identity(1, format="csr")], [R], [P], False)
+        before = ctx.launch_count()
+        got, st, _ = s.Solve()
+        launches.append(ctx.launch_count() - before)
+        if sweeps == 1:
+            np.testing.assert_array_equal(got, x)
+        s.ReleaseCudaResources()
+    more = launches[1] - launches[0]
+    assert more == 0 if block else more >= 2 * levels

@@ -21,6 +21,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <limits>
 #include <vector>
 
 using namespace dvk;
@@ -139,7 +140,8 @@ extern "C" DV_API int dv_hex_assemble_device(dv_context *ctx, const int32_t *ne,
 
 // The numbers of Ke in its symmetry blocks (HexModes): (1/64) H Ke H with the signs (-1)^(s.b) of
 // character s and corner b.  Every entry outside the blocks is zero and every entry inside is one of
-// the eight numbers, up to rounding; another element stiffness is refused.
+// the eight numbers, up to rounding; another element stiffness is refused, and so is one with a NaN.  An
+// infinite stiffness has NaN numbers: then every node is formed from Ke itself (hex_node_direct).
 static void hex_modes(const double *ke, double (&out)[8]) {
     static const int vtk[8] = {0, 1, 3, 2, 4, 5, 7, 6};
     auto sign = [](int s, int b) { return __builtin_popcount(s & b) & 1 ? -1.0L : 1.0L; };
@@ -154,7 +156,14 @@ static void hex_modes(const double *ke, double (&out)[8]) {
     const long double v[8] = {mode(1, 0, 1, 0) - normal, normal, mode(3, 1, 3, 1), mode(3, 1, 5, 2),
                               mode(2, 0, 2, 0),          mode(7, 2, 7, 2), mode(6, 0, 6, 0) - high, high};
     for (int i = 0; i < 8; ++i) out[i] = (double)v[i];
-    const long double tol = 1e-13L * (std::abs(v[0]) + std::abs(v[1]));
+    bool infinite = false;
+    for (int i = 0; i < 576; ++i) {
+        DV_REQUIRE(!std::isnan(ke[i]), DV_ERR_UNSUPPORTED, "element stiffness with a NaN");
+        infinite |= std::isinf(ke[i]);
+    }
+    if (infinite) return;
+    // ke's own rounding: relative, and of a subnormal (a stiffness of 1e-310) absolute
+    const long double tol = 1e-13L * (std::abs(v[0]) + std::abs(v[1])) + 64 * std::numeric_limits<double>::denorm_min();
     for (int s = 0; s < 8; ++s)
         for (int d = 0; d < 3; ++d)
             for (int t = 0; t < 8; ++t)

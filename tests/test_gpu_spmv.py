@@ -610,3 +610,22 @@ def test_matrix_free_hex_operator_near_overflow(ctx, native, prec):
     got = _device_product(ctx, H, x, dt).astype(np.float64)
     assert np.all(np.isfinite(got))
     assert rowwise_rel(got * 2.0 ** -12, A @ (x * 2.0 ** -12), A, x * 2.0 ** -12) <= bar
+
+
+@pytest.mark.parametrize("E,nu", [(1.0, 0.0), (1.0, 0.499999999), (1e-312, 0.25), (1e-320, 0.3), (1e308, 0.3), (1.0, 0.5)])
+def test_matrix_free_hex_operator_extreme_materials(ctx, native, rng, E, nu):
+    # Every stiffness without a NaN is accepted, subnormal and infinite ones too, and its product is that of Ke's
+    # entries; a NaN (0 times an infinite modulus) is refused.
+    ne = (4, 3, 2)
+    H = native.SparseMatrix.hex_operator(ctx, ne, E=E, nu=nu)
+    A = native.hex_stiffness(ne, E=E, nu=nu)
+    x = rng.standard_normal(A.shape[1])
+    y = H.Multiply(x)
+    if 1e-300 < E and np.all(np.isfinite(A.data)):
+        assert rowwise_rel(y, A @ x, A, x) <= REL64
+    elif E < 1e-300:   # each of a row's at most 192 products rounds to a multiple of the smallest subnormal
+        assert np.max(np.abs(y - A @ x)) <= 200 * 2.0 ** -1074 + REL64 * np.max(abs(A) @ np.abs(x))
+    else:
+        assert not np.any(np.isfinite(y))
+    with pytest.raises(native.DuviError):
+        native.SparseMatrix.hex_operator(ctx, ne, E=0.0, nu=0.5)

@@ -200,8 +200,7 @@ extern "C" DV_API int dv_adjoint_create(dv_context *ctx, const int32_t *ne, cons
         std::vector<dv_csr_host> av, pv;
         for (auto &a : A) av.push_back(a.view());
         for (auto &p : P) pv.push_back(p.view());
-        int st = dv_mgpcg_create(ctx, (int32_t)av.size(), av.data(), pv.data(), cfg, &s->solver);
-        DV_REQUIRE(st == DV_OK, st, dv_last_error());
+        s->solver = dv_mgpcg_build(ctx, (int32_t)av.size(), av.data(), pv.data(), cfg).release();
         // The finest operator K(rho) has a factor per element and no repeating rows: the solver
         // applies it matrix-free (element kernel) in the outer FP64 loop and in the finest level
         // of the Jacobi V-cycle; the coarse Galerkin levels stay assembled.  DV_MATRIX_FREE=0
@@ -210,7 +209,7 @@ extern "C" DV_API int dv_adjoint_create(dv_context *ctx, const int32_t *ne, cons
         if (!(mf && mf[0] == '0') && cfg->smoother == DV_SMOOTHER_JACOBI) {
             dv_mgpcg *m = s->solver;
             dv_matrix *h64 = nullptr;
-            st = dv_matrix_create_hex(ctx, ne, scale_e.data(), 1.0, E0, nu, DV_F64, &h64);
+            int st = dv_matrix_create_hex(ctx, ne, scale_e.data(), 1.0, E0, nu, DV_F64, &h64);
             DV_REQUIRE(st == DV_OK, st, dv_last_error());
             m->Aout.reset(h64);
             if (m->v32) {
@@ -226,6 +225,7 @@ extern "C" DV_API int dv_adjoint_create(dv_context *ctx, const int32_t *ne, cons
             }
             s->matrix_free = true;
         }
+        s->solver->use_entries();
         // device copies
         cudaStream_t stream = ctx->stream;
         std::vector<double> ke(576);

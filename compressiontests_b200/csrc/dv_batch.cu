@@ -397,7 +397,6 @@ std::unique_ptr<BCycle<T>> build_bcycle(dv_batch *B, const int32_t *nlev, const 
             hr.nc = pv.n_rows;
             dv_csr_host rv = hr.view();
             L.R.reset(dv_matrix_build(ctx, rv, B->cfg.format, prec, 0, 1e-10));
-            for (dv_matrix *m : {L.A.get(), L.P.get(), L.R.get()}) dv_use_entries(m);
             for (double d : L.A->host_diag) DV_REQUIRE(d != 0.0, DV_ERR_SINGULAR, "zero diagonal entry");
             double om = B->cfg.omega;
             if (B->cfg.omega_mode == DV_OMEGA_SPECTRAL) {
@@ -620,85 +619,106 @@ void permute(dv_batch *B, const double *src, double *dst, bool to_internal, cuda
 
 }  // namespace
 
+// The batched solver without decoded entries, for a caller that replaces operators first.
+static std::unique_ptr<dv_batch> batch_build(dv_context *ctx, int32_t n_meshes, const int32_t *n_levels,
+                                             const dv_csr_host *const *A, const dv_csr_host *const *P,
+                                             const dv_mgpcg_config *cfg) {
+    DV_REQUIRE(ctx && n_levels && A && P && cfg && n_meshes >= 1, DV_ERR_ARG, "null argument");
+    DV_REQUIRE(cfg->precision == DV_F64 || cfg->precision == DV_MIXED, DV_ERR_ARG, "precision must be DV_F64 or DV_MIXED");
+    DV_REQUIRE(cfg->nu >= 1 && cfg->max_iterations >= 1 && cfg->tol > 0, DV_ERR_ARG, "bad smoothing or stop parameters");
+    DV_REQUIRE(cfg->smoother == DV_SMOOTHER_JACOBI, DV_ERR_UNSUPPORTED, "batched meshes smooth with weighted Jacobi only");
+    dv_ctx_check(ctx);
+    for (int32_t m = 0; m < n_meshes; ++m) {
+        DV_REQUIRE(n_levels[m] >= 1 && A[m] && (n_levels[m] == 1 || P[m]), DV_ERR_ARG, "mesh without levels");
+        for (int32_t l = 0; l < n_levels[m]; ++l)
+            DV_REQUIRE(A[m][l].n_rows == A[m][l].n_cols && A[m][l].n_rows >= 1, DV_ERR_ARG, "level operators must be square");
+        for (int32_t l = 0; l + 1 < n_levels[m]; ++l)
+            DV_REQUIRE(P[m][l].n_rows == A[m][l].n_rows && P[m][l].n_cols == A[m][l + 1].n_rows, DV_ERR_ARG,
+                       "prolongation shape does not match the levels");
+    }
+    auto B = std::make_unique<dv_batch>();
+    B->ctx = ctx;
+    B->cfg = *cfg;
+    B->nmesh = n_meshes;
+    B->order.resize(n_meshes);
+    std::iota(B->order.begin(), B->order.end(), 0);
+    std::stable_sort(B->order.begin(), B->order.end(), [&](int32_t a, int32_t b) { return n_levels[a] > n_levels[b]; });
+    B->nfine.resize(n_meshes);
+    B->user_off.assign(n_meshes + 1, 0);
+    for (int32_t m = 0; m < n_meshes; ++m) {
+        B->nfine[m] = A[m][0].n_rows;
+        B->user_off[m + 1] = B->user_off[m] + B->nfine[m];
+    }
+    DV_REQUIRE(B->user_off[n_meshes] < INT32_MAX, DV_ERR_ARG, "batch exceeds int32 rows");
+    B->n = (int32_t)B->user_off[n_meshes];
+    B->int_off.assign(n_meshes + 1, 0);
+    for (int32_t pos = 0; pos < n_meshes; ++pos) B->int_off[pos + 1] = B->int_off[pos] + B->nfine[B->order[pos]];
+    B->ws = std::make_unique<SolverWs>(ctx);
+    // outer FP64 operator over all meshes
+    {
+        std::vector<const dv_csr_host *> a0;
+        for (int32_t m : B->order) a0.push_back(&A[m][0]);
+        HostCsr h = blockdiag(a0);
+        dv_csr_host v = h.view();
+        B->Aout.reset(dv_matrix_build(ctx, v, cfg->outer_format, DV_F64, 0, 1e-10));
+    }
+    if (cfg->precision == DV_MIXED) B->c32 = build_bcycle<float>(B.get(), n_levels, A, P);
+    else B->c64 = build_bcycle<double>(B.get(), n_levels, A, P);
+    // reduction chunks: <= kChunkRows rows, never across a mesh
+    std::vector<int32_t> cseg, cbeg, cend, segc(1, 0), segof(B->n);
+    for (int32_t pos = 0; pos < n_meshes; ++pos) {
+        const int32_t r0 = (int32_t)B->int_off[pos], r1 = (int32_t)B->int_off[pos + 1];
+        for (int32_t r = r0; r < r1; r += kChunkRows) {
+            cseg.push_back(pos);
+            cbeg.push_back(r);
+            cend.push_back(std::min(r1, r + kChunkRows));
+        }
+        segc.push_back((int32_t)cseg.size());
+        std::fill(segof.begin() + r0, segof.begin() + r1, pos);
+    }
+    B->nchunks = (int32_t)cseg.size();
+    cudaStream_t st = ctx->stream;
+    auto up = [&](DevMem &d, const std::vector<int32_t> &v) {
+        d.alloc(4 * v.size());
+        DV_CUDA(cudaMemcpyAsync(d.p, v.data(), 4 * v.size(), cudaMemcpyHostToDevice, st));
+    };
+    up(B->chunk_seg, cseg);
+    up(B->chunk_begin, cbeg);
+    up(B->chunk_end, cend);
+    up(B->seg_chunk, segc);
+    up(B->seg_of, segof);
+    DV_CUDA(cudaStreamSynchronize(st));
+    const size_t nb = 8 * (size_t)B->n;
+    B->b.alloc(nb);
+    B->x.alloc(nb);
+    B->r.alloc(nb);
+    B->p.alloc(nb);
+    B->q.alloc(nb);
+    if (cfg->precision == DV_MIXED) B->r32.alloc(4 * (size_t)B->n);
+    B->ms.alloc(sizeof(MeshScalars) * (size_t)n_meshes);
+    B->red.alloc(64 + sizeof(double) * 2 * (size_t)B->nchunks);
+    return B;
+}
+
+// Small operators on their decoded entries (dv_use_entries), once every operator is the one kept.
+static void batch_use_entries(dv_batch *B) {
+    std::vector<dv_matrix *> ops{B->Aout.get()};
+    auto add = [&](auto &c) {
+        if (c)
+            for (auto &l : c->lv) ops.insert(ops.end(), {l.A.get(), l.P.get(), l.R.get()});
+    };
+    add(B->c32);
+    add(B->c64);
+    dv_use_entries(B->ctx, ops);
+}
+
 extern "C" DV_API int dv_batch_create(dv_context *ctx, int32_t n_meshes, const int32_t *n_levels,
                                       const dv_csr_host *const *A, const dv_csr_host *const *P,
                                       const dv_mgpcg_config *cfg, dv_batch **out) {
     return dv_guard([&] {
-        DV_REQUIRE(ctx && n_levels && A && P && cfg && out && n_meshes >= 1, DV_ERR_ARG, "null argument");
-        DV_REQUIRE(cfg->precision == DV_F64 || cfg->precision == DV_MIXED, DV_ERR_ARG, "precision must be DV_F64 or DV_MIXED");
-        DV_REQUIRE(cfg->nu >= 1 && cfg->max_iterations >= 1 && cfg->tol > 0, DV_ERR_ARG, "bad smoothing or stop parameters");
-        DV_REQUIRE(cfg->smoother == DV_SMOOTHER_JACOBI, DV_ERR_UNSUPPORTED, "batched meshes smooth with weighted Jacobi only");
-        dv_ctx_check(ctx);
-        for (int32_t m = 0; m < n_meshes; ++m) {
-            DV_REQUIRE(n_levels[m] >= 1 && A[m] && (n_levels[m] == 1 || P[m]), DV_ERR_ARG, "mesh without levels");
-            for (int32_t l = 0; l < n_levels[m]; ++l)
-                DV_REQUIRE(A[m][l].n_rows == A[m][l].n_cols && A[m][l].n_rows >= 1, DV_ERR_ARG, "level operators must be square");
-            for (int32_t l = 0; l + 1 < n_levels[m]; ++l)
-                DV_REQUIRE(P[m][l].n_rows == A[m][l].n_rows && P[m][l].n_cols == A[m][l + 1].n_rows, DV_ERR_ARG,
-                           "prolongation shape does not match the levels");
-        }
-        auto B = std::make_unique<dv_batch>();
-        B->ctx = ctx;
-        B->cfg = *cfg;
-        B->nmesh = n_meshes;
-        B->order.resize(n_meshes);
-        std::iota(B->order.begin(), B->order.end(), 0);
-        std::stable_sort(B->order.begin(), B->order.end(), [&](int32_t a, int32_t b) { return n_levels[a] > n_levels[b]; });
-        B->nfine.resize(n_meshes);
-        B->user_off.assign(n_meshes + 1, 0);
-        for (int32_t m = 0; m < n_meshes; ++m) {
-            B->nfine[m] = A[m][0].n_rows;
-            B->user_off[m + 1] = B->user_off[m] + B->nfine[m];
-        }
-        DV_REQUIRE(B->user_off[n_meshes] < INT32_MAX, DV_ERR_ARG, "batch exceeds int32 rows");
-        B->n = (int32_t)B->user_off[n_meshes];
-        B->int_off.assign(n_meshes + 1, 0);
-        for (int32_t pos = 0; pos < n_meshes; ++pos) B->int_off[pos + 1] = B->int_off[pos] + B->nfine[B->order[pos]];
-        B->ws = std::make_unique<SolverWs>(ctx);
-        // outer FP64 operator over all meshes
-        {
-            std::vector<const dv_csr_host *> a0;
-            for (int32_t m : B->order) a0.push_back(&A[m][0]);
-            HostCsr h = blockdiag(a0);
-            dv_csr_host v = h.view();
-            B->Aout.reset(dv_matrix_build(ctx, v, cfg->outer_format, DV_F64, 0, 1e-10));
-            dv_use_entries(B->Aout.get());
-        }
-        if (cfg->precision == DV_MIXED) B->c32 = build_bcycle<float>(B.get(), n_levels, A, P);
-        else B->c64 = build_bcycle<double>(B.get(), n_levels, A, P);
-        // reduction chunks: <= kChunkRows rows, never across a mesh
-        std::vector<int32_t> cseg, cbeg, cend, segc(1, 0), segof(B->n);
-        for (int32_t pos = 0; pos < n_meshes; ++pos) {
-            const int32_t r0 = (int32_t)B->int_off[pos], r1 = (int32_t)B->int_off[pos + 1];
-            for (int32_t r = r0; r < r1; r += kChunkRows) {
-                cseg.push_back(pos);
-                cbeg.push_back(r);
-                cend.push_back(std::min(r1, r + kChunkRows));
-            }
-            segc.push_back((int32_t)cseg.size());
-            std::fill(segof.begin() + r0, segof.begin() + r1, pos);
-        }
-        B->nchunks = (int32_t)cseg.size();
-        cudaStream_t st = ctx->stream;
-        auto up = [&](DevMem &d, const std::vector<int32_t> &v) {
-            d.alloc(4 * v.size());
-            DV_CUDA(cudaMemcpyAsync(d.p, v.data(), 4 * v.size(), cudaMemcpyHostToDevice, st));
-        };
-        up(B->chunk_seg, cseg);
-        up(B->chunk_begin, cbeg);
-        up(B->chunk_end, cend);
-        up(B->seg_chunk, segc);
-        up(B->seg_of, segof);
-        DV_CUDA(cudaStreamSynchronize(st));
-        const size_t nb = 8 * (size_t)B->n;
-        B->b.alloc(nb);
-        B->x.alloc(nb);
-        B->r.alloc(nb);
-        B->p.alloc(nb);
-        B->q.alloc(nb);
-        if (cfg->precision == DV_MIXED) B->r32.alloc(4 * (size_t)B->n);
-        B->ms.alloc(sizeof(MeshScalars) * (size_t)n_meshes);
-        B->red.alloc(64 + sizeof(double) * 2 * (size_t)B->nchunks);
+        DV_REQUIRE(out, DV_ERR_ARG, "null argument");
+        auto B = batch_build(ctx, n_meshes, n_levels, A, P, cfg);
+        batch_use_entries(B.get());
         *out = B.release();
     });
 }
@@ -758,10 +778,7 @@ extern "C" DV_API int dv_batch_create_hex(dv_context *ctx, int32_t n_meshes, con
             pp[m] = pv[m].data();
             nlev[m] = (int32_t)A[m].size();
         }
-        dv_batch *B = nullptr;
-        int st = dv_batch_create(ctx, n_meshes, nlev.data(), ap.data(), pp.data(), cfg, &B);
-        DV_REQUIRE(st == DV_OK, st, dv_last_error());
-        std::unique_ptr<dv_batch, int (*)(dv_batch *)> guard(B, dv_batch_destroy);
+        auto B = batch_build(ctx, n_meshes, nlev.data(), ap.data(), pp.data(), cfg);
         // the finest operators applied matrix-free: the outer FP64 one over every mesh, the V-cycle's level 0
         // over the meshes that smooth there (internal order, the block-diagonal layout of the batch)
         const char *mf = getenv("DV_MATRIX_FREE");
@@ -778,7 +795,8 @@ extern "C" DV_API int dv_batch_create_hex(dv_context *ctx, int32_t n_meshes, con
                 else B->c64->lv[0].A.reset(dv_hex_operator_build(ctx, ns, smoothed.data(), nullptr, 1.0, E, nu, DV_F64));
             }
         }
-        *out = guard.release();
+        batch_use_entries(B.get());
+        *out = B.release();
     });
 }
 

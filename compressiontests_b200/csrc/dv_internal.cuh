@@ -353,9 +353,9 @@ dv_matrix *dv_trilinear_build(dv_context *ctx, const int32_t *ne_fine, int restr
 // Matrix-free hexahedral operator of nmesh meshes placed block-diagonally (dv_assemble.cu).
 dv_matrix *dv_hex_operator_build(dv_context *ctx, int32_t nmesh, const int32_t *ne, const double *elem_E, double scale,
                                  double E, double nu, int32_t precision);
-// Decodes a solver's own small DuVi operator into columns and values and lets its products run on
-// them (dv_matrix.cu).
-void dv_use_entries(dv_matrix *m);
+// Decodes a solver's own small DuVi operators into columns and values and lets their products run on
+// them (dv_matrix.cu): the operators it keeps, once all are in place (null pointers are skipped).
+void dv_use_entries(dv_context *ctx, const std::vector<dv_matrix *> &operators);
 // Times the launch shapes of m's product and keeps the fastest (matrices of >= 100k rows).
 void dv_autotune(dv_matrix *m);
 

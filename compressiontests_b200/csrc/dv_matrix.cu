@@ -381,21 +381,26 @@ void dv_autotune(dv_matrix *m) { autotune(m); }
 // The grid's line holds for every matrix that has the grid layout, whatever the trial launches chose: with a
 // 104,544-row level of the 128^3 hierarchy on its 47 MB of entries the mixed solve took 6.97 ms, on the grid 6.62.
 // DV_ENTRIES=<MB> moves the line (0: never; A/B comparisons).
-void dv_use_entries(dv_matrix *m) {
-    int64_t limit = (m->grid_ok ? 12ll : 48ll) << 20;
-    if (const char *v = getenv("DV_ENTRIES")) limit = atoll(v) << 20;
-    if (m->format != DV_FORMAT_DUVI || m->entries_ok || m->n_rows == 0) return;
-    const int64_t vs = m->precision == DV_F64 ? 8 : 4;
-    const bool nodes = m->row_group == 3 && !m->lanes_shift && !m->pat_shift && m->n_rows % 3 == 0;
-    const double mean_nnz = (double)m->nnz / m->n_rows;
-    if (m->nnz * vs + m->nnz * 4 / (nodes ? 3 : 1) > limit || (!nodes && mean_nnz > 32)) return;
-    m->col.alloc(4 * (size_t)m->nnz);
-    m->val.alloc(vs * (size_t)m->nnz);
-    if (m->precision == DV_F64) dvk::duvi_decode<double>(m, m->col.as<int32_t>(), m->val.as<double>());
-    else dvk::duvi_decode<float>(m, m->col.as<int32_t>(), m->val.as<float>());
-    m->csr_tpr = nodes ? row_lanes(3, mean_nnz) : 1;
-    DV_CUDA(cudaStreamSynchronize(m->ctx->stream));
-    m->entries_ok = 1;
+void dv_use_entries(dv_context *ctx, const std::vector<dv_matrix *> &operators) {
+    std::vector<dv_matrix *> decoded;
+    for (dv_matrix *m : operators) {
+        if (!m || m->format != DV_FORMAT_DUVI || m->entries_ok || m->n_rows == 0) continue;
+        int64_t limit = (m->grid_ok ? 12ll : 48ll) << 20;
+        if (const char *v = getenv("DV_ENTRIES")) limit = atoll(v) << 20;
+        const int64_t vs = m->precision == DV_F64 ? 8 : 4;
+        const bool nodes = m->row_group == 3 && !m->lanes_shift && !m->pat_shift && m->n_rows % 3 == 0;
+        const double mean_nnz = (double)m->nnz / m->n_rows;
+        if (m->nnz * vs + m->nnz * 4 / (nodes ? 3 : 1) > limit || (!nodes && mean_nnz > 32)) continue;
+        m->col.alloc(4 * (size_t)m->nnz);
+        m->val.alloc(vs * (size_t)m->nnz);
+        if (m->precision == DV_F64) dvk::duvi_decode<double>(m, m->col.as<int32_t>(), m->val.as<double>());
+        else dvk::duvi_decode<float>(m, m->col.as<int32_t>(), m->val.as<float>());
+        m->csr_tpr = nodes ? row_lanes(3, mean_nnz) : 1;
+        decoded.push_back(m);
+    }
+    if (decoded.empty()) return;
+    DV_CUDA(cudaStreamSynchronize(ctx->stream));
+    for (dv_matrix *m : decoded) m->entries_ok = 1;
 }
 
 dv_matrix *dv_matrix_build(dv_context *ctx, const dv_csr_host &a, int format, int precision, int vi_bits, double tol,

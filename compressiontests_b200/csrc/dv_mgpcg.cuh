@@ -148,6 +148,21 @@ struct dv_mgpcg {
     std::vector<double> omega_eff;
     int64_t launches_last = 0;
     MultiHolder *multi = nullptr;   // block (multi-right-hand-side) work buffers, created on first use
+    // Small operators on their decoded entries (dv_use_entries); called when every operator is the one kept.
+    void use_entries() {
+        std::vector<dv_matrix *> ops{Aout.get()};
+        auto add = [&](auto &v) {
+            if (v)
+                for (auto &l : v->lv) ops.insert(ops.end(), {l.A.get(), l.P.get(), l.R.get()});
+        };
+        add(v32);
+        add(v64);
+        dv_use_entries(ctx, ops);
+    }
     ~dv_mgpcg() { dv_mgpcg_multi_release(multi); }
 };
+
+// dv_mgpcg_create without use_entries, for a caller that replaces operators first.
+std::unique_ptr<dv_mgpcg> dv_mgpcg_build(dv_context *ctx, int32_t L, const dv_csr_host *A, const dv_csr_host *P,
+                                         const dv_mgpcg_config *cfg);
 

@@ -491,7 +491,6 @@ static std::unique_ptr<VCycle<T>> build_vcycle(dv_context *ctx, SolverWs &ws, in
             dv_csr_host rt{P[l].n_cols, P[l].n_rows, rp.data(), ci.data(), va.data()};
             lv.R.reset(dv_matrix_build(ctx, rt, cfg.format, prec, 0, 1e-10));
         }
-        for (dv_matrix *m : {lv.A.get(), lv.P.get(), lv.R.get()}) dv_use_entries(m);
         for (double d : lv.A->host_diag) DV_REQUIRE(d != 0.0, DV_ERR_SINGULAR, "zero diagonal entry");
         double om = cfg.omega;
         if (cfg.omega_mode == DV_OMEGA_SPECTRAL) {
@@ -600,10 +599,7 @@ extern "C" DV_API int dv_mgpcg_create_hex(dv_context *ctx, const int32_t *ne, do
                 dv_autotune(m.get());
                 return m;
             };
-            if (l == 0) {
-                s->Aout = build(DV_F64);
-                dv_use_entries(s->Aout.get());
-            }
+            if (l == 0) s->Aout = build(DV_F64);
             prebuilt.push_back(build(prec));
             Ash[l] = dv_csr_host{nr, nr, nullptr, nullptr, nullptr};
             // trilinear prolongation to this level from the next: matrix-free, or host CSR when
@@ -637,41 +633,49 @@ extern "C" DV_API int dv_mgpcg_create_hex(dv_context *ctx, const int32_t *ne, do
             s->wb32.alloc(4 * (size_t)s->n);
         }
         DV_CUDA(cudaStreamSynchronize(st));
+        s->use_entries();
         *out = s.release();
     });
+}
+
+std::unique_ptr<dv_mgpcg> dv_mgpcg_build(dv_context *ctx, int32_t L, const dv_csr_host *A, const dv_csr_host *P,
+                                         const dv_mgpcg_config *cfg) {
+    DV_REQUIRE(A && cfg && L >= 1 && (L == 1 || P), DV_ERR_ARG, "null argument");
+    check_mgpcg_config(cfg);
+    DV_REQUIRE(L >= 2, DV_ERR_ARG, "need at least two levels");
+    dv_ctx_check(ctx);
+    auto s = std::make_unique<dv_mgpcg>();
+    s->ctx = ctx;
+    s->cfg = *cfg;
+    s->ws = std::make_unique<SolverWs>(ctx);
+    s->n = A[0].n_rows;
+    // the finest operator is encoded once for the outer matrix and the V-cycle's level 0
+    const bool outer_duvi = cfg->outer_format == DV_FORMAT_DUVI, inner_duvi = cfg->format == DV_FORMAT_DUVI;
+    DuviHost h0;
+    if (outer_duvi && inner_duvi) {
+        dv_check_csr(A[0]);
+        dv_encode_duvi(A[0], 1e-10, 0, h0);
+    }
+    const DuviHost *shared = outer_duvi && inner_duvi ? &h0 : nullptr;
+    s->Aout.reset(dv_matrix_build(ctx, A[0], cfg->outer_format, DV_F64, 0, 1e-10, shared));
+    if (cfg->precision == DV_MIXED) s->v32 = build_vcycle<float>(ctx, *s->ws, L, A, P, *cfg, s->omega_eff, shared);
+    else s->v64 = build_vcycle<double>(ctx, *s->ws, L, A, P, *cfg, s->omega_eff, shared);
+    const size_t nb = 8 * (size_t)s->n;
+    s->b.alloc(nb); s->x.alloc(nb); s->r.alloc(nb); s->p.alloc(nb); s->q.alloc(nb);
+    if (cfg->precision == DV_MIXED) {
+        s->r32.alloc(4 * (size_t)s->n);
+        s->wb32.alloc(4 * (size_t)s->n);
+    }
+    DV_CUDA(cudaStreamSynchronize(ctx->stream));
+    return s;
 }
 
 extern "C" DV_API int dv_mgpcg_create(dv_context *ctx, int32_t L, const dv_csr_host *A, const dv_csr_host *P,
                                       const dv_mgpcg_config *cfg, dv_mgpcg **out) {
     return dv_guard([&] {
-        DV_REQUIRE(A && cfg && out && L >= 1 && (L == 1 || P), DV_ERR_ARG, "null argument");
-        check_mgpcg_config(cfg);
-        DV_REQUIRE(L >= 2, DV_ERR_ARG, "need at least two levels");
-        dv_ctx_check(ctx);
-        auto s = std::make_unique<dv_mgpcg>();
-        s->ctx = ctx;
-        s->cfg = *cfg;
-        s->ws = std::make_unique<SolverWs>(ctx);
-        s->n = A[0].n_rows;
-        // the finest operator is encoded once for the outer matrix and the V-cycle's level 0
-        const bool outer_duvi = cfg->outer_format == DV_FORMAT_DUVI, inner_duvi = cfg->format == DV_FORMAT_DUVI;
-        DuviHost h0;
-        if (outer_duvi && inner_duvi) {
-            dv_check_csr(A[0]);
-            dv_encode_duvi(A[0], 1e-10, 0, h0);
-        }
-        const DuviHost *shared = outer_duvi && inner_duvi ? &h0 : nullptr;
-        s->Aout.reset(dv_matrix_build(ctx, A[0], cfg->outer_format, DV_F64, 0, 1e-10, shared));
-        dv_use_entries(s->Aout.get());
-        if (cfg->precision == DV_MIXED) s->v32 = build_vcycle<float>(ctx, *s->ws, L, A, P, *cfg, s->omega_eff, shared);
-        else s->v64 = build_vcycle<double>(ctx, *s->ws, L, A, P, *cfg, s->omega_eff, shared);
-        const size_t nb = 8 * (size_t)s->n;
-        s->b.alloc(nb); s->x.alloc(nb); s->r.alloc(nb); s->p.alloc(nb); s->q.alloc(nb);
-        if (cfg->precision == DV_MIXED) {
-            s->r32.alloc(4 * (size_t)s->n);
-            s->wb32.alloc(4 * (size_t)s->n);
-        }
-        DV_CUDA(cudaStreamSynchronize(ctx->stream));
+        DV_REQUIRE(out, DV_ERR_ARG, "null argument");
+        auto s = dv_mgpcg_build(ctx, L, A, P, cfg);
+        s->use_entries();
         *out = s.release();
     });
 }

@@ -507,3 +507,26 @@ def test_gauss_seidel_row_order_wide_levels(ctx, native, fmt, levels, width, gro
         s.ReleaseCudaResources()
     more = launches[1] - launches[0]
     assert more == 0 if block else more >= 2 * levels
+
+
+def test_decoded_entries_of_kept_operators_only(ctx, native, monkeypatch):
+    # A solver's small DuVi operators are decoded once all are in place: one launch each, none for the finest operators
+    # that the adjoint and the batch replace by the matrix-free one.
+    def decodes(make):
+        counts = []
+        for limit in ("0", None):
+            monkeypatch.delenv("DV_ENTRIES", raising=False)
+            if limit is not None:
+                monkeypatch.setenv("DV_ENTRIES", limit)
+            before = ctx.launch_count()
+            s = make()
+            counts.append(ctx.launch_count() - before)
+            s.release()
+        return counts[1] - counts[0]
+
+    ne, rho = (8, 4, 4), np.random.default_rng(1).uniform(0.1, 1.0, 8 * 4 * 4)
+    assert decodes(lambda: native.AdjointCantilever(ctx, ne, rho, max_coarse_dofs=300)) == 2   # P and R
+    assert decodes(lambda: native.BatchedMultigridSolver.from_hex(ctx, [ne, (6, 4, 5)], max_coarse_dofs=300)) == 2
+    A, P = native.hex_hierarchy(ne, coarse_ne=2)
+    assert decodes(lambda: native.MultigridPcgSolver(ctx, A, P, precision="mixed", fmt="duvi")) == 4   # outer, A, P, R
+    assert decodes(lambda: native.MultigridPcgSolver.from_hex(ctx, ne, coarse_ne=2)) == 2   # outer, A

@@ -376,26 +376,51 @@ void dv_autotune(dv_matrix *m) { autotune(m); }
 // Measured with against without: solve of 12 uneven meshes 3.43 -> 2.53 ms, adjoint pair 48x24x24 10.4
 // -> 6.6 ms, mixed solve 16^3 1.31 -> 0.99 ms (a 12,168-row level's sweep 25.7 us on the lane layout, 16
 // blocks).  The line against the grid stencil, by mixed and FP64 solves: 6.0 and 9.4 MB of entries (16^3
-// in FP32 and FP64) gain 12 and 16 %, 20 MB (24^3 in FP32) lose 14 %; the other layouts are further behind
-// and give way as long as the entries stay in the 126 MB L2 cache beside the vectors.
+// in FP32 and FP64) gain 12 and 16 %, 20 MB (24^3 in FP32) lose 14 %.  The other layouts are further behind: a host-built
+// hierarchy of 32 x 26 x 25 elements (outer and finest operator 47 MB each in FP64) solves in 4.07 ms on
+// the lane layout, in 2.74 with both decoded, although their sum of 106 MB does not stay in the L2 cache beside the vectors.
+// Their line bounds the memory: four operators of a solver can be that large (outer, finest, its transfers), so
+// the copies take 220 MB at most; the smallest are made first, and one that has no room is not made.
 // The grid's line holds for every matrix that has the grid layout, whatever the trial launches chose: with a
 // 104,544-row level of the 128^3 hierarchy on its 47 MB of entries the mixed solve took 6.97 ms, on the grid 6.62.
 // DV_ENTRIES=<MB> moves the line (0: never; A/B comparisons).
 void dv_use_entries(dv_context *ctx, const std::vector<dv_matrix *> &operators) {
-    std::vector<dv_matrix *> decoded;
+    int64_t line = 48ll << 20, grid_line = 12ll << 20;   // bytes an operator
+    if (const char *v = getenv("DV_ENTRIES")) line = grid_line = atoll(v) << 20;
+    struct Candidate {
+        dv_matrix *m;
+        int64_t bytes;
+        bool nodes;
+    };
+    std::vector<Candidate> candidates;
     for (dv_matrix *m : operators) {
         if (!m || m->format != DV_FORMAT_DUVI || m->entries_ok || m->n_rows == 0) continue;
-        int64_t limit = (m->grid_ok ? 12ll : 48ll) << 20;
-        if (const char *v = getenv("DV_ENTRIES")) limit = atoll(v) << 20;
         const int64_t vs = m->precision == DV_F64 ? 8 : 4;
         const bool nodes = m->row_group == 3 && !m->lanes_shift && !m->pat_shift && m->n_rows % 3 == 0;
-        const double mean_nnz = (double)m->nnz / m->n_rows;
-        if (m->nnz * vs + m->nnz * 4 / (nodes ? 3 : 1) > limit || (!nodes && mean_nnz > 32)) continue;
-        m->col.alloc(4 * (size_t)m->nnz);
-        m->val.alloc(vs * (size_t)m->nnz);
+        const int64_t bytes = m->nnz * vs + m->nnz * 4 / (nodes ? 3 : 1);   // of a product's reads
+        if (bytes <= (m->grid_ok ? grid_line : line) && (nodes || m->nnz <= 32 * (int64_t)m->n_rows))
+            candidates.push_back({m, bytes, nodes});
+    }
+    std::stable_sort(candidates.begin(), candidates.end(),
+                     [](const Candidate &a, const Candidate &b) { return a.bytes < b.bytes; });
+    std::vector<dv_matrix *> decoded;
+    for (const Candidate &c : candidates) {
+        dv_matrix *m = c.m;
+        DevMem col, val;
+        try {
+            col.alloc(4 * (size_t)m->nnz);
+            val.alloc((m->precision == DV_F64 ? 8 : 4) * (size_t)m->nnz);
+        } catch (const DvError &e) {   // no room for a copy: this operator and the larger ones stay on their layouts
+            if (e.code != DV_ERR_NOMEM) throw;
+            cudaGetLastError();
+            break;
+        }
+        m->col = std::move(col);
+        m->val = std::move(val);
         if (m->precision == DV_F64) dvk::duvi_decode<double>(m, m->col.as<int32_t>(), m->val.as<double>());
         else dvk::duvi_decode<float>(m, m->col.as<int32_t>(), m->val.as<float>());
-        m->csr_tpr = nodes ? row_lanes(3, mean_nnz) : 1;
+        m->csr_tpr = c.nodes ? row_lanes(3, (double)m->nnz / m->n_rows) : 1;
+        m->device_bytes = c.bytes + 4 * ((int64_t)m->n_rows + 1);
         decoded.push_back(m);
     }
     if (decoded.empty()) return;

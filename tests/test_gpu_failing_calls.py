@@ -1,0 +1,84 @@
+"""CUDA calls that fail: what the library does when an allocation has no room or a launch is refused.
+
+The failure comes from a stand-in for the runtime's entry point, preloaded into a child process: it returns the
+error code and calls nothing, so the GPU is not involved in it.
+"""
+import json
+import os
+import subprocess
+import sys
+
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+STAND_IN = r"""
+#define _GNU_SOURCE
+#include <dlfcn.h>
+#include <stddef.h>
+static size_t lo = 1, hi = 0;   /* allocations of lo .. hi bytes fail */
+static int fail_cooperative, failed;
+void fail_allocations(size_t from, size_t to) { lo = from; hi = to; }
+void fail_cooperative_launches(int on) { fail_cooperative = on; }
+int failed_calls(void) { return failed; }
+static void *real(const char *name) {
+    void *lib = dlopen("libcudart.so.12", RTLD_LAZY | RTLD_NOLOAD);
+    return dlsym(lib, name);
+}
+int cudaMalloc(void **p, size_t bytes) {
+    if (bytes >= lo && bytes <= hi) { failed++; return 2; }   /* cudaErrorMemoryAllocation */
+    return ((int (*)(void **, size_t))real("cudaMalloc"))(p, bytes);
+}
+typedef struct { unsigned x, y, z; } Dim;
+int cudaLaunchCooperativeKernel(const void *f, Dim grid, Dim block, void **args, size_t smem, void *stream) {
+    if (fail_cooperative) { failed++; return 720; }   /* cudaErrorCooperativeLaunchTooLarge */
+    return ((int (*)(const void *, Dim, Dim, void **, size_t, void *))real("cudaLaunchCooperativeKernel"))(f, grid, block, args,
+                                                                                                           smem, stream);
+}
+"""
+PRELUDE = """
+import ctypes, json, sys
+import numpy as np
+import compressiontests_b200 as cb
+fake = ctypes.CDLL(None)
+fake.fail_allocations.argtypes = [ctypes.c_size_t, ctypes.c_size_t]
+ctx = cb.CudaContext(0)
+"""
+
+
+@pytest.fixture(scope="module")
+def child(tmp_path_factory):
+    """Runs a script in a process with the stand-in loaded first; the script prints one JSON line."""
+    d = tmp_path_factory.mktemp("stand_in")
+    (d / "f.c").write_text(STAND_IN)
+    subprocess.run(["gcc", "-shared", "-fPIC", "-O1", "-o", str(d / "f.so"), str(d / "f.c"), "-ldl"], check=True)
+
+    def run(script):
+        env = dict(os.environ, LD_PRELOAD=str(d / "f.so"), PYTHONPATH=ROOT)
+        r = subprocess.run([sys.executable, "-c", PRELUDE + script], cwd=ROOT, env=env, capture_output=True, text=True, timeout=300)
+        assert r.returncode == 0, r.stdout + r.stderr
+        return json.loads(r.stdout.strip().splitlines()[-1])
+
+    return run
+
+
+def test_solver_without_room_for_decoded_entries(child):
+    # The decoded copy of the outer operator has no room: the solver keeps that operator on its layout and solves as with the copy.
+    r = child("""
+ne = (12, 8, 8)
+A, P = cb.hex_hierarchy(ne, coarse_ne=4)
+b = cb.traction_rhs(ne)
+out = []
+for fail in (False, True):
+    n = 8 * A[0].nnz + 64
+    if fail: fake.fail_allocations(n, n)
+    s = cb.MultigridPcgSolver(ctx, A, P, precision="mixed", fmt="duvi")
+    fake.fail_allocations(1, 0)
+    x, st = s.Solve(b)
+    out.append((x, st.HasConverged, st.NumIterationsRequired))
+print(json.dumps(dict(failed=fake.failed_calls(), ok=[o[1] for o in out], its=[o[2] for o in out],
+                      diff=float(np.max(np.abs(out[0][0] - out[1][0])) / np.max(np.abs(out[0][0]))))))
+""")
+    # two solves to a relative residual of 1e-8, each within 1e-6 of the solution
+    assert r["failed"] == 1 and r["ok"] == [True, True] and r["its"][0] == r["its"][1] and r["diff"] < 2e-6, r

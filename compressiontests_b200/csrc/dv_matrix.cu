@@ -320,10 +320,12 @@ static void autotune(dv_matrix *m) {
             dvk::launch_rows<float>(e, m, dvk::GatherVec<float, float>{x.as<float>()}, op);
         }
     };
-    // CSR: threads per row; DuVi: 4 / 9 = staged kernel with that batch width, 100 = lane kernel
-    // (48 / 96: 16 / 32 lanes per 3-row node group, where the rows come in such groups)
+    // CSR: threads per row, and where row_lanes takes the node kernel 48 / 96 = 16 / 32 lanes per 3-row node group
+    // (600,000 rows in groups, best width of the row kernel against the node kernel: 9 entries 25.7 against 30.8 us, 16
+    // entries 28.6 against 35.1, 27 entries 38.3 against 40.3, 81 entries 104.7 against 81.4);
+    // DuVi: 4 / 9 = staged kernel with that batch width, 100 = lane kernel
     std::vector<int> cand = m->format == DV_FORMAT_CSR ? std::vector<int>{8, 16, 32} : std::vector<int>{4, 9};
-    if (m->format == DV_FORMAT_CSR && m->row_group == 3) cand = {3 * 16, 3 * 32};
+    if (m->format == DV_FORMAT_CSR && m->csr_tpr >= 3 * 16) cand.insert(cand.end(), {3 * 16, 3 * 32});
     if (m->format == DV_FORMAT_DUVI && m->lanes_ok) cand.push_back(100);
     if (m->format == DV_FORMAT_DUVI && m->pat_ok) cand.push_back(200);
     if (m->format == DV_FORMAT_DUVI && m->grid_ok) cand.push_back(300);

@@ -629,3 +629,18 @@ def test_matrix_free_hex_operator_extreme_materials(ctx, native, rng, E, nu):
         assert not np.any(np.isfinite(y))
     with pytest.raises(native.DuviError):
         native.SparseMatrix.hex_operator(ctx, ne, E=0.0, nu=0.5)
+
+
+@pytest.mark.parametrize("width,variants", [(9, (8, 16, 32)), (15, (8, 16, 32)), (16, (8, 16, 32, 48, 96)), (81, (48, 96))])
+def test_csr_trials_keep_the_rule(ctx, native, rng, width, variants):
+    # Matrices large enough for trial launches, rows in groups of 3 with one column list: short rows stay on the row
+    # kernel, whose widths are tried (below 16 entries most lanes of the node kernel idle); 81 entries end on the node kernel.
+    ng = 34000
+    first = rng.integers(0, 3 * ng - width, ng)
+    cols = np.repeat(first[:, None] + np.arange(width), 3, axis=0).ravel()
+    A = sp.csr_matrix((rng.standard_normal(cols.size), cols, width * np.arange(3 * ng + 1)), shape=(3 * ng, 3 * ng))
+    M = native.SparseMatrix(ctx, A, "csr", "f64")
+    info = M.info()
+    assert info["row_group"] == 3 and info["kernel_variant"] in variants
+    x = rng.standard_normal(A.shape[1])
+    assert rowwise_rel(M.Multiply(x), A @ x, A, x) <= REL64

@@ -200,7 +200,7 @@ struct dv_matrix {
     int precision = DV_F64;
     // CSR
     DevMem rowptr, col, val;
-    int csr_tpr = 16;          // threads per row (autotuned)
+    int csr_tpr = 16;          // threads per row (autotuned), or 3 x the lanes per node group
     int entries_ok = 0;        // DuVi: columns and values also decoded into col / val (dv_use_entries)
     // DuVi SoA
     int vi_bits = 8;

@@ -2252,6 +2252,15 @@ void launch_rows(const LaunchEnv &e, const dv_matrix *m, Gather g, Op op) {
     launch_csr<AT>(e, m, g, op);
 }
 
+// r = b - A x for the residual that a PCG solve reports.  Close to the limit of FP64 its last digits depend on the order
+// of the row sums, so it does not follow the kernel that is fastest for the iterations: CSR rows are summed one
+// thread a row in the stored order, as DuVi rows are and as a host would.
+template <class Gather, class Op>
+void launch_reported_residual(const LaunchEnv &e, const dv_matrix *m, Gather g, Op op) {
+    if (m->format == DV_FORMAT_CSR) launch_csr_tpr<1, double>(e, m, g, op);
+    else launch_rows<double>(e, m, g, op);
+}
+
 // ---------------------------------------------------------------------------
 // vector kernels
 // ---------------------------------------------------------------------------

@@ -223,14 +223,10 @@ extern "C" DV_API int dv_pcg_solve_noalloc(dv_matrix *A, const double *d_b, doub
             DV_CUDA(cudaMemcpyAsync(&h, sc, sizeof(h), cudaMemcpyDeviceToHost, st));
             DV_CUDA(cudaStreamSynchronize(st));
         }
-        // relative residual of the returned x in FP64: z = b - A x (z is free now), ||b||, ||z||.  Close to the
-        // limit of FP64 its last digits depend on the order of the row sums: a small system's CSR rows are
-        // summed one thread a row in the stored order, as DuVi rows are and as a host would.
+        // relative residual of the returned x in FP64: z = b - A x (z is free now), ||b||, ||z||
         {
             OpResid<double> op{{}, d_b, z};
-            const GatherVec<double, double> x{d_x};
-            if (resident && A->format == DV_FORMAT_CSR) launch_csr_tpr<1, double>(e, A, x, op);
-            else launch_rows<double>(e, A, x, op);
+            launch_reported_residual(e, A, GatherVec<double, double>{d_x}, op);
             k_na_norms<<<grid, kThreads, 0, st>>>(d_b, z, n, sc, partials, ticket);
             DV_CUDA(cudaGetLastError());
             ctx->count();

@@ -412,14 +412,10 @@ extern "C" DV_API int dv_pcg_solve(dv_pcg *s, const double *b, const double *x0,
         }
         DV_CUDA(cudaEventRecord(e1, st));
         DV_CUDA(cudaMemcpyAsync(xout, s->x.p, nb, cudaMemcpyDeviceToHost, st));
-        // relative residual of the returned x, recomputed in FP64: z = b - A x, ||z||^2.  Close to the limit of
-        // FP64 its last digits depend on the order of the row sums: a small system's CSR rows are summed
-        // one thread a row in the stored order, as DuVi rows are and as a host would.
+        // relative residual of the returned x, recomputed in FP64: z = b - A x, ||z||^2
         {
             OpResid<double> op{{}, s->b.as<double>(), s->z.as<double>()};
-            const GatherVec<double, double> x{s->x.as<double>()};
-            if (s->work.p && s->A->format == DV_FORMAT_CSR) launch_csr_tpr<1, double>(e, s->A.get(), x, op);
-            else launch_rows<double>(e, s->A.get(), x, op);
+            launch_reported_residual(e, s->A.get(), GatherVec<double, double>{s->x.as<double>()}, op);
             k_norm2<<<g, kThreads, 0, st>>>(s->z.as<double>(), n, s->ws->sc(), 1, e.partials, e.ticket);
             DV_CUDA(cudaGetLastError());
             ctx->count();

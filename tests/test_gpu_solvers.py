@@ -530,3 +530,26 @@ def test_decoded_entries_of_kept_operators_only(ctx, native, monkeypatch):
     A, P = native.hex_hierarchy(ne, coarse_ne=2)
     assert decodes(lambda: native.MultigridPcgSolver(ctx, A, P, precision="mixed", fmt="duvi")) == 4   # outer, A, P, R
     assert decodes(lambda: native.MultigridPcgSolver.from_hex(ctx, ne, coarse_ne=2)) == 2   # outer, A
+
+
+@pytest.mark.parametrize("ne", [(16, 4, 4), (33, 32, 31), (36, 32, 32)])
+def test_pcg_reports_the_stored_order_residual(ctx, native, ne):
+    # Solved to where rounding dominates the residual, on both sides of the one-kernel solve's size: the relative residual
+    # that is reported is that of the returned x with every row summed in the stored order, as numpy does here.
+    A = native.hex_stiffness(ne)
+    b = native.traction_rhs(ne)
+    s = native.CudaCsrPcgSolver(ctx, 20000, 1e-13, fmt="csr", tol_kind="rel_l2").Initialize(A=A, b=b)
+    x, st = s.Solve()
+    s.ReleaseCudaResources()
+    r = b.copy()
+    sums = np.zeros_like(b)
+    length = np.diff(A.indptr)
+    for k in range(int(length.max())):   # entry k of every row that has one
+        rows = np.nonzero(length > k)[0]
+        at = A.indptr[rows] + k
+        sums[rows] += A.data[at] * x[A.indices[at]]
+    r -= sums
+    true_rel = np.linalg.norm(r) / np.linalg.norm(b)
+    assert true_rel < 1e-11
+    # the two norms of n terms are summed in another order
+    assert abs(st.RelativeResidual - true_rel) <= 2 * len(b) * 2.0 ** -53 * true_rel

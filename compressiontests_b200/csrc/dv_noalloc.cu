@@ -202,9 +202,8 @@ extern "C" DV_API int dv_pcg_solve_noalloc(dv_matrix *A, const double *d_b, doub
         LaunchEnv ed = e;
         ed.done = &sc->done;
         SolverScalars h{};
-        if (resident) {
-            DV_REQUIRE(dv_pcg_resident_bytes(ctx) <= kPartialBytes, DV_ERR_CUDA, "too many SMs for the fixed array");
-            dv_pcg_resident(A, A->diag.as<double>(), 1, d_x, r, z, ap + len, p, ap, partials, sc, tol, 0);
+        if (resident && dv_pcg_resident_bytes(ctx) <= kPartialBytes &&
+            dv_pcg_resident(A, A->diag.as<double>(), 1, d_x, r, z, ap + len, p, ap, partials, sc, tol, 0)) {
             DV_CUDA(cudaMemcpyAsync(&h, sc, sizeof(h), cudaMemcpyDeviceToHost, st));
             DV_CUDA(cudaStreamSynchronize(st));
             DV_REQUIRE(h.done, DV_ERR_CUDA, "the blocks of the one-kernel PCG lost one another");

@@ -215,14 +215,20 @@ __global__ void __launch_bounds__(kThreadsR) k_pcg_resident(Groups G, ResidentAr
 }
 
 template <class Groups>
-void launch_resident(dv_context *ctx, const Groups &G, ResidentArgs a, size_t smem) {
+bool launch_resident(dv_context *ctx, const Groups &G, ResidentArgs a, size_t smem) {
     auto kern = k_pcg_resident<Groups>;
     static SmemLimit limit;   // per instantiation and device
     limit.raise(kern, smem, ctx->device);
     void *args[] = {const_cast<Groups *>(&G), &a};
-    DV_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<void *>(kern), dim3(ctx->num_sms), dim3(kThreadsR), args, smem,
-                                        ctx->stream));   // one block an SM
+    const cudaError_t err = cudaLaunchCooperativeKernel(reinterpret_cast<void *>(kern), dim3(ctx->num_sms), dim3(kThreadsR),
+                                                        args, smem, ctx->stream);   // one block an SM
+    if (err == cudaErrorCooperativeLaunchTooLarge || err == cudaErrorNotSupported) {
+        cudaGetLastError();
+        return false;
+    }
+    DV_CUDA(err);
     ctx->count();
+    return true;
 }
 
 }  // namespace
@@ -233,10 +239,11 @@ bool dv_pcg_resident_ok(const dv_matrix *A) {
     if (A->precision != DV_F64 || A->n_rows > kPcgResidentRows || A->n_rows % 3 != 0 || A->n_rows == 0) return false;
     if (A->format == DV_FORMAT_CSR) return A->row_group == 3;
     return A->n_rows <= kPcgResidentPatternRows && A->format == DV_FORMAT_DUVI && A->pat_ok && A->lanes_group == 3 && !A->pat_based && !A->pat_shift &&
-           sizeof(PatRec<double>) * (size_t)A->pat_entries + 4 * ((size_t)A->pat_count + 1) <= 160 * 1024;
+           sizeof(PatRec<double>) * (size_t)A->pat_entries + 4 * ((size_t)A->pat_count + 1) <=
+               (size_t)std::min(160 * 1024, A->ctx->max_smem_optin - 2048);   // less the sums' own shared memory
 }
 
-void dv_pcg_resident(dv_matrix *A, const double *M, int invert, double *x, double *r, double *z, double *p0, double *p1, double *ap,
+bool dv_pcg_resident(dv_matrix *A, const double *M, int invert, double *x, double *r, double *z, double *p0, double *p1, double *ap,
                      void *work, SolverScalars *sc, double tol, int rel_l2) {
     dv_context *ctx = A->ctx;
     ResidentArgs a;
@@ -257,10 +264,9 @@ void dv_pcg_resident(dv_matrix *A, const double *M, int invert, double *x, doubl
     DV_CUDA(cudaMemsetAsync(work, 0, 64, ctx->stream));
     DV_CUDA(cudaMemsetAsync(p0, 0, sizeof(double) * (size_t)A->n_rows, ctx->stream));   // read with beta = 0 first
     if (A->format == DV_FORMAT_CSR)
-        launch_resident(ctx, CsrGroups{A->rowptr.as<int32_t>(), A->col.as<int32_t>(), A->val.as<double>()}, a, 0);
-    else
-        launch_resident(ctx, PatternGroups{A->pat_id.as<uint16_t>(), A->pat_start.as<uint32_t>(),
-                                           static_cast<const PatRec<double> *>(A->pat_rec.p), A->pat_count,
-                                           A->pat_entries}, a,
-                        sizeof(PatRec<double>) * (size_t)A->pat_entries + 4 * ((size_t)A->pat_count + 1));
+        return launch_resident(ctx, CsrGroups{A->rowptr.as<int32_t>(), A->col.as<int32_t>(), A->val.as<double>()}, a, 0);
+    return launch_resident(ctx, PatternGroups{A->pat_id.as<uint16_t>(), A->pat_start.as<uint32_t>(),
+                                              static_cast<const PatRec<double> *>(A->pat_rec.p), A->pat_count,
+                                              A->pat_entries}, a,
+                           sizeof(PatRec<double>) * (size_t)A->pat_entries + 4 * ((size_t)A->pat_count + 1));
 }

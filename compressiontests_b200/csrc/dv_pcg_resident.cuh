@@ -18,6 +18,8 @@ size_t dv_pcg_resident_bytes(dv_context *ctx);
 // Iterates from r, z = M r and sc (rz, bb, it, max_it) until sc->done, the same steps and stop test as
 // dv_pcg_solve's chunks; M is the inverse diagonal, or with invert the diagonal; p0, p1, ap are work
 // vectors.  Context stream, asynchronous.  sc->done stays
-// 0 if the blocks lost one another (a bounded wait ran out).
-void dv_pcg_resident(dv_matrix *A, const double *M, int invert, double *x, double *r, double *z, double *p0, double *p1, double *ap,
+// 0 if the blocks lost one another (a bounded wait ran out).  False where the driver does not take the
+// cooperative launch (fewer SMs for this process than the device has): p1, r, z and sc are then as they came, and the
+// caller iterates in chunks.
+bool dv_pcg_resident(dv_matrix *A, const double *M, int invert, double *x, double *r, double *z, double *p0, double *p1, double *ap,
                      void *work, dvk::SolverScalars *sc, double tol, int rel_l2);

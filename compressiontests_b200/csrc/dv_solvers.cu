@@ -399,10 +399,9 @@ extern "C" DV_API int dv_pcg_solve(dv_pcg *s, const double *b, const double *x0,
                 ctx->count(2);
             }
         };
-        if (s->work.p) {   // every iteration in one kernel
-            dv_pcg_resident(s->A.get(), s->M.as<double>(), 0, s->x.as<double>(), s->r.as<double>(), s->z.as<double>(),
-                            s->p1.as<double>(), s->p.as<double>(), s->ap.as<double>(), s->work.p, s->ws->sc(), s->tol,
-                            rel_l2);
+        if (s->work.p && dv_pcg_resident(s->A.get(), s->M.as<double>(), 0, s->x.as<double>(), s->r.as<double>(),
+                                         s->z.as<double>(), s->p1.as<double>(), s->p.as<double>(), s->ap.as<double>(),
+                                         s->work.p, s->ws->sc(), s->tol, rel_l2)) {   // every iteration in one kernel
             s->ws->pull();
             DV_REQUIRE(h.done, DV_ERR_CUDA, "the blocks of the one-kernel PCG lost one another");
         }

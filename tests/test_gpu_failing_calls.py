@@ -82,3 +82,34 @@ print(json.dumps(dict(failed=fake.failed_calls(), ok=[o[1] for o in out], its=[o
 """)
     # two solves to a relative residual of 1e-8, each within 1e-6 of the solution
     assert r["failed"] == 1 and r["ok"] == [True, True] and r["its"][0] == r["its"][1] and r["diff"] < 2e-6, r
+
+
+@pytest.mark.parametrize("fmt", ["csr", "duvi"])
+def test_pcg_where_the_cooperative_launch_is_refused(child, fmt):
+    # A process that has fewer SMs than the device reports: the driver refuses the one-kernel solve and the solvers
+    # iterate in chunks, with and without a start vector.
+    r = child(f"""
+import torch
+N = cb._native
+ne = (16, 6, 5)
+A, b = cb.hex_stiffness(ne), cb.traction_rhs(ne)
+out = []
+for fail in (0, 1):
+    fake.fail_cooperative_launches(fail)
+    s = cb.CudaCsrPcgSolver(ctx, 2000, 1e-9, fmt="{fmt}").Initialize(A=A, b=b)
+    x, st = s.Solve()
+    x2, st2 = s.Solve(xInitialGuess=0.5 * x)
+    M = cb.SparseMatrix(ctx, A, "{fmt}", "f64")
+    db = torch.from_numpy(b).cuda()
+    dx = torch.zeros_like(db)
+    torch.cuda.synchronize()
+    sn = N.Stats()
+    N.check(N.lib().dv_pcg_solve_noalloc(M.h, ctypes.c_void_p(db.data_ptr()), ctypes.c_void_p(dx.data_ptr()), 0, 2000, 1e-9,
+                                         ctypes.byref(sn)))
+    out.append(([x, x2, dx.cpu().numpy()], [st.HasConverged, st2.HasConverged, bool(sn.converged)],
+                [st.NumIterationsRequired, st2.NumIterationsRequired, sn.iterations]))
+print(json.dumps(dict(failed=fake.failed_calls(), ok=[o[1] for o in out], its=[o[2] for o in out],
+                      diff=[float(np.max(np.abs(p - q)) / np.max(np.abs(p))) for p, q in zip(out[0][0], out[1][0])])))
+""")
+    assert r["failed"] == 3 and all(r["ok"][0]) and all(r["ok"][1]), r
+    assert all(abs(p - q) <= 1 for p, q in zip(*r["its"])) and max(r["diff"]) < 1e-7, r

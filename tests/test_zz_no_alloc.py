@@ -77,3 +77,30 @@ def test_noalloc_rejects_systems_above_the_limit(ctx, native):
     assert status == N.DV_ERR_ARG
     assert b"131072" in N.lib().dv_last_error()
     M.release()
+
+
+@pytest.mark.parametrize("fmt,ne", [("csr", (33, 32, 31)), ("csr", (42, 31, 31)), ("duvi", (30, 28, 28)), ("duvi", (42, 31, 31)),
+                                    ("csr", (35, 29, 32)), ("duvi", (27, 27, 27))])
+def test_noalloc_pcg_sizes(ctx, native, fmt, ne):
+    # Systems that iterate by launches (CSR from 104,001 rows, node patterns from 65,537, up to the array's 131,072), and those
+    # just below, whose five vectors of n rows share the array (103,950 rows in CSR; 63,504 on patterns).
+    import torch
+    N = native._native
+    A, b = native.hex_stiffness(ne), native.traction_rhs(ne)
+    ref = native.CudaCsrPcgSolver(ctx, 2000, 1e-8, fmt=fmt).Initialize(A=A, b=b)
+    x_ref, st_ref = ref.Solve()
+    assert st_ref.HasConverged
+    M = native.SparseMatrix(ctx, A, fmt, "f64")
+    db = torch.from_numpy(b).cuda()
+    for guess in (0, 1):
+        dx = torch.from_numpy(0.5 * x_ref).cuda() if guess else torch.full_like(db, float("nan"))
+        torch.cuda.synchronize()
+        st = N.Stats()
+        N.check(N.lib().dv_pcg_solve_noalloc(M.h, C.c_void_p(db.data_ptr()), C.c_void_p(dx.data_ptr()), guess, 2000, 1e-8,
+                                             C.byref(st)))
+        assert st.converged and not st.failed
+        assert guess or abs(st.iterations - st_ref.NumIterationsRequired) <= 1
+        x = dx.cpu().numpy()
+        assert np.max(np.abs(x - x_ref)) <= REL * np.max(np.abs(x_ref))
+    ref.ReleaseCudaResources()
+    M.release()

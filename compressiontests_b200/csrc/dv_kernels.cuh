@@ -2254,10 +2254,13 @@ void launch_rows(const LaunchEnv &e, const dv_matrix *m, Gather g, Op op) {
 
 // r = b - A x for the residual that a PCG solve reports.  Close to the limit of FP64 its last digits depend on the order
 // of the row sums, so it does not follow the kernel that is fastest for the iterations: CSR rows are summed one
-// thread a row in the stored order, as DuVi rows are and as a host would.
+// thread a row in the stored order, as DuVi rows are and as a host would.  Long rows, on the average, are split as
+// the products split them: one after another, 1,200 and 3,000 entries a row took 0.28 and 0.6 ms of a solve of
+// 22 iterations (0.8 and 1.5 ms); 81 entries a row take 0.03 ms of 1.5 (13,872 rows) and 0.14 of 8.9 (117,612).
+constexpr int64_t kStoredOrderEntries = 96;   // a row
 template <class Gather, class Op>
 void launch_reported_residual(const LaunchEnv &e, const dv_matrix *m, Gather g, Op op) {
-    if (m->format == DV_FORMAT_CSR) launch_csr_tpr<1, double>(e, m, g, op);
+    if (m->format == DV_FORMAT_CSR && m->nnz <= kStoredOrderEntries * m->n_rows) launch_csr_tpr<1, double>(e, m, g, op);
     else launch_rows<double>(e, m, g, op);
 }
 

@@ -326,25 +326,27 @@ void multi_solve(dv_mgpcg *s, VCycle<T> &vc, MultiState<T> &M, int k, const doub
     const size_t nk = (size_t)n * ld;
     if (M.k != k) {   // (re)size the block buffers
         M = MultiState<T>();
-        M.k = k;
+        MultiState<T> N;   // taken over when it is whole: an allocation may fail
+        N.k = k;
         for (auto &L : vc.lv) {
             const size_t b = sizeof(T) * (size_t)L.n * ld;
-            M.W.x.emplace_back(b);
-            M.W.t.emplace_back(b);
-            M.W.r.emplace_back(b);
-            M.W.b.emplace_back(b);
+            N.W.x.emplace_back(b);
+            N.W.t.emplace_back(b);
+            N.W.r.emplace_back(b);
+            N.W.b.emplace_back(b);
         }
-        M.W.bc.alloc(sizeof(T) * (size_t)vc.nc * ld);
-        M.W.xc.alloc(sizeof(T) * (size_t)vc.nc * ld);
-        M.B.alloc(8 * nk);
-        M.X.alloc(8 * nk);
-        M.R.alloc(8 * nk);
-        M.Pv.alloc(8 * nk);
-        M.Q.alloc(8 * nk);
-        if (kMixed) M.Rlow.alloc(4 * nk);
-        M.cols.alloc(sizeof(ColScalars) * (size_t)k);
-        M.red.alloc(64 + sizeof(double) * 2 * (size_t)kMaxK * ctx->num_sms * dvb::kReduceBlocksPerSm);
-        M.ws = std::make_unique<SolverWs>(ctx);
+        N.W.bc.alloc(sizeof(T) * (size_t)vc.nc * ld);
+        N.W.xc.alloc(sizeof(T) * (size_t)vc.nc * ld);
+        N.B.alloc(8 * nk);
+        N.X.alloc(8 * nk);
+        N.R.alloc(8 * nk);
+        N.Pv.alloc(8 * nk);
+        N.Q.alloc(8 * nk);
+        if (kMixed) N.Rlow.alloc(4 * nk);
+        N.cols.alloc(sizeof(ColScalars) * (size_t)k);
+        N.red.alloc(64 + sizeof(double) * 2 * (size_t)kMaxK * ctx->num_sms * dvb::kReduceBlocksPerSm);
+        N.ws = std::make_unique<SolverWs>(ctx);
+        M = std::move(N);
     }
     SolverWs &ws = *M.ws;
     dvk::SolverScalars &h = *ws.host_scal;

@@ -113,3 +113,28 @@ print(json.dumps(dict(failed=fake.failed_calls(), ok=[o[1] for o in out], its=[o
 """)
     assert r["failed"] == 3 and all(r["ok"][0]) and all(r["ok"][1]), r
     assert all(abs(p - q) <= 1 for p, q in zip(*r["its"])) and max(r["diff"]) < 1e-7, r
+
+
+@pytest.mark.parametrize("which", ["V-cycle block", "outer block", "scalars"])
+def test_load_cases_after_an_allocation_failed(child, which):
+    # Resizing the block buffers for another number of load cases has no room once: that call raises, the next one with the
+    # same number allocates them anew and solves (8 columns in FP32 and FP64 blocks, 8 columns' scalars).
+    r = child(f"""
+ne, k = (12, 8, 8), 8
+B = cb.random_face_loads(ne, k, seed=2)
+s = cb.MultigridPcgSolver.from_hex(ctx, ne, coarse_ne=4, precision="mixed", tol=1e-9)
+ref = s.solve_many(B)[0]
+s.solve_many(B[:, :3])
+n = {{"V-cycle block": 4 * k * B.shape[0] + 64, "outer block": 8 * k * B.shape[0] + 64}}.get("{which}")
+if n is None: fake.fail_allocations(64 + 8 * k, 1024)
+else: fake.fail_allocations(n, n)
+raised = ""
+try:
+    s.solve_many(B)
+except cb.DuviError as e:
+    raised = str(e)
+fake.fail_allocations(1, 0)
+X, st, conv = s.solve_many(B)
+print(json.dumps(dict(raised=raised, ok=bool(conv.all()), same=bool(np.array_equal(X, ref)))))
+""")
+    assert "memory" in r["raised"] and r["ok"] and r["same"], r

@@ -160,3 +160,38 @@ def test_block_grid_stencil_solver_equals_pattern_solver(ctx, native, problem, m
         s.release()
     assert res["1"][1] == res["0"][1]
     np.testing.assert_array_equal(res["1"][0], res["0"][0])
+
+
+@pytest.mark.parametrize("k", [5, 33, 66])
+def test_grid_outer_product_equals_pattern_outer_product(ctx, native, problem, k, monkeypatch):
+    # The FP64 outer product of the mixed solver on the grid-stencil block kernel, rows of k columns padded to 16 bytes: the
+    # pattern kernel's solver (the structural zeros multiplied too) takes the same iterations to the same solution.
+    ne, A, P = problem
+    B = native.random_face_loads(ne, k, seed=9)
+    res = {}
+    for flag in ("1", "0"):
+        monkeypatch.setenv("DV_BGRID", flag)
+        s = native.MultigridPcgSolver.from_hex(ctx, ne, coarse_ne=4, precision="mixed", tol=1e-10)
+        X, st, conv = s.solve_many(B)
+        assert conv.all() and st.RelativeResidual <= 1e-10
+        res[flag] = (X, st.NumIterationsRequired)
+        s.release()
+    assert res["1"][1] == res["0"][1]
+    # two solutions to a relative residual of 1e-10 each
+    assert max(rel(res["1"][0][:, j], res["0"][0][:, j]) for j in range(k)) < 1e-7
+
+
+@pytest.mark.parametrize("precision", ["mixed", "f64"])
+def test_load_cases_across_changes_of_their_number(ctx, native, precision):
+    # The block buffers and the captured iterations are kept while k stays: other loads, another k and back give
+    # a new solver's bits.
+    ne = (12, 8, 8)
+    s = native.MultigridPcgSolver.from_hex(ctx, ne, coarse_ne=4, precision=precision, tol=1e-9)
+    for k, seed in ((8, 1), (8, 2), (3, 3), (8, 2), (33, 4), (3, 3), (3, 5)):
+        B = native.random_face_loads(ne, k, seed=seed)
+        X, st, conv = s.solve_many(B)
+        fresh = native.MultigridPcgSolver.from_hex(ctx, ne, coarse_ne=4, precision=precision, tol=1e-9)
+        X1, st1, conv1 = fresh.solve_many(B)
+        fresh.release()
+        assert conv.all() and conv1.all() and st.NumIterationsRequired == st1.NumIterationsRequired
+        np.testing.assert_array_equal(X, X1)

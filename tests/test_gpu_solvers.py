@@ -553,3 +553,28 @@ def test_pcg_reports_the_stored_order_residual(ctx, native, ne):
     assert true_rel < 1e-11
     # the two norms of n terms are summed in another order
     assert abs(st.RelativeResidual - true_rel) <= 2 * len(b) * 2.0 ** -53 * true_rel
+
+
+@pytest.mark.parametrize("precision", ["mixed", "f64"])
+@pytest.mark.parametrize("build", ["hex", "hierarchy", "heterogeneous"])
+def test_decoded_entries_against_the_layouts(ctx, native, precision, build, monkeypatch):
+    # A solver on decoded entries and one on the DuVi layouts: the same iterations, the same solution.
+    ne = (16, 12, 8)
+    b = native.traction_rhs(ne)
+    E = 10.0 ** np.random.default_rng(2).uniform(-1.0, 0.0, int(np.prod(ne))) if build == "heterogeneous" else None
+    A, P = native.hex_hierarchy(ne, coarse_ne=4, elem_E=E)
+    out = []
+    for limit in ("0", None):
+        monkeypatch.delenv("DV_ENTRIES", raising=False)
+        if limit is not None:
+            monkeypatch.setenv("DV_ENTRIES", limit)
+        if build == "hex":
+            s = native.MultigridPcgSolver.from_hex(ctx, ne, coarse_ne=4, precision=precision, tol=1e-10)
+        else:
+            s = native.MultigridPcgSolver(ctx, A, P, precision=precision, fmt="duvi", tol=1e-10)
+        x, st = s.Solve(b)
+        s.release()
+        assert st.HasConverged and st.RelativeResidual <= 1e-10
+        out.append((x, st.NumIterationsRequired))
+    assert out[0][1] == out[1][1]
+    assert rel(out[0][0], out[1][0]) < 1e-7

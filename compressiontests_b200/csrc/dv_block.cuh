@@ -56,10 +56,18 @@ __device__ __forceinline__ void col_reduce(double (&acc)[U][NC], int kc, double 
     __syncthreads();
     if (!is_last) return;
     __threadfence();
-    // warp w sums quantities q = w, w + 8, ...: lanes stride over blocks, then a fixed butterfly
+    // warp w sums quantities q = w, w + 8, ...: lanes stride over blocks, then a fixed butterfly.  With four column slots
+    // (65 to 128 columns) this is most of a reduction, and eight loads are kept in flight: the compiler's own choice
+    // took k_bfcg_red from 171 to 257 us (97 columns, FP64, 45,000 rows) when its loop above changed; 145 us so.
+    // With one or two slots its choice is the better one (64 columns, CSR FP64 solve 12.4 against 13.0 ms).
     for (int q = warp; q < nq; q += kWarps) {
         double t = 0.0;
-        for (unsigned b = lane; b < gridDim.x; b += 32) t += __ldcg(partials + (size_t)b * nq + q);
+        if constexpr (U == 4) {
+#pragma unroll 8
+            for (unsigned b = lane; b < gridDim.x; b += 32) t += __ldcg(partials + (size_t)b * nq + q);
+        } else {
+            for (unsigned b = lane; b < gridDim.x; b += 32) t += __ldcg(partials + (size_t)b * nq + q);
+        }
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
         if (lane == 0) sh[0][q] = t;   // sh[0] is free: every warp finished reading it above

@@ -439,7 +439,9 @@ __global__ void __launch_bounds__(kThreads) k_bprod_pattern(const uint16_t *__re
         for (int t = 0; t < G; ++t)
 #pragma unroll
             for (int u = 0; u < U; ++u) acc[t][u] = AT(0);
-#pragma unroll 2
+        // FP32: four records' loads in flight (with two, and the registers the compiler gave the loop, 33 columns of a 200,000-row
+        // hex operator took 138.8 us, 99 columns 241; 117 and 193 so); FP64 has no registers for more than two
+#pragma unroll (sizeof(AT) == 4 ? 4 : 2)
         for (uint32_t k = b; k < e; ++k) {
             const dvk::PatRec<AT> q = rec[k];
             const uint32_t c = c0 + (uint32_t)q.off;

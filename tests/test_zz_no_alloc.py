@@ -104,3 +104,40 @@ def test_noalloc_pcg_sizes(ctx, native, fmt, ne):
         assert np.max(np.abs(x - x_ref)) <= REL * np.max(np.abs(x_ref))
     ref.ReleaseCudaResources()
     M.release()
+
+
+@pytest.mark.parametrize("fmt", ["csr", "duvi"])
+@pytest.mark.parametrize("first", [0, 1])
+def test_noalloc_after_one_call_with_the_format(fmt, first):
+    # After one call with the format, in a fresh process, another call takes no device memory: a small system solved in one kernel
+    # and then a large one by launches from a start vector, or the other way round.
+    import json
+    import os
+    import subprocess
+    import sys
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", f"""
+import ctypes as C, json
+import numpy as np, torch
+import compressiontests_b200 as cb
+N, ctx = cb._native, cb.CudaContext(0)
+calls = []
+for ne in ((16, 4, 4), (36, 32, 32)):
+    A, b = cb.hex_stiffness(ne), cb.traction_rhs(ne)
+    M = cb.SparseMatrix(ctx, A, "{fmt}", "f64")
+    db = torch.from_numpy(b).cuda()
+    calls.append((M, db, torch.zeros_like(db)))
+if {first}: calls.reverse()
+torch.cuda.synchronize()
+free, ok = [], []
+for k, (M, db, dx) in enumerate(calls):
+    st = N.Stats()
+    free.append(torch.cuda.mem_get_info()[0])
+    N.check(N.lib().dv_pcg_solve_noalloc(M.h, C.c_void_p(db.data_ptr()), C.c_void_p(dx.data_ptr()), k, 2000, 1e-6, C.byref(st)))
+    ok.append(bool(st.converged))
+free.append(torch.cuda.mem_get_info()[0])
+print(json.dumps([ok, free]))
+"""], cwd=root, env=dict(os.environ, PYTHONPATH=root), capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stdout + r.stderr
+    ok, free = json.loads(r.stdout.strip().splitlines()[-1])
+    assert all(ok) and free[1] == free[2], (ok, free)

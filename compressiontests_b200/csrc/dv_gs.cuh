@@ -135,7 +135,7 @@ __global__ void __launch_bounds__(256) k_gs_pattern(const uint16_t *__restrict__
 // they are subtracted one after another in column order: products and differences are rounded
 // one by one as in gs_row_csr, so the result is the same bit for bit (the diagonal and the padding
 // subtract +0, which changes nothing).  Bound by that chain of dependent subtractions.
-// 12 x 4 x 4 elements, two levels, to 1e-3: 1,040 -> 109 ms (13.8 -> about 1.2 us a dependency level).
+// 12 x 4 x 4 elements, two levels, to 1e-3: 950 -> 109 ms (about 12 -> 1.3 us a dependency level).
 // ---------------------------------------------------------------------------
 constexpr int kGsWarps = 32;
 constexpr int kGsLane = 3;   // entries of a row a lane holds at a time (96 a warp)

@@ -1749,7 +1749,7 @@ void launch_csr_nodes(const LaunchEnv &e, const dv_matrix *m, Gather g, Op op) {
 // (hex_tile).  Elements outside the mesh have factor 0 and clamped or outside nodes have x = 0,
 // so face and edge nodes need no special case.  The sum order differs from the assembled
 // operator's, so FP64 products agree with the assembled matrix to rounding (not bit for bit).
-// 128^3, log-uniform moduli, FP64 product: 212.9 -> 79.9 us (119 MB of vectors and factors: 18 us;
+// 128^3, log-uniform moduli, FP64 product: 212.9 -> 68 us (119 MB of vectors and factors: 18 us;
 // 170 FP64 operations a node: 19 us), relative error against 64 bits 4.7e-16 -> 2.1e-16.
 // Sums and differences over corners turn an infinite x into Inf - Inf, and overflow for a finite x near
 // the type's limit: a node whose sums are not finite is formed again from the entries of Ke

@@ -76,7 +76,12 @@ struct DevMem {
         // The zero fill runs on the legacy stream, which does not order against the
         // non-blocking context streams: finish it before anyone writes the buffer.
         if (b) {
-            DV_CUDA(cudaMalloc(&p, b + 64));
+            const cudaError_t err = cudaMalloc(&p, b + 64);
+            if (err != cudaSuccess) {
+                cudaGetLastError();   // reported here, not by the next launch's check
+                p = nullptr;
+                DV_CUDA(err);
+            }
             DV_CUDA(cudaMemsetAsync(p, 0, b + 64, 0));
             DV_CUDA(cudaStreamSynchronize(0));
         }

@@ -414,7 +414,6 @@ void dv_use_entries(dv_context *ctx, const std::vector<dv_matrix *> &operators) 
             val.alloc((m->precision == DV_F64 ? 8 : 4) * (size_t)m->nnz);
         } catch (const DvError &e) {   // no room for a copy: this operator and the larger ones stay on their layouts
             if (e.code != DV_ERR_NOMEM) throw;
-            cudaGetLastError();
             break;
         }
         m->col = std::move(col);

@@ -1,7 +1,7 @@
 """CUDA calls that fail: what the library does when an allocation has no room or a launch is refused.
 
-The failure comes from a stand-in for the runtime's entry point, preloaded into a child process: it returns the
-error code and calls nothing, so the GPU is not involved in it.
+The failure comes from a stand-in for the runtime's entry point, preloaded into a child process: it asks for more memory
+than there is, or returns the launch's error code and calls nothing, so nothing runs on the GPU.
 """
 import json
 import os
@@ -27,7 +27,7 @@ static void *real(const char *name) {
     return dlsym(lib, name);
 }
 int cudaMalloc(void **p, size_t bytes) {
-    if (bytes >= lo && bytes <= hi) { failed++; return 2; }   /* cudaErrorMemoryAllocation */
+    if (bytes >= lo && bytes <= hi) { failed++; bytes = (size_t)1 << 50; }   /* more than any device has: out of memory */
     return ((int (*)(void **, size_t))real("cudaMalloc"))(p, bytes);
 }
 typedef struct { unsigned x, y, z; } Dim;
